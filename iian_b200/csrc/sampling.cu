@@ -12,10 +12,12 @@
 // order when it sorted), and the uniform number comes from the caller (a counter-based stream per
 // request) instead of a per-request mt19937_64.  The distribution is the same.
 //
-// One block per row.  The k-th largest value and the top-p cut are found exactly by bisection over
-// the order-preserving integer image of the float values (32 counting passes over the row, which
-// stays in L2).
+// The k-th largest value and the top-p cut are found exactly, over the order-preserving integer image of the float values.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace iian {
 
@@ -141,196 +143,377 @@ __global__ void argmax_final_kernel(const float * __restrict__ part_val, const i
     if (lane == 0) out[row] = bi == 0x7fffffff ? 0 : bi;
 }
 
-__global__ void __launch_bounds__(kSampleThreads) sample_kernel(
-    const float * __restrict__ logits, int V, size_t stride,
-    const float * __restrict__ temperature, const int * __restrict__ top_k, const float * __restrict__ top_p,
-    const float * __restrict__ min_p, const float * __restrict__ uniform, int * __restrict__ out) {
+// ---- temperature sampling ------------------------------------------------------------------------------------------
+// A row is worked on by a thread-block cluster: each CTA keeps a slice of the row in shared memory as ordered integer keys,
+// so the row is read from global memory once (V > 8 x kStagedMax: read again per pass) and a row of 150,000 entries has up
+// to 8 SMs.  The k-th largest value and the top-p cut are found exactly by narrowing an interval of keys eight ways per pass:
+// a pass counts (and for top-p adds the probability of) the keys at or above seven borders inside the interval, looking
+// only at keys inside it -- what lies above is known --, and the CTAs swap their numbers through each other's shared
+// memory behind one cluster barrier.  A search ends when one key is left inside.
+// Every sum has an order fixed by V alone (entries of a thread, lanes, warps, CTAs): the same row gives the same token
+// whatever else is in the batch.
+// What bounds it: latency of the passes (a scan of a slice, two block barriers, a cluster barrier: about 1 us, some 20 of them),
+// not the bytes.  Rows of 151,936, the usual mix of settings: 48 rows 131 us, 8 rows 82 us, one row with top-k and top-p 51 us (one
+// block per row with 32 one-bit passes per search over the L2: 2,208 us for 48 rows).
+constexpr int kDrawThreads = 512;
+constexpr int kDrawWarps = kDrawThreads / 32;
+constexpr int kDrawCluster = 8;                  // CTAs per row, at most
+constexpr int kStagedMax = 50 * 1024;            // entries of a slice that shared memory holds (200 KB)
+constexpr int kBorders = 7;
+
+__device__ __forceinline__ unsigned draw_key(float z) { return z != z ? 0u : order_key(z); }      // NaN: below every key that is looked at
+__device__ __forceinline__ float key_value(unsigned k) { return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k); }
+
+struct DrawShared {
+    double inbox_m[2][kDrawCluster][8];          // what every CTA of the cluster sent: masses (or a value of the kind at hand)
+    int inbox_c[2][kDrawCluster][8];             // and counts
+    float warp_m[kDrawWarps][8];
+    int warp_c[kDrawWarps][8];
+    double warp_d[kDrawWarps];
+    int warp_i[kDrawWarps];
+    int pick;
+};
+
+template <bool STAGED>
+struct Draw {
+    DrawShared & sh;
+    const unsigned * keys;                       // staged slice
+    const float * slice;                         // the same entries in global memory
+    int n;                                       // entries of this CTA
+    float inv_t, zmax;
+    int rank, ctas, turn;
+    __device__ __forceinline__ unsigned key(int i) const { return STAGED ? keys[i] : draw_key(slice[i] * inv_t); }
+    __device__ __forceinline__ float mass(unsigned k) const { return expf(key_value(k) - zmax); }
+
+    // Lane j of every warp gets (count, mass) of the keys in [max(border j, lo), hi) over the whole row, j < 7; border in lane j.
+    template <bool MASS>
+    __device__ __forceinline__ void pass(unsigned border, unsigned lo, unsigned hi, int & count, double & m) {
+        const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+        unsigned t[kBorders];
+#pragma unroll
+        for (int j = 0; j < kBorders; j++) t[j] = __shfl_sync(0xffffffffu, border, j);
+        int c[kBorders];
+        float a[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) { a[j] = 0.0f; if (j < kBorders) c[j] = 0; }
+        for (int i = tid; i < n; i += kDrawThreads) {
+            const unsigned k = key(i);
+            if (k >= lo && k < hi) {
+                const float e = MASS ? mass(k) : 0.0f;
+#pragma unroll
+                for (int j = 0; j < kBorders; j++) {
+                    const bool in = k >= t[j];
+                    c[j] += in;
+                    if (MASS) a[j] += in ? e : 0.0f;
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kBorders; j++) c[j] = __reduce_add_sync(0xffffffffu, c[j]);
+        if (MASS) {
+            // eight sums over 32 lanes: halve the values a lane carries with every exchange; lane ends with value lane >> 2
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const bool up = lane & 16;
+                const float give = up ? a[j] : a[j + 4], keep = up ? a[j + 4] : a[j];
+                a[j] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const bool up = lane & 8;
+                const float give = up ? a[j] : a[j + 2], keep = up ? a[j + 2] : a[j];
+                a[j] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+            }
+            {
+                const bool up = lane & 4;
+                const float give = up ? a[0] : a[1], keep = up ? a[1] : a[0];
+                a[0] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+            }
+            a[0] += __shfl_xor_sync(0xffffffffu, a[0], 2);
+            a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
+            if ((lane & 3) == 0) sh.warp_m[warp][lane >> 2] = a[0];
+        }
+        if (lane == 0) {
+#pragma unroll
+            for (int j = 0; j < kBorders; j++) sh.warp_c[warp][j] = c[j];
+        }
+        __syncthreads();
+        if (warp < kBorders) {                   // warp j puts border j's numbers together and sends them to every CTA
+            const int w = lane & (kDrawWarps - 1);
+            double d = MASS && lane < kDrawWarps ? (double) sh.warp_m[w][warp] : 0.0;
+            const int cc = __reduce_add_sync(0xffffffffu, lane < kDrawWarps ? sh.warp_c[w][warp] : 0);
+            if (MASS) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+            }
+            send(lane, warp, d, cc);
+        }
+        swap();
+        count = 0;
+        m = 0.0;
+        if (lane < kBorders) {
+            for (int r = 0; r < ctas; r++) {
+                count += sh.inbox_c[turn][r][lane];
+                if (MASS) m += sh.inbox_m[turn][r][lane];
+            }
+        }
+        turn ^= 1;
+    }
+    // lane r < ctas: value `which` of this CTA goes to CTA r
+    __device__ __forceinline__ void send(int lane, int which, double d, int c) {
+        if (lane < ctas) {
+            cg::cluster_group cl = cg::this_cluster();
+            DrawShared * to = cl.map_shared_rank(&sh, lane);
+            to->inbox_m[turn][rank][which] = d;
+            to->inbox_c[turn][rank][which] = c;
+        }
+    }
+    // what was sent before is there afterwards.  The two inboxes take turns: one is written again only behind the barrier of
+    // the turn between, which a CTA reaches after it has read this one.
+    __device__ __forceinline__ void swap() { cg::this_cluster().sync(); }
+
+    // The largest key K in [lo, hi) whose count (or mass) of keys at or above it reaches the goal; it does at lo and does not at hi.
+    // In: the aggregates at lo and hi.  Out: lo = K and the aggregates of the keys at or above it and above it.
+    template <bool MASS>
+    __device__ __forceinline__ void search(unsigned & lo, unsigned hi, int & c_lo, int & c_hi, double & m_hi, double goal) {
+        const int lane = threadIdx.x & 31;
+        bool first = true;
+        while (hi - lo > 1) {
+            if (c_lo - c_hi == 1) {              // one key left inside: it is K
+                unsigned found = 0;
+                for (int i = threadIdx.x; i < n; i += kDrawThreads) {
+                    const unsigned k = key(i);
+                    if (k >= lo && k < hi) found = k;
+                }
+                found = __reduce_max_sync(0xffffffffu, found);
+                if (lane == 0) sh.warp_i[threadIdx.x >> 5] = (int) found;
+                __syncthreads();
+                if (threadIdx.x < 32) {
+                    found = __reduce_max_sync(0xffffffffu, lane < kDrawWarps ? (unsigned) sh.warp_i[lane] : 0u);
+                    send(lane, 0, 0.0, (int) found);
+                }
+                swap();
+                found = __reduce_max_sync(0xffffffffu, lane < ctas ? (unsigned) sh.inbox_c[turn][lane][0] : 0u);
+                turn ^= 1;
+                lo = found;
+                return;
+            }
+            unsigned border;
+            if (first) {                         // distances from the largest value: 32, 16, ..., 0.5
+                border = order_key(zmax - exp2f((float) (5 - min(lane, kBorders - 1))));
+                border = min(max(border, lo), hi);
+            } else border = lo + (unsigned) (((unsigned long long) (hi - lo) * (unsigned) (min(lane, kBorders - 1) + 1)) >> 3);
+            first = false;
+            int c;
+            double m;
+            pass<MASS>(border, lo, hi, c, m);
+            c += c_hi;
+            m += m_hi;
+            const unsigned ok = __ballot_sync(0xffffffffu, lane < kBorders && (MASS ? m >= goal : (double) c >= goal));
+            const int reached = __popc(ok);      // the borders ascend: the first `reached` of them reach the goal
+            const int up = min(reached, kBorders - 1), down = max(reached - 1, 0);
+            const unsigned b_up = __shfl_sync(0xffffffffu, border, up), b_down = __shfl_sync(0xffffffffu, border, down);
+            const int c_up = __shfl_sync(0xffffffffu, c, up), c_down = __shfl_sync(0xffffffffu, c, down);
+            const double m_up = __shfl_sync(0xffffffffu, m, up);
+            if (reached < kBorders) { hi = b_up; c_hi = c_up; m_hi = m_up; }
+            if (reached > 0) { lo = b_down; c_lo = c_down; }
+        }
+    }
+};
+
+template <bool STAGED>
+__global__ void __launch_bounds__(kDrawThreads) sample_kernel(
+    const float * __restrict__ logits, int V, size_t stride, int slice, const float * __restrict__ temperature,
+    const int * __restrict__ top_k, const float * __restrict__ top_p, const float * __restrict__ min_p,
+    const float * __restrict__ uniform, int * __restrict__ out) {
+    extern __shared__ unsigned staged[];
+    __shared__ DrawShared sh;
     __shared__ float fs[32];
     __shared__ int is[32];
-    __shared__ float chunk_mass[kSampleThreads];
-    __shared__ int chunk_ties[kSampleThreads];
-    __shared__ int pick_thread;
-    __shared__ float pick_before;
-    __shared__ int pick_ties_before;
+    cg::cluster_group cl = cg::this_cluster();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ctas = (int) cl.num_blocks(), rank = (int) cl.block_rank(), row = blockIdx.x / ctas;
+    const int begin = (int) min((long long) V, (long long) rank * slice), n = (int) min((long long) V, (long long) begin + slice) - begin;
+    const float * src = logits + (size_t) row * stride + begin;
+    const float T = temperature[row];
+    const bool greedy = T < 1e-5f;
+    const float inv_t = greedy ? 1.0f : 1.0f / T;
 
-    const float * row = logits + (size_t) blockIdx.x * stride;
-    const float T = temperature[blockIdx.x];
-    if (T < 1e-5f) {
-        float b; int bi;
-        block_argmax(row, V, 1.0f, b, bi, fs, is);
-        if (threadIdx.x == 0) out[blockIdx.x] = bi;
+    // the slice into shared memory; the row's largest value and the lowest id that holds it
+    float best = -INFINITY;
+    int best_i = 0x7fffffff;
+#pragma unroll 8
+    for (int i = tid; i < n; i += kDrawThreads) {
+        const float z = src[i] * inv_t;
+        if (STAGED) staged[i] = draw_key(z);
+        if (z > best || (z == best && begin + i < best_i)) { best = z; best_i = begin + i; }        // NaN compares false
+    }
+    auto better = [&](float ob, int oi) { if (ob > best || (ob == best && oi < best_i)) { best = ob; best_i = oi; } };
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
+        better(ob, oi);
+    }
+    if (lane == 0) { fs[warp] = best; is[warp] = best_i; }
+    cl.sync();                                   // every CTA of the cluster runs before its shared memory is written; orders fs, is and staged too
+    Draw<STAGED> d{sh, staged, src, n, inv_t, 0.0f, rank, ctas, 0};
+    if (warp == 0) {
+        best = lane < kDrawWarps ? fs[lane] : -INFINITY;
+        best_i = lane < kDrawWarps ? is[lane] : 0x7fffffff;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
+            better(ob, oi);
+        }
+        d.send(lane, 0, (double) best, best_i);
+    }
+    d.swap();
+    best = -INFINITY;
+    best_i = 0x7fffffff;
+    for (int r = 0; r < ctas; r++) better((float) sh.inbox_m[d.turn][r][0], sh.inbox_c[d.turn][r][0]);
+    d.turn ^= 1;
+    const int imax = best_i == 0x7fffffff ? 0 : best_i;
+    d.zmax = best;
+    const float P = top_p[row];
+    // nothing to draw from: a greedy row, an infinite or missing largest value, or a share of the mass that keeps none (these
+    // tests see the same numbers in every CTA, so a cluster leaves together; what was sent has been read by its receiver only
+    // after the barrier above, and nothing is sent after it)
+    if (greedy || !(fabsf(best) < INFINITY) || P <= 0.0f) {
+        if (rank == 0 && tid == 0) out[row] = imax;
         return;
     }
-    const float inv_t = 1.0f / T;
-    float zmax; int imax;
-    block_argmax(row, V, inv_t, zmax, imax, fs, is);
-
-    // candidate set: key > cut, plus the first n_tie elements (by id) with key == cut
-    unsigned cut = 0u;                 // 0 is below every finite or infinite value's key
+    const unsigned top = order_key(best) + 1;    // above every key
+    // candidates: keys above `cut`, and the first n_tie entries (by id) whose key is `cut`
+    unsigned cut = 1u;
     int n_tie = 0x7fffffff;
-    const float mp = min_p[blockIdx.x];
-    if (mp > 0.0f) cut = order_key(zmax + logf(mp)), n_tie = 0x7fffffff;
-    // keys >= cut are candidates; express "all ties" as n_tie = INT_MAX
-
-    int count = 0;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) count += order_key(row[i] * inv_t) >= cut;
-    count = block_sum_int(count, is);
-
-    const int k = top_k[blockIdx.x];
-    if (k > 0 && k < count) {
-        unsigned K = 0u;
-        for (int bit = 31; bit >= 0; bit--) {
-            const unsigned trial = K | (1u << bit);
-            int c = 0;
-            for (int i = threadIdx.x; i < V; i += blockDim.x) c += order_key(row[i] * inv_t) >= trial;
-            c = block_sum_int(c, is);
-            if (c >= k) K = trial;
+    const float mp = min_p[row];
+    if (mp > 0.0f) cut = order_key(best + logf(mp));
+    const int k = top_k[row];
+    if (k > 0 && cut < top) {
+        int c;
+        double m;
+        d.template pass<false>(cut, cut, top, c, m);
+        int count = __shfl_sync(0xffffffffu, c, 0), above = 0;
+        double none = 0.0;
+        if (k < count) {
+            d.template search<false>(cut, top, count, above, none, (double) k);
+            n_tie = k - above;
         }
-        int gt = 0;
-        for (int i = threadIdx.x; i < V; i += blockDim.x) gt += order_key(row[i] * inv_t) > K;
-        gt = block_sum_int(gt, is);
-        cut = K;
-        n_tie = k - gt;
     }
-
-    const float P = top_p[blockIdx.x];
-    if (P < 1.0f) {
-        // mass of the current set; ties at `cut` all have the same value, so only their count matters
-        float mass_gt = 0.0f;
-        int ties = 0;
-        float cut_val = 0.0f;
-        for (int i = threadIdx.x; i < V; i += blockDim.x) {
-            const float z = row[i] * inv_t;
-            const unsigned key = order_key(z);
-            if (key > cut) mass_gt += expf(z - zmax);
-            else if (key == cut) { ties++; cut_val = z; }
-        }
-        mass_gt = block_sum(mass_gt, fs);
-        ties = block_sum_int(ties, is);
-        // every thread needs the tied value: take it from the key itself
-        const unsigned cb = (cut & 0x80000000u) ? (cut & 0x7fffffffu) : ~cut;
-        cut_val = __uint_as_float(cb);
-        const int ties_in = min(ties, n_tie);
-        const float pe_cut = ties_in > 0 ? expf(cut_val - zmax) : 0.0f;
-        const float total = mass_gt + (float) ties_in * pe_cut;
-        const float target = P * total;
-        // largest key Kp (> cut) with mass(key >= Kp) >= target; if none, the cut itself stays
-        unsigned Kp = cut;
-        bool moved = false;
-        {
-            unsigned K = 0u;
-            for (int bit = 31; bit >= 0; bit--) {
-                const unsigned trial = K | (1u << bit);
-                bool ok;
-                if (trial <= cut) ok = true;
-                else {
-                    float ms = 0.0f;
-                    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-                        const float z = row[i] * inv_t;
-                        if (order_key(z) >= trial) ms += expf(z - zmax);
-                    }
-                    ms = block_sum(ms, fs);
-                    ok = ms >= target;
-                }
-                if (ok) K = trial;
-            }
-            if (K > cut) { Kp = K; moved = true; }
-        }
-        if (moved) {
-            float above = 0.0f;
-            int tie_p = 0;
-            for (int i = threadIdx.x; i < V; i += blockDim.x) {
-                const float z = row[i] * inv_t;
-                const unsigned key = order_key(z);
-                if (key > Kp) above += expf(z - zmax);
-                else if (key == Kp) tie_p++;
-            }
-            above = block_sum(above, fs);
-            tie_p = block_sum_int(tie_p, is);
-            const unsigned pb = (Kp & 0x80000000u) ? (Kp & 0x7fffffffu) : ~Kp;
-            const float pe = expf(__uint_as_float(pb) - zmax);
-            int need = pe > 0.0f ? (int) ceilf((target - above) / pe) : tie_p;
-            need = max(1, min(need, tie_p));
-            cut = Kp;
-            n_tie = need;
+    if (P < 1.0f && cut < top) {
+        // borders: cut in lane 0, cut + 1 in the others (entries equal to the cut: the difference of the counts)
+        int c;
+        double m;
+        d.template pass<true>(cut + (lane > 0 ? 1u : 0u), cut, top, c, m);
+        const int c_all = __shfl_sync(0xffffffffu, c, 0);
+        int c_gt = __shfl_sync(0xffffffffu, c, 1);
+        const double m_gt = __shfl_sync(0xffffffffu, m, 1);
+        const int ties_in = min(c_all - c_gt, n_tie);
+        const float pe_cut = ties_in > 0 ? d.mass(cut) : 0.0f;
+        const double target = (double) P * (m_gt + (double) ties_in * (double) pe_cut);
+        if (target > 0.0 && m_gt >= target) {    // the cut moves up: the largest key whose mass from there on reaches the target
+            unsigned K = cut + 1;
+            int c_above = 0;
+            double m_above = 0.0;
+            d.template search<true>(K, top, c_gt, c_above, m_above, target);
+            const int tie_p = c_gt - c_above;
+            const float pe = d.mass(K);
+            const int need = pe > 0.0f ? (int) fmin(ceil((target - m_above) / (double) pe), 2147483647.0) : tie_p;
+            cut = K;
+            n_tie = max(1, min(need, tie_p));
         } else if (ties_in > 0 && pe_cut > 0.0f) {
-            int need = (int) ceilf((target - mass_gt) / pe_cut);
-            n_tie = max(mass_gt >= target ? 0 : 1, min(need, ties_in));
-            if (mass_gt <= 0.0f) n_tie = max(n_tie, 1);
+            const int need = (int) fmin(ceil((target - m_gt) / (double) pe_cut), 2147483647.0);
+            n_tie = max(m_gt >= target ? 0 : 1, min(need, ties_in));
+            if (m_gt <= 0.0) n_tie = max(n_tie, 1);
         }
     }
 
-    // inverse CDF in vocabulary order: thread t owns ids [t * per, (t + 1) * per)
-    const int per = (V + blockDim.x - 1) / blockDim.x;
-    const int begin = min(V, (int) threadIdx.x * per), end = min(V, begin + per);
-    float cm = 0.0f;
-    int ct = 0;
-    for (int i = begin; i < end; i++) {
-        const unsigned key = order_key(row[i] * inv_t);
-        if (key == cut) ct++;
+    // inverse CDF in vocabulary order: thread t owns `per` neighbouring entries (an odd number: no two lanes in one bank)
+    const int per = ((n + kDrawThreads - 1) / kDrawThreads) | 1;
+    const int i0 = (int) min((long long) n, (long long) tid * per), i1 = min(n, i0 + per);
+    int ties = 0;
+    for (int i = i0; i < i1; i++) ties += d.key(i) == cut;
+    int tie_rank = ties;                         // inclusive scan over the CTA, then the CTAs before
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, tie_rank, o);
+        if (lane >= o) tie_rank += v;
     }
-    chunk_ties[threadIdx.x] = ct;
+    __syncthreads();                             // sh.warp_i may still be read from the search
+    if (lane == 31) sh.warp_i[warp] = tie_rank;
     __syncthreads();
-    if (threadIdx.x == 0) {     // exclusive scan of tie counts (1024 entries)
-        int run = 0;
-        for (int t = 0; t < blockDim.x; t++) { const int c = chunk_ties[t]; chunk_ties[t] = run; run += c; }
+    if (warp == 0) {
+        const int w = lane < kDrawWarps ? sh.warp_i[lane] : 0;
+        d.send(lane, 0, 0.0, __reduce_add_sync(0xffffffffu, w));
     }
-    __syncthreads();
-    int tie_rank = chunk_ties[threadIdx.x];
-    const int tie_rank0 = tie_rank;
-    for (int i = begin; i < end; i++) {
-        const float z = row[i] * inv_t;
-        const unsigned key = order_key(z);
-        if (key > cut) cm += expf(z - zmax);
-        else if (key == cut) { if (tie_rank < n_tie) cm += expf(z - zmax); tie_rank++; }
+    d.swap();
+    tie_rank -= ties;
+    for (int w = 0; w < warp; w++) tie_rank += sh.warp_i[w];
+    for (int r = 0; r < rank; r++) tie_rank += sh.inbox_c[d.turn][r][0];
+    d.turn ^= 1;
+    double cm = 0.0;
+    int tr = tie_rank;
+    for (int i = i0; i < i1; i++) {
+        const unsigned kk = d.key(i);
+        if (kk > cut) cm += (double) d.mass(kk);
+        else if (kk == cut) { if (tr < n_tie) cm += (double) d.mass(kk); tr++; }
     }
-    chunk_mass[threadIdx.x] = cm;
+    double incl = cm;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) sh.warp_d[warp] = incl;
+    if (tid == 0) sh.pick = -1;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float total = 0.0f;
-        for (int t = 0; t < blockDim.x; t++) total += chunk_mass[t];
-        const float r = uniform[blockIdx.x] * total;
-        float run = 0.0f;
-        int pt = -1;
-        for (int t = 0; t < blockDim.x; t++) {
-            if (chunk_mass[t] > 0.0f && run + chunk_mass[t] > r) { pt = t; break; }
-            run += chunk_mass[t];
+    double before = 0.0, all = 0.0;
+    for (int w = 0; w < kDrawWarps; w++) {
+        if (w == warp) before = all;
+        all += sh.warp_d[w];
+    }
+    if (warp == 0) d.send(lane, 0, all, 0);
+    d.swap();
+    double total = 0.0;
+    for (int r = 0; r < ctas; r++) total += sh.inbox_m[d.turn][r][0];
+    const double u = (double) uniform[row] * total;
+    // the CTA the draw falls into: the first whose running sum passes it, else (rounding) the last that holds mass
+    int owner = -1;
+    double run = 0.0, ahead = 0.0;
+    for (int r = 0; r < ctas; r++) {
+        const double v = sh.inbox_m[d.turn][r][0];
+        if (v > 0.0) { owner = r; ahead = run; if (run + v > u) break; }
+        run += v;
+    }
+    if (owner < 0) {                             // no candidate holds mass
+        if (rank == 0 && tid == 0) out[row] = imax;
+        return;
+    }
+    if (rank != owner) return;
+    // the thread: the same way
+    const double lead = ahead + before;
+    if (cm > 0.0) atomicMax(&sh.pick, lead + incl > u ? kDrawThreads * 2 - tid : tid);     // the first past the draw, else the last
+    __syncthreads();
+    const int pick = sh.pick >= kDrawThreads ? kDrawThreads * 2 - sh.pick : sh.pick;
+    if (tid != pick) return;
+    double at = lead + (incl - cm);
+    int chosen = -1, last = -1;
+    tr = tie_rank;
+    for (int i = i0; i < i1; i++) {
+        const unsigned kk = d.key(i);
+        float e = 0.0f;
+        if (kk > cut) e = d.mass(kk);
+        else if (kk == cut) { if (tr < n_tie) e = d.mass(kk); tr++; }
+        if (e > 0.0f) {
+            last = i;
+            at += (double) e;
+            if (at > u) { chosen = i; break; }
         }
-        if (pt < 0) {           // r == total (rounding): last chunk that holds mass
-            run = 0.0f;
-            float before = 0.0f;
-            for (int t = 0; t < blockDim.x; t++) { if (chunk_mass[t] > 0.0f) { pt = t; before = run; } run += chunk_mass[t]; }
-            run = before;
-        }
-        pick_thread = pt;
-        pick_before = run;
-        pick_ties_before = 0;
-        (void) pick_ties_before;
-        // r is re-derived by the owner from `uniform` and `total`
-        fs[0] = r;
     }
-    __syncthreads();
-    if ((int) threadIdx.x == pick_thread) {
-        const float r = fs[0];
-        float run = pick_before;
-        int tr = tie_rank0;
-        int chosen = -1, last = -1;
-        for (int i = begin; i < end; i++) {
-            const float z = row[i] * inv_t;
-            const unsigned key = order_key(z);
-            float pe = 0.0f;
-            if (key > cut) pe = expf(z - zmax);
-            else if (key == cut) { if (tr < n_tie) pe = expf(z - zmax); tr++; }
-            if (pe > 0.0f) {
-                last = i;
-                run += pe;
-                if (run > r) { chosen = i; break; }
-            }
-        }
-        if (chosen < 0) chosen = last >= 0 ? last : imax;
-        out[blockIdx.x] = chosen;
-    }
-    if (pick_thread < 0 && threadIdx.x == 0) out[blockIdx.x] = imax;
+    if (chosen < 0) chosen = last;
+    out[row] = chosen >= 0 ? begin + chosen : imax;
 }
 
 // Logits processors in the reference's order (src/iian/sampler.cpp:72-109), as lists the host prepares per row:
@@ -456,14 +639,37 @@ IIAN_API int iian_argmax_wide(const float * logits, int R, int V, long long stri
     return iian_launch(argmax_final_kernel, dim3(R), dim3(32), 0, stream, (const float *) pv, (const int *) pi, parts, out);
 }
 
+// CTAs per row: slices of 4,096 entries and more, up to 8 CTAs (a smaller slice is scanned in less time than the cluster's
+// barrier takes).
 IIAN_API int iian_sample(const float * logits, int R, int V, long long stride, const float * temperature,
                          const int * top_k, const float * top_p, const float * min_p, const float * uniform,
                          int * out, cudaStream_t stream) {
     if (R <= 0) return IIAN_OK;
     if (V <= 0) return IIAN_ERR_SHAPE;
-    sample_kernel<<<R, kSampleThreads, 0, stream>>>(logits, V, (size_t) stride, temperature, top_k, top_p, min_p,
-                                                    uniform, out);
-    return iian_launch_status();
+    int ctas = 1;
+    while (ctas < kDrawCluster && V > ctas * 4096) ctas *= 2;
+    const int slice = (V - 1) / ctas + 1;
+    const bool staged = slice <= kStagedMax;
+    const size_t smem = staged ? (size_t) slice * sizeof(unsigned) : 0;
+    auto kernel = staged ? sample_kernel<true> : sample_kernel<false>;
+    if (smem > 40 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+        if (e != cudaSuccess) return 1000 + (int) e;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(kDrawThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned) ctas;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3((unsigned) R * (unsigned) ctas);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, logits, V, (size_t) stride, slice, temperature, top_k, top_p, min_p,
+                                             uniform, out);
+    return e == cudaSuccess ? IIAN_OK : 1000 + (int) e;
 }
 
 // logits [R, V] float32, changed in place.  allow_off / edit_off: [R + 1] int32 prefix sums; a token may appear in
