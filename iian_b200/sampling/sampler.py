@@ -15,6 +15,7 @@ from __future__ import annotations
 
 from typing import List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from .. import ops
@@ -35,6 +36,20 @@ def uniform(seed: int, index: int) -> float:
     """Number ``index`` of the stream ``seed``: a float32-exact value in [0, 1)."""
     h = _splitmix64(_splitmix64(seed & _MASK) ^ ((index * 0xD1B54A32D192ED03) & _MASK))
     return (h >> 40) / float(1 << 24)
+
+
+def uniforms(seeds: Sequence[int], indices: Sequence[int]) -> np.ndarray:
+    """``uniform`` of every (seed, index) pair, float32: the same integers on arrays (they wrap modulo 2^64)."""
+    def mix(x):
+        x = x + np.uint64(GOLDEN)
+        x = (x ^ (x >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+        x = (x ^ (x >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+        return x ^ (x >> np.uint64(31))
+
+    s = np.array([v & _MASK for v in seeds], dtype=np.uint64)
+    i = np.array([v & _MASK for v in indices], dtype=np.uint64)
+    h = mix(mix(s) ^ (i * np.uint64(0xD1B54A32D192ED03)))
+    return (h >> np.uint64(40)).astype(np.float32) * np.float32(2.0 ** -24)
 
 
 def request_seed(params: SamplingParams, engine_seed: int, request_id: int) -> int:
@@ -130,16 +145,15 @@ class Sampler:
         if all(p.is_greedy for p in params):
             k.argmax(logits, out)
             return out.tolist()
-        host = torch.empty((5, r), dtype=torch.float32)
-        for i, p in enumerate(params):
-            host[0, i] = p.temperature
-            host[1, i] = p.top_p
-            host[2, i] = p.min_p
-            host[3, i] = uniform(seeds[i], indices[i])
-            host[4, i] = float(max(p.top_k, 0))
-        dev = host.to(logits.device, non_blocking=False)
-        top_k = dev[4].to(torch.int32)
-        k.sample(logits, dev[0].contiguous(), top_k, dev[1].contiguous(), dev[2].contiguous(), dev[3].contiguous(), out)
+        # one array for the whole step, one upload: filled element by element through torch it took 0.7 ms of host time for 48 rows
+        host = np.empty((5, r), dtype=np.float32)
+        host[0] = [p.temperature for p in params]
+        host[1] = [p.top_p for p in params]
+        host[2] = [p.min_p for p in params]
+        host[3] = uniforms(seeds, indices)
+        host[4].view(np.int32)[:] = [min(max(p.top_k, 0), 0x7FFFFFFF) for p in params]
+        dev = torch.from_numpy(host).to(logits.device, non_blocking=False)
+        k.sample(logits, dev[0], dev[4].view(torch.int32), dev[1], dev[2], dev[3], out)
         return out.tolist()
 
     def logprobs(self, raw_logits: torch.Tensor, tokens: Sequence[int], params: Sequence[SamplingParams]):

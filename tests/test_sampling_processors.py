@@ -175,3 +175,12 @@ def test_logprobs_through_the_engine_are_those_of_the_raw_distribution(tmp_path)
         assert abs(lp - ref[tok].item()) < 1e-3
         assert len(top) == 3 and top[0][0] == int(torch.argmax(ref)) and abs(top[0][1] - ref.max().item()) < 1e-3
         toks.append(tok)
+
+
+def test_uniform_streams_of_a_step_are_the_requests_own():
+    import random
+    from iian_b200.sampling.sampler import uniform, uniforms
+    rng = random.Random(5)
+    seeds = [rng.getrandbits(64) for _ in range(200)] + [0, -3, 2 ** 64 - 1, 2 ** 70]
+    indices = [rng.randrange(1 << 20) for _ in range(200)] + [0, 1, 2, 3]
+    assert uniforms(seeds, indices).tolist() == [uniform(s, i) for s, i in zip(seeds, indices)]
