@@ -573,3 +573,16 @@ def test_paged_attention_mma(case, standout, mode):
     K().paged_attention_mma(q, kc, vc, out, m, num_heads=nh, num_kv_heads=nkv, head_dim=hd, scale=scale, window=window, **kw)
     err = (out.double().cpu() - want).abs().max().item()
     assert err < tol(dtype, max(1.0, want.abs().max().item())), err
+
+
+@pytest.mark.parametrize("od", DT)
+@pytest.mark.parametrize("N", [1, 2, 4, 5, 8, 9, 16, 17, 33, 64, 65, 130])
+@pytest.mark.parametrize("M,K_", [(1, 4), (33, 132), (130, 260), (257, 1000), (6151, 48)])
+def test_gemm_simt_forms_give_the_same_bits(od, N, M, K_):
+    """The streaming and the tiled form against the plain one, which operands that do not start on 16 bytes are left to."""
+    x, w = rnd(N, K_, seed=40), rnd(M, K_, seed=41)
+    odd = torch.empty(N * K_ + 1, dtype=torch.float32, device="cuda")[1:].view(N, K_).copy_(x)
+    a, b = (torch.full((N, M), float("nan"), dtype=od, device="cuda") for _ in range(2))
+    K().gemm_simt(x, w, a)
+    K().gemm_simt(odd, w, b)
+    assert torch.equal(a, b)
