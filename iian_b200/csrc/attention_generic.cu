@@ -12,6 +12,8 @@
 // Two options beyond the reference's formula, for mixers that have them: a sink per head (a logit with no key and no
 // value that joins the softmax's denominator once, unscaled: the running softmax simply starts at maximum sink_h with
 // denominator 1), and an output gate (o *= sigmoid(g) element by element, g read from rows of a wider matrix).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace iian {
@@ -19,18 +21,35 @@ namespace iian {
 constexpr int kGenMaxHeadDim = 512;
 constexpr int kGenWarps = 4;
 
-template <typename A>
+constexpr int kTileItems = 32;      // (token, head) pairs of a CTA of the tiled kernel: 32 / (heads of a group) tokens
+constexpr int kTileRuns = 4;        // requests whose tokens may lie side by side in such a CTA
+constexpr int kTileMinTokens = 8;   // tokens of a step from which the tiled kernel is launched
+
+// Whether the tokens [t0, t0 + tokens) of the step are the tiled kernel's: at most kTileRuns requests, no padding.  Both kernels ask.
+// A whole warp calls it (at most 32 tokens a tile).
+__device__ __forceinline__ bool tile_is_shared(const int * __restrict__ seq_of_token, int t0, int tokens, int N) {
+    const int lane = threadIdx.x & 31;
+    const bool in = lane < tokens && t0 + lane < N;
+    const int s = in ? seq_of_token[t0 + lane] : 0;
+    const int before = __shfl_up_sync(0xffffffffu, s, 1);
+    const unsigned padding = __ballot_sync(0xffffffffu, in && s < 0), starts = __ballot_sync(0xffffffffu, in && (lane == 0 || s != before));
+    return padding == 0 && __popc(starts) <= kTileRuns;
+}
+
+// VEC: rows of keys are whole 16-byte pieces.  NACC: output entries per lane (hd <= 32 * NACC).
+template <typename A, int NACC, bool VEC>
 __global__ void paged_attention_generic_kernel(
     const A * __restrict__ q, const A * __restrict__ k_cache, const A * __restrict__ v_cache,
     A * __restrict__ out, const int * __restrict__ positions, const int * __restrict__ seq_of_token,
     const int * __restrict__ block_table, int max_blocks, const int * __restrict__ ctx_len,
     int N, int nh, int nkv, int hd, int page_size, int num_pages, float scale, int window,
-    const float * __restrict__ sink, const A * __restrict__ gate, long long ld_gate) {
-    __shared__ float qs[kGenWarps][kGenMaxHeadDim];
+    const float * __restrict__ sink, const A * __restrict__ gate, long long ld_gate, int tile_tokens) {
+    __shared__ __align__(16) float qs[kGenWarps][kGenMaxHeadDim];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long item = (long long) blockIdx.x * kGenWarps + warp;
     if (item >= (long long) N * nh) return;
     const int t = (int) (item / nh), h = (int) (item % nh);
+    if (tile_tokens > 0 && tile_is_shared(seq_of_token, t / tile_tokens * tile_tokens, tile_tokens, N)) return;
     const int kvh = h / (nh / nkv);
     A * o = out + ((size_t) t * nh + h) * hd;
     const int s = seq_of_token[t];
@@ -47,10 +66,9 @@ __global__ void paged_attention_generic_kernel(
     for (int d = lane; d < hd; d += 32) qs[warp][d] = to_f32(qp[d]);
     __syncwarp();
 
-    constexpr int kAcc = kGenMaxHeadDim / 32;
-    float acc[kAcc];
+    float acc[NACC];
 #pragma unroll
-    for (int i = 0; i < kAcc; i++) acc[i] = 0.0f;
+    for (int i = 0; i < NACC; i++) acc[i] = 0.0f;
     float m = sink != nullptr ? sink[h] : -INFINITY, l = sink != nullptr ? 1.0f : 0.0f;
     const int * bt = block_table + (size_t) s * max_blocks;
 
@@ -72,7 +90,17 @@ __global__ void paged_attention_generic_kernel(
         float sc = -INFINITY;
         if (valid) {
             float dot = 0.0f;
-            for (int d = 0; d < hd; d++) dot += qs[warp][d] * to_f32(kp[d]);
+            if (VEC) {
+                constexpr int PIECE = 16 / sizeof(A);
+#pragma unroll 8
+                for (int d = 0; d < hd; d += PIECE) {
+                    const uint4 raw = __ldg(reinterpret_cast<const uint4 *>(kp + d));
+                    const A * kk = reinterpret_cast<const A *>(&raw);
+#pragma unroll
+                    for (int e = 0; e < PIECE; e++) dot = fmaf(qs[warp][d + e], to_f32(kk[e]), dot);
+                }
+            } else
+                for (int d = 0; d < hd; d++) dot = fmaf(qs[warp][d], to_f32(kp[d]), dot);
             sc = dot * scale;
         }
         const float tile_max = warp_max(sc);
@@ -82,23 +110,34 @@ __global__ void paged_attention_generic_kernel(
         const float corr = (m == -INFINITY) ? 0.0f : expf(m - m_new);
         l = l * corr + warp_sum(pj);
 #pragma unroll
-        for (int i = 0; i < kAcc; i++) acc[i] *= corr;
+        for (int i = 0; i < NACC; i++) acc[i] *= corr;
         m = m_new;
-        for (int jj = 0; jj < 32; jj++) {
-            const float pjj = __shfl_sync(0xffffffffu, pj, jj);
-            const unsigned long long vaddr = __shfl_sync(0xffffffffu, (unsigned long long) vp, jj);
-            if (pjj == 0.0f) continue;
-            const A * vrow = (const A *) vaddr;
+        // eight value rows are loaded before the first is added
+        constexpr int AT_ONCE = NACC <= 4 ? 8 : 4;
 #pragma unroll
-            for (int i = 0; i < kAcc; i++) {
-                const int d = lane + 32 * i;
-                if (d < hd) acc[i] += pjj * to_f32(vrow[d]);
+        for (int j0 = 0; j0 < 32; j0 += AT_ONCE) {
+            float pr[AT_ONCE], vr[AT_ONCE][NACC];
+#pragma unroll
+            for (int e = 0; e < AT_ONCE; e++) {
+                pr[e] = __shfl_sync(0xffffffffu, pj, j0 + e);
+                const A * vrow = (const A *) __shfl_sync(0xffffffffu, (unsigned long long) vp, j0 + e);
+#pragma unroll
+                for (int i = 0; i < NACC; i++) {
+                    const int d = lane + 32 * i;
+                    vr[e][i] = pr[e] != 0.0f && d < hd ? to_f32(vrow[d]) : 0.0f;
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < AT_ONCE; e++) {
+                if (pr[e] == 0.0f) continue;
+#pragma unroll
+                for (int i = 0; i < NACC; i++) acc[i] = fmaf(pr[e], vr[e][i], acc[i]);
             }
         }
     }
     const float inv = l > 0.0f ? 1.0f / l : 0.0f;     // a row that sees no key yields zeros
 #pragma unroll
-    for (int i = 0; i < kAcc; i++) {
+    for (int i = 0; i < NACC; i++) {
         const int d = lane + 32 * i;
         if (d < hd) {
             float v = acc[i] * inv;
@@ -106,6 +145,242 @@ __global__ void paged_attention_generic_kernel(
             o[d] = from_f32<A>(v);
         }
     }
+}
+
+__device__ __forceinline__ unsigned long long ag_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ unsigned long long ag_pair(float x, float y) {
+    unsigned long long d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+    return d;
+}
+__device__ __forceinline__ float2 ag_halves(unsigned long long v) {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+}
+__device__ __forceinline__ void ag_cp16(float * dst, const float * src, bool valid) {
+    const unsigned d = (unsigned) __cvta_generic_to_shared(dst);
+    const int n = valid ? 16 : 0;                      // src-size 0: zeros are written, nothing is read
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n));
+}
+
+// The same attention in float32 for neighbouring tokens: a CTA owns 32 (token, head) items of one KV head, eight a warp, and its key
+// tiles -- the same 32 keys from the same multiples of 32 -- come once through two stages of shared memory for all of them.  Every
+// item's arithmetic is the kernel's above term by term (a lane is a key in the scores and four output entries in the sum; packed
+// multiply-adds of two items, or of two entries, round as single ones do), so an item has the same bits whichever kernel it falls to.
+// What bounds it: reads of shared memory (a tile's keys and values per warp against eight items' multiply-adds).  2 requests,
+// 301 tokens x 16 heads of 128: 487 -> 77 us; 2,048 tokens 19.6 -> 1.2 ms (a warp per item, each reading its keys row by row from
+// global memory).
+constexpr int kTileHeadDim = 128;
+constexpr int kTileLd = kTileHeadDim + 4;
+constexpr size_t kTileSmem = (size_t) (2 * 2 * 32 * kTileLd + kTileItems * kTileHeadDim + kGenWarps * 8 * 64) * sizeof(float);
+
+__global__ void __launch_bounds__(kGenWarps * 32)
+paged_attention_tile_kernel(
+    const float * __restrict__ q, const float * __restrict__ k_cache, const float * __restrict__ v_cache,
+    float * __restrict__ out, const int * __restrict__ positions, const int * __restrict__ seq_of_token,
+    const int * __restrict__ block_table, int max_blocks, const int * __restrict__ ctx_len,
+    int N, int nh, int nkv, int hd, int page_size, int num_pages, float scale, int window,
+    const float * __restrict__ sink, const float * __restrict__ gate, long long ld_gate) {
+    extern __shared__ __align__(16) float sm[];
+    float * stages = sm;                               // [2][keys | values][32][kTileLd]
+    float * qs = sm + 2 * 2 * 32 * kTileLd;            // [16 pairs of items][hd][2]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float * ps = qs + kTileItems * kTileHeadDim + warp * 8 * 64;       // [8 items][32 keys][2]: probabilities, each twice
+    __shared__ unsigned good[2];                       // keys of a stage whose page exists
+    const int G = nh / nkv, tokens = kTileItems / G;
+    const int t0 = blockIdx.x * tokens, kvh = blockIdx.y;
+    if (!tile_is_shared(seq_of_token, t0, tokens, N)) return;
+    const int n_tok = min(tokens, N - t0), n_items = n_tok * G;
+    for (int e = tid; e < kTileItems * hd; e += kGenWarps * 32) {
+        const int item = e / hd, d = e % hd;
+        const float v = item < n_items ? q[((size_t) (t0 + item / G) * nh + kvh * G + item % G) * hd + d] : 0.0f;
+        qs[((item >> 1) * hd + d) * 2 + (item & 1)] = v;
+    }
+    unsigned long long acc[8][2];
+    float m[8], l[8];
+    int lo[8], hi[8], sq[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int item = warp * 8 + i, t = t0 + item / G;
+        const bool real = item < n_items;
+        const float sk = sink != nullptr ? sink[kvh * G + item % G] : -INFINITY;
+        m[i] = sk;
+        l[i] = sink != nullptr ? 1.0f : 0.0f;
+        sq[i] = real ? seq_of_token[t] : -1;
+        const int p = real ? positions[t] : -1;
+        hi[i] = real && ctx_len != nullptr ? min(p, ctx_len[sq[i]] - 1) : p;
+        lo[i] = window > 0 ? max(0, p - window + 1) : 0;
+        acc[i][0] = acc[i][1] = 0ull;
+    }
+    const int pieces = hd / 4;
+    int first = t0;
+    while (first < t0 + n_tok) {                       // one request's tokens after the other's
+        const int s = seq_of_token[first];
+        int end = first, k_lo = 0x7fffffff, k_hi = -1;
+        for (; end < t0 + n_tok && seq_of_token[end] == s; end++) {
+            const int p = positions[end];
+            k_hi = max(k_hi, ctx_len != nullptr ? min(p, ctx_len[s] - 1) : p);
+            k_lo = min(k_lo, window > 0 ? max(0, p - window + 1) : 0);
+        }
+        first = end;
+        const int * bt = block_table + (size_t) s * max_blocks;
+        const int kb0 = (k_lo / 32) * 32;
+        auto fill = [&](int kb, int stage) {           // four lanes a key
+            if (kb <= k_hi) {
+                const int r = tid >> 2, j = kb + r;
+                int page = -1;
+                if (j <= k_hi) page = bt[j / page_size];
+                const bool ok = page >= 0 && page < num_pages;
+                const size_t cell = ok ? (((size_t) page * nkv + kvh) * page_size + (j % page_size)) * hd : 0;
+                float * to = stages + (size_t) stage * 2 * 32 * kTileLd + r * kTileLd;
+                for (int c = tid & 3; c < pieces; c += 4) {
+                    ag_cp16(to + c * 4, k_cache + cell + c * 4, ok);
+                    ag_cp16(to + 32 * kTileLd + c * 4, v_cache + cell + c * 4, ok);
+                }
+                const unsigned b = __ballot_sync(0xffffffffu, ok);       // this warp's eight keys, four bits each
+                if (lane == 0) {
+                    unsigned mine = 0;
+                    for (int e = 0; e < 8; e++) mine |= ((b >> (4 * e)) & 1u) << e;
+                    reinterpret_cast<unsigned char *>(&good[stage])[warp] = (unsigned char) mine;
+                }
+            }
+            asm volatile("cp.async.commit_group;");
+        };
+        fill(kb0, 0);
+        int stage = 0;
+        for (int kb = kb0; kb <= k_hi; kb += 32, stage ^= 1) {
+            fill(kb + 32, stage ^ 1);
+            asm volatile("cp.async.wait_group 1;");
+            __syncthreads();
+            const float * ks = stages + (size_t) stage * 2 * 32 * kTileLd;
+            const float * vs = ks + 32 * kTileLd;
+            const bool here = (good[stage] >> lane) & 1u;
+            const int j = kb + lane;
+            bool any = false;
+#pragma unroll
+            for (int i = 0; i < 8; i++) any |= sq[i] == s && kb <= hi[i] && kb + 31 >= lo[i];
+            if (any) {                                 // the same for all lanes: an item's numbers are the warp's
+                unsigned long long dot[4] = {0ull, 0ull, 0ull, 0ull};
+                const float * kr = ks + lane * kTileLd;
+                const float * qw = qs + (size_t) warp * 4 * hd * 2;
+#pragma unroll 4
+                for (int d = 0; d < hd; d += 4) {
+                    const float4 k4 = *reinterpret_cast<const float4 *>(kr + d);
+                    const unsigned long long k0 = ag_pair(k4.x, k4.x), k1 = ag_pair(k4.y, k4.y), k2 = ag_pair(k4.z, k4.z), k3 = ag_pair(k4.w, k4.w);
+#pragma unroll
+                    for (int pr = 0; pr < 4; pr++) {
+                        const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(qw + (pr * hd + d) * 2);
+                        const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(qw + (pr * hd + d + 2) * 2);
+                        dot[pr] = ag_fma2(a.x, k0, dot[pr]);
+                        dot[pr] = ag_fma2(a.y, k1, dot[pr]);
+                        dot[pr] = ag_fma2(b.x, k2, dot[pr]);
+                        dot[pr] = ag_fma2(b.y, k3, dot[pr]);
+                    }
+                }
+                bool full = true;                      // every item weighs every key of the tile: no term is left out below
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const float2 two = ag_halves(dot[i >> 1]);
+                    const bool valid = here && sq[i] == s && j >= lo[i] && j <= hi[i];
+                    const float sc = valid ? ((i & 1) ? two.y : two.x) * scale : -INFINITY;
+                    const float tile_max = warp_max(sc);
+                    float pj = 0.0f;
+                    if (tile_max != -INFINITY) {
+                        const float m_new = fmaxf(m[i], tile_max);
+                        pj = valid ? expf(sc - m_new) : 0.0f;
+                        const float corr = (m[i] == -INFINITY) ? 0.0f : expf(m[i] - m_new);
+                        l[i] = l[i] * corr + warp_sum(pj);
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            const float2 v = ag_halves(acc[i][e]);
+                            acc[i][e] = ag_pair(v.x * corr, v.y * corr);
+                        }
+                        m[i] = m_new;
+                    }
+                    full &= pj != 0.0f;
+                    *reinterpret_cast<float2 *>(ps + (i * 32 + lane) * 2) = make_float2(pj, pj);
+                }
+                full = __all_sync(0xffffffffu, full);
+                __syncwarp();
+                if (full && lane < pieces) {
+#pragma unroll 4
+                    for (int jj = 0; jj < 32; jj += 2) {
+                        const ulonglong2 v0 = *reinterpret_cast<const ulonglong2 *>(vs + jj * kTileLd + lane * 4);
+                        const ulonglong2 v1 = *reinterpret_cast<const ulonglong2 *>(vs + (jj + 1) * kTileLd + lane * 4);
+#pragma unroll
+                        for (int i = 0; i < 8; i++) {
+                            const ulonglong2 p2 = *reinterpret_cast<const ulonglong2 *>(ps + (i * 32 + jj) * 2);
+                            acc[i][0] = ag_fma2(p2.x, v0.x, acc[i][0]);
+                            acc[i][1] = ag_fma2(p2.x, v0.y, acc[i][1]);
+                            acc[i][0] = ag_fma2(p2.y, v1.x, acc[i][0]);
+                            acc[i][1] = ag_fma2(p2.y, v1.y, acc[i][1]);
+                        }
+                    }
+                } else if (lane < pieces) {
+#pragma unroll 4
+                    for (int jj = 0; jj < 32; jj += 2) {
+                        const ulonglong2 v0 = *reinterpret_cast<const ulonglong2 *>(vs + jj * kTileLd + lane * 4);
+                        const ulonglong2 v1 = *reinterpret_cast<const ulonglong2 *>(vs + (jj + 1) * kTileLd + lane * 4);
+#pragma unroll
+                        for (int i = 0; i < 8; i++) {
+                            const ulonglong2 p2 = *reinterpret_cast<const ulonglong2 *>(ps + (i * 32 + jj) * 2);
+                            if (ag_halves(p2.x).x != 0.0f) { acc[i][0] = ag_fma2(p2.x, v0.x, acc[i][0]); acc[i][1] = ag_fma2(p2.x, v0.y, acc[i][1]); }
+                            if (ag_halves(p2.y).x != 0.0f) { acc[i][0] = ag_fma2(p2.y, v1.x, acc[i][0]); acc[i][1] = ag_fma2(p2.y, v1.y, acc[i][1]); }
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            __syncthreads();                           // everyone is done with this stage before it is filled again
+        }
+        asm volatile("cp.async.wait_group 0;");
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int item = warp * 8 + i;
+        if (item >= n_items || lane >= pieces) continue;
+        const int t = t0 + item / G, h = kvh * G + item % G;
+        const float inv = l[i] > 0.0f ? 1.0f / l[i] : 0.0f;
+        const float2 x = ag_halves(acc[i][0]), y = ag_halves(acc[i][1]);
+        float4 v = make_float4(x.x * inv, x.y * inv, y.x * inv, y.y * inv);
+        if (gate != nullptr) {
+            const float * g = gate + (size_t) t * ld_gate + h * hd + lane * 4;
+            v.x *= 1.0f / (1.0f + expf(-g[0]));
+            v.y *= 1.0f / (1.0f + expf(-g[1]));
+            v.z *= 1.0f / (1.0f + expf(-g[2]));
+            v.w *= 1.0f / (1.0f + expf(-g[3]));
+        }
+        float * o = out + ((size_t) t * nh + h) * hd + lane * 4;
+        *reinterpret_cast<float4 *>(o) = v;
+    }
+}
+
+template <typename A>
+static int launch_generic(const A * q, const A * k_cache, const A * v_cache, A * out, const int * positions, const int * seq_of_token,
+                          const int * block_table, int max_blocks, const int * ctx_len, int N, int nh, int nkv, int hd, int page_size,
+                          int num_pages, float scale, int window, const float * sink, const A * gate, long long ld_gate, int tile_tokens,
+                          cudaStream_t stream) {
+    const unsigned blocks = (unsigned) (((long long) N * nh + kGenWarps - 1) / kGenWarps);
+    const bool vec = (size_t) hd * sizeof(A) % 16 == 0 && (uintptr_t) k_cache % 16 == 0;
+    auto go = [&](auto nacc, auto v) {
+        paged_attention_generic_kernel<A, decltype(nacc)::value, decltype(v)::value><<<blocks, kGenWarps * 32, 0, stream>>>(
+            q, k_cache, v_cache, out, positions, seq_of_token, block_table, max_blocks, ctx_len, N, nh, nkv, hd, page_size, num_pages,
+            scale, window, sink, gate, ld_gate, tile_tokens);
+    };
+    auto pick = [&](auto v) {
+        if (hd <= 64) go(std::integral_constant<int, 2>(), v);
+        else if (hd <= 128) go(std::integral_constant<int, 4>(), v);
+        else go(std::integral_constant<int, kGenMaxHeadDim / 32>(), v);
+    };
+    if (vec) pick(std::true_type());
+    else pick(std::false_type());
+    return iian_launch_status();
 }
 
 }  // namespace iian
@@ -122,21 +397,29 @@ IIAN_API int iian_paged_attention_sink(
     float scale, int window, const float * sink, const void * gate, long long ld_gate, cudaStream_t stream) {
     if (N <= 0) return IIAN_OK;
     if (hd <= 0 || hd > kGenMaxHeadDim || nkv <= 0 || nh % nkv != 0 || page_size <= 0) return IIAN_ERR_SHAPE;
-    const long long items = (long long) N * nh;
-    const unsigned blocks = (unsigned) ((items + kGenWarps - 1) / kGenWarps);
-    const int threads = kGenWarps * 32;
-    if (act_dtype == IIAN_F32)
-        paged_attention_generic_kernel<float><<<blocks, threads, 0, stream>>>(
-            (const float *) q, (const float *) k_cache, (const float *) v_cache, (float *) out, positions,
-            seq_of_token, block_table, max_blocks, ctx_len, N, nh, nkv, hd, page_size, num_pages, scale, window, sink,
-            (const float *) gate, ld_gate);
-    else if (act_dtype == IIAN_BF16)
-        paged_attention_generic_kernel<__nv_bfloat16><<<blocks, threads, 0, stream>>>(
-            (const __nv_bfloat16 *) q, (const __nv_bfloat16 *) k_cache, (const __nv_bfloat16 *) v_cache,
-            (__nv_bfloat16 *) out, positions, seq_of_token, block_table, max_blocks, ctx_len, N, nh, nkv, hd,
-            page_size, num_pages, scale, window, sink, (const __nv_bfloat16 *) gate, ld_gate);
-    else return IIAN_ERR_DTYPE;
-    return iian_launch_status();
+    if (act_dtype == IIAN_BF16)
+        return launch_generic((const __nv_bfloat16 *) q, (const __nv_bfloat16 *) k_cache, (const __nv_bfloat16 *) v_cache, (__nv_bfloat16 *) out,
+                              positions, seq_of_token, block_table, max_blocks, ctx_len, N, nh, nkv, hd, page_size, num_pages, scale, window,
+                              sink, (const __nv_bfloat16 *) gate, ld_gate, 0, stream);
+    if (act_dtype != IIAN_F32) return IIAN_ERR_DTYPE;
+    // neighbouring tokens of a request share their key tiles where the sizes allow it; what is left (tokens of many requests side by
+    // side, as when decoding) goes to the kernel with a warp per item, which leaves the others out
+    const int group = nh / nkv;
+    const uintptr_t all = (uintptr_t) k_cache | (uintptr_t) v_cache | (uintptr_t) out;
+    int tile_tokens = 0;
+    if (N >= kTileMinTokens && group <= 8 && kTileItems % group == 0 && hd <= kTileHeadDim && hd % 4 == 0 && all % 16 == 0 && nkv <= 65535) {
+        tile_tokens = kTileItems / group;
+        const cudaError_t e = cudaFuncSetAttribute(paged_attention_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kTileSmem);
+        if (e != cudaSuccess) return 1000 + (int) e;
+        paged_attention_tile_kernel<<<dim3((N + tile_tokens - 1) / tile_tokens, nkv), kGenWarps * 32, kTileSmem, stream>>>(
+            (const float *) q, (const float *) k_cache, (const float *) v_cache, (float *) out, positions, seq_of_token, block_table,
+            max_blocks, ctx_len, N, nh, nkv, hd, page_size, num_pages, scale, window, sink, (const float *) gate, ld_gate);
+        const int rc = iian_launch_status();
+        if (rc != IIAN_OK) return rc;
+    }
+    return launch_generic((const float *) q, (const float *) k_cache, (const float *) v_cache, (float *) out, positions, seq_of_token,
+                          block_table, max_blocks, ctx_len, N, nh, nkv, hd, page_size, num_pages, scale, window, sink, (const float *) gate,
+                          ld_gate, tile_tokens, stream);
 }
 
 IIAN_API int iian_paged_attention_generic(

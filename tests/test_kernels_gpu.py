@@ -586,3 +586,22 @@ def test_gemm_simt_forms_give_the_same_bits(od, N, M, K_):
     K().gemm_simt(x, w, a)
     K().gemm_simt(odd, w, b)
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("window", [0, 19])
+@pytest.mark.parametrize("ctx_lens,q_lens", [([8], [8]), ([45], [40]), ([75, 266], [75, 226]), ([23, 101, 20], [20, 1, 13]),
+                                             ([13, 22, 39, 41, 67], [3, 2, 9, 1, 17]), ([2, 3, 4, 5, 6, 7, 36], [2, 2, 2, 2, 2, 2, 30])])
+@pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 16), (8, 1, 64), (16, 8, 128), (5, 5, 36), (6, 2, 64), (4, 4, 132)])
+def test_paged_attention_generic_bits_do_not_depend_on_the_neighbours(nh, nkv, hd, ctx_lens, q_lens, window):
+    """Tokens that share their key tiles with neighbours against the same tokens alone, one call each: the same bits."""
+    q, kc, vc, m, _, scale = attention_case(torch.float32, nh, nkv, hd, 16, ctx_lens, q_lens, window, seed=9, standout=None)
+    run = lambda q_, m_, out: K().paged_attention_generic(q_, kc, vc, out, m_, num_heads=nh, num_kv_heads=nkv, head_dim=hd, scale=scale,
+                                                          window=window)
+    out = torch.full((q.shape[0], nh * hd), float("nan")).cuda()
+    run(q, m, out)
+    for t in sorted({0, 1, q.shape[0] // 2, q.shape[0] - 2, q.shape[0] - 1}):
+        class One:
+            positions, seq_of_token, block_table, ctx_len = m.positions[t:t + 1], m.seq_of_token[t:t + 1], m.block_table, m.ctx_len
+        one = torch.empty(1, nh * hd).cuda()
+        run(q[t:t + 1].contiguous(), One, one)
+        assert torch.equal(one[0], out[t]), t
