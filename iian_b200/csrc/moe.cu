@@ -20,6 +20,10 @@ constexpr int kTileM = 64, kTileN = 64, kTileK = 16;
 // One warp per token.  ids / wts: [N, top].
 // mode 0: the weight of a chosen expert is sigmoid(logit); mode 1: the softmax over the chosen logits only.  bias (optional,
 // float32 [E]) is added to the logits before anything else.
+// SLOTS: a lane's logits e = lane, lane + 32, ... held in registers (E <= 32 * SLOTS), 0: read again for every choice.  A chain of
+// `top` reductions over the warp bounds it; lane k keeps choice k (top <= 32), so that nothing is read back.  2,048 tokens, 5 of 64
+// experts: 28 us when every choice went through memory.
+template <int SLOTS>
 __global__ void moe_route_kernel(const float * __restrict__ logits, long long ld, int E, int top, int * __restrict__ ids,
                                  float * __restrict__ wts, int N, const float * __restrict__ bias, int mode) {
     pdl_wait();
@@ -28,14 +32,35 @@ __global__ void moe_route_kernel(const float * __restrict__ logits, long long ld
     const long long t = (long long) blockIdx.x * (blockDim.x >> 5) + warp;
     if (t >= N) return;
     const float * z = logits + t * ld;
+    float held[SLOTS > 0 ? SLOTS : 1];
+    if (SLOTS > 0) {
+#pragma unroll
+        for (int i = 0; i < SLOTS; i++) {
+            const int e = lane + 32 * i;
+            held[i] = e < E ? (bias != nullptr ? z[e] + bias[e] : z[e]) : -INFINITY;
+        }
+    }
     unsigned long long taken_lo = 0;          // experts already chosen, for the lanes' own candidates (by slot i / 32)
+    float mine = 0.0f;                        // choice `lane`: its weight, or in mode 1 its logit
+    int mine_e = 0;
+    float first = 0.0f;
+    const bool in_lanes = top <= 32;
     for (int k = 0; k < top; k++) {
         float best = -INFINITY;
         int best_e = 0x7fffffff;
-        for (int e = lane, i = 0; e < E; e += 32, i++) {
-            if (i < 64 && ((taken_lo >> i) & 1ull)) continue;
-            const float v = bias != nullptr ? z[e] + bias[e] : z[e];
-            if (v > best || (v == best && e < best_e)) { best = v; best_e = e; }
+        if (SLOTS > 0) {
+#pragma unroll
+            for (int i = 0; i < SLOTS; i++) {
+                const int e = lane + 32 * i;
+                if (e >= E || ((taken_lo >> i) & 1ull)) continue;
+                if (held[i] > best || (held[i] == best && e < best_e)) { best = held[i]; best_e = e; }
+            }
+        } else {
+            for (int e = lane, i = 0; e < E; e += 32, i++) {
+                if (i < 64 && ((taken_lo >> i) & 1ull)) continue;
+                const float v = bias != nullptr ? z[e] + bias[e] : z[e];
+                if (v > best || (v == best && e < best_e)) { best = v; best_e = e; }
+            }
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -43,17 +68,30 @@ __global__ void moe_route_kernel(const float * __restrict__ logits, long long ld
             const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
             if (ov > best || (ov == best && oe < best_e)) { best = ov; best_e = oe; }
         }
-        if (best_e != 0x7fffffff && (best_e & 31) == lane) taken_lo |= 1ull << (best_e >> 5);
-        if (lane == 0) {
-            ids[t * top + k] = best_e == 0x7fffffff ? 0 : best_e;
-            wts[t * top + k] = best_e == 0x7fffffff ? (mode == 1 ? -INFINITY : 0.0f) : mode == 1 ? best : 1.0f / (1.0f + expf(-best));
+        const bool none = best_e == 0x7fffffff;
+        if (!none && (best_e & 31) == lane) taken_lo |= 1ull << (best_e >> 5);
+        const float w = none ? (mode == 1 ? -INFINITY : 0.0f) : best;
+        if (k == 0) first = w;
+        if (in_lanes) {
+            if (lane == k) { mine = mode == 1 || none ? w : 1.0f / (1.0f + expf(-w)); mine_e = none ? 0 : best_e; }
+        } else if (lane == 0) {
+            ids[t * top + k] = none ? 0 : best_e;
+            wts[t * top + k] = mode == 1 || none ? w : 1.0f / (1.0f + expf(-w));
         }
     }
-    if (mode == 1 && lane == 0) {      // the chosen logits came in falling order: the first is their maximum
-        const float mx = wts[t * top];
+    // mode 1: the chosen logits came in falling order, the first is their maximum; the sum in the order of the choices
+    if (in_lanes) {
+        if (mode == 1) {
+            const float e = lane < top ? expf(mine - first) : 0.0f;
+            float sum = 0.0f;
+            for (int k = 0; k < top; k++) sum += __shfl_sync(0xffffffffu, e, k);
+            mine = e / sum;
+        }
+        if (lane < top) { ids[t * top + lane] = mine_e; wts[t * top + lane] = mine; }
+    } else if (mode == 1 && lane == 0) {
         float sum = 0.0f;
         for (int k = 0; k < top; k++) {
-            const float e = expf(wts[t * top + k] - mx);
+            const float e = expf(wts[t * top + k] - first);
             wts[t * top + k] = e;
             sum += e;
         }
@@ -133,56 +171,101 @@ __global__ void moe_plan_kernel(const int * __restrict__ ids, int M, int E, int 
     for (int i = threadIdx.x; i < M; i += blockDim.x)
         if ((unsigned) ids[i] < (unsigned) E) atomicAdd(&counts[ids[i]], 1);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0, nt = 0;
-        for (int e = 0; e < E; e++) {
+    if (threadIdx.x < 32) {                   // one warp: a lane takes neighbouring experts, rows and tiles are counted up over the lanes
+        const int lane = threadIdx.x, per = (E + 31) / 32, e0 = min(E, lane * per), e1 = min(E, e0 + per);
+        int rows = 0, nt = 0;
+        for (int e = e0; e < e1; e++) { rows += counts[e]; nt += (counts[e] + tile_rows - 1) / tile_rows; }
+        const int own_rows = rows, own_tiles = nt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int r = __shfl_up_sync(0xffffffffu, rows, o), n = __shfl_up_sync(0xffffffffu, nt, o);
+            if (lane >= o) { rows += r; nt += n; }
+        }
+        if (lane == 31) { offsets[E] = rows; tiles[0] = min(nt, max_tiles); }
+        int run = rows - own_rows, at = nt - own_tiles;
+        for (int e = e0; e < e1; e++) {
             offsets[e] = run;
             cursor[e] = run;
-            for (int r = 0; r < counts[e] && nt < max_tiles; r += tile_rows) {
-                tiles[1 + 2 * nt] = e;
-                tiles[2 + 2 * nt] = run + r;
-                nt++;
-            }
+            // tiles of more than 64 rows (the tensor cores', which end where the next begins): an expert's rows in equal shares of 16s
+            const int share = tile_rows > kTileM && counts[e] > tile_rows
+                ? min(tile_rows, (((counts[e] - 1) / ((counts[e] + tile_rows - 1) / tile_rows) + 1) + 15) / 16 * 16) : tile_rows;
+            for (int r = 0; r < counts[e]; r += share, at++)
+                if (at < max_tiles) {
+                    tiles[1 + 2 * at] = e;
+                    tiles[2 + 2 * at] = run + r;
+                }
             run += counts[e];
         }
-        offsets[E] = run;
-        tiles[0] = nt;
     }
     __syncthreads();
     // the order of an expert's rows among themselves is left to the atomics: a row's arithmetic does not depend on it
     for (int i = threadIdx.x; i < M; i += blockDim.x) pos[i] = (unsigned) ids[i] < (unsigned) E ? atomicAdd(&cursor[ids[i]], 1) : -1;
 }
 
-// xs[pos[t * top + k], :] = A(w[t, k] * h[t, :]);  rows[pos] = t * top + k
-template <typename A>
+// V neighbouring values as one access: V = 1, or 16 bytes
+template <typename A, int V> __device__ __forceinline__ void moe_load(const A * src, float * f) {
+    if constexpr (V == 8) unpack8(*reinterpret_cast<const uint4 *>(src), f);
+    else if constexpr (V == 4) { const float4 q = *reinterpret_cast<const float4 *>(src); f[0] = q.x; f[1] = q.y; f[2] = q.z; f[3] = q.w; }
+    else f[0] = to_f32(*src);
+}
+template <typename A, int V> __device__ __forceinline__ void moe_store(A * dst, const float * f) {
+    if constexpr (V == 8) {
+        __nv_bfloat162 r[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) r[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+        *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<uint4 *>(r);
+    } else if constexpr (V == 4) *reinterpret_cast<float4 *>(dst) = make_float4(f[0], f[1], f[2], f[3]);
+    else *dst = from_f32<A>(f[0]);
+}
+
+// xs[pos[t * top + k], :] = A(w[t, k] * h[t, :]).  A CTA takes a token (and with gridDim.y a share of its columns): the row is read once
+// for all its choices, 16 bytes an access.  2,048 tokens x 5 rows of 2,048 bf16: 40 us with a CTA per choice and scalar accesses.
+template <typename A, int V>
 __global__ void moe_scatter_kernel(const A * __restrict__ h, const int * __restrict__ pos, const float * __restrict__ wts,
                                    A * __restrict__ xs, int W, int top) {
     pdl_wait();
     pdl_launch_dependents();
-    const size_t i = blockIdx.x;              // (token, choice)
-    const size_t t = i / top;
-    if (pos[i] < 0) return;                   // no expert behind this choice
-    const float w = wts != nullptr ? wts[i] : 1.0f;
-    const A * src = h + t * W;
-    A * dst = xs + (size_t) pos[i] * W;
-    for (int c = threadIdx.x; c < W; c += blockDim.x) dst[c] = from_f32<A>(w * to_f32(src[c]));
+    const size_t t = blockIdx.x;
+    for (int c = V * (blockIdx.y * blockDim.x + threadIdx.x); c < W; c += V * blockDim.x * gridDim.y) {
+        float f[V], g[V];
+        moe_load<A, V>(h + t * W + c, f);
+        for (int k = 0; k < top; k++) {
+            const int p = pos[t * top + k];
+            if (p < 0) continue;              // no expert behind this choice
+            const float w = wts != nullptr ? wts[t * top + k] : 1.0f;
+#pragma unroll
+            for (int i = 0; i < V; i++) g[i] = w * f[i];
+            moe_store<A, V>(xs + (size_t) p * W + c, g);
+        }
+    }
 }
 
 // out[t, :] = sum_k [wts[t, k] *] ys[pos[t * top + k], :]  (k ascending)
-template <typename A>
+// V columns a thread, gridDim.y shares of the columns.  2,048 tokens x 5 rows of 2,048 bf16 and an addend: 35 us with scalar accesses;
+// 24 tokens 17 us with one CTA a token.
+template <typename A, int V>
 __global__ void moe_combine_kernel(const A * __restrict__ ys, const int * __restrict__ pos, const float * __restrict__ wts,
                                    A * __restrict__ out, int W, int top, const A * add) {
     pdl_wait();
     pdl_launch_dependents();
     const size_t t = blockIdx.x;
-    for (int c = threadIdx.x; c < W; c += blockDim.x) {
-        float acc = 0.0f;
+    for (int c = V * (blockIdx.y * blockDim.x + threadIdx.x); c < W; c += V * blockDim.x * gridDim.y) {
+        float acc[V], y[V];
+#pragma unroll
+        for (int i = 0; i < V; i++) acc[i] = 0.0f;
+#pragma unroll 4
         for (int k = 0; k < top; k++) {
-            const float y = to_f32(ys[(size_t) pos[t * top + k] * W + c]);
-            acc += wts != nullptr ? wts[t * top + k] * y : y;
+            moe_load<A, V>(ys + (size_t) pos[t * top + k] * W + c, y);
+            const float w = wts != nullptr ? wts[t * top + k] : 1.0f;
+#pragma unroll
+            for (int i = 0; i < V; i++) acc[i] = fmaf(w, y[i], acc[i]);
         }
-        if (add != nullptr) acc += to_f32(add[t * W + c]);        // may be `out` itself: read before it is written
-        out[t * W + c] = from_f32<A>(acc);
+        if (add != nullptr) {
+            moe_load<A, V>(add + t * W + c, y);        // may be `out` itself: read before it is written
+#pragma unroll
+            for (int i = 0; i < V; i++) acc[i] += y[i];
+        }
+        moe_store<A, V>(out + t * W + c, acc);
     }
 }
 
@@ -318,13 +401,20 @@ using namespace iian;
 
 IIAN_API int iian_moe_tile_rows() { return kTileM; }
 
+static int launch_route(const float * logits, long long ld, int E, int top, int * ids, float * wts, int N, const float * bias, int mode,
+                        cudaStream_t stream) {
+    const int warps = 4;
+    const dim3 grid((N + warps - 1) / warps), block(warps * 32);
+    if (E <= 64) return iian_launch(moe_route_kernel<2>, grid, block, 0, stream, logits, ld, E, top, ids, wts, N, bias, mode);
+    if (E <= 256) return iian_launch(moe_route_kernel<8>, grid, block, 0, stream, logits, ld, E, top, ids, wts, N, bias, mode);
+    return iian_launch(moe_route_kernel<0>, grid, block, 0, stream, logits, ld, E, top, ids, wts, N, bias, mode);
+}
+
 // logits f32 (row stride ld) -> ids i32 [N, top], wts f32 [N, top]
 IIAN_API int iian_moe_route(const float * logits, long long ld, int E, int top, int * ids, float * wts, int N, cudaStream_t stream) {
     if (N <= 0) return IIAN_OK;
     if (E <= 0 || top <= 0 || top > E || E > 2048) return IIAN_ERR_SHAPE;
-    const int warps = 4;
-    return iian_launch(moe_route_kernel, dim3((N + warps - 1) / warps), dim3(warps * 32), 0, stream, logits, ld, E, top, ids, wts, N,
-                       (const float *) nullptr, 0);
+    return launch_route(logits, ld, E, top, ids, wts, N, nullptr, 0, stream);
 }
 
 // The same with a bias on the logits (float32 [E] or null) and the weights as the softmax over the chosen logits only.
@@ -332,9 +422,7 @@ IIAN_API int iian_moe_route_softmax(const float * logits, long long ld, const fl
                                     int N, cudaStream_t stream) {
     if (N <= 0) return IIAN_OK;
     if (E <= 0 || top <= 0 || top > E || E > 2048) return IIAN_ERR_SHAPE;
-    const int warps = 4;
-    return iian_launch(moe_route_kernel, dim3((N + warps - 1) / warps), dim3(warps * 32), 0, stream, logits, ld, E, top, ids, wts, N,
-                       bias, 1);
+    return launch_route(logits, ld, E, top, ids, wts, N, bias, 1, stream);
 }
 
 // Softmax over all E outputs, choice by score + correction (float32 [E] or null), weights scale * score.
@@ -366,14 +454,28 @@ IIAN_API int iian_moe_plan(const int * ids, int M, int E, int * offsets, int * p
                        max_tiles, tile_rows);
 }
 
+// How rows of W values are spread: 16-byte pieces where rows and pointers allow it, a CTA per row, more where there are few rows.
+static bool row_shares(int N, int W, int act_dtype, uintptr_t pointers, dim3 & grid, int & threads) {
+    const int V = act_dtype == IIAN_F32 ? 4 : 8;
+    const bool vec = W % V == 0 && (pointers & 15) == 0;
+    const int cols = vec ? W / V : W;
+    threads = cols >= 256 ? 256 : (cols + 31) / 32 * 32;
+    if (N < 128 && cols > 64) threads = 64;
+    grid = dim3(N, N >= 1024 ? 1 : min((cols + threads - 1) / threads, 8));
+    return vec;
+}
+
 IIAN_API int iian_moe_scatter(const void * h, const int * pos, const float * wts, void * xs, int act_dtype, int N, int W, int top,
                               cudaStream_t stream) {
     if (N <= 0) return IIAN_OK;
-    const int threads = W >= 1024 ? 256 : 128;
-    const unsigned blocks = (unsigned) ((size_t) N * top);
-    if (act_dtype == IIAN_F32) return iian_launch(moe_scatter_kernel<float>, dim3(blocks), dim3(threads), 0, stream, (const float *) h, pos, wts, (float *) xs, W, top);
-    if (act_dtype == IIAN_BF16) return iian_launch(moe_scatter_kernel<__nv_bfloat16>, dim3(blocks), dim3(threads), 0, stream, (const __nv_bfloat16 *) h, pos, wts, (__nv_bfloat16 *) xs, W, top);
-    return IIAN_ERR_DTYPE;
+    if (act_dtype != IIAN_F32 && act_dtype != IIAN_BF16) return IIAN_ERR_DTYPE;
+    int threads;
+    dim3 grid;
+    const bool vec = row_shares(N, W, act_dtype, (uintptr_t) h | (uintptr_t) xs, grid, threads);
+#define IIAN_SCATTER(A, V) iian_launch(moe_scatter_kernel<A, V>, grid, dim3(threads), 0, stream, (const A *) h, pos, wts, (A *) xs, W, top)
+    if (act_dtype == IIAN_F32) return vec ? IIAN_SCATTER(float, 4) : IIAN_SCATTER(float, 1);
+    return vec ? IIAN_SCATTER(__nv_bfloat16, 8) : IIAN_SCATTER(__nv_bfloat16, 1);
+#undef IIAN_SCATTER
 }
 
 // wts: f32 [N, top], the weight of each expert's OUTPUT in the sum, or null (plain sum); add: A [N, W] or null, rows added
@@ -381,10 +483,14 @@ IIAN_API int iian_moe_scatter(const void * h, const int * pos, const float * wts
 IIAN_API int iian_moe_combine_add(const void * ys, const int * pos, const float * wts, const void * add, void * out, int act_dtype,
                                   int N, int W, int top, cudaStream_t stream) {
     if (N <= 0) return IIAN_OK;
-    const int threads = W >= 1024 ? 256 : 128;
-    if (act_dtype == IIAN_F32) return iian_launch(moe_combine_kernel<float>, dim3(N), dim3(threads), 0, stream, (const float *) ys, pos, wts, (float *) out, W, top, (const float *) add);
-    if (act_dtype == IIAN_BF16) return iian_launch(moe_combine_kernel<__nv_bfloat16>, dim3(N), dim3(threads), 0, stream, (const __nv_bfloat16 *) ys, pos, wts, (__nv_bfloat16 *) out, W, top, (const __nv_bfloat16 *) add);
-    return IIAN_ERR_DTYPE;
+    if (act_dtype != IIAN_F32 && act_dtype != IIAN_BF16) return IIAN_ERR_DTYPE;
+    int threads;
+    dim3 grid;
+    const bool vec = row_shares(N, W, act_dtype, (uintptr_t) ys | (uintptr_t) add | (uintptr_t) out, grid, threads);
+#define IIAN_SUM(A, V) iian_launch(moe_combine_kernel<A, V>, grid, dim3(threads), 0, stream, (const A *) ys, pos, wts, (A *) out, W, top, (const A *) add)
+    if (act_dtype == IIAN_F32) return vec ? IIAN_SUM(float, 4) : IIAN_SUM(float, 1);
+    return vec ? IIAN_SUM(__nv_bfloat16, 8) : IIAN_SUM(__nv_bfloat16, 1);
+#undef IIAN_SUM
 }
 
 // wts: f32 [N, top]; h: A [N, W], the rows choices without an expert (pos < 0) pass on; add: A [N, W] or null (it may be `out`),
@@ -394,11 +500,9 @@ IIAN_API int iian_moe_combine_mixed(const void * ys, const int * pos, const floa
                                     cudaStream_t stream) {
     if (N <= 0) return IIAN_OK;
     if (act_dtype != IIAN_F32 && act_dtype != IIAN_BF16) return IIAN_ERR_DTYPE;
-    const int V = act_dtype == IIAN_F32 ? 4 : 8;
-    const bool vec = W % V == 0 && (((uintptr_t) ys | (uintptr_t) h | (uintptr_t) add | (uintptr_t) out) & 15) == 0;
-    const int cols = vec ? W / V : W;
-    const int threads = cols >= 256 ? 256 : (cols + 31) / 32 * 32;
-    const dim3 grid(N, N >= 1024 ? 1 : min((cols + threads - 1) / threads, 8));
+    int threads;
+    dim3 grid;
+    const bool vec = row_shares(N, W, act_dtype, (uintptr_t) ys | (uintptr_t) h | (uintptr_t) add | (uintptr_t) out, grid, threads);
 #define IIAN_MIX(A, V) iian_launch(moe_combine_mixed_kernel<A, V>, grid, dim3(threads), 0, stream, (const A *) ys, pos, wts, (const A *) h, \
                                    (A *) out, W, top, (const A *) add, add_gate, ld_gate)
     if (act_dtype == IIAN_F32) return vec ? IIAN_MIX(float, 4) : IIAN_MIX(float, 1);
