@@ -154,10 +154,11 @@ def run(peaks: dict, width: int = 2048, heads: int = 16) -> dict:
         ctx_ = StepContext(Workspace(dev))
         part.forward(h, ctx_)                   # sizes the buffers and leaves a plan
         m = n * top
-        offsets, tiles = ctx_.buf("expert_offsets", (E + 1,), torch.int32), ctx_.buf("expert_tiles", (1 + 2 * k.moe_max_tiles(m, E, 128),), torch.int32)
+        tr = k.moe_tc_tile_rows(m, E)
+        offsets, tiles = ctx_.buf("expert_offsets", (E + 1,), torch.int32), ctx_.buf("expert_tiles", (1 + 2 * k.moe_max_tiles(m, E, tr),), torch.int32)
         xs, act, ys = ctx_.buf("expert_in", (m, width), bf), ctx_.buf("expert_act", (m, ff), bf), ctx_.buf("expert_out", (m, width), bf)
-        ms1 = _timed(lambda: k.moe_grouped_gemm_tc(xs, part.w_gate_up, act, offsets, tiles, gated=True))
-        ms2 = _timed(lambda: k.moe_grouped_gemm_tc(act, part.w_down, ys, offsets, tiles, gated=False))
+        ms1 = _timed(lambda: k.moe_grouped_gemm_tc(xs, part.w_gate_up, act, offsets, tiles, gated=True, tile_rows=tr))
+        ms2 = _timed(lambda: k.moe_grouped_gemm_tc(act, part.w_down, ys, offsets, tiles, gated=False, tile_rows=tr))
         ms_all = _timed(lambda: part.forward(h, ctx_))
         if n >= 128:
             flop_row(f"expert_gate_up_{n}", ms1, 2.0 * m * 2 * ff * width)

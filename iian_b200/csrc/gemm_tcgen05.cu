@@ -21,6 +21,8 @@
 // that gave up has written garbage; the host checks `status` after the stream has been synchronised.
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "gated.cuh"
 
@@ -31,7 +33,7 @@ constexpr int TC_BK = 64;                 // 64 bf16 = 128 bytes = one swizzle a
 constexpr int TC_THREADS = 192;           // warp 0: TMA, warp 1: MMA + TMEM, warps 2..5: epilogue
 constexpr unsigned kSpinLimit = 2u * 1000u * 1000u;
 
-enum { EPI_STORE = 0, EPI_SWIGLU8 = 1, EPI_RESNORM = 2, EPI_RELU2 = 3, EPI_GATED8 = 4 };      // EPI_RELU2 (grouped form): max(z, 0)^2;
+enum { EPI_STORE = 0, EPI_SWIGLU8 = 1, EPI_RESNORM = 2, EPI_RELU2 = 3, EPI_GATED8 = 4 };      // EPI_RELU2 (grouped product): max(z, 0)^2;
                                                   // EPI_GATED8: EPI_SWIGLU8 with the activation `act`
 
 struct TcStatus { int code; int where; };
@@ -50,13 +52,6 @@ struct TcExtra {
     float * res;
     const float * norm_w;
     float * out_partial;
-    // Grouped form (single-SM kernel only; null: one weight matrix for all rows).  The rows of x are sorted by group;
-    // g_tiles holds the number of row tiles and then (group, first row) per row tile of 128 rows, g_offsets [groups + 1]
-    // the first row of every group; group e multiplies with rows [e * g_rows, (e + 1) * g_rows) of w.  A row tile
-    // reads 128 rows from its first row on and stores only those that belong to its group.
-    const int * g_tiles;
-    const int * g_offsets;
-    int g_rows;
     int act;                    // EPI_GATED8: the activation (gated.cuh), `limit` for the clamped one
     float limit;
 };
@@ -138,14 +133,7 @@ __device__ __forceinline__ void epilogue_store32(unsigned * r, OutT * __restrict
 #pragma unroll
         for (int i = 0; i < 32; i++) r[i] = __float_as_uint(__uint_as_float(r[i]) * rs);
     }
-    if (EPI == EPI_RELU2) {
-#pragma unroll
-        for (int i = 0; i < 32; i++) {
-            const float z = fmaxf(__uint_as_float(r[i]), 0.0f);
-            r[i] = __float_as_uint(z * z);
-        }
-    }
-    if (EPI == EPI_STORE || EPI == EPI_RELU2) {
+    if (EPI == EPI_STORE) {
         OutT * dst = out + (size_t) row * ldo + col0;
         if (col0 + 32 <= N && (((uintptr_t) dst) & 15) == 0) {
             if (sizeof(OutT) == 2) {
@@ -258,8 +246,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int num_kb = (K + TC_BK - 1) / TC_BK;
-    const bool grouped = ex.g_tiles != nullptr;
-    const int m_tiles = grouped ? ex.g_tiles[0] : (T + TC_BM - 1) / TC_BM, n_tiles = (N + BN - 1) / BN;
+    const int m_tiles = (T + TC_BM - 1) / TC_BM, n_tiles = (N + BN - 1) / BN;
     const int num_tiles = m_tiles * n_tiles;
 
     if (threadIdx.x == 0) {
@@ -281,9 +268,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(
         // ---- producer: the stage ring runs on across tiles -------------------------------------------
         int it = 0;
         for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-            const int mt = tile % m_tiles;
-            const int m0 = grouped ? ex.g_tiles[2 + 2 * mt] : mt * TC_BM;
-            const int n0 = (tile / m_tiles) * BN + (grouped ? ex.g_tiles[1 + 2 * mt] * ex.g_rows : 0);     // row of w
+            const int m0 = (tile % m_tiles) * TC_BM, n0 = (tile / m_tiles) * BN;
             for (int kb = 0; kb < num_kb; kb++, it++) {
                 const int s = it % STAGES;
                 const unsigned phase = (it / STAGES) & 1;
@@ -325,9 +310,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(
         for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, use++) {
             const int buf = use & 1;
             const unsigned acc_phase = (use >> 1) & 1;
-            const int mt = tile % m_tiles;
-            const int m0 = grouped ? ex.g_tiles[2 + 2 * mt] : mt * TC_BM, n0 = (tile / m_tiles) * BN;
-            const int row_end = grouped ? min(T, ex.g_offsets[ex.g_tiles[1 + 2 * mt] + 1]) : T;
+            const int m0 = (tile % m_tiles) * TC_BM, n0 = (tile / m_tiles) * BN;
             if (!mbar_wait(smem_addr(&acc_full[buf]), acc_phase)) {
                 if (lane == 0) { status->code = 3; status->where = use; }
                 failed = 1;
@@ -336,7 +319,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(
             tc_fence_after();
             const int row = m0 + q * 32 + lane;
             float rs = 1.0f;
-            if (ex.in_partial != nullptr && row < row_end) {          // this row's factor: its partial sums in a fixed order
+            if (ex.in_partial != nullptr && row < T) {          // this row's factor: its partial sums in a fixed order
                 float a = 0.0f;
                 for (int i = 0; i < ex.in_tiles; i++) a += ex.in_partial[(size_t) row * ex.in_tiles + i];
                 rs = rsqrtf(a * ex.inv_width + ex.eps);
@@ -347,7 +330,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(
                 unsigned r[32];
                 tc_ld32(tmem_base + ((unsigned) (q * 32) << 16) + (unsigned) (buf * BN + c0), r);
                 tc_wait_ld();
-                if (row < row_end) {
+                if (row < T) {
                     if constexpr (EPI == EPI_RESNORM)
                         sq += epilogue_resnorm32(r, reinterpret_cast<__nv_bfloat16 *>(out), ex.res, ex.norm_w, row, n0 + c0, N, rs);
                     else
@@ -355,7 +338,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(
                 }
             }
             if constexpr (EPI == EPI_RESNORM) {
-                if (row < row_end) ex.out_partial[(size_t) row * n_tiles + tile / m_tiles] = sq;
+                if (row < T) ex.out_partial[(size_t) row * n_tiles + tile / m_tiles] = sq;
             }
             tc_fence_before();
             __syncwarp();
@@ -364,6 +347,164 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(
     }
 done:
     // ---- common exit: everybody arrives here, also after a wait that gave up -------------------------
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    }
+}
+
+// ---- the grouped product: rows sorted by group, a weight block per group -----------------------------------
+// The weights are the M operand and the rows the N operand: a tile is 128 weight rows x all rows of a group (up to COLS), rounded
+// up to 16, so that a group of 160 rows costs 160 columns and not two row tiles of 128, and a group of two rows 16.  The
+// accumulator comes out transposed (a lane is an output feature, a column a row of x): the epilogue swaps neighbouring lanes'
+// values so that a warp stores pairs of features, 64 bytes of a row at a time.
+// Group tiles come from the plan on the device: (group, first row) each, ending where the next begins; the weight blocks of a
+// group tile are walked first, so a group's rows are read from the L2 and every weight from memory once per group tile.
+// COLS = 256: four stages of 48 KB; COLS = 64, for steps whose groups have few rows: eight of 24 KB.
+// What bounds it: the weights' bytes (64 experts of 2 x 1,408 x 2,048 and 1,408 x 2,048, 5 a token, from a flushed L2: 2,048 tokens 172 and
+// 91 us, row tiles of 128 as the M operand 192 and 91 us; 24 tokens 125 and 75 us).
+template <int COLS, int STAGES, int EPI>
+__global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_grouped_kernel(
+    const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, __nv_bfloat16 * __restrict__ out,
+    int T, int N, int K, int ldo, TcStatus * status, const int * __restrict__ tiles, const int * __restrict__ offsets, int groups,
+    int act, float limit) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char * smem = (unsigned char *) (((uintptr_t) smem_raw + 1023) & ~(uintptr_t) 1023);
+    constexpr int W_BYTES = TC_BM * TC_BK * 2, BOX_ROWS = 32, BOX_BYTES = BOX_ROWS * TC_BK * 2, STAGE_BYTES = W_BYTES + COLS * TC_BK * 2;
+    constexpr unsigned TMEM_COLS = 2 * COLS;
+    __shared__ __align__(8) unsigned long long full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
+    __shared__ unsigned tmem_base_s;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int num_kb = (K + TC_BK - 1) / TC_BK;
+    const int w_tiles = (N + TC_BM - 1) / TC_BM, g_tiles = tiles[0], num_tiles = g_tiles * w_tiles;
+    // first row and number of rows of a group tile (COLS of them at most are multiplied; the plan makes no larger ones)
+    auto rows_of = [&](int gt, int & r0) {
+        r0 = tiles[2 + 2 * gt];
+        const int end = gt + 1 < g_tiles ? tiles[2 + 2 * (gt + 1)] : offsets[groups];
+        return max(1, min(min(end, T) - r0, COLS));
+    };
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; s++) { mbar_init(smem_addr(&full_bar[s]), 1); mbar_init(smem_addr(&empty_bar[s]), 1); }
+        for (int b = 0; b < 2; b++) { mbar_init(smem_addr(&acc_full[b]), 1); mbar_init(smem_addr(&acc_empty[b]), 4); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_s)), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem_base = tmem_base_s;
+
+    if (warp == 0 && lane == 0) {
+        int it = 0;
+        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+            const int gt = tile / w_tiles;
+            int r0;
+            const int boxes = (rows_of(gt, r0) + BOX_ROWS - 1) / BOX_ROWS;
+            const int w0 = tiles[1 + 2 * gt] * N + (tile - gt * w_tiles) * TC_BM;
+            for (int kb = 0; kb < num_kb; kb++, it++) {
+                const int s = it % STAGES;
+                if (!mbar_wait(smem_addr(&empty_bar[s]), ((it / STAGES) & 1) ^ 1)) { status->code = 1; status->where = it; goto done; }
+                const unsigned bar = smem_addr(&full_bar[s]), to = smem_addr(smem + s * STAGE_BYTES);
+                mbar_expect_tx(bar, W_BYTES + boxes * BOX_BYTES);
+                tma_load_2d(to, &map_w, kb * TC_BK, w0, bar);
+                for (int b = 0; b < boxes; b++) tma_load_2d(to + W_BYTES + b * BOX_BYTES, &map_x, kb * TC_BK, r0 + b * BOX_ROWS, bar);
+            }
+        }
+    } else if (warp == 1 && lane == 0) {
+        int it = 0, use = 0;
+        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, use++) {
+            const int buf = use & 1;
+            int r0;
+            const unsigned idesc = instr_desc_bf16(TC_BM, (rows_of(tile / w_tiles, r0) + 15) & ~15);
+            if (!mbar_wait(smem_addr(&acc_empty[buf]), ((use >> 1) & 1) ^ 1)) { status->code = 4; status->where = use; goto done; }
+            tc_fence_after();
+            const unsigned d_tmem = tmem_base + (unsigned) (buf * COLS);
+            for (int kb = 0; kb < num_kb; kb++, it++) {
+                const int s = it % STAGES;
+                if (!mbar_wait(smem_addr(&full_bar[s]), (it / STAGES) & 1)) { status->code = 2; status->where = it; goto done; }
+                tc_fence_after();
+                const unsigned long long dw = smem_desc_sw128(smem_addr(smem + s * STAGE_BYTES));
+                const unsigned long long dx = smem_desc_sw128(smem_addr(smem + s * STAGE_BYTES + W_BYTES));
+#pragma unroll
+                for (int k = 0; k < TC_BK / 16; k++)
+                    tc_mma(d_tmem, dw + (unsigned long long) (k * 2), dx + (unsigned long long) (k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                tc_commit(smem_addr(&empty_bar[s]));
+            }
+            tc_commit(smem_addr(&acc_full[buf]));
+        }
+    } else if (warp >= 2) {
+        const int q = warp & 3;
+        const bool pairs = ldo % 2 == 0 && ((uintptr_t) out & 3) == 0;
+        auto put = [&](int c, int feature, __nv_bfloat162 v, int r0, bool both) {
+            __nv_bfloat16 * to = out + (size_t) (r0 + c) * ldo + feature;
+            if (pairs) *reinterpret_cast<__nv_bfloat162 *>(to) = v;
+            else {
+                to[0] = v.x;
+                if (both) to[1] = v.y;
+            }
+        };
+        int use = 0;
+        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, use++) {
+            const int buf = use & 1, gt = tile / w_tiles;
+            int r0;
+            const int rows = rows_of(gt, r0), f0 = (tile - gt * w_tiles) * TC_BM + q * 32;      // this warp's weight rows
+            if (!mbar_wait(smem_addr(&acc_full[buf]), (use >> 1) & 1)) {
+                if (lane == 0) { status->code = 3; status->where = use; }
+                break;
+            }
+            tc_fence_after();
+#pragma unroll 1
+            for (int c0 = 0; c0 < rows; c0 += 32) {
+                unsigned r[32];
+                tc_ld32(tmem_base + ((unsigned) (q * 32) << 16) + (unsigned) (buf * COLS + c0), r);
+                tc_wait_ld();
+                if constexpr (EPI == EPI_SWIGLU8 || EPI == EPI_GATED8) {
+                    // lanes 0..7 and 16..23 hold gates, the eight after each the ups of the same features.  A gate lane works on rows c0 + 4 i
+                    // and c0 + 4 i + 2, its up lane on the rows behind them; then lanes swap so that each has two features of one row.
+                    const bool up = lane & 8, odd = lane & 1;
+                    const int feature = f0 / 2 + (lane >> 4) * 8 + (lane & 6);
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4) {
+                        float a[2];
+#pragma unroll
+                        for (int p = 0; p < 2; p++) {
+                            const float even_row = __uint_as_float(r[i + 2 * p]), odd_row = __uint_as_float(r[i + 2 * p + 1]);
+                            const float got = __shfl_xor_sync(0xffffffffu, up ? even_row : odd_row, 8);
+                            const float g = up ? got : even_row, u = up ? odd_row : got;
+                            a[p] = EPI == EPI_GATED8 ? gated_value_fast(g, u, act, limit) : g / (1.0f + __expf(-g)) * u;
+                        }
+                        const float got = __shfl_xor_sync(0xffffffffu, odd ? a[0] : a[1], 1);
+                        const __nv_bfloat162 v = odd ? __floats2bfloat162_rn(got, a[1]) : __floats2bfloat162_rn(a[0], got);
+                        const int c = c0 + i + (up ? 1 : 0) + (odd ? 2 : 0);
+                        if (c < rows && 2 * feature < N) put(c, feature, v, r0, true);
+                    }
+                } else {
+                    const bool odd = lane & 1;
+                    const int feature = f0 + (lane & 30);
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2) {
+                        float x = __uint_as_float(r[i]), y = __uint_as_float(r[i + 1]);
+                        if (EPI == EPI_RELU2) { x = fmaxf(x, 0.0f); x *= x; y = fmaxf(y, 0.0f); y *= y; }
+                        const float got = __shfl_xor_sync(0xffffffffu, odd ? x : y, 1);
+                        const __nv_bfloat162 v = odd ? __floats2bfloat162_rn(got, y) : __floats2bfloat162_rn(x, got);
+                        const int c = c0 + i + (odd ? 1 : 0);
+                        if (c < rows && feature < N) put(c, feature, v, r0, feature + 1 < N);
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_addr(&acc_empty[buf]));
+        }
+    }
+done:
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
@@ -584,7 +725,7 @@ static int make_map(CUtensorMap * map, const void * base, int rows, int K, int b
 
 template <int BN, int STAGES, int EPI, typename OutT>
 static int launch_tc(const CUtensorMap & ma, const CUtensorMap & mb, void * out, int T, int N, int K, int ldo, TcStatus * status,
-                     const TcExtra & ex, cudaStream_t stream, int row_tile_bound = 0) {
+                     const TcExtra & ex, cudaStream_t stream) {
     constexpr size_t smem = (size_t) STAGES * (TC_BM * TC_BK * 2 + BN * TC_BK * 2) + 1024;
     static bool configured = false;
     if (!configured) {
@@ -592,8 +733,7 @@ static int launch_tc(const CUtensorMap & ma, const CUtensorMap & mb, void * out,
         if (e != cudaSuccess) return 1000 + (int) e;
         configured = true;
     }
-    // the grouped form learns its number of row tiles on the device; the grid is sized by the caller's bound
-    const int tiles = (row_tile_bound > 0 ? row_tile_bound : (T + TC_BM - 1) / TC_BM) * ((N + BN - 1) / BN);
+    const int tiles = ((T + TC_BM - 1) / TC_BM) * ((N + BN - 1) / BN);
     static int sms = 0;
     if (sms == 0) {
         int dev = 0;
@@ -601,6 +741,26 @@ static int launch_tc(const CUtensorMap & ma, const CUtensorMap & mb, void * out,
     }
     dim3 grid(tiles < sms ? tiles : sms);
     gemm_tcgen05_kernel<BN, STAGES, EPI, OutT><<<grid, TC_THREADS, smem, stream>>>(ma, mb, (OutT *) out, T, N, K, ldo, status, ex);
+    return iian_launch_status();
+}
+
+template <int COLS, int STAGES, int EPI>
+static int launch_grouped(const CUtensorMap & mw, const CUtensorMap & mx, void * out, int T, int N, int K, int ldo, TcStatus * status,
+                          const int * tiles, const int * offsets, int groups, int act, float limit, int max_tiles, cudaStream_t stream) {
+    constexpr size_t smem = (size_t) STAGES * (TC_BM + COLS) * TC_BK * 2 + 1024;
+    auto kernel = gemm_tcgen05_grouped_kernel<COLS, STAGES, EPI>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    if (e != cudaSuccess) return 1000 + (int) e;
+    static int sms = 0;
+    if (sms == 0) {
+        int dev = 0, n = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        sms = n;
+    }
+    // how many group tiles there are is known on the device alone: the grid is sized by the caller's bound
+    const long long bound = (long long) max_tiles * ((N + TC_BM - 1) / TC_BM);
+    kernel<<<(unsigned) (bound < sms ? bound : sms), TC_THREADS, smem, stream>>>(mw, mx, (__nv_bfloat16 *) out, T, N, K, ldo, status, tiles,
+                                                                                  offsets, groups, act, limit);
     return iian_launch_status();
 }
 
@@ -699,10 +859,11 @@ static int tc_entry(const void * x, const void * w, void * out, int out_dtype, i
 }
 
 // The grouped product: x [T, K] bf16 with its rows sorted by group, w [groups * N, K] bf16 (group e's matrix in rows
-// e * N ..), out [T, N] or, with epilogue 1 or 4 (act and limit as in gated.cuh), [T, N / 2] (epilogue 3: max(z, 0)^2 of every entry); tiles = {row tiles, then (group, first row) per row tile of 128
-// rows}, offsets [groups + 1], both on the device; max_tiles bounds the row tiles (it sizes the grid).  bn: 128 or 256.
+// e * N ..), out [T, N] or, with epilogue 1 or 4 (act and limit as in gated.cuh), [T, N / 2] (epilogue 3: max(z, 0)^2 of every entry);
+// tiles = {group tiles, then (group, first row) per tile}, each ending where the next begins, offsets [groups + 1], both on the
+// device; max_tiles bounds the group tiles (it sizes the grid).  cols: 64 or 256, the most rows a tile of the plan has.
 IIAN_API int iian_gemm_tcgen05_grouped(const void * x, const void * w, void * out, int out_dtype, int T, int N, int groups, int K,
-                                       int epilogue, int act, float limit, int bn, int * status, const int * tiles, const int * offsets,
+                                       int epilogue, int act, float limit, int cols, int * status, const int * tiles, const int * offsets,
                                        int max_tiles, cudaStream_t stream) {
     if (T <= 0 || N <= 0 || groups <= 0 || max_tiles <= 0) return IIAN_OK;
     if (K <= 0 || K % 8 != 0 || tiles == nullptr || offsets == nullptr || status == nullptr) return IIAN_ERR_SHAPE;
@@ -711,28 +872,24 @@ IIAN_API int iian_gemm_tcgen05_grouped(const void * x, const void * w, void * ou
     if (!gated && epilogue != EPI_STORE && epilogue != EPI_RELU2) return IIAN_ERR_SHAPE;
     if (epilogue == EPI_GATED8 && act != ACT_SILU && act != ACT_CLAMPED && act != ACT_RELU) return IIAN_ERR_SHAPE;
     if (gated && N % 16 != 0) return IIAN_ERR_SHAPE;
-    if (bn != 128 && bn != 256) return IIAN_ERR_SHAPE;
+    if (cols != 64 && cols != 256) return IIAN_ERR_SHAPE;
     if (out_dtype != IIAN_BF16) return IIAN_ERR_DTYPE;
-    if ((long long) groups * N > 2147483647LL) return IIAN_ERR_LIMIT;
-    CUtensorMap ma, mb;
-    int rc = make_map(&ma, x, T, K, TC_BM);
+    if ((long long) groups * N > 2147483647LL || (long long) max_tiles * ((N + TC_BM - 1) / TC_BM) > 2147483647LL) return IIAN_ERR_LIMIT;
+    CUtensorMap mw, mx;
+    int rc = make_map(&mw, w, groups * N, K, TC_BM);
     if (rc != IIAN_OK) return rc;
-    rc = make_map(&mb, w, groups * N, K, bn);
+    rc = make_map(&mx, x, T, K, 32);
     if (rc != IIAN_OK) return rc;
     TcStatus * st = (TcStatus *) status;
     const int ldo = gated ? N / 2 : N;
-    const TcExtra ex = {nullptr, 0, 0.0f, 0.0f, nullptr, nullptr, nullptr, tiles, offsets, N, act, limit};
-    if (epilogue == EPI_GATED8)
-        return bn == 256 ? launch_tc<256, 4, EPI_GATED8, __nv_bfloat16>(ma, mb, out, T, N, K, ldo, st, ex, stream, max_tiles)
-                         : launch_tc<128, 6, EPI_GATED8, __nv_bfloat16>(ma, mb, out, T, N, K, ldo, st, ex, stream, max_tiles);
-    if (epilogue == EPI_RELU2)
-        return bn == 256 ? launch_tc<256, 4, EPI_RELU2, __nv_bfloat16>(ma, mb, out, T, N, K, ldo, st, ex, stream, max_tiles)
-                         : launch_tc<128, 6, EPI_RELU2, __nv_bfloat16>(ma, mb, out, T, N, K, ldo, st, ex, stream, max_tiles);
-    if (bn == 256)
-        return epilogue == EPI_STORE ? launch_tc<256, 4, EPI_STORE, __nv_bfloat16>(ma, mb, out, T, N, K, ldo, st, ex, stream, max_tiles)
-                                     : launch_tc<256, 4, EPI_SWIGLU8, __nv_bfloat16>(ma, mb, out, T, N, K, ldo, st, ex, stream, max_tiles);
-    return epilogue == EPI_STORE ? launch_tc<128, 6, EPI_STORE, __nv_bfloat16>(ma, mb, out, T, N, K, ldo, st, ex, stream, max_tiles)
-                                 : launch_tc<128, 6, EPI_SWIGLU8, __nv_bfloat16>(ma, mb, out, T, N, K, ldo, st, ex, stream, max_tiles);
+    auto go = [&](auto epi) {
+        constexpr int E = decltype(epi)::value;
+        return cols == 64 ? launch_grouped<64, 8, E>(mw, mx, out, T, N, K, ldo, st, tiles, offsets, groups, act, limit, max_tiles, stream)
+                          : launch_grouped<256, 4, E>(mw, mx, out, T, N, K, ldo, st, tiles, offsets, groups, act, limit, max_tiles, stream);
+    };
+    if (epilogue == EPI_GATED8) return go(std::integral_constant<int, EPI_GATED8>());
+    if (epilogue == EPI_RELU2) return go(std::integral_constant<int, EPI_RELU2>());
+    return epilogue == EPI_STORE ? go(std::integral_constant<int, EPI_STORE>()) : go(std::integral_constant<int, EPI_SWIGLU8>());
 }
 
 // x: [T, K] bf16, w: [N, K] bf16; out: [T, N] (epilogue 0) or [T, N / 2] (epilogue 1: SiLU(gate) * up over

@@ -1139,9 +1139,14 @@ class CudaKernels:
         """Upper bound of the row tiles of a grouped product over ``n_rows`` rows sorted by expert."""
         return -(-n_rows // (tile_rows or self.moe_tile_rows())) + num_experts
 
-    # grouped products on tcgen05 (csrc/gemm_tcgen05.cu, row tiles of 128); IIAN_MOE_TCGEN05=0: the general kernel
+    # grouped products on tcgen05 (csrc/gemm_tcgen05.cu); IIAN_MOE_TCGEN05=0: the general kernel
     MOE_TCGEN05 = os.environ.get("IIAN_MOE_TCGEN05", "1") not in ("0", "false", "off")
-    MOE_TC_TILE_ROWS = 128
+
+    @staticmethod
+    def moe_tc_tile_rows(n_rows: int, num_experts: int) -> int:
+        """The most rows of a plan's tile for the tcgen05 product: 64, whose stages are smaller and more, where an expert gets 32
+        rows or fewer on average (the product is bound by the weights' bytes), else 256 (by the tensor pipe)."""
+        return 64 if n_rows <= 32 * num_experts else 256
 
     def moe_tcgen05_ok(self, dtype: torch.dtype, hidden: int, inter: int, activation: str) -> bool:
         """Whether both grouped products of an expert feed-forward can run on the tcgen05 kernel: bfloat16, rows of 16
@@ -1150,16 +1155,17 @@ class CudaKernels:
                 and activation in ("silu", "clamped_swish", "relu", "relu2") and hidden % 8 == 0 and inter % 8 == 0)
 
     def moe_grouped_gemm_tc(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, offsets: torch.Tensor, tiles: torch.Tensor,
-                            gated: bool, relu2: bool = False, activation: str = "silu", limit: float = 0.0) -> None:
+                            gated: bool, relu2: bool = False, activation: str = "silu", limit: float = 0.0, tile_rows: int = 128) -> None:
         """Rows of ``x`` sorted by expert times that expert's block of ``w`` [E, n, K] on tcgen05; ``gated``: the block's
         rows are gate and up interleaved in groups of 8 and ``out`` [M, n / 2] = act(gate, up) (``activation`` as in ``gated_act``);
-        ``relu2`` (not gated): ``out`` = max(product, 0)^2.  The plan's row tiles are of 128 rows."""
+        ``relu2`` (not gated): ``out`` = max(product, 0)^2.  The plan's tiles have ``tile_rows`` rows at most (256 or fewer)."""
         m, k = x.shape
         e, n = w.shape[0], w.shape[1]
         if w.shape[2] != k or out.shape != (m, n // 2 if gated else n) or x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 \
                 or out.dtype != torch.bfloat16:
             raise KernelError(f"moe_grouped_gemm_tc: x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)} do not fit")
-        bn = 256 if n % 256 == 0 or n > 2048 else 128
+        if tile_rows > 256:
+            raise KernelError("moe_grouped_gemm_tc: the plan's tiles may have 256 rows")
         status = self.tcgen05_status_buffer(x.device).data_ptr()
         CudaKernels._tc_used = True
         fn = _fn("gemm_tcgen05", "iian_gemm_tcgen05_grouped",
@@ -1167,7 +1173,7 @@ class CudaKernels:
                   c_void_p, c_int, c_void_p])
         epilogue = (1 if activation == "silu" else 4) if gated else 3 if relu2 else 0
         _check(fn(_cuda(x, "moe rows"), _cuda(w, "expert weights"), _cuda(out, "moe out"), BF16, m, n, e, k, epilogue,
-                  self.ACTIVATIONS[activation], limit, bn, status, _cuda(tiles, "tiles", torch.int32), _cuda(offsets, "offsets", torch.int32), (tiles.numel() - 1) // 2,
+                  self.ACTIVATIONS[activation], limit, 64 if tile_rows <= 64 else 256, status, _cuda(tiles, "tiles", torch.int32), _cuda(offsets, "offsets", torch.int32), (tiles.numel() - 1) // 2,
                   _stream()), "gemm_tcgen05_grouped")
 
     def moe_route(self, logits: torch.Tensor, top: int, ids: torch.Tensor, weights: torch.Tensor) -> None:

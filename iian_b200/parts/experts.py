@@ -194,7 +194,7 @@ class RoutedExperts(FeedForward):
         on_input = self.weight_on == "input"
         on_tc = ((self.w_gate_up is not None or self.activation == "relu2") and hasattr(k, "moe_tcgen05_ok")
                  and k.moe_tcgen05_ok(self.dtype, self.hidden, self.inter, self.activation))
-        tile_rows = k.MOE_TC_TILE_ROWS if on_tc else k.moe_tile_rows()
+        tile_rows = k.moe_tc_tile_rows(m, E) if on_tc else k.moe_tile_rows()
         max_tiles = k.moe_max_tiles(m, E, tile_rows)
         offsets = ctx.buf("expert_offsets", (E + 1,), torch.int32)
         pos = ctx.buf("expert_pos", (m,), torch.int32)
@@ -206,14 +206,15 @@ class RoutedExperts(FeedForward):
         ys = ctx.buf("expert_out", (m, self.hidden), self.dtype)
         if self.activation == "relu2":
             if on_tc:
-                k.moe_grouped_gemm_tc(xs, self.w_up, act, offsets, tiles, gated=False, relu2=True)
-                k.moe_grouped_gemm_tc(act, self.w_down, ys, offsets, tiles, gated=False)
+                k.moe_grouped_gemm_tc(xs, self.w_up, act, offsets, tiles, gated=False, relu2=True, tile_rows=tile_rows)
+                k.moe_grouped_gemm_tc(act, self.w_down, ys, offsets, tiles, gated=False, tile_rows=tile_rows)
             else:
                 k.moe_grouped_gemm(xs, self.w_up, None, act, offsets, tiles, "relu2")
                 k.moe_grouped_gemm(act, self.w_down, None, ys, offsets, tiles)
         elif on_tc:
-            k.moe_grouped_gemm_tc(xs, self.w_gate_up, act, offsets, tiles, gated=True, activation=self.activation, limit=self.limit)
-            k.moe_grouped_gemm_tc(act, self.w_down, ys, offsets, tiles, gated=False)
+            k.moe_grouped_gemm_tc(xs, self.w_gate_up, act, offsets, tiles, gated=True, activation=self.activation, limit=self.limit,
+                                  tile_rows=tile_rows)
+            k.moe_grouped_gemm_tc(act, self.w_down, ys, offsets, tiles, gated=False, tile_rows=tile_rows)
         else:
             if self.w_gate_up is not None:
                 k.moe_grouped_gemm(xs, self.w_gate_up, self.w_gate_up, act, offsets, tiles, self.activation, self.limit)

@@ -88,3 +88,32 @@ def test_a_kernel_that_gave_up_is_reported_at_the_next_host_wait():
     with pytest.raises(KernelError, match="gave up"):
         k.check_device_status()
     assert k.tcgen05_status_buffer(x.device).tolist() == [0, 0]
+
+
+@pytest.mark.parametrize("tile_rows", [64, 128, 256])
+@pytest.mark.parametrize("counts", [[1], [5, 0, 3], [16, 17, 1, 0, 31, 33], [64, 65, 100, 2], [255, 256, 257, 1, 0, 500]])
+@pytest.mark.parametrize("n,k", [(16, 8), (96, 72), (272, 200), (129, 64)])
+def test_grouped_rows(n, k, counts, tile_rows):
+    """Groups around the tiles' edges (16 columns of a product, 32 rows of a copy, 64 and 256 rows of a tile), weight blocks that are
+    no multiple of 128 rows; plain and gated."""
+    from iian_b200.ops.cuda_backend import CudaKernels
+    K = CudaKernels()
+    g = torch.Generator("cuda").manual_seed(n * k + len(counts))
+    E, m = len(counts), sum(counts)
+    x = torch.randn(m, k, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(E, n, k, device="cuda", generator=g) * k ** -0.5).bfloat16()
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(counts)).int().cuda()
+    offsets, pos = torch.empty(E + 1, dtype=torch.int32, device="cuda"), torch.empty(m, dtype=torch.int32, device="cuda")
+    tiles = torch.empty(1 + 2 * K.moe_max_tiles(m, E, tile_rows), dtype=torch.int32, device="cuda")
+    K.moe_plan(ids, E, offsets, pos, tiles, tile_rows)
+    want = torch.cat([x[a:b].double() @ w[e].double().T for e, (a, b) in enumerate(zip(offsets.tolist(), offsets.tolist()[1:]))])
+    for gated in ([False, True] if n % 16 == 0 else [False]):
+        out = torch.full((m, n // 2 if gated else n), float("nan"), device="cuda", dtype=torch.bfloat16)
+        K.moe_grouped_gemm_tc(x, w, out, offsets, tiles, gated=gated, tile_rows=tile_rows)
+        K.tcgen05_check(x.device)
+        ref = want
+        if gated:
+            pair = want.view(m, n // 16, 2, 8)
+            ref = (torch.nn.functional.silu(pair[:, :, 0]) * pair[:, :, 1]).reshape(m, n // 2)
+        # one rounding to bfloat16 (2^-9 of the value) and 32-bit sums
+        assert ((out.double() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-4).all()
