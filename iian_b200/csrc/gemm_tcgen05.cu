@@ -362,23 +362,25 @@ done:
 // values so that a warp stores pairs of features, 64 bytes of a row at a time.
 // Group tiles come from the plan on the device: (group, first row) each, ending where the next begins; the weight blocks of a
 // group tile are walked first, so a group's rows are read from the L2 and every weight from memory once per group tile.
-// COLS = 256: four stages of 48 KB; COLS = 64, for steps whose groups have few rows: eight of 24 KB.
+// COLS = 256: four stages of 48 KB; COLS = 64, for steps whose groups have few rows: four of 48 KB that hold two K blocks, so that 256
+// bytes of a weight row are asked for together (24 tokens 123 -> 118 us against eight stages of one block; rings of their own for
+// weights and rows: 141 us, the issuing thread then waits and commits twice per block).
 // What bounds it: the weights' bytes (64 experts of 2 x 1,408 x 2,048 and 1,408 x 2,048, 5 a token, from a flushed L2: 2,048 tokens 172 and
-// 91 us, row tiles of 128 as the M operand 192 and 91 us; 24 tokens 125 and 75 us).
-template <int COLS, int STAGES, int EPI>
+// 92 us, row tiles of 128 as the M operand 192 and 91 us; 24 tokens 118 and 68 us).
+template <int COLS, int STAGES, int KPS, int EPI>
 __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_grouped_kernel(
     const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, __nv_bfloat16 * __restrict__ out,
     int T, int N, int K, int ldo, TcStatus * status, const int * __restrict__ tiles, const int * __restrict__ offsets, int groups,
     int act, float limit) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char * smem = (unsigned char *) (((uintptr_t) smem_raw + 1023) & ~(uintptr_t) 1023);
-    constexpr int W_BYTES = TC_BM * TC_BK * 2, BOX_ROWS = 32, BOX_BYTES = BOX_ROWS * TC_BK * 2, STAGE_BYTES = W_BYTES + COLS * TC_BK * 2;
+    constexpr int W_BYTES = TC_BM * TC_BK * 2, BOX_ROWS = 32, BOX_BYTES = BOX_ROWS * TC_BK * 2, X_BYTES = COLS * TC_BK * 2, STAGE_BYTES = KPS * (W_BYTES + X_BYTES);
     constexpr unsigned TMEM_COLS = 2 * COLS;
     __shared__ __align__(8) unsigned long long full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
     __shared__ unsigned tmem_base_s;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int num_kb = (K + TC_BK - 1) / TC_BK;
+    const int num_kb = ((K + TC_BK - 1) / TC_BK + KPS - 1) / KPS;        // (blocks past the end of K are filled with zeros)
     const int w_tiles = (N + TC_BM - 1) / TC_BM, g_tiles = tiles[0], num_tiles = g_tiles * w_tiles;
     // first row and number of rows of a group tile (COLS of them at most are multiplied; the plan makes no larger ones)
     auto rows_of = [&](int gt, int & r0) {
@@ -412,9 +414,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_grouped_kernel(
                 const int s = it % STAGES;
                 if (!mbar_wait(smem_addr(&empty_bar[s]), ((it / STAGES) & 1) ^ 1)) { status->code = 1; status->where = it; goto done; }
                 const unsigned bar = smem_addr(&full_bar[s]), to = smem_addr(smem + s * STAGE_BYTES);
-                mbar_expect_tx(bar, W_BYTES + boxes * BOX_BYTES);
-                tma_load_2d(to, &map_w, kb * TC_BK, w0, bar);
-                for (int b = 0; b < boxes; b++) tma_load_2d(to + W_BYTES + b * BOX_BYTES, &map_x, kb * TC_BK, r0 + b * BOX_ROWS, bar);
+                mbar_expect_tx(bar, KPS * (W_BYTES + boxes * BOX_BYTES));
+#pragma unroll
+                for (int j = 0; j < KPS; j++) tma_load_2d(to + j * W_BYTES, &map_w, (kb * KPS + j) * TC_BK, w0, bar);
+                for (int b = 0; b < boxes; b++)
+#pragma unroll
+                    for (int j = 0; j < KPS; j++)
+                        tma_load_2d(to + KPS * W_BYTES + j * X_BYTES + b * BOX_BYTES, &map_x, (kb * KPS + j) * TC_BK, r0 + b * BOX_ROWS, bar);
             }
         }
     } else if (warp == 1 && lane == 0) {
@@ -430,11 +436,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_grouped_kernel(
                 const int s = it % STAGES;
                 if (!mbar_wait(smem_addr(&full_bar[s]), (it / STAGES) & 1)) { status->code = 2; status->where = it; goto done; }
                 tc_fence_after();
-                const unsigned long long dw = smem_desc_sw128(smem_addr(smem + s * STAGE_BYTES));
-                const unsigned long long dx = smem_desc_sw128(smem_addr(smem + s * STAGE_BYTES + W_BYTES));
 #pragma unroll
-                for (int k = 0; k < TC_BK / 16; k++)
-                    tc_mma(d_tmem, dw + (unsigned long long) (k * 2), dx + (unsigned long long) (k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                for (int j = 0; j < KPS; j++) {
+                    const unsigned long long dw = smem_desc_sw128(smem_addr(smem + s * STAGE_BYTES + j * W_BYTES));
+                    const unsigned long long dx = smem_desc_sw128(smem_addr(smem + s * STAGE_BYTES + KPS * W_BYTES + j * X_BYTES));
+#pragma unroll
+                    for (int k = 0; k < TC_BK / 16; k++)
+                        tc_mma(d_tmem, dw + (unsigned long long) (k * 2), dx + (unsigned long long) (k * 2), idesc, (kb > 0 || j > 0 || k > 0) ? 1u : 0u);
+                }
                 tc_commit(smem_addr(&empty_bar[s]));
             }
             tc_commit(smem_addr(&acc_full[buf]));
@@ -744,11 +753,11 @@ static int launch_tc(const CUtensorMap & ma, const CUtensorMap & mb, void * out,
     return iian_launch_status();
 }
 
-template <int COLS, int STAGES, int EPI>
+template <int COLS, int STAGES, int KPS, int EPI>
 static int launch_grouped(const CUtensorMap & mw, const CUtensorMap & mx, void * out, int T, int N, int K, int ldo, TcStatus * status,
                           const int * tiles, const int * offsets, int groups, int act, float limit, int max_tiles, cudaStream_t stream) {
-    constexpr size_t smem = (size_t) STAGES * (TC_BM + COLS) * TC_BK * 2 + 1024;
-    auto kernel = gemm_tcgen05_grouped_kernel<COLS, STAGES, EPI>;
+    constexpr size_t smem = (size_t) STAGES * KPS * (TC_BM + COLS) * TC_BK * 2 + 1024;
+    auto kernel = gemm_tcgen05_grouped_kernel<COLS, STAGES, KPS, EPI>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
     if (e != cudaSuccess) return 1000 + (int) e;
     static int sms = 0;
@@ -884,8 +893,8 @@ IIAN_API int iian_gemm_tcgen05_grouped(const void * x, const void * w, void * ou
     const int ldo = gated ? N / 2 : N;
     auto go = [&](auto epi) {
         constexpr int E = decltype(epi)::value;
-        return cols == 64 ? launch_grouped<64, 8, E>(mw, mx, out, T, N, K, ldo, st, tiles, offsets, groups, act, limit, max_tiles, stream)
-                          : launch_grouped<256, 4, E>(mw, mx, out, T, N, K, ldo, st, tiles, offsets, groups, act, limit, max_tiles, stream);
+        return cols == 64 ? launch_grouped<64, 4, 2, E>(mw, mx, out, T, N, K, ldo, st, tiles, offsets, groups, act, limit, max_tiles, stream)
+                          : launch_grouped<256, 4, 1, E>(mw, mx, out, T, N, K, ldo, st, tiles, offsets, groups, act, limit, max_tiles, stream);
     };
     if (epilogue == EPI_GATED8) return go(std::integral_constant<int, EPI_GATED8>());
     if (epilogue == EPI_RELU2) return go(std::integral_constant<int, EPI_RELU2>());
