@@ -47,6 +47,7 @@ struct AttnParams {
     const int * slots;              // [N] cache cell of each token (page * page_size + offset), < 0: not stored
     float eps;
     int write_kv;
+    int longest_first = 0;          // decode kernel, unsplit keys: the CTAs take the sequences in falling order of their contexts
     int * status;                   // TMA form of the decode kernel: {code, where}, zero before the launch
     // a sink per head: a logit without key and value that joins the softmax's denominator once, not scaled
     const float * sink = nullptr;   // [nh] or null
@@ -441,7 +442,25 @@ __global__ void __launch_bounds__(128, STAGES == 2 ? 3 : 2) attention_decode_ker
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g_ = lane >> 2, t_ = lane & 3;
     const int kvh = blockIdx.y;
-    const int s = blockIdx.z / p.n_split, split = blockIdx.z % p.n_split;
+    const int split = blockIdx.z % p.n_split;
+    int s = blockIdx.z / p.n_split;
+    if (p.longest_first) {
+        // the sequences in falling order of their contexts (ties in their own order)
+        __shared__ int ranked;
+        const int S = gridDim.z;
+        for (int t = threadIdx.x; t < S; t += blockDim.x) {
+            const int own = p.ctx_len[t];
+            int rank = 0;
+#pragma unroll 8
+            for (int u = 0; u < S; u++) {
+                const int other = __ldg(p.ctx_len + u);
+                rank += other > own || (other == own && u < t);
+            }
+            if (rank == s) ranked = t;
+        }
+        __syncthreads();
+        s = ranked;
+    }
     const int G = p.nh / p.nkv;
     const int q0 = p.cu_q[s];
     const int q_len = p.cu_q[s + 1] - q0;
@@ -1008,7 +1027,8 @@ static int launch_decode_st(const AttnParams & p, const KvMaps & maps, int S, in
 static int g_decode_stages = 2;
 static int g_unsplit_stages = 0;        // 0: the rule below; 2 or 3: that many for unsplit keys
 template <int HD, bool CLUSTER, bool FUSED = false, bool KEPT = false>
-static int launch_decode(const AttnParams & p, int S, int max_rows, cudaStream_t stream) {
+static int launch_decode(const AttnParams & asked, int S, int max_rows, cudaStream_t stream) {
+    AttnParams p = asked;
     // unsplit keys mean many sequences, each CTA walking a whole context: the deeper pipeline pays there
     bool deep = g_decode_stages == 3;
     if (p.n_split == 1) {
@@ -1020,6 +1040,9 @@ static int launch_decode(const AttnParams & p, int S, int max_rows, cudaStream_t
         const long long ctas = (long long) ((max_rows + 15) / 16) * p.nkv * S;
         const long long waves3 = (ctas + 2 * sms - 1) / (2 * sms), waves2 = (ctas + 3 * sms - 1) / (3 * sms);
         deep = g_unsplit_stages != 0 ? g_unsplit_stages == 3 : waves3 * 100 <= waves2 * 115;
+        // With more CTAs than are resident at once those of the long contexts go first; the ranking costs a CTA about half a
+        // microsecond, so a single wave keeps the order of the batch, and so does a batch too large to be ranked in passing.
+        p.longest_first = ctas > (deep ? 2 : 3) * sms && S <= 256;
     }
     KvMaps maps = {};
     if constexpr (HD == 128) {
