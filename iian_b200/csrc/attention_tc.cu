@@ -58,7 +58,7 @@ struct TcAttnParams {
     const int * cu_q;               // [S + 1]
     const int * ctx_len;            // [S]
     const int * block_table;        // [S, max_blocks]
-    int max_blocks, nh, nkv, page_size, num_pages, window;
+    int max_blocks, nh, nkv, page_size, num_pages, window, num_seqs;
     float scale_log2;               // scale * log2(e)
     int * status;                   // {code, where}; zero before the launch
     // a sink per head: a logit without key and value that joins the softmax's denominator once, not scaled
@@ -257,6 +257,83 @@ template <int N> __device__ __forceinline__ void at_capped_row(unsigned * v, con
     }
 }
 
+// Which request and row tile the `unit`-th CTA of a KV head works on: the row tiles of all requests in falling order of the keys they
+// see, so that the longest walks start first and the short ones fill the gaps at the end (in the order of the grid the longest tiles of
+// the last request or head began when the GPU was already running empty).  A row tile of `rows` rows sees ceil((pos0 + last token + 1)
+// / AT_BN) key tiles, which grows with its number; the number of row tiles of a request that see L key tiles or more is a closed
+// form, and a warp finds the L of the unit by bisection over L with its lanes over the requests.  Every warp asks for itself.
+__device__ __forceinline__ bool at_row_tile(const TcAttnParams & p, int G, int rows, int unit, int & s, int & tile) {
+    if (p.num_seqs == 1) {
+        s = 0;
+        tile = ((p.cu_q[1] - p.cu_q[0]) * G + rows - 1) / rows - 1 - unit;
+        return tile >= 0;
+    }
+    const int lane = threadIdx.x & 31;
+    auto request = [&](int i, int & q_len, int & pos0) {
+        q_len = p.cu_q[i + 1] - p.cu_q[i];
+        pos0 = p.ctx_len[i] - q_len;
+    };
+    auto tiles_from = [&](int q_len, int pos0, int L) {      // row tiles of a request that see L key tiles or more
+        const int n = (q_len * G + rows - 1) / rows, x = (L - 1) * AT_BN - pos0;
+        if (x <= 0) return n;
+        if (x > q_len - 1) return 0;
+        return n - min((x * G + rows) / rows - 1, n - 1);    // the first of them holds row x * G
+    };
+    int q_len0 = 0, pos00 = 0, most = 0;                     // the lane's first request, kept
+    if (lane < p.num_seqs) request(lane, q_len0, pos00);
+    for (int i = lane; i < p.num_seqs; i += 32) {
+        int q_len = q_len0, pos0 = pos00;
+        if (i >= 32) request(i, q_len, pos0);
+        most = max(most, q_len > 0 ? pos0 + q_len : 0);
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    auto count = [&](int L) {
+        int c = 0;
+        for (int i = lane; i < p.num_seqs; i += 32) {
+            int q_len = q_len0, pos0 = pos00;
+            if (i >= 32) request(i, q_len, pos0);
+            c += tiles_from(q_len, pos0, L);
+        }
+        return __reduce_add_sync(0xffffffffu, c);
+    };
+    if (count(1) <= unit) return false;
+    int lo = 1, hi = (most + AT_BN - 1) / AT_BN + 1, above = 0;        // count(lo) > unit >= count(hi) = above
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1, c = count(mid);
+        if (c > unit) lo = mid;
+        else { hi = mid; above = c; }
+    }
+    int rest = unit - above;                                 // among the row tiles that see exactly lo key tiles, request by request
+    for (int base = 0; base < p.num_seqs; base += 32) {
+        const int i = base + lane;
+        int q_len = q_len0, pos0 = pos00;
+        if (base > 0 && i < p.num_seqs) request(i, q_len, pos0);
+        const int more = i < p.num_seqs ? tiles_from(q_len, pos0, lo + 1) : 0, c = i < p.num_seqs ? tiles_from(q_len, pos0, lo) - more : 0;
+        int upto = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        const unsigned here = __ballot_sync(0xffffffffu, upto > rest);
+        if (here != 0) {
+            const int l = __ffs(here) - 1;
+            s = base + l;
+            const int n = (q_len * G + rows - 1) / rows;
+            tile = __shfl_sync(0xffffffffu, n - 1 - more - (rest - (upto - c)), l);
+            return true;
+        }
+        rest -= __shfl_sync(0xffffffffu, upto, 31);
+    }
+    return false;
+}
+
+// CTAs for the row tiles of a step: no request has more than ceil(max_rows / rows), all together not more than N G / rows + S.
+static inline unsigned at_grid(int N, int S, int max_q_len, int nh, int nkv, int rows) {
+    const long long G = nh / nkv, each = (max_q_len * G + rows - 1) / rows * S, all = (long long) N * G / rows + S;
+    return (unsigned) ((each < all ? each : all) * nkv);
+}
+
 template <int FORM>
 __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
     const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const TcAttnParams p) {
@@ -271,15 +348,16 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
     __shared__ unsigned tmem_base_s;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kvh = blockIdx.y, s = blockIdx.z;
     const int G = p.nh / p.nkv;
+    int s, row_tile;
+    if (!at_row_tile(p, G, CTA_ROWS, (int) blockIdx.x / p.nkv, s, row_tile)) return;
+    const int kvh = (int) blockIdx.x % p.nkv;
     const int q0 = p.cu_q[s];
     const int q_len = p.cu_q[s + 1] - q0;
     const int ctx = p.ctx_len[s];
     const int pos0 = ctx - q_len;
     const int rows_total = q_len * G;
-    const int row0 = ((int) gridDim.x - 1 - (int) blockIdx.x) * CTA_ROWS;    // late rows see the most keys: they start first
-    if (row0 >= rows_total) return;
+    const int row0 = row_tile * CTA_ROWS;
 
     // two groups of 128 rows (A, B) share every K/V tile; B may be empty, and A may need a tile less than B
     const bool has_b = DIFF || row0 + AT_BM < rows_total;
@@ -873,7 +951,7 @@ IIAN_API int iian_attention_tc_kept(const void * q, long long ld_q, const void *
     if (rc != IIAN_OK) return rc;
     TcAttnParams p;
     p.q = (const __nv_bfloat16 *) q; p.out = (__nv_bfloat16 *) out; p.cu_q = cu_q; p.ctx_len = ctx_len; p.block_table = block_table;
-    p.max_blocks = max_blocks; p.nh = nh; p.nkv = nkv; p.page_size = page_size; p.num_pages = num_pages; p.window = window;
+    p.max_blocks = max_blocks; p.nh = nh; p.nkv = nkv; p.num_seqs = S; p.page_size = page_size; p.num_pages = num_pages; p.window = window;
     p.scale_log2 = scale * 1.4426950408889634f;
     p.status = status;
     p.sink = sink;
@@ -894,8 +972,7 @@ IIAN_API int iian_attention_tc_kept(const void * q, long long ld_q, const void *
         if (e != cudaSuccess) return 1000 + (int) e;
         configured[kept ? 1 : 0] = true;
     }
-    const int max_rows = max_q_len * (nh / nkv);
-    dim3 grid((max_rows + AT_ROWS - 1) / AT_ROWS, nkv, S);
+    const unsigned grid = at_grid(N, S, max_q_len, nh, nkv, AT_ROWS);
     if (kept) attention_tc_kernel<AT_KEPT><<<grid, AT_THREADS, smem, stream>>>(mk, mv, p);
     else attention_tc_kernel<AT_PLAIN><<<grid, AT_THREADS, smem, stream>>>(mk, mv, p);
     return iian_launch_status();
@@ -922,7 +999,7 @@ IIAN_API int iian_attention_tc_capped(const void * q, long long ld_q, const void
     if (rc != IIAN_OK) return rc;
     TcAttnParams p;
     p.q = (const __nv_bfloat16 *) q; p.out = (__nv_bfloat16 *) out; p.cu_q = cu_q; p.ctx_len = ctx_len; p.block_table = block_table;
-    p.max_blocks = max_blocks; p.nh = nh; p.nkv = nkv; p.page_size = page_size; p.num_pages = num_pages; p.window = window;
+    p.max_blocks = max_blocks; p.nh = nh; p.nkv = nkv; p.num_seqs = S; p.page_size = page_size; p.num_pages = num_pages; p.window = window;
     p.status = status;
     p.sink = sink;
     p.sink_to_raw = 1.4426950408889634f;                     // capped scores are kept in units of log2
@@ -936,8 +1013,7 @@ IIAN_API int iian_attention_tc_capped(const void * q, long long ld_q, const void
         if (e != cudaSuccess) return 1000 + (int) e;
         configured = true;
     }
-    const int max_rows = max_q_len * (nh / nkv);
-    dim3 grid((max_rows + AT_ROWS - 1) / AT_ROWS, nkv, S);
+    const unsigned grid = at_grid(N, S, max_q_len, nh, nkv, AT_ROWS);
     attention_tc_kernel<AT_CAP><<<grid, AT_THREADS, smem, stream>>>(mk, mv, p);
     return iian_launch_status();
 }
@@ -961,7 +1037,7 @@ IIAN_API int iian_attention_tc_difference(const void * q, const void * k_cache, 
     if (rc != IIAN_OK) return rc;
     TcAttnParams p;
     p.q = (const __nv_bfloat16 *) q; p.out = (__nv_bfloat16 *) out; p.cu_q = cu_q; p.ctx_len = ctx_len; p.block_table = block_table;
-    p.max_blocks = max_blocks; p.nh = nh; p.nkv = nkv; p.page_size = page_size; p.num_pages = num_pages; p.window = 0;
+    p.max_blocks = max_blocks; p.nh = nh; p.nkv = nkv; p.num_seqs = S; p.page_size = page_size; p.num_pages = num_pages; p.window = 0;
     p.scale_log2 = cap > 0.0f ? 1.0f : scale * 1.4426950408889634f;
     p.status = status;
     p.ld_q = (long long) nh * AT_HD;
@@ -974,7 +1050,7 @@ IIAN_API int iian_attention_tc_difference(const void * q, const void * k_cache, 
         if (e != cudaSuccess) return 1000 + (int) e;
         configured = true;
     }
-    dim3 grid((max_q_len * (nh / nkv) + AT_BM - 1) / AT_BM, nkv, S);
+    const unsigned grid = at_grid(N, S, max_q_len, nh, nkv, AT_BM);
     attention_tc_kernel<AT_DIFF><<<grid, AT_THREADS, smem, stream>>>(mk, mv, p);
     return iian_launch_status();
 }
