@@ -491,9 +491,328 @@ delta_scan_kernel(const float * __restrict__ qn, const float * __restrict__ kn, 
     }
 }
 
+// ---- portions of prompts, four tokens at a time ------------------------------------------------------------------
+// Over four tokens the recurrence is a product with the state before them and small sums among themselves.  With G_t the decays'
+// product from the first of the four to token t and G_ts that from the token behind s to t (both per key channel):
+//     p_t = (G_t k_t) . s,  r_t = (G_t q_t) . s        eight dot products with ONE state column s
+//     u_t = beta_t (v_t - p_t - sum_{s<t} A_ts u_s),   A_ts = sum_d k_t k_s G_ts
+//     o_t = r_t + sum_{s<=t} B_ts u_s,                 B_ts = sum_d q_t k_s G_ts
+//     s  <- G_3 s + sum_t (G_3t k_t) u_t
+// so the chain from token to token (a pass over the column, a reduction over its lanes, the write) is walked once for four tokens.
+// Everything is float32; the decays' products are of at most four factors, taken as such (no logarithms), and only ever shrink.
+//   delta_block  per four tokens and head: the 13 vectors G_t k_t, G_t q_t, G_3t k_t, G_3 and the 28 numbers beta, A, B, one piece of
+//                memory (tokens beyond a sequence's last count as k = q = 0, decay 1, beta 0: nothing changes).
+//   delta_block_scan  the recurrence: the pieces come through a ring of shared memory, kBlocksPerStage at a time.
+constexpr int kBlockNumbers = 28;               // beta [4], A (1,0) (2,0) (2,1) (3,0) (3,1) (3,2) 0 0, B [4][4] (zero above the diagonal)
+constexpr int kBlocksPerStage = 2, kBlockStages = 4;
+
+__device__ __forceinline__ unsigned long long dr_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ unsigned long long dr_mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long dr_twice(float v) {
+    unsigned long long d;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(v));
+    return d;
+}
+__device__ __forceinline__ float dr_both(unsigned long long v) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+    return x + y;
+}
+
+// Where a sequence's pieces begin.  `pieces` 0: the whole step at once, the pieces of sequence s from cu_q[s] / 4 + s on (the sequences
+// before it have no more: sum ceil(n / 4) <= floor(sum n / 4) + s); else the step in segments of that many pieces per sequence.
+__device__ __forceinline__ size_t first_piece(const int * __restrict__ cu_q, int s, int pieces) {
+    return pieces > 0 ? (size_t) s * pieces : (size_t) (cu_q[s] / 4 + s);
+}
+
+// Grid (all pieces, H) with the whole step at once, else (pieces of a segment, H, S); 128 threads; D <= 128.  Piece c of sequence s
+// holds its tokens `from` + 4 c ..
+__global__ void __launch_bounds__(128)
+delta_block_kernel(const float * __restrict__ qn, const float * __restrict__ kn, const float * __restrict__ beta,
+                   const float * __restrict__ decay, int per_head, const int * __restrict__ cu_q, const int * __restrict__ state_slots,
+                   float * __restrict__ blocks, int from, int pieces, int S, int H, int G, int D) {
+    const int h = blockIdx.y, g = h / (H / G);
+    int s = blockIdx.z, c = blockIdx.x;
+    if (pieces == 0) {                           // the last sequence that begins at or before this piece
+        int lo = 0, hi = S - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (cu_q[mid] / 4 + mid <= (int) blockIdx.x) lo = mid; else hi = mid - 1;
+        }
+        s = lo;
+        c = (int) blockIdx.x - (cu_q[s] / 4 + s);
+    }
+    const long long t0 = (long long) cu_q[s] + from + 4 * c;
+    const int n = (int) min(4ll, cu_q[s + 1] - t0);
+    if (n <= 0 || state_slots[s] < 0) return;
+    float * b = blocks + ((first_piece(cu_q, s, pieces) + c) * H + h) * (13 * D + kBlockNumbers);
+    __shared__ float red[4][16];
+    const int d = threadIdx.x, lane = d & 31, warp = d >> 5;
+    float k[4], q[4], w[4];
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+        const bool in = t < n && d < D;
+        const size_t row = (size_t) (t0 + t);
+        k[t] = in ? kn[row * G * D + g * D + d] : 0.0f;
+        q[t] = in ? qn[row * G * D + g * D + d] : 0.0f;
+        w[t] = t < n ? (per_head ? decay[row * H + h] : d < D ? decay[row * H * D + h * D + d] : 1.0f) : 1.0f;
+    }
+    const float p0 = w[0], p1 = p0 * w[1], p2 = p1 * w[2], p3 = p2 * w[3];
+    const float g21 = w[1] * w[2], g32 = w[2] * w[3], g31 = g21 * w[3];          // from the token behind 0 to 2, behind 1 to 3, behind 0 to 3
+    if (d < D) {
+        b[d] = p0 * k[0]; b[D + d] = p1 * k[1]; b[2 * D + d] = p2 * k[2]; b[3 * D + d] = p3 * k[3];
+        b[4 * D + d] = p0 * q[0]; b[5 * D + d] = p1 * q[1]; b[6 * D + d] = p2 * q[2]; b[7 * D + d] = p3 * q[3];
+        b[8 * D + d] = g31 * k[0]; b[9 * D + d] = g32 * k[1]; b[10 * D + d] = w[3] * k[2]; b[11 * D + d] = k[3];
+        b[12 * D + d] = p3;
+    }
+    const float k0_1 = k[0] * w[1], k0_2 = k[0] * g21, k0_3 = k[0] * g31, k1_2 = k[1] * w[2], k1_3 = k[1] * g32, k2_3 = k[2] * w[3];
+    float a[16] = {k[1] * k0_1, k[2] * k0_2, k[2] * k1_2, k[3] * k0_3, k[3] * k1_3, k[3] * k2_3,
+                   q[0] * k[0], q[1] * k0_1, q[1] * k[1], q[2] * k0_2, q[2] * k1_2, q[2] * k[2],
+                   q[3] * k0_3, q[3] * k1_3, q[3] * k2_3, q[3] * k[3]};
+    // sixteen sums over the warp: the values a lane carries are halved with every exchange; a lane ends with value lane >> 1
+#pragma unroll
+    for (int half = 8; half >= 1; half >>= 1) {
+        const bool up = lane & (2 * half);
+#pragma unroll
+        for (int j = 0; j < half; j++) {
+            const float give = up ? a[j] : a[j + half], keep = up ? a[j + half] : a[j];
+            a[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * half);
+        }
+    }
+    a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
+    if ((lane & 1) == 0) red[warp][lane >> 1] = a[0];
+    __syncthreads();
+    if (d < kBlockNumbers) {
+        // place of each number among the sixteen sums; -1: zero, -2: a write strength
+        const int from_sum[kBlockNumbers] = {-2, -2, -2, -2, 0, 1, 2, 3, 4, 5, -1, -1, 6, -1, -1, -1, 7, 8, -1, -1, 9, 10, 11, -1, 12, 13, 14, 15};
+        int at = -1;
+#pragma unroll
+        for (int i = 0; i < kBlockNumbers; i++) at = i == d ? from_sum[i] : at;
+        float v = 0.0f;
+        if (at >= 0) v = (red[0][at] + red[1][at]) + (red[2][at] + red[3][at]);
+        else if (at == -2 && d < n) v = beta[(size_t) (t0 + d) * H + h];
+        b[13 * D + d] = v;
+    }
+}
+
+// A CTA owns kCols columns of one (sequence, head); 16 lanes share two columns, E = D / 16 entries of each a lane (groups of four
+// neighbours, d = 4 lane + 64 i): a vector that is read serves both.  Where the time goes: some 260 instructions a warp and piece, 5 clocks
+// each with one warp per scheduler, their chain (reduction over the lanes, four writes, update) uncovered.  1,500 tokens x 16 heads: 256 us
+// (token by token 399 us).  Measured against it: eight lanes a column, each column reading every vector for itself, 300 us (128 bytes a clock
+// is what shared memory delivers to registers); 32 lanes for two columns, two warps per scheduler, 240 us, but 565 against 500 us for four
+// sequences of 2,048; a warp per eighth of D and a lane per column, the sums through shared memory, 241 and 523 us.
+// V a multiple of kCols; state and values on 16-byte boundaries.
+constexpr int kPairLanes = 16;
+
+template <int E, typename A>
+__global__ void __launch_bounds__(kCols / 2 * kPairLanes)
+delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restrict__ vv, float * __restrict__ state, long long state_stride,
+                        long long tail_off, const A * __restrict__ proj, long long ld, int col_off, int n_taps,
+                        const int * __restrict__ cu_q, const int * __restrict__ state_slots, float * __restrict__ out,
+                        int from, int pieces, int H, int G, int V) {
+    constexpr int D = E * kPairLanes, BLOCK = 13 * D + kBlockNumbers, PIECE = BLOCK + 4 * kCols, STAGE = kBlocksPerStage * PIECE;
+    constexpr int kThreads = kCols / 2 * kPairLanes;
+    extern __shared__ __align__(16) float sm[];
+    const int cb = blockIdx.x, h = blockIdx.y, s = blockIdx.z;
+    const int tid = threadIdx.x, pair = tid / kPairLanes, lane = tid % kPairLanes, j = cb * kCols + 2 * pair;
+    const int q0 = cu_q[s], q1 = cu_q[s + 1], slot = state_slots[s], HV = H * V;
+    const int t0 = q0 + from, t1 = pieces > 0 ? min(q1, t0 + 4 * pieces) : q1;
+    if (t0 >= t1) return;
+    if (slot < 0) {
+        for (int t = t0; t < t1; t++)
+            if (lane < 2) out[(size_t) t * HV + h * V + j + lane] = 0.0f;
+        return;
+    }
+    float * st = state + (size_t) slot * state_stride;
+    const int n_blocks = (t1 - t0 + 3) / 4, turns = (n_blocks + kBlocksPerStage - 1) / kBlocksPerStage;
+    const float * mine = blocks + (first_piece(cu_q, s, pieces) * H + h) * BLOCK;
+    auto fill = [&](int turn) {
+        if (turn < turns) {
+            float * to = sm + (turn % kBlockStages) * STAGE;
+#pragma unroll
+            for (int b = 0; b < kBlocksPerStage; b++) {
+                const int c = turn * kBlocksPerStage + b;
+                if (c >= n_blocks) break;
+                const float * src = mine + (size_t) c * H * BLOCK;
+                for (int e = tid; e < BLOCK / 4; e += kThreads) dr_cp16(to + b * PIECE + 4 * e, src + 4 * e);
+                if (tid < kCols) {                           // four tokens' values of the CTA's columns; beyond the last token: that one's
+                    const int t = min(t0 + 4 * c + tid / 4, t1 - 1);
+                    dr_cp16(to + b * PIECE + BLOCK + 4 * tid, vv + (size_t) t * HV + h * V + cb * kCols + 4 * (tid % 4));
+                }
+            }
+        }
+        dr_commit();
+    };
+#pragma unroll
+    for (int i = 0; i < kBlockStages - 1; i++) fill(i);
+
+    if (from == 0 && n_taps > 1) {             // the convolution's tail moves on, as in the scan above
+        const int C = 2 * G * D + HV, back = n_taps - 1, L = q1 - q0;
+        float * tail = st + tail_off;
+        const int part = h * gridDim.x + cb, parts = gridDim.x * gridDim.y;
+        for (int c = part * kThreads + tid; c < C; c += parts * kThreads) {
+            float keep[kMaxTaps];
+#pragma unroll
+            for (int i = 0; i < kMaxTaps - 1; i++) {
+                if (i >= back) break;
+                const int src = L - back + i;
+                keep[i] = src >= 0 ? to_f32(proj[(size_t) (q0 + src) * ld + col_off + c]) : tail[(size_t) (src + back) * C + c];
+            }
+#pragma unroll
+            for (int i = 0; i < kMaxTaps - 1; i++) {
+                if (i >= back) break;
+                tail[(size_t) i * C + c] = keep[i];
+            }
+        }
+    }
+    unsigned long long S[2][E / 2];
+    float * scol = st + ((size_t) h * V + j) * D;
+#pragma unroll
+    for (int x = 0; x < 2; x++)
+#pragma unroll
+        for (int i = 0; i < E / 4; i++) {
+            const ulonglong2 e = *reinterpret_cast<const ulonglong2 *>(scol + x * D + 4 * lane + 4 * kPairLanes * i);
+            S[x][2 * i] = e.x; S[x][2 * i + 1] = e.y;
+        }
+    for (int turn = 0; turn < turns; turn++) {
+        dr_wait<kBlockStages - 2>();
+        __syncthreads();                       // this turn's pieces have landed; the stage filled next was read by everyone
+        fill(turn + kBlockStages - 1);
+        const float * stage = sm + (turn % kBlockStages) * STAGE;
+#pragma unroll
+        for (int b = 0; b < kBlocksPerStage; b++) {
+            const int c = turn * kBlocksPerStage + b;
+            if (c >= n_blocks) break;
+            const float * vec = stage + b * PIECE;
+            const float * num = vec + 13 * D;
+            unsigned long long acc[2][8];
+#pragma unroll
+            for (int v = 0; v < 8; v++) acc[0][v] = acc[1][v] = 0ull;
+#pragma unroll
+            for (int i = 0; i < E / 4; i++) {
+#pragma unroll
+                for (int v = 0; v < 8; v++) {
+                    const ulonglong2 e = *reinterpret_cast<const ulonglong2 *>(vec + v * D + 4 * lane + 4 * kPairLanes * i);
+#pragma unroll
+                    for (int x = 0; x < 2; x++) {
+                        acc[x][v] = dr_fma2(e.x, S[x][2 * i], acc[x][v]);
+                        acc[x][v] = dr_fma2(e.y, S[x][2 * i + 1], acc[x][v]);
+                    }
+                }
+            }
+            float a[16];
+#pragma unroll
+            for (int v = 0; v < 16; v++) a[v] = dr_both(acc[v >> 3][v & 7]);
+            // sixteen sums over the sixteen lanes: the values a lane carries are halved with every exchange; lane l ends with sum l: p_0 ..
+            // p_3, r_0 .. r_3 of the first column, then of the second
+#pragma unroll
+            for (int half = 8; half >= 1; half >>= 1) {
+                const bool up = lane & half;
+#pragma unroll
+                for (int i = 0; i < half; i++) {
+                    const float give = up ? a[i] : a[i + half], keep = up ? a[i + half] : a[i];
+                    a[i] = keep + __shfl_xor_sync(0xffffffffu, give, half);
+                }
+            }
+            const float4 be = *reinterpret_cast<const float4 *>(num), A0 = *reinterpret_cast<const float4 *>(num + 4);
+            const float2 A1 = *reinterpret_cast<const float2 *>(num + 8);
+            const float * val = vec + BLOCK + 2 * pair;
+            float2 v[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) v[t] = *reinterpret_cast<const float2 *>(val + t * kCols);
+            float u[2][4];
+#pragma unroll
+            for (int x = 0; x < 2; x++) {
+                float p[4];
+#pragma unroll
+                for (int t = 0; t < 4; t++) p[t] = (x ? v[t].y : v[t].x) - __shfl_sync(0xffffffffu, a[0], 8 * x + t, kPairLanes);
+                u[x][0] = be.x * p[0];
+                u[x][1] = be.y * (p[1] - A0.x * u[x][0]);
+                u[x][2] = be.z * (p[2] - (A0.y * u[x][0] + A0.z * u[x][1]));
+                u[x][3] = be.w * (p[3] - (A0.w * u[x][0] + A1.x * u[x][1] + A1.y * u[x][2]));
+            }
+#pragma unroll
+            for (int i = 0; i < E / 4; i++) {
+                const int at = 4 * lane + 4 * kPairLanes * i;
+                ulonglong2 e = *reinterpret_cast<const ulonglong2 *>(vec + 12 * D + at);
+#pragma unroll
+                for (int x = 0; x < 2; x++) { S[x][2 * i] = dr_mul2(e.x, S[x][2 * i]); S[x][2 * i + 1] = dr_mul2(e.y, S[x][2 * i + 1]); }
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    e = *reinterpret_cast<const ulonglong2 *>(vec + (8 + t) * D + at);
+#pragma unroll
+                    for (int x = 0; x < 2; x++) {
+                        const unsigned long long w = dr_twice(u[x][t]);
+                        S[x][2 * i] = dr_fma2(e.x, w, S[x][2 * i]);
+                        S[x][2 * i + 1] = dr_fma2(e.y, w, S[x][2 * i + 1]);
+                    }
+                }
+            }
+            const int t = t0 + 4 * c + (lane & 7) - 4;
+            if ((lane & 4) && t < t1) {
+                const float4 B = *reinterpret_cast<const float4 *>(num + 12 + 4 * (lane & 3));
+                const bool second = lane & 8;
+                const float u0 = second ? u[1][0] : u[0][0], u1 = second ? u[1][1] : u[0][1], u2 = second ? u[1][2] : u[0][2];
+                const float u3 = second ? u[1][3] : u[0][3];
+                out[(size_t) t * HV + h * V + j + (second ? 1 : 0)] = a[0] + (B.x * u0 + B.y * u1 + B.z * u2 + B.w * u3);
+            }
+        }
+    }
+#pragma unroll
+    for (int x = 0; x < 2; x++)
+#pragma unroll
+        for (int i = 0; i < E / 4; i++) {
+            ulonglong2 e;
+            e.x = S[x][2 * i]; e.y = S[x][2 * i + 1];
+            *reinterpret_cast<ulonglong2 *>(scol + x * D + 4 * lane + 4 * kPairLanes * i) = e;
+        }
+}
+
 }  // namespace iian
 
 using namespace iian;
+
+// Floats of one four-token piece (all heads) of iian_delta_block_scan's scratch.
+IIAN_API long long iian_delta_block_floats(int H, int D) { return (long long) H * (13 * D + kBlockNumbers); }
+
+// The scan of iian_delta_scan for bfloat16 models and portions of many tokens, four tokens at a time.  blocks: scratch for N / 4 + S
+// pieces with `pieces` 0, else for S * pieces: the step is then walked in segments of 4 * pieces tokens of every sequence, max_q_len the
+// most tokens a sequence has.  D 64 or 128, V a multiple of 16.
+IIAN_API int iian_delta_block_scan(const float * qn, const float * kn, const float * vv, const float * beta, const float * decay,
+                                   float * blocks, int pieces, float * state, long long state_stride, const void * proj, long long ld,
+                                   int col_off, int n_taps, const int * cu_q, const int * state_slots, float * out, int N, int S, int H,
+                                   int G, int D, int V, int max_q_len, int per_head, cudaStream_t stream) {
+    if (N <= 0 || S <= 0 || max_q_len <= 0) return IIAN_OK;
+    if (H <= 0 || G <= 0 || H % G || (D != 64 && D != 128) || V <= 0 || V % kCols || n_taps < 1 || n_taps > kMaxTaps || pieces < 0 || S > 65535 ||
+        H > 65535) return IIAN_ERR_SHAPE;
+    if (state_stride % 4 || (((uintptr_t) blocks | (uintptr_t) vv | (uintptr_t) state) & 15)) return IIAN_ERR_ALIGN;
+    typedef __nv_bfloat16 bf;
+    const size_t smem = (size_t) kBlockStages * kBlocksPerStage * (13 * D + kBlockNumbers + 4 * kCols) * sizeof(float);
+    auto scan = D == 128 ? delta_block_scan_kernel<8, bf> : delta_block_scan_kernel<4, bf>;
+    const cudaError_t e = cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    if (e != cudaSuccess) return 1000 + (int) e;
+    const int step = pieces > 0 ? 4 * pieces : max_q_len;
+    for (int from = 0; from < max_q_len; from += step) {
+        const dim3 grid = pieces > 0 ? dim3(min(pieces, (max_q_len - from + 3) / 4), H, S) : dim3(N / 4 + S, H);
+        delta_block_kernel<<<grid, 128, 0, stream>>>(qn, kn, beta, decay, per_head, cu_q, state_slots, blocks, from, pieces, S, H, G, D);
+        int rc = iian_launch_status();
+        if (rc != IIAN_OK) return rc;
+        scan<<<dim3(V / kCols, H, S), kCols / 2 * kPairLanes, smem, stream>>>(blocks, vv, state, state_stride, (long long) H * V * D, (const bf *) proj, ld,
+                                                                      col_off, n_taps, cu_q, state_slots, out, from, pieces, H, G, V);
+        rc = iian_launch_status();
+        if (rc != IIAN_OK) return rc;
+    }
+    return IIAN_OK;
+}
+
 
 // Floats of a slot's state: S [H, V, D], then the tail [taps - 1, 2 G D + H V].
 IIAN_API long long iian_delta_state_floats(int H, int G, int D, int V, int n_taps) {

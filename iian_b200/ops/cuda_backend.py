@@ -1992,6 +1992,28 @@ class CudaKernels:
         (csrc/delta_rule.cu: iian_delta_state_floats)."""
         return num_heads * v_dim * dim + (taps - 1) * (2 * num_kv_heads * dim + num_heads * v_dim)
 
+    # the delta rule's scan over portions of prompts, four tokens at a time (bfloat16 models); IIAN_DELTA_BLOCKS=0: token by token.
+    # The 32-bit path stays token by token: there a token's bits must not depend on how its prompt was cut.
+    DELTA_BLOCKS = os.environ.get("IIAN_DELTA_BLOCKS", "1") not in ("0", "false", "off")
+    DELTA_BLOCK_MIN_TOKENS = 32            # of the longest portion (16 tokens 148 -> 150 us a layer, 100 tokens 156 -> 152, 1,500 tokens 585 -> 457)
+    DELTA_BLOCK_BYTES = 192 << 20          # of scratch for the pieces; a step that needs more is walked in segments
+
+    def _delta_block_floats(self, h: int, d: int) -> int:
+        fn = _build.load("delta_rule").iian_delta_block_floats
+        fn.restype = c_longlong
+        return int(fn(c_int(h), c_int(d)))
+
+    def _delta_pieces(self, code: int, n: int, s: int, h: int, d: int, v: int, max_q_len: int, state: torch.Tensor) -> Optional[int]:
+        """None: the scan token by token; 0: in pieces of four tokens, the whole step at once; else that many pieces of every sequence
+        at a time (a power of two)."""
+        if not self.DELTA_BLOCKS or code != BF16 or max_q_len < self.DELTA_BLOCK_MIN_TOKENS or d not in (64, 128) or v % 16 \
+                or state.shape[1] % 4 or state.data_ptr() % 16:
+            return None
+        most = self.DELTA_BLOCK_BYTES // (4 * self._delta_block_floats(h, d))
+        if n // 4 + s <= most:
+            return 0
+        return 1 << ((most // s).bit_length() - 1) if most // s >= 8 else None
+
     def delta_rule(self, proj: torch.Tensor, col_off: int, b_off: int, z: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor,
                    dt_bias: torch.Tensor, state: torch.Tensor, ctx, out: torch.Tensor, *, num_heads: int, num_kv_heads: int, dim: int,
                    v_dim: int, b_pre: Optional[torch.Tensor] = None) -> None:
@@ -1999,7 +2021,8 @@ class CudaKernels:
         column ``col_off`` and the write strengths' pre-activations at ``b_off`` (or ``b_pre`` float32 [N, heads] holds them);
         ``z`` float32 [N, heads * dim] (a decay per key channel) or [N, heads] (one per head) the decays' pre-activations
         without bias; ``z`` and ``b_pre`` may be column slices of one matrix; ``taps`` float32 [channels, taps]; ``state`` float32 [slots, state floats];
-        ``out`` float32 [N, heads * v_dim] receives ``S^T q`` per head.  Two launches: per-token preparation, then the scan."""
+        ``out`` float32 [N, heads * v_dim] receives ``S^T q`` per head.  Two launches: per-token preparation, then the scan; portions of
+        prompts in bfloat16 models walk the scan four tokens at a time (``_delta_pieces``)."""
         n = proj.shape[0]
         h, g, d, v = num_heads, num_kv_heads, dim, v_dim
         channels = 2 * g * d + h * v
@@ -2032,12 +2055,25 @@ class CudaKernels:
                   _cuda(ctx.seq_of_token, "seq_of_token", torch.int32), _cuda(ctx.cu_q, "cu_q", torch.int32),
                   _cuda(ctx.state_slots, "state slots", torch.int32), qn.data_ptr(), kn.data_ptr(), vv.data_ptr(), beta.data_ptr(),
                   decay.data_ptr(), qk.data_ptr(), n, h, g, d, v, _stream()), "delta_prep")
+        max_q_len = int(getattr(ctx, "max_q_len", 0) or 0)
+        pieces = self._delta_pieces(code, n, s, h, d, v, max_q_len, state)
+        if pieces is not None:
+            count = n // 4 + s if pieces == 0 else s * pieces
+            blocks = ctx.buf("delta_blocks", (count * self._delta_block_floats(h, d),), f32)
+            fn = _fn("delta_rule", "iian_delta_block_scan",
+                     [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_int,
+                      c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
+            _check(fn(qn.data_ptr(), kn.data_ptr(), vv.data_ptr(), beta.data_ptr(), decay.data_ptr(), blocks.data_ptr(), pieces,
+                      state.data_ptr(), state.shape[1], pp, ld, col_off, n_taps, ctx.cu_q.data_ptr(), ctx.state_slots.data_ptr(),
+                      _cuda(out, "delta out", f32), n, s, h, g, d, v, max_q_len, 1 if per_head else 0, _stream()), "delta_block_scan")
+            LAUNCHES[0] += 2 * (1 if pieces == 0 else -(-max_q_len // (4 * pieces))) - 1
+            return
         fn = _fn("delta_rule", "iian_delta_scan",
                  [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int,
                   c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
         _check(fn(qn.data_ptr(), kn.data_ptr(), vv.data_ptr(), beta.data_ptr(), decay.data_ptr(), qk.data_ptr(), state.data_ptr(),
                   state.shape[1], pp, ld, col_off, code, n_taps, ctx.cu_q.data_ptr(), ctx.state_slots.data_ptr(),
-                  _cuda(out, "delta out", f32), s, h, g, d, v, int(getattr(ctx, "max_q_len", 0) or 0), 1 if per_head else 0, _stream()),
+                  _cuda(out, "delta out", f32), s, h, g, d, v, max_q_len, 1 if per_head else 0, _stream()),
                "delta_scan")
 
     # ---- routing by a table, weights on the experts' outputs (csrc/moe.cu) ------------------------------------------------------

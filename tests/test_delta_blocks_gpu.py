@@ -1,0 +1,56 @@
+"""The delta rule's scan over portions of prompts, four tokens at a time, against the scan token by token: lengths around multiples
+of four and of a stage, sequences of a single token and padding between long ones, states that go on, the step whole and in segments."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from iian_b200.ops.cuda_backend import CudaKernels
+
+pytestmark = pytest.mark.gpu
+
+
+def walk(blocks, scratch, lens, H, G, D, V, per_head):
+    K = CudaKernels()
+    g = torch.Generator("cuda").manual_seed(sum(lens) + D + H)
+    C = 2 * G * D + H * V
+    state = torch.randn(len(lens) + 1, K.delta_state_floats(H, G, D, V, 4), device="cuda", generator=g)
+    taps = torch.randn(C, 4, device="cuda", generator=g) * 0.4
+    a_log, z_width = torch.rand(H, device="cuda", generator=g) * 2.5, H if per_head else H * D
+    dt_bias = torch.randn(z_width, device="cuda", generator=g) - 2.0
+    slots = [i if i != 1 else -1 for i in range(len(lens))]                       # the second sequence is padding
+    bufs, outs = {}, []
+    for _ in range(2):                                                              # the second step goes on from the first one's states
+        n = sum(lens)
+        proj = torch.randn(n, C + H, device="cuda", generator=g).bfloat16()
+        z = torch.randn(n, z_width, device="cuda", generator=g)
+        cu = [0]
+        for x in lens:
+            cu.append(cu[-1] + x)
+        seq = torch.tensor([i if slots[i] >= 0 else -1 for i, x in enumerate(lens) for _ in range(x)], dtype=torch.int32, device="cuda")
+        ctx = SimpleNamespace(cu_q=torch.tensor(cu, dtype=torch.int32, device="cuda"), seq_of_token=seq, max_q_len=max(lens),
+                              state_slots=torch.tensor(slots, dtype=torch.int32, device="cuda"),
+                              buf=lambda name, shape, dt: bufs.setdefault((name, tuple(shape)), torch.zeros(shape, dtype=dt, device="cuda")))
+        out = torch.full((n, H * V), 7.0, device="cuda")
+        was = CudaKernels.DELTA_BLOCKS, CudaKernels.DELTA_BLOCK_BYTES
+        CudaKernels.DELTA_BLOCKS, CudaKernels.DELTA_BLOCK_BYTES = blocks, scratch
+        try:
+            K.delta_rule(proj, 0, C, z, taps, a_log, dt_bias, state, ctx, out, num_heads=H, num_kv_heads=G, dim=D, v_dim=V)
+        finally:
+            CudaKernels.DELTA_BLOCKS, CudaKernels.DELTA_BLOCK_BYTES = was
+        outs.append(out)
+    assert not blocks or any(name == "delta_blocks" for name, _ in bufs)
+    return torch.cat(outs), state
+
+
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("H,G,D,V", [(4, 2, 128, 128), (3, 3, 64, 48), (2, 1, 128, 16)])
+@pytest.mark.parametrize("lens", [[32], [33, 3, 1], [1, 2, 47, 1, 64], [35, 1, 130]])
+def test_four_tokens_at_a_time(lens, H, G, D, V, per_head):
+    want, want_state = walk(False, 0, lens, H, G, D, V, per_head)
+    piece = 4 * H * (13 * D + 28)
+    for scratch in (192 << 20, piece * 8 * len(lens)):            # the whole step at once, and in segments of eight pieces
+        got, state = walk(True, scratch, lens, H, G, D, V, per_head)
+        # both are 32-bit sums of the same terms in another order: D of them in a dot product, the sequence's tokens in the state
+        for a, b in ((got, want), (state, want_state)):
+            assert (a - b).norm() <= 1e-5 * b.norm() and (a - b).abs().max() <= 1e-4 * b.abs().max()
