@@ -21,6 +21,8 @@
 // With ONE decay per head the two dot products are taken from the column as it is and multiplied by the decay behind the
 // reduction (g (k . s_j) = k . (g s_j)), so the multiplication of the column leaves the chain from token to token.
 // State of a slot (float32): S as [heads, vdim, dim] (a column is contiguous), then the tail [taps - 1, channels].
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace iian {
@@ -271,6 +273,144 @@ delta_prep_tile_kernel(const A * __restrict__ proj, long long ld, int col_off, i
                 const float zb = b_pre != nullptr ? b_pre[t * (size_t) ld_z + h] : to_f32(proj[t * ld + b_off + h]);
                 beta[t * H + h] = 1.0f / (1.0f + expf(-zb));
             }
+        }
+    }
+}
+
+// The same preparation for steps of many tokens of bfloat16 models with heads of 128 and four taps: a warp takes one unit of 128 channels
+// (a query/key head's q and k, 128 values, a head's decays) over kWideTokens neighbouring rows, a lane four neighbouring channels.  The
+// convolution's window slides through registers, so every input is read once, eight bytes a lane, four tokens ahead; nothing is staged
+// and no lane waits for another but in the three sums of a query/key head.  What bounds it: instruction issue (the exponentials and
+// logarithms of silu and softplus) and the latency of a window's loads.  1,500 tokens, 16 heads of 128 with a decay per channel: 37 us
+// for 66 of the tiled kernel (the inputs and results are 74 MB, 11 us).  (The sums over a head run over a lane's four channels, then the
+// lanes: another order than the kernels above keep between them for the 32-bit path, which stays with those.)
+constexpr int kWideTokens = 16, kWideWarps = 4;
+
+template <bool HEAD>
+__global__ void __launch_bounds__(kWideWarps * 32)
+delta_prep_wide_kernel(const __nv_bfloat16 * __restrict__ proj, long long ld, int col_off, int b_off, const float * __restrict__ b_pre,
+                       const float * __restrict__ z, long long ld_z, const float * __restrict__ taps,
+                       const float * __restrict__ a_log, const float * __restrict__ dt_bias,
+                       const float * __restrict__ state, long long state_stride, long long tail_off,
+                       const int * __restrict__ seq_of_token, const int * __restrict__ cu_q, const int * __restrict__ state_slots,
+                       float * __restrict__ qn, float * __restrict__ kn, float * __restrict__ vv,
+                       float * __restrict__ beta, float * __restrict__ decay, float * __restrict__ qk,
+                       int N, int H, int G, int V, float q_scale) {
+    constexpr int D = 128, TAPS = 4, AHEAD = 4;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int GD = G * D, HV = H * V, C = 2 * GD + HV, v_units = HV / 128;
+    const int t0 = blockIdx.x * kWideTokens, t1 = min(N, t0 + kWideTokens);
+    const int u = blockIdx.y * kWideWarps + warp;
+    if (u >= G + v_units + H) return;
+    if (u >= G + v_units) {                      // decays and write strength of a head
+        const int h = u - G - v_units;
+        const float rate = expf(a_log[h]);
+        if (HEAD) {                              // a lane is a token
+            const int t = t0 + lane;
+            if (lane < kWideTokens && t < t1 && seq_of_token[t] >= 0)
+                decay[(size_t) t * H + h] = expf(-rate * softplus_f32(z[(size_t) t * ld_z + h] + dt_bias[h]));
+        } else {
+            const float4 bias = *reinterpret_cast<const float4 *>(dt_bias + h * D + 4 * lane);
+#pragma unroll 4
+            for (int t = t0; t < t1; t++) {
+                const float4 x = *reinterpret_cast<const float4 *>(z + (size_t) t * ld_z + h * D + 4 * lane);
+                float4 g;
+                g.x = expf(-rate * softplus_f32(x.x + bias.x));
+                g.y = expf(-rate * softplus_f32(x.y + bias.y));
+                g.z = expf(-rate * softplus_f32(x.z + bias.z));
+                g.w = expf(-rate * softplus_f32(x.w + bias.w));
+                if (seq_of_token[t] >= 0) *reinterpret_cast<float4 *>(decay + (size_t) t * H * D + h * D + 4 * lane) = g;
+            }
+        }
+        const int t = t0 + lane;
+        if (lane < kWideTokens && t < t1 && seq_of_token[t] >= 0) {
+            const float zb = b_pre != nullptr ? b_pre[(size_t) t * ld_z + h] : __bfloat162float(proj[(size_t) t * ld + b_off + h]);
+            beta[(size_t) t * H + h] = 1.0f / (1.0f + expf(-zb));
+        }
+        return;
+    }
+    const bool is_qk = u < G;
+    // this lane's channels: four of q and four of k, or four values
+    const int c[2] = {is_qk ? u * D + 4 * lane : 2 * GD + (u - G) * 128 + 4 * lane, GD + u * D + 4 * lane};
+    const int parts = is_qk ? 2 : 1;
+    float w[2][4][TAPS], x[2][TAPS][4];          // filters; the last four inputs, the current one last
+#pragma unroll
+    for (int p = 0; p < 2; p++)
+        if (p < parts)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const float4 f = *reinterpret_cast<const float4 *>(taps + (size_t) (c[p] + e) * TAPS);
+                w[p][e][0] = f.x; w[p][e][1] = f.y; w[p][e][2] = f.z; w[p][e][3] = f.w;
+            }
+    auto input = [&](int p, long long r, float * to) {
+        const uint2 raw = *reinterpret_cast<const uint2 *>(proj + (size_t) r * ld + col_off + c[p]);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.x));
+        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.y));
+        to[0] = a.x; to[1] = a.y; to[2] = b.x; to[3] = b.y;
+    };
+    for (int tb = t0; tb < t1; tb += AHEAD) {
+        float in[AHEAD][2][4];
+        int sq[AHEAD];
+#pragma unroll
+        for (int i = 0; i < AHEAD; i++) {
+            sq[i] = tb + i < t1 ? seq_of_token[tb + i] : -1;
+#pragma unroll
+            for (int p = 0; p < 2; p++)
+                if (p < parts && tb + i < t1) input(p, tb + i, in[i][p]);
+        }
+#pragma unroll
+        for (int i = 0; i < AHEAD; i++) {
+            const int t = tb + i, s = sq[i];
+            if (s < 0) continue;                 // padding, or behind the tile (the same for all lanes)
+            const int first = cu_q[s];
+            if (t == t0 || t == first || (i == 0 ? false : sq[i - 1] != s)) {       // the window anew: rows before t, or the state's tail
+                const int slot = state_slots[s];
+                const float * tail = slot >= 0 ? state + (size_t) slot * state_stride + tail_off : nullptr;
+#pragma unroll
+                for (int j = 1; j < TAPS; j++) {
+                    const long long r = t - TAPS + j;                  // becomes the input of tap j - 1
+#pragma unroll
+                    for (int p = 0; p < 2; p++) {
+                        if (p >= parts) continue;
+                        if (r >= first) input(p, r, x[p][j]);
+                        else {
+                            const int idx = (int) (r - first) + TAPS - 1;
+#pragma unroll
+                            for (int e = 0; e < 4; e++) x[p][j][e] = tail != nullptr && idx >= 0 ? tail[(size_t) idx * C + c[p] + e] : 0.0f;
+                        }
+                    }
+                }
+            }
+            float a[2][4];
+#pragma unroll
+            for (int p = 0; p < 2; p++)
+                if (p < parts)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        x[p][0][e] = x[p][1][e]; x[p][1][e] = x[p][2][e]; x[p][2][e] = x[p][3][e]; x[p][3][e] = in[i][p][e];
+                        float acc = 0.0f;
+#pragma unroll
+                        for (int j = 0; j < TAPS; j++) acc = fmaf(w[p][e][j], x[p][j][e], acc);
+                        a[p][e] = silu_f32(acc);
+                    }
+            if (!is_qk) {
+                *reinterpret_cast<float4 *>(vv + (size_t) t * HV + c[0] - 2 * GD) = make_float4(a[0][0], a[0][1], a[0][2], a[0][3]);
+                continue;
+            }
+            float s_q = 0.0f, s_k = 0.0f, dot = 0.0f;
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                s_q = fmaf(a[0][e], a[0][e], s_q);
+                s_k = fmaf(a[1][e], a[1][e], s_k);
+                dot = fmaf(a[0][e], a[1][e], dot);
+            }
+            s_q = warp_sum(s_q);
+            s_k = warp_sum(s_k);
+            dot = warp_sum(dot);
+            const float iq = q_scale / sqrtf(s_q + 1e-6f), ik = 1.0f / sqrtf(s_k + 1e-6f);
+            *reinterpret_cast<float4 *>(qn + (size_t) t * GD + c[0]) = make_float4(a[0][0] * iq, a[0][1] * iq, a[0][2] * iq, a[0][3] * iq);
+            *reinterpret_cast<float4 *>(kn + (size_t) t * GD + c[0]) = make_float4(a[1][0] * ik, a[1][1] * ik, a[1][2] * ik, a[1][3] * ik);
+            if (lane == 0) qk[(size_t) t * G + u] = dot * iq * ik;
         }
     }
 }
@@ -827,6 +967,16 @@ static int launch_prep(const A * proj, long long ld, int col_off, int b_off, con
                        cudaStream_t stream) {
     const long long tail_off = (long long) H * V * D;
     const float q_scale = 1.0f / sqrtf((float) D);
+    if constexpr (std::is_same<A, __nv_bfloat16>::value) {
+        const bool whole = ld % 4 == 0 && col_off % 4 == 0 && ((uintptr_t) proj & 7) == 0 && (HEAD || (ld_z % 4 == 0 && ((uintptr_t) z & 15) == 0)) &&
+                           (((uintptr_t) taps | (uintptr_t) dt_bias | (uintptr_t) qn | (uintptr_t) kn | (uintptr_t) vv | (uintptr_t) decay) & 15) == 0;
+        if (N >= kPrepTileFrom && D == 128 && V % 128 == 0 && n_taps == 4 && whole) {
+            const int units = G + H * V / 128 + H;
+            return iian_launch(delta_prep_wide_kernel<HEAD>, dim3((N + kWideTokens - 1) / kWideTokens, (units + kWideWarps - 1) / kWideWarps),
+                               dim3(kWideWarps * 32), 0, stream, proj, ld, col_off, b_off, b_pre, z, ld_z, taps, a_log, dt_bias, state, state_stride,
+                               tail_off, seq_of_token, cu_q, state_slots, qn, kn, vv, beta, decay, qk, N, H, G, V, q_scale);
+        }
+    }
     // many tokens: tiles of T rows through shared memory; few: a CTA per token and unit, so that they spread over the GPU
     int T = N >= 4 * kPrepTileFrom ? 16 : N >= kPrepTileFrom ? 8 : 0;
     size_t smem = 0;
