@@ -42,13 +42,13 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "tc_attention.cuh"
 
 namespace iian {
 
 constexpr int AT_BM = 128, AT_BN = 128, AT_HD = 128;
 constexpr int AT_ROWS = 2 * AT_BM;              // rows of a CTA: two groups of 128
 constexpr int AT_THREADS = 320;
-constexpr unsigned kAtSpinLimit = 4u * 1000u * 1000u;
 constexpr int AT_HALF_BYTES = 128 * 128;          // 128 rows x 64 bf16: one 128-byte-swizzled half tile
 constexpr int AT_TILE_BYTES = 2 * AT_HALF_BYTES;  // a 128 x 128 bf16 tile
 
@@ -87,132 +87,6 @@ struct TcAttnParams {
     int cap_range = 0;              // capped form: 1: every |s| <= cap_small, 2: <= 2 cap_small, 0: not known beforehand
     float lambda = 0.0f, factor = 0.0f, eps = 0.0f;
 };
-
-__device__ __forceinline__ unsigned at_smem(const void * p) { return (unsigned) __cvta_generic_to_shared(p); }
-__device__ __forceinline__ void at_mbar_init(unsigned bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void at_expect_tx(unsigned bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void at_arrive(unsigned bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool at_wait(unsigned bar, unsigned parity) {
-    for (unsigned spin = 0; spin < kAtSpinLimit; spin++) {
-        unsigned done;
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                     : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-__device__ __forceinline__ void at_tma_4d(unsigned dst, const CUtensorMap * map, int x, int y, int z, int w, unsigned bar) {
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void at_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void at_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void at_fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void at_commit(unsigned bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void at_mma(unsigned d_tmem, unsigned long long a_desc, unsigned long long b_desc, unsigned idesc,
-                                       unsigned accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// the same with the A operand in tensor memory (lane = row, 32-bit column = two consecutive bf16 along K)
-__device__ __forceinline__ void at_mma_ts(unsigned d_tmem, unsigned a_tmem, unsigned long long b_desc, unsigned idesc,
-                                          unsigned accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
-                 ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void at_ld32(unsigned taddr, unsigned * r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                 : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void at_st32(unsigned taddr, const unsigned * r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-                 "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-                 "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
-                   "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
-                   "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-                 : "memory");
-}
-__device__ __forceinline__ void at_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void at_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// packed pairs of float32 (one instruction for two values) and the maximum of three
-__device__ __forceinline__ unsigned long long at_pack2(float a, float b) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void at_unpack2(unsigned long long v, float & a, float & b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long at_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ unsigned long long at_mul2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ float at_min3(float a, float b, float c) {
-    float r;
-    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-__device__ __forceinline__ float at_tanh(float x) {      // 1 - 2 / (1 + e^2x), absolute error of a few 1e-7
-    float e, r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * 2.8853900817779268f));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-    return fmaf(-2.0f, r, 1.0f);
-}
-__device__ __forceinline__ unsigned long long at_add2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ float at_max3(float a, float b, float c) {
-    float r;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-__device__ __forceinline__ float at_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-// Shared-memory matrix descriptor with 128-byte swizzle.  K-major operand (rows of 128 bytes along K, groups of
-// 8 rows 1024 bytes apart): lbo unused, sbo = 1024.  MN-major operand (V: a key's row holds 64 values of the
-// head, 8 keys make a 1024-byte swizzle atom): lbo = distance between the two halves of the head, sbo = 1024
-// = the next 8 keys.  Addresses and offsets in units of 16 bytes.
-__device__ __forceinline__ unsigned long long at_desc(unsigned addr, unsigned lbo_bytes, unsigned sbo_bytes) {
-    unsigned long long d = 0;
-    d |= (unsigned long long) ((addr & 0x3FFFF) >> 4);
-    d |= (unsigned long long) ((lbo_bytes >> 4) & 0x3FFF) << 16;
-    d |= (unsigned long long) ((sbo_bytes >> 4) & 0x3FFF) << 32;
-    d |= (unsigned long long) 1 << 46;
-    d |= (unsigned long long) 2 << 61;
-    return d;
-}
-// bf16 x bf16 -> f32, M x N tile; b_mn: the B operand is MN-major (else both are K-major)
-__host__ __device__ constexpr unsigned at_idesc(int m, int n, bool b_mn) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn ? (1u << 16) : 0u) | ((unsigned) (n >> 3) << 17) | ((unsigned) (m >> 4) << 24);
-}
 
 // t = s (c0 + c1 s^2 + ...) for one score
 template <int N> __device__ __forceinline__ float at_cap_one(float s, const float * c) {
@@ -257,83 +131,6 @@ template <int N> __device__ __forceinline__ void at_capped_row(unsigned * v, con
     }
 }
 
-// Which request and row tile the `unit`-th CTA of a KV head works on: the row tiles of all requests in falling order of the keys they
-// see, so that the longest walks start first and the short ones fill the gaps at the end (in the order of the grid the longest tiles of
-// the last request or head began when the GPU was already running empty).  A row tile of `rows` rows sees ceil((pos0 + last token + 1)
-// / AT_BN) key tiles, which grows with its number; the number of row tiles of a request that see L key tiles or more is a closed
-// form, and a warp finds the L of the unit by bisection over L with its lanes over the requests.  Every warp asks for itself.
-__device__ __forceinline__ bool at_row_tile(const TcAttnParams & p, int G, int rows, int unit, int & s, int & tile) {
-    if (p.num_seqs == 1) {
-        s = 0;
-        tile = ((p.cu_q[1] - p.cu_q[0]) * G + rows - 1) / rows - 1 - unit;
-        return tile >= 0;
-    }
-    const int lane = threadIdx.x & 31;
-    auto request = [&](int i, int & q_len, int & pos0) {
-        q_len = p.cu_q[i + 1] - p.cu_q[i];
-        pos0 = p.ctx_len[i] - q_len;
-    };
-    auto tiles_from = [&](int q_len, int pos0, int L) {      // row tiles of a request that see L key tiles or more
-        const int n = (q_len * G + rows - 1) / rows, x = (L - 1) * AT_BN - pos0;
-        if (x <= 0) return n;
-        if (x > q_len - 1) return 0;
-        return n - min((x * G + rows) / rows - 1, n - 1);    // the first of them holds row x * G
-    };
-    int q_len0 = 0, pos00 = 0, most = 0;                     // the lane's first request, kept
-    if (lane < p.num_seqs) request(lane, q_len0, pos00);
-    for (int i = lane; i < p.num_seqs; i += 32) {
-        int q_len = q_len0, pos0 = pos00;
-        if (i >= 32) request(i, q_len, pos0);
-        most = max(most, q_len > 0 ? pos0 + q_len : 0);
-    }
-    most = __reduce_max_sync(0xffffffffu, most);
-    auto count = [&](int L) {
-        int c = 0;
-        for (int i = lane; i < p.num_seqs; i += 32) {
-            int q_len = q_len0, pos0 = pos00;
-            if (i >= 32) request(i, q_len, pos0);
-            c += tiles_from(q_len, pos0, L);
-        }
-        return __reduce_add_sync(0xffffffffu, c);
-    };
-    if (count(1) <= unit) return false;
-    int lo = 1, hi = (most + AT_BN - 1) / AT_BN + 1, above = 0;        // count(lo) > unit >= count(hi) = above
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1, c = count(mid);
-        if (c > unit) lo = mid;
-        else { hi = mid; above = c; }
-    }
-    int rest = unit - above;                                 // among the row tiles that see exactly lo key tiles, request by request
-    for (int base = 0; base < p.num_seqs; base += 32) {
-        const int i = base + lane;
-        int q_len = q_len0, pos0 = pos00;
-        if (base > 0 && i < p.num_seqs) request(i, q_len, pos0);
-        const int more = i < p.num_seqs ? tiles_from(q_len, pos0, lo + 1) : 0, c = i < p.num_seqs ? tiles_from(q_len, pos0, lo) - more : 0;
-        int upto = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, upto, o);
-            if (lane >= o) upto += v;
-        }
-        const unsigned here = __ballot_sync(0xffffffffu, upto > rest);
-        if (here != 0) {
-            const int l = __ffs(here) - 1;
-            s = base + l;
-            const int n = (q_len * G + rows - 1) / rows;
-            tile = __shfl_sync(0xffffffffu, n - 1 - more - (rest - (upto - c)), l);
-            return true;
-        }
-        rest -= __shfl_sync(0xffffffffu, upto, 31);
-    }
-    return false;
-}
-
-// CTAs for the row tiles of a step: no request has more than ceil(max_rows / rows), all together not more than N G / rows + S.
-static inline unsigned at_grid(int N, int S, int max_q_len, int nh, int nkv, int rows) {
-    const long long G = nh / nkv, each = (max_q_len * G + rows - 1) / rows * S, all = (long long) N * G / rows + S;
-    return (unsigned) ((each < all ? each : all) * nkv);
-}
-
 template <int FORM>
 __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
     const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const TcAttnParams p) {
@@ -350,7 +147,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = p.nh / p.nkv;
     int s, row_tile;
-    if (!at_row_tile(p, G, CTA_ROWS, (int) blockIdx.x / p.nkv, s, row_tile)) return;
+    if (!at_row_tile<AT_BN>(p.cu_q, p.ctx_len, p.num_seqs, G, CTA_ROWS, (int) blockIdx.x / p.nkv, s, row_tile)) return;
     const int kvh = (int) blockIdx.x % p.nkv;
     const int q0 = p.cu_q[s];
     const int q_len = p.cu_q[s + 1] - q0;
@@ -819,21 +616,6 @@ done:
         at_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }
-}
-
-typedef CUresult (*AtEncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                               const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static AtEncodeFn at_encode_fn() {
-    static AtEncodeFn fn = nullptr;
-    if (fn == nullptr) {
-        void * p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-            fn = (AtEncodeFn) p;
-    }
-    return fn;
 }
 
 // a cache [num_pages, nkv, page_size, 128] bf16; boxes of one page and half a head: [page_size rows, 64 values]

@@ -30,11 +30,13 @@ SHARED_HEADERS = ["common.cuh"]
 # further headers that some sources share
 SOURCE_HEADERS: Dict[str, List[str]] = {"attention_mma": ["paged_mma.cuh"], "difference_attention_mma": ["paged_mma.cuh"],
                                          "moe": ["gated.cuh"], "postnorm": ["gated.cuh"], "gemm_stream": ["gated.cuh"],
-                                         "gemm_tcgen05": ["gated.cuh"]}
+                                         "gemm_tcgen05": ["gated.cuh"], "attention_tc": ["tc_attention.cuh"],
+                                         "latent_attention_tc": ["tc_attention.cuh", "latent_merge.cuh"],
+                                         "latent_attention_mma": ["latent_merge.cuh"]}
 
 # every library of the engine; build_all() compiles them all
 SOURCES = ["elementwise", "rope_kv", "attention_generic", "gemm_simt", "sampling", "gemm_skinny", "attention_mma", "prefetch", "gemm_tcgen05",
-           "attention_tc", "gemm_stream", "postnorm", "latent_attention", "moe", "latent_attention_mma",
+           "attention_tc", "gemm_stream", "postnorm", "latent_attention", "moe", "latent_attention_mma", "latent_attention_tc",
            "stream_ops", "shared_kv", "matrix_memory", "residual_ops", "chunked_attention", "delta_rule", "window_attention",
            "decay_scan", "tanh_norm", "difference_attention", "difference_attention_mma"]
 # libraries only the bfloat16 serving path uses

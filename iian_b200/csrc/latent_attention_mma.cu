@@ -16,6 +16,7 @@
 // The keys may be cut into parts (gridDim.z, up to 32) for steps with few rows; a part leaves unnormalised sums with
 // its maximum and denominator in scratch memory and a second kernel merges them.
 #include "common.cuh"
+#include "latent_merge.cuh"
 
 namespace iian {
 
@@ -50,11 +51,6 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], 
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-__device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<unsigned *>(&v);
-}
-
 // NT: n8 tiles of the output a warp owns (rank = 32 * NT); MT: m16 tiles of rows; KEYS: keys per tile (32 or 64).
 // q: [N, H, width]; cache: [num_pages * page_size, width]; out: [N, H, rank].
 // With gridDim.z > 1: part_o [N * H, parts, rank] f32 (unnormalised), part_ml [N * H, parts, 2] (maximum, denominator).
@@ -301,44 +297,6 @@ __global__ void __launch_bounds__(kWarps * 32) latent_attention_mma_kernel(
         }
 }
 
-// out[row] = sum_z o_z exp(m_z - m) / sum_z l_z exp(m_z - m),  z ascending
-__global__ void latent_merge_kernel(const float * __restrict__ part_o, const float * __restrict__ part_ml,
-                                    __nv_bfloat16 * __restrict__ out, const int * __restrict__ seq_of_token, int H, int parts,
-                                    int rank) {
-    pdl_wait();
-    pdl_launch_dependents();
-    __shared__ float wz[64];                  // the weight of every part: exp(m_z - m) / l
-    const size_t row = blockIdx.x;
-    if (seq_of_token[row / H] < 0) {
-        for (int c = threadIdx.x; c < rank; c += blockDim.x) out[row * rank + c] = __float2bfloat16_rn(0.0f);
-        return;
-    }
-    if (threadIdx.x < 32) {
-        const int z = threadIdx.x;
-        const float mz = z < parts ? part_ml[(row * parts + z) * 2] : -INFINITY;
-        const float lz = z < parts ? part_ml[(row * parts + z) * 2 + 1] : 0.0f;
-        const float m = warp_max(mz);
-        const float e = mz == -INFINITY ? 0.0f : __expf(mz - m);
-        float l = lz * e;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {     // in the order of the parts: a prefix-style sum keeps z ascending pairs together
-            l += __shfl_xor_sync(0xffffffffu, l, o);
-        }
-        wz[z] = l > 0.0f ? e / l : 0.0f;
-    }
-    __syncthreads();
-    const float * po = part_o + row * parts * rank;
-    for (int c = threadIdx.x * 2; c < rank; c += blockDim.x * 2) {
-        float a0 = 0.0f, a1 = 0.0f;
-        for (int z = 0; z < parts; z++) {
-            const float2 v = *reinterpret_cast<const float2 *>(po + (size_t) z * rank + c);
-            a0 = fmaf(v.x, wz[z], a0);
-            a1 = fmaf(v.y, wz[z], a1);
-        }
-        *reinterpret_cast<unsigned *>(out + row * rank + c) = pack_bf16(a0, a1);
-    }
-}
-
 }  // namespace iian
 
 using namespace iian;
@@ -420,6 +378,5 @@ IIAN_API int iian_latent_attention_mma(const void * q, const void * cache, void 
     else IIAN_LAT(16);
 #undef IIAN_LAT
     if (code != IIAN_OK || parts == 1) return code;
-    return iian_launch(latent_merge_kernel, dim3((unsigned) ((size_t) N * H)), dim3(rank >= 256 ? 128 : 64), 0, stream,
-                       (const float *) part_o, (const float *) part_ml, (__nv_bfloat16 *) out, seq_of_token, H, parts, rank);
+    return latent_merge(part_o, part_ml, out, seq_of_token, N, H, parts, rank, stream);
 }

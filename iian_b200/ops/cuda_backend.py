@@ -1125,6 +1125,65 @@ class CudaKernels:
         if parts > 1:
             LAUNCHES[0] += 1
 
+    # portions of prompts on tcgen05 (csrc/latent_attention_tc.cu): bfloat16, rank 256 / 512, rows of up to 576 values in chunks of 64
+    LATENT_TC = os.environ.get("IIAN_LATENT_TC", "1") not in ("0", "false", "off")
+    # (row, key) pairs of a step, times the shares of the rank, from which it is used: 48 tokens of 16 heads behind 600 cached ones take 23 us
+    # for 25 on mma.sync, 32 of them 24 for 21, 16 behind 4,000 25 for 38; rank 256: 64 behind 600 22 for 19, 128 of them 23 for 28
+    LATENT_TC_MIN_PAIRS = 900_000
+
+    def latent_attention_tc_ok(self, q_cat: torch.Tensor, cache_rows: torch.Tensor, rank: int, scale: float) -> bool:
+        """Whether the tcgen05 kernel takes these operands at all."""
+        n, h, width = q_cat.shape
+        if not (self.LATENT_MMA and self.LATENT_TC) or not scale > 0 or q_cat.dtype != torch.bfloat16 or cache_rows.dtype != torch.bfloat16 \
+                or n * h < 128:
+            return False
+        fn = _fn("latent_attention_tc", "iian_latent_attention_tc_ok", [c_int, c_int, c_int, c_int])
+        return fn(rank, width, h, cache_rows.shape[1]) == 0
+
+    def latent_attention_tc_parts(self, n: int, num_seqs: int, max_q_len: int, num_heads: int, rank: int, max_ctx: int,
+                                  window: Optional[int]) -> int:
+        """Into how many parts the tcgen05 kernel cuts the keys of a step, 0 where the mma.sync kernel is the better one."""
+        shares = max(1, rank // 256)
+        keys = min(max_ctx, window + max_q_len) if window else max_ctx
+        if max_q_len == 1 or n * num_heads * shares * keys < self.LATENT_TC_MIN_PAIRS:
+            return 0
+        # row tiles of 128 (token, head) rows the step has at most; single tokens beside short portions leave most of one empty: 240 of
+        # them behind 1,000 cached tokens 172 us for 151 on mma.sync
+        units = min(num_seqs * -(-max_q_len * num_heads // 128), n * num_heads // 128 + num_seqs)
+        if units * shares > 3 * self.sm_count() and n * num_heads < 32 * units:
+            return 0
+        # as many as fill the GPU once (a second wave costs more than the cut gives: 200 tokens behind 4,000 cached take 79 us in two
+        # parts, 113 in three); a part keeps at least two tiles of keys
+        return max(1, min(self.sm_count() // (units * shares), (-(-keys // 64) + 1) // 2, 32))
+
+    def latent_attention_tc(self, q_cat: torch.Tensor, cache_rows: torch.Tensor, out: torch.Tensor, sink: Optional[torch.Tensor],
+                            meta, *, num_heads: int, rank: int, scale: float, window: Optional[int],
+                            parts: Optional[int] = None) -> None:
+        n, h, width = q_cat.shape
+        if h != num_heads or cache_rows.shape[-1] != width or out.shape != (n, h, rank) or q_cat.dtype != torch.bfloat16 \
+                or cache_rows.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or (sink is not None and sink.numel() != h):
+            raise KernelError(f"latent_attention_tc: q {tuple(q_cat.shape)}, cache {tuple(cache_rows.shape)}, out {tuple(out.shape)} do not fit")
+        status = self.tcgen05_status_buffer(q_cat.device)
+        CudaKernels._tc_used = True
+        if parts is None:
+            parts = max(1, self.latent_attention_tc_parts(n, meta.num_seqs, meta.max_q_len, h, rank, meta.max_ctx, window))
+        part_o = part_ml = 0
+        if parts > 1:
+            scratch = self.attention_scratch(q_cat.device, n * h * parts * (rank + 2))
+            part_o = scratch.data_ptr()
+            part_ml = part_o + n * h * parts * rank * 4
+        bt = meta.block_table
+        fn = _fn("latent_attention_tc", "iian_latent_attention_tc",
+                 [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                  c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_void_p])
+        _check(fn(_cuda(q_cat, "q_cat"), _cuda(cache_rows, "latent cache"), _cuda(out, "attention out"), part_o, part_ml,
+                  _cuda(sink, "sink", torch.float32), _cuda(meta.cu_q, "cu_q", torch.int32), _cuda(meta.ctx_len, "ctx_len", torch.int32),
+                  _cuda(meta.seq_of_token, "seq_of_token", torch.int32), _cuda(bt, "block table", torch.int32), bt.shape[1], n,
+                  meta.num_seqs, meta.max_q_len, h, rank, width, cache_rows.shape[1], cache_rows.shape[0], scale, window or 0, parts,
+                  status.data_ptr(), _stream()), "latent_attention_tc")
+        if parts > 1:
+            LAUNCHES[0] += 1
+
     # ---- routed experts (csrc/moe.cu) -----------------------------------------------------------------------------
     _moe_tile_rows = None
 

@@ -115,7 +115,7 @@ class LatentAttention(Mixer):
         return RowNeed(self.width, int(self.window) if self.window is not None else None)
 
     def kernel_libraries(self):
-        return ("latent_attention", "gemm_simt") + (("latent_attention_mma",) if self.dtype == torch.bfloat16 else ()) \
+        return ("latent_attention", "gemm_simt") + (("latent_attention_mma", "latent_attention_tc") if self.dtype == torch.bfloat16 else ()) \
             + (("residual_ops",) if self.q_rank is not None else ()) + (("stream_ops",) if self.has_gate else ())
 
     def graph_plan(self, num_seqs: int, max_ctx: int):
@@ -154,7 +154,13 @@ class LatentAttention(Mixer):
         k.head_linear(qd if queries is None else queries, 0, self.dim + self.rot, self.w_uk, self.dim * self.rank, self.rank, 1,
                       q_cat.view(n, self.nh * self.width), 0, self.width, num_heads=self.nh, n_in=self.dim, n_out=self.rank)
         lat = ctx.buf("latent_ctx", (n, self.nh, self.rank), self.dtype)
-        if hasattr(k, "latent_attention_mma_ok") and k.latent_attention_mma_ok(q_cat, cache.rows, self.rank):
+        tc = 0
+        if hasattr(k, "latent_attention_tc_ok") and k.latent_attention_tc_ok(q_cat, cache.rows, self.rank, self.scale):
+            tc = k.latent_attention_tc_parts(n, meta.num_seqs, meta.max_q_len, self.nh, self.rank, meta.max_ctx, self.window)
+        if tc:
+            k.latent_attention_tc(q_cat, cache.rows, lat, self.sink, meta, num_heads=self.nh, rank=self.rank, scale=self.scale,
+                                  window=self.window, parts=tc)
+        elif hasattr(k, "latent_attention_mma_ok") and k.latent_attention_mma_ok(q_cat, cache.rows, self.rank):
             plan = ctx.graph_plan(self)
             k.latent_attention_mma(q_cat, cache.rows, lat, self.sink, meta, num_heads=self.nh, rank=self.rank, scale=self.scale,
                                    window=self.window, parts=plan["parts"] if plan else None)

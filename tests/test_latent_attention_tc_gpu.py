@@ -1,0 +1,53 @@
+"""Attention over a cached latent for portions of prompts on tcgen05 against float64: row tiles that end inside a request, key tiles that
+end inside a page, windows, both ranks, widths with and without chunks outside the values; what lies in the cache behind the newest key (here
+NaN) must not reach the output."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from iian_b200.ops.cuda_backend import CudaKernels
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rank,rot,heads,page", [(512, 64, 16, 16), (512, 64, 5, 64), (512, 0, 16, 8), (256, 64, 3, 32), (256, 0, 128, 16)])
+@pytest.mark.parametrize("cached,news,window", [([0], [64], 0), ([0, 70, 5], [130, 33, 1], 0), ([200, 63, 0], [65, 64, 63], 50),
+                                                ([17] * 40, [1 + i % 9 for i in range(40)], 0), ([100 + 61 * i for i in range(50)], [1] * 50, 0)])
+def test_portions_against_float64(rank, rot, heads, page, cached, news, window):
+    g = torch.Generator("cuda").manual_seed(rank + heads + len(news))
+    width, n = rank + rot, sum(news)
+    blocks = [-(-(c + m) // page) for c, m in zip(cached, news)]
+    order = torch.randperm(sum(blocks) + 1, generator=torch.Generator().manual_seed(7)).tolist()
+    rows = torch.full((sum(blocks) + 1, page, width), float("nan"), device="cuda", dtype=torch.bfloat16)
+    bt = torch.full((len(news), max(blocks)), -1, dtype=torch.int32)
+    q = (2 * torch.randn(n, heads, width, device="cuda", generator=g)).bfloat16()
+    sink = torch.randn(heads, device="cuda", generator=g)
+    scale, cu, want, bound = width ** -0.5, [0], [], []
+    for i, (c, m) in enumerate(zip(cached, news)):
+        keys = torch.randn(c + m, width, device="cuda", generator=g).bfloat16()
+        for b in range(blocks[i]):
+            bt[i, b] = order.pop()
+            part = keys[b * page: (b + 1) * page]
+            rows[int(bt[i, b]), : len(part)] = part
+        pos, j = torch.arange(c, c + m, device="cuda")[:, None], torch.arange(c + m, device="cuda")[None]
+        hidden = (j > pos) | (pos - j >= window if window else False)
+        z = torch.einsum("thw,kw->thk", q[cu[-1]: cu[-1] + m].double(), keys.double()) * scale
+        z = torch.cat([z.masked_fill(hidden[:, None], float("-inf")), sink.double()[None, :, None].expand(m, -1, 1)], 2)
+        p = torch.softmax(z, 2)[..., :-1]
+        want.append(p @ keys[:, :rank].double())
+        bound.append(p @ keys[:, :rank].double().abs())
+        cu.append(cu[-1] + m)
+    cuda = lambda x: torch.as_tensor(x, dtype=torch.int32).cuda()
+    meta = SimpleNamespace(cu_q=cuda(cu), ctx_len=cuda([c + m for c, m in zip(cached, news)]), block_table=bt.cuda(), num_seqs=len(news),
+                           max_q_len=max(news), seq_of_token=cuda([i for i, m in enumerate(news) for _ in range(m)]))
+    K, outs = CudaKernels(), []
+    for parts in (1, 2, 5):                    # the keys whole and cut; parts without keys among them
+        outs.append(torch.full((n, heads, rank), 7.0, device="cuda", dtype=torch.bfloat16))
+        K.latent_attention_tc(q, rows, outs[-1], sink, meta, num_heads=heads, rank=rank, scale=scale, window=window or None, parts=parts)
+        K.tcgen05_check(q.device)
+    # the weights and the result are rounded to bfloat16, whose significand has 8 bits: by 2^-8 of each term and 2^-8 of the sum at most;
+    # the scores are 32-bit sums of up to 576 products whose exponentials are off by 1e-4 at most
+    want, bound = torch.cat(want), torch.cat(bound)
+    for out in outs:
+        assert bool(((out.double() - want).abs() <= (2.0 ** -7 + 2e-4) * bound).all())
