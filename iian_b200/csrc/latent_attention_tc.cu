@@ -1,4 +1,5 @@
-// Attention over a cached low-rank latent for portions of prompts (bfloat16) on the fifth-generation tensor cores.
+// Attention over a cached low-rank latent (bfloat16) on the fifth-generation tensor cores: portions of prompts, and decoded tokens of
+// models with many heads.
 //
 // As in latent_attention_mma.cu the rows of a product are (token, head) pairs: all heads of a token score the same cached rows
 // (c_j, kr_j), and the values are the front of those rows.  Neighbouring rows of a request are neighbouring rows of q, so a CTA's 128 rows

@@ -1125,7 +1125,7 @@ class CudaKernels:
         if parts > 1:
             LAUNCHES[0] += 1
 
-    # portions of prompts on tcgen05 (csrc/latent_attention_tc.cu): bfloat16, rank 256 / 512, rows of up to 576 values in chunks of 64
+    # portions of prompts and, from 32 heads on, decoded tokens on tcgen05 (csrc/latent_attention_tc.cu): bfloat16, rank 256 / 512, rows of up to 576 values in chunks of 64
     LATENT_TC = os.environ.get("IIAN_LATENT_TC", "1") not in ("0", "false", "off")
     # (row, key) pairs of a step, times the shares of the rank, from which it is used: 48 tokens of 16 heads behind 600 cached ones take 23 us
     # for 25 on mma.sync, 32 of them 24 for 21, 16 behind 4,000 25 for 38; rank 256: 64 behind 600 22 for 19, 128 of them 23 for 28
@@ -1143,9 +1143,13 @@ class CudaKernels:
     def latent_attention_tc_parts(self, n: int, num_seqs: int, max_q_len: int, num_heads: int, rank: int, max_ctx: int,
                                   window: Optional[int]) -> int:
         """Into how many parts the tcgen05 kernel cuts the keys of a step, 0 where the mma.sync kernel is the better one."""
+        # decoded tokens: a CTA takes one token's heads, so 16 of them leave too much of a row tile empty (48 tokens behind 800 to 4,000
+        # cached 75 us for 77), 32 do not (64 behind 4,000 125 us for 216, 8 of them 28 for 33; with 128 heads 128 for 821 and 36 for 111)
+        if max_q_len == 1 and num_heads < 32:
+            return 0
         shares = max(1, rank // 256)
         keys = min(max_ctx, window + max_q_len) if window else max_ctx
-        if max_q_len == 1 or n * num_heads * shares * keys < self.LATENT_TC_MIN_PAIRS:
+        if n * num_heads * shares * keys < self.LATENT_TC_MIN_PAIRS:
             return 0
         # row tiles of 128 (token, head) rows the step has at most; single tokens beside short portions leave most of one empty: 240 of
         # them behind 1,000 cached tokens 172 us for 151 on mma.sync

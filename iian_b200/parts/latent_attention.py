@@ -119,11 +119,12 @@ class LatentAttention(Mixer):
             + (("residual_ops",) if self.q_rank is not None else ()) + (("stream_ops",) if self.has_gate else ())
 
     def graph_plan(self, num_seqs: int, max_ctx: int):
-        """The number of key parts of the tensor-core kernel is part of a captured graph (its grid)."""
+        """Which tensor-core kernel runs and its number of key parts are part of a captured graph (its grid)."""
         k = ops.kernels()
         if not hasattr(k, "latent_attention_parts"):
             return None
-        return {"parts": k.latent_attention_parts(num_seqs, 1, self.nh, max_ctx, self.window)}
+        return {"parts": k.latent_attention_parts(num_seqs, 1, self.nh, max_ctx, self.window),
+                "tc": k.latent_attention_tc_parts(num_seqs, num_seqs, 1, self.nh, self.rank, max_ctx, self.window)}
 
     def forward(self, x, ctx, cache, writes_cache: bool, with_extra: bool = False):
         """``x`` [N, hidden] in the activation dtype.  Returns the mixer's output [N, hidden], or with ``with_extra`` the
@@ -154,14 +155,14 @@ class LatentAttention(Mixer):
         k.head_linear(qd if queries is None else queries, 0, self.dim + self.rot, self.w_uk, self.dim * self.rank, self.rank, 1,
                       q_cat.view(n, self.nh * self.width), 0, self.width, num_heads=self.nh, n_in=self.dim, n_out=self.rank)
         lat = ctx.buf("latent_ctx", (n, self.nh, self.rank), self.dtype)
-        tc = 0
-        if hasattr(k, "latent_attention_tc_ok") and k.latent_attention_tc_ok(q_cat, cache.rows, self.rank, self.scale):
-            tc = k.latent_attention_tc_parts(n, meta.num_seqs, meta.max_q_len, self.nh, self.rank, meta.max_ctx, self.window)
-        if tc:
+        plan, tc = ctx.graph_plan(self), 0
+        if hasattr(k, "latent_attention_tc_parts"):
+            tc = plan["tc"] if plan else k.latent_attention_tc_parts(n, meta.num_seqs, meta.max_q_len, self.nh, self.rank, meta.max_ctx,
+                                                                     self.window)
+        if tc and k.latent_attention_tc_ok(q_cat, cache.rows, self.rank, self.scale):
             k.latent_attention_tc(q_cat, cache.rows, lat, self.sink, meta, num_heads=self.nh, rank=self.rank, scale=self.scale,
                                   window=self.window, parts=tc)
         elif hasattr(k, "latent_attention_mma_ok") and k.latent_attention_mma_ok(q_cat, cache.rows, self.rank):
-            plan = ctx.graph_plan(self)
             k.latent_attention_mma(q_cat, cache.rows, lat, self.sink, meta, num_heads=self.nh, rank=self.rank, scale=self.scale,
                                    window=self.window, parts=plan["parts"] if plan else None)
         else:
