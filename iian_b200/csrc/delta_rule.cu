@@ -296,6 +296,8 @@ delta_prep_wide_kernel(const __nv_bfloat16 * __restrict__ proj, long long ld, in
                        float * __restrict__ qn, float * __restrict__ kn, float * __restrict__ vv,
                        float * __restrict__ beta, float * __restrict__ decay, float * __restrict__ qk,
                        int N, int H, int G, int V, float q_scale) {
+    pdl_wait();
+    pdl_launch_dependents();
     constexpr int D = 128, TAPS = 4, AHEAD = 4;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int GD = G * D, HV = H * V, C = 2 * GD + HV, v_units = HV / 128;
