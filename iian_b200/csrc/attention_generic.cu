@@ -203,7 +203,7 @@ paged_attention_tile_kernel(
     }
     unsigned long long acc[8][2];
     float m[8], l[8];
-    int lo[8], hi[8], sq[8];
+    int lo[8], hi[8], tok[8];                          // first and last key; the token, -1: no item
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int item = warp * 8 + i, t = t0 + item / G;
@@ -211,16 +211,16 @@ paged_attention_tile_kernel(
         const float sk = sink != nullptr ? sink[kvh * G + item % G] : -INFINITY;
         m[i] = sk;
         l[i] = sink != nullptr ? 1.0f : 0.0f;
-        sq[i] = real ? seq_of_token[t] : -1;
+        tok[i] = real ? t : -1;
         const int p = real ? positions[t] : -1;
-        hi[i] = real && ctx_len != nullptr ? min(p, ctx_len[sq[i]] - 1) : p;
+        hi[i] = real && ctx_len != nullptr ? min(p, ctx_len[seq_of_token[t]] - 1) : p;
         lo[i] = window > 0 ? max(0, p - window + 1) : 0;
         acc[i][0] = acc[i][1] = 0ull;
     }
     const int pieces = hd / 4;
     int first = t0;
-    while (first < t0 + n_tok) {                       // one request's tokens after the other's
-        const int s = seq_of_token[first];
+    while (first < t0 + n_tok) {                       // run after run of one request's tokens; an item walks the keys in its own run alone
+        const int s = seq_of_token[first], begin = first;
         int end = first, k_lo = 0x7fffffff, k_hi = -1;
         for (; end < t0 + n_tok && seq_of_token[end] == s; end++) {
             const int p = positions[end];
@@ -263,7 +263,7 @@ paged_attention_tile_kernel(
             const int j = kb + lane;
             bool any = false;
 #pragma unroll
-            for (int i = 0; i < 8; i++) any |= sq[i] == s && kb <= hi[i] && kb + 31 >= lo[i];
+            for (int i = 0; i < 8; i++) any |= tok[i] >= begin && tok[i] < end && kb <= hi[i] && kb + 31 >= lo[i];
             if (any) {                                 // the same for all lanes: an item's numbers are the warp's
                 unsigned long long dot[4] = {0ull, 0ull, 0ull, 0ull};
                 const float * kr = ks + lane * kTileLd;
@@ -286,7 +286,7 @@ paged_attention_tile_kernel(
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
                     const float2 two = ag_halves(dot[i >> 1]);
-                    const bool valid = here && sq[i] == s && j >= lo[i] && j <= hi[i];
+                    const bool valid = here && tok[i] >= begin && tok[i] < end && j >= lo[i] && j <= hi[i];
                     const float sc = valid ? ((i & 1) ? two.y : two.x) * scale : -INFINITY;
                     const float tile_max = warp_max(sc);
                     float pj = 0.0f;

@@ -605,3 +605,29 @@ def test_paged_attention_generic_bits_do_not_depend_on_the_neighbours(nh, nkv, h
         one = torch.empty(1, nh * hd).cuda()
         run(q[t:t + 1].contiguous(), One, one)
         assert torch.equal(one[0], out[t]), t
+
+
+@pytest.mark.parametrize("G", [1, 2])
+@pytest.mark.parametrize("runs", [[(0, 3), (1, 2), (0, 4)], [(1, 2), (0, 5), (1, 6), (0, 1)]])
+def test_paged_attention_generic_takes_a_requests_tokens_in_several_runs(G, runs):
+    """Tokens of two requests in turns, as nothing in the op's interface forbids: every token as when it is alone, bit for bit."""
+    nkv, hd, lens = 2, 64, [40, 70]
+    q, kc, vc, m, _, scale = attention_case(torch.float32, nkv * G, nkv, hd, 16, lens, [sum(n for s, n in runs if s == i) for i in (0, 1)], 0,
+                                            seed=12, standout=None)
+    begin, order = [0, sum(n for s, n in runs if s == 0)], []
+    for s, n in runs:
+        order += range(begin[s], begin[s] + n)
+        begin[s] += n
+    at = torch.tensor(order, device="cuda")
+
+    class Turns:
+        positions, seq_of_token, block_table, ctx_len = m.positions[at], m.seq_of_token[at], m.block_table, m.ctx_len
+    out = torch.full((len(order), nkv * G * hd), float("nan")).cuda()
+    call = lambda q_, m_, o: K().paged_attention_generic(q_, kc, vc, o, m_, num_heads=nkv * G, num_kv_heads=nkv, head_dim=hd, scale=scale, window=0)
+    call(q[at].contiguous(), Turns, out)
+    for i, t in enumerate(order):
+        class One:
+            positions, seq_of_token, block_table, ctx_len = m.positions[t:t + 1], m.seq_of_token[t:t + 1], m.block_table, m.ctx_len
+        one = torch.empty(1, nkv * G * hd).cuda()
+        call(q[t:t + 1].contiguous(), One, one)
+        assert torch.equal(one[0], out[i]), (i, t)
