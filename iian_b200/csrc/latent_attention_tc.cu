@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(
     const int q0 = p.cu_q[s], q_len = p.cu_q[s + 1] - q0, ctx = p.ctx_len[s], pos0 = ctx - q_len;
     const int rows_total = q_len * H, row0 = row_tile * LT_ROWS;
     const int k_lo = p.window > 0 ? max(0, pos0 + row0 / H - p.window + 1) : 0;
-    const int k_hi = pos0 + min(rows_total - 1, row0 + LT_ROWS - 1) / H;
+    const int k_hi = max(-1, pos0 + min(rows_total - 1, row0 + LT_ROWS - 1) / H);      // -1: rows without a key, one tile with nothing in it
     int tile_lo = k_lo / LT_KEYS, n_tiles = k_hi / LT_KEYS - tile_lo + 1;
     const int parts = (int) gridDim.y;
     if (parts > 1) {

@@ -51,3 +51,29 @@ def test_portions_against_float64(rank, rot, heads, page, cached, news, window):
     want, bound = torch.cat(want), torch.cat(bound)
     for out in outs:
         assert bool(((out.double() - want).abs() <= (2.0 ** -7 + 2e-4) * bound).all())
+
+
+@pytest.mark.parametrize("rank,rot,heads", [(512, 64, 16), (256, 0, 16), (256, 64, 3)])
+@pytest.mark.parametrize("parts", [1, 3])
+def test_tokens_without_a_key_give_zeros(rank, rot, heads, parts):
+    """Long portions of requests that have no context, or less than they have tokens: rows before the first key are zeros, as the other kernel
+    writes them; the rest sees what there is."""
+    g = torch.Generator("cuda").manual_seed(rank + heads)
+    width, page, news, ctx = rank + rot, 16, [100, 90, 130, 1], [0, 33, 0, 0]
+    n = sum(news)
+    rows = torch.randn(3, page, width, device="cuda", generator=g).bfloat16()
+    q = torch.randn(n, heads, width, device="cuda", generator=g).bfloat16()
+    sink = torch.randn(heads, device="cuda", generator=g)
+    cuda = lambda x: torch.as_tensor(x, dtype=torch.int32).cuda()
+    meta = SimpleNamespace(cu_q=cuda([0, 100, 190, 320, 321]), ctx_len=cuda(ctx), block_table=cuda([[-1] * 3, [0, 1, 2], [-1] * 3, [-1] * 3]), num_seqs=4,
+                           max_q_len=130, max_ctx=130, seq_of_token=cuda([i for i, m in enumerate(news) for _ in range(m)]))
+    K, out = CudaKernels(), torch.full((n, heads, rank), 7.0, device="cuda", dtype=torch.bfloat16)
+    K.latent_attention_tc(q, rows, out, sink, meta, num_heads=heads, rank=rank, scale=width ** -0.5, window=None, parts=parts)
+    K.tcgen05_check(q.device)
+    assert not out[:157].any() and not out[190:].any()              # the second request's first 57 tokens lie before its first key
+    keys = rows.view(-1, width)[:33].double()
+    z = torch.einsum("thw,kw->thk", q[157:190].double(), keys) * width ** -0.5
+    z = z.masked_fill(torch.arange(33, device="cuda")[None, None] > torch.arange(33, device="cuda")[:, None, None], float("-inf"))
+    p = torch.softmax(torch.cat([z, sink.double()[None, :, None].expand(33, -1, 1)], 2), 2)[..., :-1]
+    # as above
+    assert bool(((out[157:190].double() - p @ keys[:, :rank]).abs() <= (2.0 ** -7 + 2e-4) * (p @ keys[:, :rank].abs())).all())
