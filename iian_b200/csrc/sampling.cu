@@ -161,7 +161,8 @@ constexpr int kDrawCluster = 8;                  // CTAs per row, at most
 constexpr int kStagedMax = 50 * 1024;            // entries of a slice that shared memory holds (200 KB)
 constexpr int kBorders = 7;
 
-__device__ __forceinline__ unsigned draw_key(float z) { return z != z ? 0u : order_key(z); }      // NaN: below every key that is looked at
+// NaN: below every key that is looked at; the two zeros are equal values and get one key
+__device__ __forceinline__ unsigned draw_key(float z) { return z != z ? 0u : order_key(z + 0.0f); }
 __device__ __forceinline__ float key_value(unsigned k) { return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k); }
 
 struct DrawShared {
@@ -384,7 +385,7 @@ __global__ void __launch_bounds__(kDrawThreads) sample_kernel(
         if (rank == 0 && tid == 0) out[row] = imax;
         return;
     }
-    const unsigned top = order_key(best) + 1;    // above every key
+    const unsigned top = draw_key(best) + 1;     // above every key
     // candidates: keys above `cut`, and the first n_tie entries (by id) whose key is `cut`
     unsigned cut = 1u;
     int n_tie = 0x7fffffff;

@@ -55,3 +55,13 @@ def test_rows_without_a_largest_value():
     logits[3, 4500] = -3.0
     s = [(1.0, 5, 0.9, 0.0)] * 4
     assert draw(logits, s, torch.full((4,), 0.5)) == [0, 0, 4999, 4500]
+
+
+@pytest.mark.parametrize("V,low,high", [(3000, 5, 2000), (3000, 2000, 5), (40000, 5, 39990)])
+def test_the_two_zeros_are_one_value(V, low, high):
+    """A largest value held by a -0.0 (at ``low``) and a +0.0 (at ``high``): ties, the lower id first."""
+    logits = torch.full((6, V), -60.0)
+    logits[:, low], logits[:, high] = -0.0, 0.0
+    a, b = sorted((low, high))
+    s = [(1.0, 1, 1.0, 0.0), (1.0, 2, 1.0, 0.0), (1.0, 0, 0.3, 0.0), (1.0, 0, 0.9, 0.0), (1.0, 0, 0.9, 0.0), (0.0, 0, 1.0, 0.0)]
+    assert draw(logits, s, torch.tensor([0.9, 0.9, 0.9, 0.9, 0.1, 0.5])) == [a, b, a, b, a, a]
