@@ -500,6 +500,8 @@ class ModelRunner:
             self._graphs[key] = slot
         ctx = self.build_decode_context(entries, slot)
         slot.graph.replay()
+        if slot.reports:
+            ops.kernels().expect_status()
         self.launches += slot.launches
         self.last_upload_bytes = ctx.upload_bytes
         return slot.logits[:n]
@@ -528,6 +530,12 @@ class ModelRunner:
         # weights.  The step that asked for this graph then runs exactly once, as the first replay: a mixer
         # with state of its own must not see a step twice.
         ctx = self.build_context([], slot)
+        with k.status_use() as seen:
+            self._record(slot, ctx, k)
+        slot.reports = seen.reports
+        return slot
+
+    def _record(self, slot: "_GraphSlot", ctx: StepContext, k) -> None:
         prefetch = self.weight_prefetch and hasattr(k, "weight_log")
         if prefetch:
             k.weight_log = []
@@ -554,7 +562,6 @@ class ModelRunner:
                     k.prefetcher = None
         slot.launches = _launch_count() - before
         slot.graph = graph
-        return slot
 
 
 class _GraphSlot:
@@ -564,6 +571,7 @@ class _GraphSlot:
     staging = pinned = workspace = copy_done = graph = logits = plans = None
     layout = host_ptr = sig = c_caches = c_tokens = c_starts = c_fresh = ctx = None      # kept between steps by build_decode_context
     n_last = -1
+    reports = False                # kernels that write to the status words are among the graph's
 
 
 def _launch_count() -> int:

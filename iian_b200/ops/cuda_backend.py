@@ -9,9 +9,11 @@ mat-vec kernels do not cover).
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
+from types import SimpleNamespace
 from typing import Optional
 
 import torch
@@ -495,13 +497,30 @@ class CudaKernels:
     _tc_status = {}
 
     def tcgen05_status_buffer(self, device) -> torch.Tensor:
+        """Two words in pinned host memory, which kernels write to only when they give up and the host reads without a copy."""
         t = self._tc_status.get(device)
         if t is None:
-            t = torch.zeros(2, dtype=torch.int32, device=device)
+            t = torch.zeros(2, dtype=torch.int32, pin_memory=True)
             self._tc_status[device] = t
         return t
 
     _tc_used = False           # a tcgen05 kernel was launched since the status was last read
+
+    @contextlib.contextmanager
+    def status_use(self):
+        """Yields an object whose ``reports`` says afterwards whether a kernel that writes to the status words ran within: what a captured
+        step has to know, since its replays pass through none of the wrappers below."""
+        was, CudaKernels._tc_used = CudaKernels._tc_used, False
+        seen = SimpleNamespace(reports=False)
+        try:
+            yield seen
+        finally:
+            seen.reports = CudaKernels._tc_used
+            CudaKernels._tc_used = was or seen.reports
+
+    def expect_status(self) -> None:
+        """Such kernels were launched by other means (a replay): the words are read at the next host wait."""
+        CudaKernels._tc_used = True
 
     def check_device_status(self) -> None:
         """Called where the host has just waited for the device anyway (tokens or logits were read): if a tcgen05
@@ -509,10 +528,14 @@ class CudaKernels:
         if not CudaKernels._tc_used:
             return
         for device in list(self._tc_status):
-            self.tcgen05_check(device)
+            self._read_status(device)
 
     def tcgen05_check(self, device) -> None:
         """Synchronise and raise if a tcgen05 kernel gave up waiting (its output would be garbage)."""
+        torch.cuda.synchronize(device)
+        self._read_status(device)
+
+    def _read_status(self, device) -> None:
         CudaKernels._tc_used = False
         t = self._tc_status.get(device)
         if t is None:
