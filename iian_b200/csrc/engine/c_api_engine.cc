@@ -115,6 +115,7 @@ long long iian_runner_get(void * runner, int what) {
         case 0: return r->launches();
         case 1: return r->num_graphs();
         case 2: return r->last_upload_bytes();
+        case 3: return (long long) (uintptr_t) r->status_words();
     }
     return -1;
 }

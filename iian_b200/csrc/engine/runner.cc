@@ -203,7 +203,6 @@ struct NativeRunner::Impl {
     Workspace * cur_ws = nullptr;
     Staging staging;
     int * tc_status = nullptr;
-    bool tc_used = false;
     cublasHandle_t blas = nullptr;
     void * blas_ws = nullptr;
     // scratch of split attention and split products (shared by all launches: the stream orders them)
@@ -308,7 +307,6 @@ struct NativeRunner::Impl {
 
     void plain_stream_product(const void * x, const MatrixDesc & w, void * out, int out_dtype, int n, int epilogue) {
         if (opt.stream_product) {
-            tc_used = true;
             check(k.gemm_stream(x, w.ptr, out, out_dtype, n, w.rows, w.cols, epilogue, nullptr, 0, 0.0f, 0.0f, nullptr, nullptr, nullptr,
                                 tc_status, stream), "gemm_stream");
         } else {
@@ -319,7 +317,6 @@ struct NativeRunner::Impl {
                            float * res, const float * norm_w, float * out_partial) {
         before_stream_product();
         if (opt.stream_product) {
-            tc_used = true;
             check(k.gemm_stream(x, w.ptr, out, out_dtype, n, w.rows, w.cols, epilogue,
                                 scale ? scale->partials : nullptr, scale ? scale->parts : 0,
                                 scale ? 1.0f / (float) scale->width : 0.0f, scale ? scale->eps : 0.0f,
@@ -334,7 +331,6 @@ struct NativeRunner::Impl {
     }
     void gemm_tcgen05(const void * x, const MatrixDesc & w, void * out, int out_dtype, int n, int epilogue, const Rows * scale,
                       float * res, const float * norm_w, float * out_partial) {
-        tc_used = true;
         const int bn = tcgen05_tile(n, w.rows);
         if (scale == nullptr && res == nullptr) {
             check(k.gemm_tcgen05(x, w.ptr, out, out_dtype, n, w.rows, w.cols, epilogue, bn, tc_status, stream), "gemm_tcgen05");
@@ -420,7 +416,6 @@ struct NativeRunner::Impl {
     // them it copies with cp.async.
     int * decode_status() {
         if (!opt.decode_tma) return nullptr;
-        tc_used = true;
         return tc_status;
     }
     void paged_attention(const void * q, const CallDesc & c, const LayerDesc & L, void * out, const StepInts & si) {
@@ -429,7 +424,6 @@ struct NativeRunner::Impl {
         const int mb = si.max_blocks[g];
         const bool pow2_page = ps == 8 || ps == 16 || ps == 32 || ps == 64 || ps == 128;
         if (opt.attention_tc && bf16_mode() && hd == 128 && pow2_page && nkv > 0 && nh % nkv == 0 && si.max_q_len * (nh / nkv) >= 64) {
-            tc_used = true;
             const int Sd = si.decode_seqs;
             if (Sd > 0 && opt.split_mixed && nh / nkv <= 16) {
                 // A mixed step: the single decoded tokens (the first Sd sequences) go to the decode kernel, which reads
@@ -949,8 +943,9 @@ NativeRunner::NativeRunner(const ModelDesc & model, const KernelLibraries & libs
             bind(h, "iian_set_pdl", set_pdl, libs.gemm_stream);
             set_pdl(opt.pdl_stream ? 1 : 0);
         } else if (opt.stream_product) fail("the gemm_stream kernel library is required for bfloat16");
-        cuda_ok(cudaMalloc(reinterpret_cast<void **>(&m.tc_status), 2 * sizeof(int)), "cudaMalloc (status)");
-        cuda_ok(cudaMemset(m.tc_status, 0, 2 * sizeof(int)), "cudaMemset");
+        // pinned host memory: kernels write there only when they give up, and the host looks after every step, replayed or not, without a copy
+        cuda_ok(cudaHostAlloc(reinterpret_cast<void **>(&m.tc_status), 2 * sizeof(int), cudaHostAllocPortable), "cudaHostAlloc (status)");
+        m.tc_status[0] = m.tc_status[1] = 0;
     }
 }
 
@@ -960,7 +955,7 @@ NativeRunner::~NativeRunner() {
     m.graphs.clear();
     if (m.blas) cublasDestroy(m.blas);
     if (m.blas_ws) cudaFree(m.blas_ws);
-    if (m.tc_status) cudaFree(m.tc_status);
+    if (m.tc_status) cudaFreeHost(m.tc_status);
     if (m.attn_scratch) cudaFree(m.attn_scratch);
     if (m.attn_counters) cudaFree(m.attn_counters);
     for (void * p : m.retired_scratch) cudaFree(p);
@@ -988,6 +983,7 @@ int NativeRunner::vocab() const { return impl_->model.vocab; }
 long long NativeRunner::launches() const { return impl_->launches; }
 int NativeRunner::num_graphs() const { return (int) impl_->graphs.size(); }
 int NativeRunner::last_upload_bytes() const { return impl_->last_upload; }
+const int * NativeRunner::status_words() const { return impl_->tc_status; }
 long long NativeRunner::launches_of(const char * entry) const {
     auto it = impl_->by_entry.find(entry);
     return it == impl_->by_entry.end() ? 0 : it->second;
@@ -996,15 +992,11 @@ long long NativeRunner::launches_of(const char * entry) const {
 void NativeRunner::set_cuda_graphs(bool on) { impl_->opt.cuda_graphs = on; }
 
 void NativeRunner::check_status() {
-    Impl & m = *impl_;
-    if (!m.tc_used || m.tc_status == nullptr) return;
-    m.tc_used = false;
-    int host[2] = {0, 0};
-    cuda_ok(cudaMemcpy(host, m.tc_status, sizeof(host), cudaMemcpyDeviceToHost), "cudaMemcpy (status)");
-    if (host[0] != 0) {
-        cudaMemset(m.tc_status, 0, sizeof(host));
-        fail("a kernel gave up waiting on a barrier (wait " + std::to_string(host[0]) + ", iteration " + std::to_string(host[1]) + "); its result is not valid");
-    }
+    volatile int * words = impl_->tc_status;
+    if (words == nullptr || words[0] == 0) return;
+    const int code = words[0], where = words[1];
+    words[0] = words[1] = 0;
+    fail("a kernel gave up waiting on a barrier (wait " + std::to_string(code) + ", iteration " + std::to_string(where) + "); its result is not valid");
 }
 
 }  // namespace iian_b200

@@ -142,7 +142,8 @@ public:
     int num_graphs() const;
     int last_upload_bytes() const;
     long long launches_of(const char * entry) const;    // by entry point ("attention_tc", "library_gemm", ...)
-    void check_status();                    // throws if a tcgen05 kernel gave up on a barrier since the last call
+    void check_status();                    // once a step's results are on the host: throws if one of its kernels gave up on a barrier
+    const int * status_words() const;       // two words in host memory those kernels write to (null: none does)
     void set_cuda_graphs(bool on);          // replay decode-only steps from captured graphs from now on (or stop doing so)
     struct Impl;
 private:

@@ -52,7 +52,7 @@ void iian_runner_delete(void * runner);
 // until the next step (null if nothing is wanted).
 int iian_runner_step(void * runner, void * const * caches, const int32_t * tokens, const int * n_tokens, const int * starts,
                      const int32_t * want, const int * n_want, int n_entries, void * stream, const float ** logits, int * n_rows);
-// what: 0 launches, 1 graphs captured, 2 bytes of the last upload
+// what: 0 launches, 1 graphs captured, 2 bytes of the last upload, 3 address of the status words (0: none)
 long long iian_runner_get(void * runner, int what);
 long long iian_runner_launches_of(void * runner, const char * entry);
 int iian_runner_check_status(void * runner);

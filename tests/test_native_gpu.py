@@ -189,3 +189,24 @@ def test_a_mixed_step_in_any_order_of_its_entries(folders, dtype, monkeypatch):
         assert err <= limit, (dtype, err, where)
     if dtype == "float32":
         assert all(torch.equal(got[0][k], got[1][k]) for k in got[0])
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+def test_a_kernel_that_gave_up_in_a_native_step_is_reported(folders, graphs):
+    """Also in a replayed step: the words such a kernel writes are set by hand behind the step (none is made to give up)."""
+    import ctypes
+    from iian_b200.engine import native
+    from iian_b200.engine.replay import TraceReplayer
+    reqs = requests_for("B", [9, 40], 3)
+    rp = TraceReplayer.from_folder(folders["B"], "bfloat16", 256, BLOCK_SIZE["B"], 4)
+    assert rp.runner.native is not None
+    rp.runner.cuda_graphs = graphs
+    replay_and_collect(rp, trace_tail(reqs, 5))
+    torch.cuda.synchronize()
+    words = (ctypes.c_int * 2).from_address(native.lib().iian_runner_get(rp.runner.native._h, 3))
+    for _ in range(2):
+        rp.runner.check_device_status()                 # a clean run, or one that has been reported
+        words[0], words[1] = 3, 9
+        with pytest.raises(Exception, match="gave up"):
+            rp.runner.check_device_status()
+        assert list(words) == [0, 0]
