@@ -25,15 +25,18 @@ constexpr int kTileItems = 32;      // (token, head) pairs of a CTA of the tiled
 constexpr int kTileRuns = 4;        // requests whose tokens may lie side by side in such a CTA
 constexpr int kTileMinTokens = 8;   // tokens of a step from which the tiled kernel is launched
 
-// Whether the tokens [t0, t0 + tokens) of the step are the tiled kernel's: at most kTileRuns requests, no padding.  Both kernels ask.
-// A whole warp calls it (at most 32 tokens a tile).
+// Whether the tokens [t0, t0 + tokens) of the step are the tiled kernel's: at most kTileRuns runs of a request's tokens, two tokens each on
+// average (a CTA walks the runs one after the other: decoded tokens are better off with a warp for every item side by side) unless they
+// are the end of a longer portion, and no padding.  Both kernels ask.  A whole warp calls it (at most 32 tokens a tile).
 __device__ __forceinline__ bool tile_is_shared(const int * __restrict__ seq_of_token, int t0, int tokens, int N) {
     const int lane = threadIdx.x & 31;
     const bool in = lane < tokens && t0 + lane < N;
     const int s = in ? seq_of_token[t0 + lane] : 0;
     const int before = __shfl_up_sync(0xffffffffu, s, 1);
     const unsigned padding = __ballot_sync(0xffffffffu, in && s < 0), starts = __ballot_sync(0xffffffffu, in && (lane == 0 || s != before));
-    return padding == 0 && __popc(starts) <= kTileRuns;
+    const int runs = __popc(starts), n = min(tokens, N - t0);
+    const int ahead = t0 > 0 ? seq_of_token[t0 - 1] : -1, first = __shfl_sync(0xffffffffu, s, 0);
+    return padding == 0 && runs <= kTileRuns && (n >= 2 * runs || (runs == 1 && ahead == first));
 }
 
 // VEC: rows of keys are whole 16-byte pieces.  NACC: output entries per lane (hd <= 32 * NACC).
@@ -403,7 +406,8 @@ IIAN_API int iian_paged_attention_sink(
                               sink, (const __nv_bfloat16 *) gate, ld_gate, 0, stream);
     if (act_dtype != IIAN_F32) return IIAN_ERR_DTYPE;
     // neighbouring tokens of a request share their key tiles where the sizes allow it; what is left (tokens of many requests side by
-    // side, as when decoding) goes to the kernel with a warp per item, which leaves the others out
+    // side, as when decoding) goes to the kernel with a warp per item, which leaves the others out (8 heads of 64 on one KV head, eight
+    // requests behind 1,500: 244 us, 848 when a tile walks its four requests in turn; 16 on 2 of 128: 734 and 1,027)
     const int group = nh / nkv;
     const uintptr_t all = (uintptr_t) k_cache | (uintptr_t) v_cache | (uintptr_t) out;
     int tile_tokens = 0;
