@@ -115,8 +115,9 @@ __global__ void paged_attention_generic_kernel(
 #pragma unroll
         for (int i = 0; i < NACC; i++) acc[i] *= corr;
         m = m_new;
-        // eight value rows are loaded before the first is added
-        constexpr int AT_ONCE = NACC <= 4 ? 8 : 4;
+        // value rows loaded before the first is added (heads of 160 to 256, 8 bfloat16 tokens behind 1,000: two rows 529 and 696 us, four 921 and
+        // 1,333, eight 919 and 1,324; a row at a time over 16 entries a lane 795 and 1,152)
+        constexpr int AT_ONCE = NACC <= 4 ? 8 : NACC <= 8 ? 2 : 4;
 #pragma unroll
         for (int j0 = 0; j0 < 32; j0 += AT_ONCE) {
             float pr[AT_ONCE], vr[AT_ONCE][NACC];
@@ -379,6 +380,7 @@ static int launch_generic(const A * q, const A * k_cache, const A * v_cache, A *
     auto pick = [&](auto v) {
         if (hd <= 64) go(std::integral_constant<int, 2>(), v);
         else if (hd <= 128) go(std::integral_constant<int, 4>(), v);
+        else if (hd <= 256) go(std::integral_constant<int, 8>(), v);
         else go(std::integral_constant<int, kGenMaxHeadDim / 32>(), v);
     };
     if (vec) pick(std::true_type());
