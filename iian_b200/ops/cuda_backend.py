@@ -1179,6 +1179,12 @@ class CudaKernels:
         units = min(num_seqs * -(-max_q_len * num_heads // 128), n * num_heads // 128 + num_seqs)
         if units * shares > 3 * self.sm_count() and n * num_heads < 32 * units:
             return 0
+        # more CTAs than fit at once with a tile of keys each: setting up and closing a CTA (12 us a round) is most of the time; rank 512, 16
+        # prompts of 30 tokens with 32 heads 27 us for 21 on mma.sync, 60 of 20 with 128 heads 218 for 146, 16 of 60 166 for 144; 4 of 100 82
+        # for 84; rank 256 43 for 36 (16 of 30, 128 heads), but 23 for 26 (16 of 60, 32 heads).  The same with two tiles and a quarter of the
+        # rows in use: 200 portions of 2 tokens behind 100, 16 heads, 30 us for 25
+        if units * shares > self.sm_count() and (keys <= 32 * shares or (keys <= 128 and n * num_heads <= 32 * units)):
+            return 0
         # as many as fill the GPU once (a second wave costs more than the cut gives: 200 tokens behind 4,000 cached take 79 us in two
         # parts, 113 in three); a part keeps at least two tiles of keys
         return max(1, min(self.sm_count() // (units * shares), (-(-keys // 64) + 1) // 2, 32))
