@@ -47,7 +47,8 @@ struct AttnParams {
     const int * slots;              // [N] cache cell of each token (page * page_size + offset), < 0: not stored
     float eps;
     int write_kv;
-    int longest_first = 0;          // decode kernel, unsplit keys: the CTAs take the sequences in falling order of their contexts
+    int longest_first = 0;          // decode kernel, unsplit keys: the CTAs take the sequences in falling order of their contexts where the
+                                    // longest is so many per cent of the mean (0: never)
     int * status;                   // TMA form of the decode kernel: {code, where}, zero before the launch
     // a sink per head: a logit without key and value that joins the softmax's denominator once, not scaled
     const float * sink = nullptr;   // [nh] or null
@@ -398,6 +399,51 @@ __global__ void __launch_bounds__(NW * 32, 3) attention_mma_kernel(const AttnPar
     }
 }
 
+// The sequence of the `place`-th CTA when those of the long contexts go first, to one part in 16 of the longest (ties in their own order): the
+// place-th largest by a bisection over five bits, with the warp's lanes over the sequences (S <= 256).  The order of the batch stays where
+// the longest is not `percent` of the mean: there the last CTAs are not much longer than the first.  Every warp asks for itself.
+__device__ __forceinline__ int longest_first(const int * __restrict__ ctx_len, int S, int place, int percent) {
+    constexpr int HELD = 8;
+    const int lane = threadIdx.x & 31;
+    int v[HELD], most = 0, sum = 0;
+#pragma unroll
+    for (int i = 0; i < HELD; i++) {
+        const int t = lane + 32 * i;
+        v[i] = t < S ? __ldg(ctx_len + t) : -1;
+        most = max(most, v[i]);
+        sum += max(v[i], 0);
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if ((float) most * (float) (100 * S) < (float) percent * (float) sum) return place;
+    const int drop = max(0, 27 - __clz(most));
+#pragma unroll
+    for (int i = 0; i < HELD; i++) v[i] >>= drop;
+    int K = 0;                                   // the largest value that more than `place` contexts reach
+#pragma unroll 1
+    for (int bit = 16; bit > 0; bit >>= 1) {
+        const int trial = K | bit;
+        int c = 0;
+#pragma unroll
+        for (int i = 0; i < HELD; i++)
+            if (32 * i < S) c += __popc(__ballot_sync(0xffffffffu, v[i] >= trial));
+        if (c > place) K = trial;
+    }
+    int rest = place;                            // among the contexts of K
+#pragma unroll
+    for (int i = 0; i < HELD; i++)
+        if (32 * i < S) rest -= __popc(__ballot_sync(0xffffffffu, v[i] > K));
+#pragma unroll
+    for (int i = 0; i < HELD; i++)
+        if (32 * i < S) {
+            const unsigned here = __ballot_sync(0xffffffffu, v[i] == K);
+            const int n = __popc(here);
+            if (rest < n) return 32 * i + __ffs(__ballot_sync(0xffffffffu, v[i] == K && __popc(here & ((1u << lane) - 1u)) == rest)) - 1;
+            rest -= n;
+        }
+    return place;
+}
+
 // Decode form: few rows (the G heads of one token, up to 16 rows per CTA), many keys.  The four warps
 // of a CTA share the rows and split the KEYS of every 64-key tile (16 each); each warp keeps a running
 // (max, sum, output) of its own, and the four are merged through shared memory at the end.  Three
@@ -444,27 +490,13 @@ __global__ void __launch_bounds__(128, STAGES == 2 ? 3 : 2) attention_decode_ker
     const int kvh = blockIdx.y;
     const int split = blockIdx.z % p.n_split;
     int s = blockIdx.z / p.n_split;
+    int q0 = p.cu_q[s], q_end = p.cu_q[s + 1], ctx = p.ctx_len[s];       // (on their way while the ranking waits for its own loads)
     if (p.longest_first) {
-        // the sequences in falling order of their contexts (ties in their own order)
-        __shared__ int ranked;
-        const int S = gridDim.z;
-        for (int t = threadIdx.x; t < S; t += blockDim.x) {
-            const int own = p.ctx_len[t];
-            int rank = 0;
-#pragma unroll 8
-            for (int u = 0; u < S; u++) {
-                const int other = __ldg(p.ctx_len + u);
-                rank += other > own || (other == own && u < t);
-            }
-            if (rank == s) ranked = t;
-        }
-        __syncthreads();
-        s = ranked;
+        const int t = longest_first(p.ctx_len, gridDim.z, s, p.longest_first);
+        if (t != s) { s = t; q0 = p.cu_q[s]; q_end = p.cu_q[s + 1]; ctx = p.ctx_len[s]; }
     }
     const int G = p.nh / p.nkv;
-    const int q0 = p.cu_q[s];
-    const int q_len = p.cu_q[s + 1] - q0;
-    const int ctx = p.ctx_len[s];
+    const int q_len = q_end - q0;
     const int pos0 = ctx - q_len;
     const int rows_total = q_len * G;
     const int row0 = blockIdx.x * BM;
@@ -1040,10 +1072,12 @@ static int launch_decode(const AttnParams & asked, int S, int max_rows, cudaStre
         const long long ctas = (long long) ((max_rows + 15) / 16) * p.nkv * S;
         const long long waves3 = (ctas + 2 * sms - 1) / (2 * sms), waves2 = (ctas + 3 * sms - 1) / (3 * sms);
         deep = g_unsplit_stages != 0 ? g_unsplit_stages == 3 : waves3 * 100 <= waves2 * 115;
-        // With more CTAs than are resident at once those of the long contexts go first (61 requests of 100 to 2,100 tokens, 8 KV heads: 90
-        // us in the order of the batch, 64 so); the ranking costs a CTA about half a microsecond, so a single wave keeps the
-        // order of the batch, and so does a batch too large to be ranked in passing.
-        p.longest_first = ctas > (deep ? 2 : 3) * sms && S <= 256;
+        // With more CTAs than are resident at once those of the long contexts go first.  The less the last ones are of the whole, the more
+        // the contexts have to differ before that pays (32 heads of 128, 8 KV heads; us in the batch's order and ranked: 64 sequences, 1.2 rounds
+        // of CTAs, of 1,000 to 1,333 tokens 74 and 75, to 1,500 80 and 75; 128 of 200 to 800 62 and 63, of 100 to 2,100 118 and 102; 256 105 and 112,
+        // 202 and 194).  A batch too large to be ranked in passing keeps its order.
+        const int slots = (deep ? 2 : 3) * sms;
+        p.longest_first = ctas <= slots || S > 256 ? 0 : ctas * 2 <= 3 * slots ? 118 : 175;
     }
     KvMaps maps = {};
     if constexpr (HD == 128) {
