@@ -59,6 +59,7 @@ struct TcAttnParams {
     const int * ctx_len;            // [S]
     const int * block_table;        // [S, max_blocks]
     int max_blocks, nh, nkv, page_size, num_pages, window, num_seqs;
+    int single;                     // no request has more than one row tile
     float scale_log2;               // scale * log2(e)
     int * status;                   // {code, where}; zero before the launch
     // a sink per head: a logit without key and value that joins the softmax's denominator once, not scaled
@@ -131,6 +132,13 @@ template <int N> __device__ __forceinline__ void at_capped_row(unsigned * v, con
     }
 }
 
+// A step's grid: the KV heads, then the row tiles as `unit` counts them (no division in front of a CTA's first load).
+constexpr int kAtUnits = 32768;
+static inline dim3 at_grid(int N, int S, int max_q_len, int nh, int nkv, int rows) {
+    const long long units = at_units(N, S, max_q_len, nh / nkv, rows);
+    return dim3((unsigned) nkv, (unsigned) (units < kAtUnits ? units : kAtUnits), (unsigned) ((units + kAtUnits - 1) / kAtUnits));
+}
+
 template <int FORM>
 __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
     const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const TcAttnParams p) {
@@ -146,31 +154,31 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = p.nh / p.nkv;
-    int s, row_tile;
-    if (!at_row_tile<AT_BN>(p.cu_q, p.ctx_len, p.num_seqs, G, CTA_ROWS, (int) blockIdx.x / p.nkv, s, row_tile)) return;
-    const int kvh = (int) blockIdx.x % p.nkv;
-    const int q0 = p.cu_q[s];
-    const int q_len = p.cu_q[s + 1] - q0;
-    const int ctx = p.ctx_len[s];
-    const int pos0 = ctx - q_len;
-    const int rows_total = q_len * G;
-    const int row0 = row_tile * CTA_ROWS;
-
-    // two groups of 128 rows (A, B) share every K/V tile; B may be empty, and A may need a tile less than B
-    const bool has_b = DIFF || row0 + AT_BM < rows_total;
-    const int tok_min = row0 / G;
-    const int k_hi_a = pos0 + min(rows_total - 1, row0 + AT_BM - 1) / G;
-    const int k_hi = pos0 + min(rows_total - 1, row0 + CTA_ROWS - 1) / G;
-    const int k_lo = p.window > 0 ? max(0, pos0 + tok_min - p.window + 1)
-                                  : p.chunk > 0 ? (pos0 + tok_min) - (pos0 + tok_min) % p.chunk : 0;
-    const int tile_lo = k_lo / AT_BN, tile_hi = k_hi / AT_BN;
-    const int n_keep = (KEPT && p.keep_first > 0 && p.window > 0) ? min((p.keep_first + AT_BN - 1) / AT_BN, tile_lo) : 0;
-    auto phys = [&](int i) { return KEPT && i < n_keep ? i : tile_lo + i - n_keep; };        // the cache tile of the i-th tile walked
-    const int n_tiles = tile_hi - tile_lo + 1 + n_keep;
-    const int n_grp[2] = {k_hi_a / AT_BN - tile_lo + 1 + n_keep, has_b ? n_tiles : 0};
-    const int * bt = p.block_table + (size_t) s * p.max_blocks;
-    int * status = p.status;
-
+    const int kvh = blockIdx.x;
+    // Which rows are this CTA's.  Where it takes a search (some hundred instructions, which ten warps would issue in half a microsecond) it is
+    // one warp's work, beside the barriers' and tensor memory's set-up.
+    __shared__ AtPlace place;                                // (s < 0: none left)
+    __shared__ int span_s[3];
+    const bool search = p.num_seqs > 1 && p.single == 0;
+    AtPlace at;
+    at.s = -1;
+    int tile_lo = 0, k_hi_a = 0, k_hi = 0;                   // first key tile; last key of the first group of rows, of all
+    if (!search || warp == 2) {
+        const bool mine = at_row_tile<AT_BN>(p.cu_q, p.ctx_len, p.num_seqs, p.single != 0, G, CTA_ROWS, (int) (blockIdx.z * kAtUnits + blockIdx.y), at);
+        if (!mine && !search) return;
+        if (mine) {
+            const int pos0 = at.ctx - at.q_len, row0 = at.tile * CTA_ROWS, last = at.q_len * G - 1, first = pos0 + row0 / G;
+            tile_lo = (p.window > 0 ? max(0, first - p.window + 1) : p.chunk > 0 ? first - first % p.chunk : 0) / AT_BN;
+            k_hi_a = pos0 + min(last, row0 + AT_BM - 1) / G;
+            k_hi = pos0 + min(last, row0 + CTA_ROWS - 1) / G;
+            if (warp == (search ? 2 : 0)) {                  // the producer's first reads of the block table
+                const int j0 = tile_lo * AT_BN + lane * p.page_size;
+                if (lane < AT_BN / p.page_size && j0 <= k_hi)
+                    asm volatile("prefetch.global.L1 [%0];" ::"l"(p.block_table + (size_t) at.s * p.max_blocks + j0 / p.page_size));
+            }
+        } else at.s = -1;
+        if (search && lane == 0) { place = at; span_s[0] = tile_lo; span_s[1] = k_hi_a; span_s[2] = k_hi; }
+    }
     if (threadIdx.x == 0) {
         for (int g = 0; g < 2; g++) {
             at_mbar_init(at_smem(&s_full[g]), 1);
@@ -180,14 +188,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
         }
         at_mbar_init(at_smem(&q_full), AT_THREADS / 32 - 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) {          // the producer's first reads: the descriptors and the block table's first entries
-        if (lane == 0) {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
-        }
-        const int j0 = tile_lo * AT_BN + lane * p.page_size;
-        if (lane < AT_BN / p.page_size && j0 <= k_hi) asm volatile("prefetch.global.L1 [%0];" ::"l"(bt + j0 / p.page_size));
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
     }
     if (warp == 1) {          // tensor memory: S of both groups (2 x 128 columns), O of both groups (2 x 128 columns)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at_smem(&tmem_base_s)), "r"(512u) : "memory");
@@ -197,6 +199,23 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
     __syncthreads();
     at_fence_after();
     const unsigned tmem_base = tmem_base_s;
+    if (search) { at = place; tile_lo = span_s[0]; k_hi_a = span_s[1]; k_hi = span_s[2]; }
+    const int s = at.s, row0 = at.tile * CTA_ROWS, q0 = at.q0, q_len = at.q_len, pos0 = at.ctx - q_len;
+    if (s < 0) {
+        if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+        return;
+    }
+    const int rows_total = q_len * G;
+
+    // two groups of 128 rows (A, B) share every K/V tile; B may be empty, and A may need a tile less than B
+    const bool has_b = DIFF || row0 + AT_BM < rows_total;
+    const int tile_hi = k_hi / AT_BN;
+    const int n_keep = (KEPT && p.keep_first > 0 && p.window > 0) ? min((p.keep_first + AT_BN - 1) / AT_BN, tile_lo) : 0;
+    auto phys = [&](int i) { return KEPT && i < n_keep ? i : tile_lo + i - n_keep; };        // the cache tile of the i-th tile walked
+    const int n_tiles = tile_hi - tile_lo + 1 + n_keep;
+    const int n_grp[2] = {k_hi_a / AT_BN - tile_lo + 1 + n_keep, has_b ? n_tiles : 0};
+    const int * bt = p.block_table + (size_t) s * p.max_blocks;
+    int * status = p.status;
 
     if (warp > 0) {
         // Q rows into the swizzled K-major layout: row r, 16-byte chunk c of half h at h * 16 KB + r * 128 + ((c ^ (r & 7)) << 4).
@@ -754,7 +773,8 @@ IIAN_API int iian_attention_tc_kept(const void * q, long long ld_q, const void *
         if (e != cudaSuccess) return 1000 + (int) e;
         configured[kept ? 1 : 0] = true;
     }
-    const unsigned grid = at_grid(N, S, max_q_len, nh, nkv, AT_ROWS);
+    const dim3 grid = at_grid(N, S, max_q_len, nh, nkv, AT_ROWS);
+    p.single = at_tiles(max_q_len, nh / nkv, AT_ROWS) <= 1;
     if (kept) attention_tc_kernel<AT_KEPT><<<grid, AT_THREADS, smem, stream>>>(mk, mv, p);
     else attention_tc_kernel<AT_PLAIN><<<grid, AT_THREADS, smem, stream>>>(mk, mv, p);
     return iian_launch_status();
@@ -795,7 +815,8 @@ IIAN_API int iian_attention_tc_capped(const void * q, long long ld_q, const void
         if (e != cudaSuccess) return 1000 + (int) e;
         configured = true;
     }
-    const unsigned grid = at_grid(N, S, max_q_len, nh, nkv, AT_ROWS);
+    const dim3 grid = at_grid(N, S, max_q_len, nh, nkv, AT_ROWS);
+    p.single = at_tiles(max_q_len, nh / nkv, AT_ROWS) <= 1;
     attention_tc_kernel<AT_CAP><<<grid, AT_THREADS, smem, stream>>>(mk, mv, p);
     return iian_launch_status();
 }
@@ -832,7 +853,8 @@ IIAN_API int iian_attention_tc_difference(const void * q, const void * k_cache, 
         if (e != cudaSuccess) return 1000 + (int) e;
         configured = true;
     }
-    const unsigned grid = at_grid(N, S, max_q_len, nh, nkv, AT_BM);
+    const dim3 grid = at_grid(N, S, max_q_len, nh, nkv, AT_BM);
+    p.single = at_tiles(max_q_len, nh / nkv, AT_BM) <= 1;
     attention_tc_kernel<AT_DIFF><<<grid, AT_THREADS, smem, stream>>>(mk, mv, p);
     return iian_launch_status();
 }

@@ -47,6 +47,7 @@ struct LatentTcParams {
     const float * sink;             // [H] or null
     int * status;                   // {code, where}; zero before the launch
     int num_seqs, max_blocks, H, rank, width, page_size, num_pages, window;
+    int single;                     // no request has more than one row tile
     float scale, scale_log2, sink_to_raw;
 };
 
@@ -76,12 +77,13 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(
     constexpr int CHUNKS = REST + LT_OWN;
     const int shares = p.rank / LT_SHARE;
     const int H = p.H;
-    int s, row_tile;
-    if (!at_row_tile<LT_KEYS>(p.cu_q, p.ctx_len, p.num_seqs, H, LT_ROWS, (int) blockIdx.x / shares, s, row_tile)) return;
+    AtPlace at;
+    if (!at_row_tile<LT_KEYS>(p.cu_q, p.ctx_len, p.num_seqs, p.single != 0, H, LT_ROWS, (int) blockIdx.x / shares, at)) return;
+    const int s = at.s, row_tile = at.tile;
     const int part = (int) blockIdx.x % shares;                    // this CTA's share of the values: chunks own .. own + LT_OWN - 1
     const int own = part * LT_OWN;
     auto column = [&](int slot) { return (slot >= REST ? own + slot - REST : slot < own ? slot : slot + LT_OWN) * LT_CHUNK; };
-    const int q0 = p.cu_q[s], q_len = p.cu_q[s + 1] - q0, ctx = p.ctx_len[s], pos0 = ctx - q_len;
+    const int q0 = at.q0, q_len = at.q_len, pos0 = at.ctx - q_len;
     const int rows_total = q_len * H, row0 = row_tile * LT_ROWS;
     const int k_lo = p.window > 0 ? max(0, pos0 + row0 / H - p.window + 1) : 0;
     const int k_hi = max(-1, pos0 + min(rows_total - 1, row0 + LT_ROWS - 1) / H);      // -1: rows without a key, one tile with nothing in it
@@ -453,7 +455,8 @@ IIAN_API int iian_latent_attention_tc(const void * q, const void * cache, void *
     p.window = window;
     p.scale_log2 = scale * 1.4426950408889634f;
     p.sink_to_raw = 1.0f / scale;
-    const dim3 grid(at_grid(N, S, max_q_len, H, 1, LT_ROWS) * (unsigned) (rank / LT_SHARE), (unsigned) parts);
+    p.single = at_tiles(max_q_len, H, LT_ROWS) <= 1;
+    const dim3 grid((unsigned) (at_units(N, S, max_q_len, H, LT_ROWS) * (rank / LT_SHARE)), (unsigned) parts);
     int rc2 = IIAN_OK;
     switch (width / LT_CHUNK - LT_OWN) {
         case 0: rc2 = lt_launch<0>(mq, mk, p, grid, stream); break;

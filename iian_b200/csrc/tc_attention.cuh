@@ -135,61 +135,84 @@ __host__ __device__ constexpr unsigned at_idesc(int m, int n, bool b_mn) {
     return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn ? (1u << 16) : 0u) | ((unsigned) (n >> 3) << 17) | ((unsigned) (m >> 4) << 24);
 }
 
+// The row tile a CTA works on: of which request, its number there, and that request's numbers.
+struct AtPlace { int s, tile, q0, q_len, ctx; };
+
 // Which request and row tile the `unit`-th CTA works on: the row tiles of all requests in falling order of the keys they
 // see, so that the longest walks start first and the short ones fill the gaps at the end (in the order of the grid the longest tiles of
-// the last request or head began when the GPU was already running empty: 204 against 156 us for three portions, 1,361 tokens together,
-// behind 200 to 6,000 cached ones, heads of 128).  A row tile of `rows` rows sees ceil((pos0 + last token + 1)
-// / KEYS) key tiles, which grows with its number; the number of row tiles of a request that see L key tiles or more is a closed
-// form, and a warp finds the L of the unit by bisection over L with its lanes over the requests.  Every warp asks for itself.
+// the last request or head began when the GPU was already running empty: 197 against 138 us for three portions, 1,361 tokens together,
+// behind 200 to 6,000 cached ones, heads of 128).  A row tile of `rows` rows sees ceil((pos0 + last token + 1) / KEYS) key tiles, which
+// grows with its number; the number of row tiles of a request that see L key tiles or more is a closed form, and a warp finds the L of the
+// unit by bisection with its lanes over the requests -- to an eighth of the longest walk, which balances as well and takes three
+// steps of some hundred cycles.  `single`: no request has more than one row tile; then the order of the batch, which needs no search, is
+// kept (68 portions of 30 tokens 37.6 us, ranked 41.8).  A whole warp calls it.
 template <int KEYS>
-__device__ __forceinline__ bool at_row_tile(const int * __restrict__ cu_q, const int * __restrict__ ctx_len, int num_seqs, int G, int rows,
-                                            int unit, int & s, int & tile) {
-    if (num_seqs == 1) {
-        s = 0;
-        tile = ((cu_q[1] - cu_q[0]) * G + rows - 1) / rows - 1 - unit;
+__device__ __forceinline__ bool at_row_tile(const int * __restrict__ cu_q, const int * __restrict__ ctx_len, int num_seqs, bool single, int G,
+                                            int rows, int unit, AtPlace & at) {
+    auto place = [&](int s, int q0, int q_len, int ctx, int tile) {
+        at.s = s; at.q0 = q0; at.q_len = q_len; at.ctx = ctx; at.tile = tile;
         return tile >= 0;
+    };
+    if (num_seqs == 1 || single) {
+        const int s = num_seqs == 1 ? 0 : unit;
+        if (s >= num_seqs) return false;
+        const int q0 = cu_q[s], q_len = cu_q[s + 1] - q0, ctx = ctx_len[s];
+        return place(s, q0, q_len, ctx, (q_len * G + rows - 1) / rows - 1 - (num_seqs == 1 ? unit : 0));
     }
     const int lane = threadIdx.x & 31;
-    auto request = [&](int i, int & q_len, int & pos0) {
-        q_len = cu_q[i + 1] - cu_q[i];
-        pos0 = max(ctx_len[i] - q_len, 0);                  // (a request without context: its rows see no key, but are written)
+    constexpr int HELD = 4;                                  // requests a lane holds: lane, lane + 32, ...; further ones are read again
+    auto request = [&](int i, int & len, int & pos0) {
+        len = pos0 = 0;                                      // (none: no tokens, no row tiles)
+        if (i < num_seqs) { len = cu_q[i + 1] - cu_q[i]; pos0 = max(ctx_len[i] - len, 0); }         // without context: sees no key, but is written
     };
-    auto tiles_from = [&](int q_len, int pos0, int L) {      // row tiles of a request that see L key tiles or more
-        const int n = (q_len * G + rows - 1) / rows, x = (L - 1) * KEYS - pos0;
+    auto tiles_from = [&](int len, int pos0, int L) {        // row tiles of a request that see L key tiles or more
+        const int n = (len * G + rows - 1) / rows, x = (L - 1) * KEYS - pos0;
         if (x <= 0) return n;
-        if (x > q_len - 1) return 0;
-        return n - min((x * G + rows) / rows - 1, n - 1);    // the first of them holds row x * G
+        return x < len ? n - x * G / rows : 0;               // the first of them holds row x * G
     };
-    int q_len0 = 0, pos00 = 0, most = 0;                     // the lane's first request, kept
-    if (lane < num_seqs) request(lane, q_len0, pos00);
-    for (int i = lane; i < num_seqs; i += 32) {
-        int q_len = q_len0, pos0 = pos00;
-        if (i >= 32) request(i, q_len, pos0);
-        most = max(most, q_len > 0 ? pos0 + q_len : 0);
+    int len[HELD], pos0[HELD], all = 0, most = 0;
+    auto add = [&](int q, int p) {
+        all += tiles_from(q, p, 1);
+        most = max(most, q > 0 ? p + q : 0);
+    };
+#pragma unroll
+    for (int h = 0; h < HELD; h++) request(lane + 32 * h, len[h], pos0[h]);
+#pragma unroll
+    for (int h = 0; h < HELD; h++) add(len[h], pos0[h]);
+#pragma unroll 1
+    for (int i = lane + 32 * HELD; i < num_seqs; i += 32) {
+        int q, p;
+        request(i, q, p);
+        add(q, p);
     }
+    all = __reduce_add_sync(0xffffffffu, all);
     most = __reduce_max_sync(0xffffffffu, most);
-    auto count = [&](int L) {
+    if (all <= unit) return false;
+    const int step = (most + 8 * KEYS - 1) / (8 * KEYS);     // key tiles to an eighth
+    int lo = 0, above = 0;                                   // row tiles that see 1 + step * lo or more > unit >= those of a higher eighth = above
+#pragma unroll 1
+    for (int bit = 4; bit > 0; bit >>= 1) {
+        const int L = 1 + step * (lo | bit);
         int c = 0;
-        for (int i = lane; i < num_seqs; i += 32) {
-            int q_len = q_len0, pos0 = pos00;
-            if (i >= 32) request(i, q_len, pos0);
-            c += tiles_from(q_len, pos0, L);
+#pragma unroll
+        for (int h = 0; h < HELD; h++)
+            if (32 * h < num_seqs) c += tiles_from(len[h], pos0[h], L);
+#pragma unroll 1
+        for (int i = lane + 32 * HELD; i < num_seqs; i += 32) {
+            int q, p;
+            request(i, q, p);
+            c += tiles_from(q, p, L);
         }
-        return __reduce_add_sync(0xffffffffu, c);
-    };
-    if (count(1) <= unit) return false;
-    int lo = 1, hi = (most + KEYS - 1) / KEYS + 1, above = 0;        // count(lo) > unit >= count(hi) = above
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1, c = count(mid);
-        if (c > unit) lo = mid;
-        else { hi = mid; above = c; }
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (c > unit) lo |= bit;
+        else above = c;
     }
-    int rest = unit - above;                                 // among the row tiles that see exactly lo key tiles, request by request
+    int rest = unit - above;                                 // among the row tiles of this eighth, request by request
+#pragma unroll 1
     for (int base = 0; base < num_seqs; base += 32) {
-        const int i = base + lane;
-        int q_len = q_len0, pos0 = pos00;
-        if (base > 0 && i < num_seqs) request(i, q_len, pos0);
-        const int more = i < num_seqs ? tiles_from(q_len, pos0, lo + 1) : 0, c = i < num_seqs ? tiles_from(q_len, pos0, lo) - more : 0;
+        int q, p;
+        request(base + lane, q, p);
+        const int more = tiles_from(q, p, 1 + step * (lo + 1)), c = tiles_from(q, p, 1 + step * lo) - more;
         int upto = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -198,21 +221,20 @@ __device__ __forceinline__ bool at_row_tile(const int * __restrict__ cu_q, const
         }
         const unsigned here = __ballot_sync(0xffffffffu, upto > rest);
         if (here != 0) {
-            const int l = __ffs(here) - 1;
-            s = base + l;
-            const int n = (q_len * G + rows - 1) / rows;
-            tile = __shfl_sync(0xffffffffu, n - 1 - more - (rest - (upto - c)), l);
-            return true;
+            const int l = __ffs(here) - 1, s = base + l;
+            const int tile = __shfl_sync(0xffffffffu, (q * G + rows - 1) / rows - 1 - more - (rest - (upto - c)), l);
+            return place(s, cu_q[s], __shfl_sync(0xffffffffu, q, l), ctx_len[s], tile);
         }
         rest -= __shfl_sync(0xffffffffu, upto, 31);
     }
     return false;
 }
 
-// CTAs for the row tiles of a step: no request has more than ceil(max_rows / rows), all together not more than N G / rows + S.
-static inline unsigned at_grid(int N, int S, int max_q_len, int nh, int nkv, int rows) {
-    const long long G = nh / nkv, each = (max_q_len * G + rows - 1) / rows * S, all = (long long) N * G / rows + S;
-    return (unsigned) ((each < all ? each : all) * nkv);
+// Row tiles a request may have, and those of a step: all together not more than N G / rows + S.
+static inline long long at_tiles(int max_q_len, int G, int rows) { return ((long long) max_q_len * G + rows - 1) / rows; }
+static inline long long at_units(int N, int S, int max_q_len, int G, int rows) {
+    const long long each = at_tiles(max_q_len, G, rows) * S, all = (long long) N * G / rows + S;
+    return each < all ? each : all;
 }
 
 typedef CUresult (*AtEncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
