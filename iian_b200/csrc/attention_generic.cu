@@ -15,6 +15,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "packed.cuh"
 
 namespace iian {
 
@@ -151,27 +152,6 @@ __global__ void paged_attention_generic_kernel(
     }
 }
 
-__device__ __forceinline__ unsigned long long ag_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ unsigned long long ag_pair(float x, float y) {
-    unsigned long long d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
-    return d;
-}
-__device__ __forceinline__ float2 ag_halves(unsigned long long v) {
-    float2 f;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
-    return f;
-}
-__device__ __forceinline__ void ag_cp16(float * dst, const float * src, bool valid) {
-    const unsigned d = (unsigned) __cvta_generic_to_shared(dst);
-    const int n = valid ? 16 : 0;                      // src-size 0: zeros are written, nothing is read
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n));
-}
-
 // The same attention in float32 for neighbouring tokens: a CTA owns 32 (token, head) items of one KV head, eight a warp, and its key
 // tiles -- the same 32 keys from the same multiples of 32 -- come once through two stages of shared memory for all of them.  Every
 // item's arithmetic is the kernel's above term by term (a lane is a key in the scores and four output entries in the sum; packed
@@ -243,8 +223,8 @@ paged_attention_tile_kernel(
                 const size_t cell = ok ? (((size_t) page * nkv + kvh) * page_size + (j % page_size)) * hd : 0;
                 float * to = stages + (size_t) stage * 2 * 32 * kTileLd + r * kTileLd;
                 for (int c = tid & 3; c < pieces; c += 4) {
-                    ag_cp16(to + c * 4, k_cache + cell + c * 4, ok);
-                    ag_cp16(to + 32 * kTileLd + c * 4, v_cache + cell + c * 4, ok);
+                    copy16(to + c * 4, k_cache + cell + c * 4, ok);
+                    copy16(to + 32 * kTileLd + c * 4, v_cache + cell + c * 4, ok);
                 }
                 const unsigned b = __ballot_sync(0xffffffffu, ok);       // this warp's eight keys, four bits each
                 if (lane == 0) {
@@ -275,21 +255,21 @@ paged_attention_tile_kernel(
 #pragma unroll 4
                 for (int d = 0; d < hd; d += 4) {
                     const float4 k4 = *reinterpret_cast<const float4 *>(kr + d);
-                    const unsigned long long k0 = ag_pair(k4.x, k4.x), k1 = ag_pair(k4.y, k4.y), k2 = ag_pair(k4.z, k4.z), k3 = ag_pair(k4.w, k4.w);
+                    const unsigned long long k0 = pack2(k4.x, k4.x), k1 = pack2(k4.y, k4.y), k2 = pack2(k4.z, k4.z), k3 = pack2(k4.w, k4.w);
 #pragma unroll
                     for (int pr = 0; pr < 4; pr++) {
                         const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(qw + (pr * hd + d) * 2);
                         const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(qw + (pr * hd + d + 2) * 2);
-                        dot[pr] = ag_fma2(a.x, k0, dot[pr]);
-                        dot[pr] = ag_fma2(a.y, k1, dot[pr]);
-                        dot[pr] = ag_fma2(b.x, k2, dot[pr]);
-                        dot[pr] = ag_fma2(b.y, k3, dot[pr]);
+                        dot[pr] = fma2(a.x, k0, dot[pr]);
+                        dot[pr] = fma2(a.y, k1, dot[pr]);
+                        dot[pr] = fma2(b.x, k2, dot[pr]);
+                        dot[pr] = fma2(b.y, k3, dot[pr]);
                     }
                 }
                 bool full = true;                      // every item weighs every key of the tile: no term is left out below
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
-                    const float2 two = ag_halves(dot[i >> 1]);
+                    const float2 two = unpack2(dot[i >> 1]);
                     const bool valid = here && tok[i] >= begin && tok[i] < end && j >= lo[i] && j <= hi[i];
                     const float sc = valid ? ((i & 1) ? two.y : two.x) * scale : -INFINITY;
                     const float tile_max = warp_max(sc);
@@ -301,8 +281,8 @@ paged_attention_tile_kernel(
                         l[i] = l[i] * corr + warp_sum(pj);
 #pragma unroll
                         for (int e = 0; e < 2; e++) {
-                            const float2 v = ag_halves(acc[i][e]);
-                            acc[i][e] = ag_pair(v.x * corr, v.y * corr);
+                            const float2 v = unpack2(acc[i][e]);
+                            acc[i][e] = pack2(v.x * corr, v.y * corr);
                         }
                         m[i] = m_new;
                     }
@@ -319,10 +299,10 @@ paged_attention_tile_kernel(
 #pragma unroll
                         for (int i = 0; i < 8; i++) {
                             const ulonglong2 p2 = *reinterpret_cast<const ulonglong2 *>(ps + (i * 32 + jj) * 2);
-                            acc[i][0] = ag_fma2(p2.x, v0.x, acc[i][0]);
-                            acc[i][1] = ag_fma2(p2.x, v0.y, acc[i][1]);
-                            acc[i][0] = ag_fma2(p2.y, v1.x, acc[i][0]);
-                            acc[i][1] = ag_fma2(p2.y, v1.y, acc[i][1]);
+                            acc[i][0] = fma2(p2.x, v0.x, acc[i][0]);
+                            acc[i][1] = fma2(p2.x, v0.y, acc[i][1]);
+                            acc[i][0] = fma2(p2.y, v1.x, acc[i][0]);
+                            acc[i][1] = fma2(p2.y, v1.y, acc[i][1]);
                         }
                     }
                 } else if (lane < pieces) {
@@ -333,8 +313,8 @@ paged_attention_tile_kernel(
 #pragma unroll
                         for (int i = 0; i < 8; i++) {
                             const ulonglong2 p2 = *reinterpret_cast<const ulonglong2 *>(ps + (i * 32 + jj) * 2);
-                            if (ag_halves(p2.x).x != 0.0f) { acc[i][0] = ag_fma2(p2.x, v0.x, acc[i][0]); acc[i][1] = ag_fma2(p2.x, v0.y, acc[i][1]); }
-                            if (ag_halves(p2.y).x != 0.0f) { acc[i][0] = ag_fma2(p2.y, v1.x, acc[i][0]); acc[i][1] = ag_fma2(p2.y, v1.y, acc[i][1]); }
+                            if (unpack2(p2.x).x != 0.0f) { acc[i][0] = fma2(p2.x, v0.x, acc[i][0]); acc[i][1] = fma2(p2.x, v0.y, acc[i][1]); }
+                            if (unpack2(p2.y).x != 0.0f) { acc[i][0] = fma2(p2.y, v1.x, acc[i][0]); acc[i][1] = fma2(p2.y, v1.y, acc[i][1]); }
                         }
                     }
                 }
@@ -351,7 +331,7 @@ paged_attention_tile_kernel(
         if (item >= n_items || lane >= pieces) continue;
         const int t = t0 + item / G, h = kvh * G + item % G;
         const float inv = l[i] > 0.0f ? 1.0f / l[i] : 0.0f;
-        const float2 x = ag_halves(acc[i][0]), y = ag_halves(acc[i][1]);
+        const float2 x = unpack2(acc[i][0]), y = unpack2(acc[i][1]);
         float4 v = make_float4(x.x * inv, x.y * inv, y.x * inv, y.y * inv);
         if (gate != nullptr) {
             const float * g = gate + (size_t) t * ld_gate + h * hd + lane * 4;

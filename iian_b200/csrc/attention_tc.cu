@@ -99,11 +99,11 @@ template <int N> __device__ __forceinline__ float at_cap_one(float s, const floa
 }
 // Two packed scores minus the maximum (neg2 = -max): x * (c0 + c1 x^2 + ...) + neg2
 template <int N> __device__ __forceinline__ unsigned long long at_cap_two(unsigned long long x, const unsigned long long * c, unsigned long long neg2) {
-    const unsigned long long x2 = at_mul2(x, x);
+    const unsigned long long x2 = mul2(x, x);
     unsigned long long y = c[N - 1];
 #pragma unroll
-    for (int i = N - 2; i >= 0; i--) y = at_fma2(x2, y, c[i]);
-    return at_fma2(x, y, neg2);
+    for (int i = N - 2; i >= 0; i--) y = fma2(x2, y, c[i]);
+    return fma2(x, y, neg2);
 }
 
 // The form with kept first keys and a gate per head (AT_KEPT), the difference form (AT_DIFF) and the capped form (AT_CAP) are
@@ -115,17 +115,17 @@ enum { AT_PLAIN = 0, AT_KEPT = 1, AT_DIFF = 2, AT_CAP = 3 };
 template <int N> __device__ __forceinline__ void at_capped_row(unsigned * v, const float * coef, float neg, unsigned long long * sum2) {
     unsigned long long c[N];
 #pragma unroll
-    for (int i = 0; i < N; i++) c[i] = at_pack2(coef[i], coef[i]);
-    const unsigned long long neg2 = at_pack2(-neg, -neg);
+    for (int i = 0; i < N; i++) c[i] = pack2(coef[i], coef[i]);
+    const unsigned long long neg2 = pack2(-neg, -neg);
 #pragma unroll
     for (int j = 0; j < AT_BN; j += 4) {
 #pragma unroll
         for (int e = 0; e < 2; e++) {
-            const unsigned long long t = at_cap_two<N>(at_pack2(__uint_as_float(v[j + 2 * e]), __uint_as_float(v[j + 2 * e + 1])), c, neg2);
+            const unsigned long long t = at_cap_two<N>(pack2(__uint_as_float(v[j + 2 * e]), __uint_as_float(v[j + 2 * e + 1])), c, neg2);
             float t0, t1;
-            at_unpack2(t, t0, t1);
+            unpack2(t, t0, t1);
             const float p0 = at_exp2(t0), p1 = at_exp2(t1);
-            sum2[e] = at_add2(sum2[e], at_pack2(p0, p1));
+            sum2[e] = add2(sum2[e], pack2(p0, p1));
             __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
             v[(j >> 1) + e] = *reinterpret_cast<unsigned *>(&h);
         }
@@ -415,32 +415,32 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
                     float far = fmaxf(fmaxf(hi4[0], hi4[1]), -fminf(lo4[0], lo4[1]));
                     if (CAP && p.cap_range != 0) far = 0.75f * (float) p.cap_range * p.cap_small;       // within the range's bound
                     if (__all_sync(0xffffffffu, far <= p.cap_small)) {
-                        const unsigned long long c0 = at_pack2(p.cap_poly[0], p.cap_poly[0]), c1 = at_pack2(p.cap_poly[1], p.cap_poly[1]);
-                        const unsigned long long c2 = at_pack2(p.cap_poly[2], p.cap_poly[2]), c3 = at_pack2(p.cap_poly[3], p.cap_poly[3]);
+                        const unsigned long long c0 = pack2(p.cap_poly[0], p.cap_poly[0]), c1 = pack2(p.cap_poly[1], p.cap_poly[1]);
+                        const unsigned long long c2 = pack2(p.cap_poly[2], p.cap_poly[2]), c3 = pack2(p.cap_poly[3], p.cap_poly[3]);
 #pragma unroll
                         for (int j = 0; j < AT_BN; j += 2) {
-                            const unsigned long long x = at_pack2(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
-                            const unsigned long long x2 = at_mul2(x, x);
-                            const unsigned long long y = at_mul2(x, at_fma2(x2, at_fma2(x2, at_fma2(x2, c3, c2), c1), c0));
+                            const unsigned long long x = pack2(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
+                            const unsigned long long x2 = mul2(x, x);
+                            const unsigned long long y = mul2(x, fma2(x2, fma2(x2, fma2(x2, c3, c2), c1), c0));
                             float y0, y1;
-                            at_unpack2(y, y0, y1);
+                            unpack2(y, y0, y1);
                             v[j] = __float_as_uint(y0);
                             v[j + 1] = __float_as_uint(y1);
                         }
                     } else if (__all_sync(0xffffffffu, far <= 2.0f * p.cap_small)) {
                         unsigned long long c[6];
 #pragma unroll
-                        for (int i2 = 0; i2 < 6; i2++) c[i2] = at_pack2(p.cap_wide[i2], p.cap_wide[i2]);
+                        for (int i2 = 0; i2 < 6; i2++) c[i2] = pack2(p.cap_wide[i2], p.cap_wide[i2]);
 #pragma unroll
                         for (int j = 0; j < AT_BN; j += 2) {
-                            const unsigned long long x = at_pack2(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
-                            const unsigned long long x2 = at_mul2(x, x);
-                            unsigned long long y = at_fma2(x2, c[5], c[4]);
+                            const unsigned long long x = pack2(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
+                            const unsigned long long x2 = mul2(x, x);
+                            unsigned long long y = fma2(x2, c[5], c[4]);
 #pragma unroll
-                            for (int i2 = 3; i2 >= 0; i2--) y = at_fma2(x2, y, c[i2]);
-                            y = at_mul2(x, y);
+                            for (int i2 = 3; i2 >= 0; i2--) y = fma2(x2, y, c[i2]);
+                            y = mul2(x, y);
                             float y0, y1;
-                            at_unpack2(y, y0, y1);
+                            unpack2(y, y0, y1);
                             v[j] = __float_as_uint(y0);
                             v[j + 1] = __float_as_uint(y1);
                         }
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
             // s * scale - max for two keys per instruction (packed float32 pairs), the exponentials one by one, the
             // sums in pairs again; the pair of probabilities is rounded to bfloat16 at once, into a register whose
             // values have been used already
-            const unsigned long long sl2 = at_pack2(sl, sl), neg2 = at_pack2(-neg, -neg);
+            const unsigned long long sl2 = pack2(sl, sl), neg2 = pack2(-neg, -neg);
             unsigned long long sum2[2] = {0ull, 0ull};
             if (riding) {
                 if (p.cap_range == 1) at_capped_row<4>(v, p.cap_poly, neg, sum2);
@@ -499,18 +499,18 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
             for (int j = 0; j < AT_BN; j += 4) {
 #pragma unroll
                 for (int e = 0; e < 2; e++) {
-                    const unsigned long long t = at_fma2(at_pack2(__uint_as_float(v[j + 2 * e]), __uint_as_float(v[j + 2 * e + 1])), sl2, neg2);
+                    const unsigned long long t = fma2(pack2(__uint_as_float(v[j + 2 * e]), __uint_as_float(v[j + 2 * e + 1])), sl2, neg2);
                     float t0, t1;
-                    at_unpack2(t, t0, t1);
+                    unpack2(t, t0, t1);
                     const float p0 = at_exp2(t0), p1 = at_exp2(t1);                // 2^-inf = 0 for masked keys
-                    sum2[e] = at_add2(sum2[e], at_pack2(p0, p1));
+                    sum2[e] = add2(sum2[e], pack2(p0, p1));
                     __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
                     v[(j >> 1) + e] = *reinterpret_cast<unsigned *>(&h);
                 }
             }
             float s0, s1, s2, s3;
-            at_unpack2(sum2[0], s0, s1);
-            at_unpack2(sum2[1], s2, s3);
+            unpack2(sum2[0], s0, s1);
+            unpack2(sum2[1], s2, s3);
             l_run = l_run * corr + ((s0 + s1) + (s2 + s3));
             if (i > 0) {        // P (and O, if it has to be rescaled) are free once the product of the tile before is complete
                 if (!at_wait(at_smem(&pv_done[g]), ph ^ 1u)) { if (lane == 0) { status[0] = 8; status[1] = i; } failed = true; break; }

@@ -30,9 +30,10 @@ SHARED_HEADERS = ["common.cuh"]
 # further headers that some sources share
 SOURCE_HEADERS: Dict[str, List[str]] = {"attention_mma": ["paged_mma.cuh"], "difference_attention_mma": ["paged_mma.cuh"],
                                          "moe": ["gated.cuh"], "postnorm": ["gated.cuh"], "gemm_stream": ["gated.cuh"],
-                                         "gemm_tcgen05": ["gated.cuh"], "attention_tc": ["tc_attention.cuh"],
-                                         "latent_attention_tc": ["tc_attention.cuh", "latent_merge.cuh"],
-                                         "latent_attention_mma": ["latent_merge.cuh"]}
+                                         "gemm_tcgen05": ["gated.cuh"], "attention_tc": ["tc_attention.cuh", "packed.cuh"],
+                                         "latent_attention_tc": ["tc_attention.cuh", "packed.cuh", "latent_merge.cuh"],
+                                         "latent_attention_mma": ["latent_merge.cuh"], "gemm_simt": ["packed.cuh"],
+                                         "attention_generic": ["packed.cuh"], "delta_rule": ["packed.cuh"]}
 
 # every library of the engine; build_all() compiles them all
 SOURCES = ["elementwise", "rope_kv", "attention_generic", "gemm_simt", "sampling", "gemm_skinny", "attention_mma", "prefetch", "gemm_tcgen05",

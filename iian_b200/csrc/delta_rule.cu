@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "packed.cuh"
 
 namespace iian {
 
@@ -425,10 +426,6 @@ __device__ __forceinline__ void dr_cp4(float * dst, const float * src, bool vali
     const int n = valid ? 4 : 0;                             // src-size 0: the word is zero-filled, nothing is read
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(n));
 }
-__device__ __forceinline__ void dr_cp16(float * dst, const float * src) {
-    const unsigned d = (unsigned) __cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src));
-}
 __device__ __forceinline__ void dr_commit() { asm volatile("cp.async.commit_group;"); }
 template <int N> __device__ __forceinline__ void dr_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N)); }
 
@@ -477,9 +474,9 @@ delta_scan_kernel(const float * __restrict__ qn, const float * __restrict__ kn, 
             for (int e = threadIdx.x; e < nt * per; e += blockDim.x) {
                 const int tt = e / per, d = (e - tt * per) << 2;
                 const size_t t = c0 + tt;
-                dr_cp16(s_q + tt * Dp + d, qn + t * GD + g * D + d);
-                dr_cp16(s_k + tt * Dp + d, kn + t * GD + g * D + d);
-                if (!HEAD) dr_cp16(s_g + tt * Dp + d, decay + t * HD + h * D + d);
+                copy16(s_q + tt * Dp + d, qn + t * GD + g * D + d);
+                copy16(s_k + tt * Dp + d, kn + t * GD + g * D + d);
+                if (!HEAD) copy16(s_g + tt * Dp + d, decay + t * HD + h * D + d);
             }
         } else {
             for (int e = threadIdx.x; e < nt * D; e += blockDim.x) {
@@ -648,25 +645,9 @@ delta_scan_kernel(const float * __restrict__ qn, const float * __restrict__ kn, 
 constexpr int kBlockNumbers = 28;               // beta [4], A (1,0) (2,0) (2,1) (3,0) (3,1) (3,2) 0 0, B [4][4] (zero above the diagonal)
 constexpr int kBlocksPerStage = 2, kBlockStages = 4;
 
-__device__ __forceinline__ unsigned long long dr_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ unsigned long long dr_mul2(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ unsigned long long dr_twice(float v) {
-    unsigned long long d;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(v));
-    return d;
-}
 __device__ __forceinline__ float dr_both(unsigned long long v) {
-    float x, y;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
-    return x + y;
+    const float2 f = unpack2(v);
+    return f.x + f.y;
 }
 
 // Where a sequence's pieces begin.  `pieces` 0: the whole step at once, the pieces of sequence s from cu_q[s] / 4 + s on (the sequences
@@ -784,10 +765,10 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
                 const int c = turn * kBlocksPerStage + b;
                 if (c >= n_blocks) break;
                 const float * src = mine + (size_t) c * H * BLOCK;
-                for (int e = tid; e < BLOCK / 4; e += kThreads) dr_cp16(to + b * PIECE + 4 * e, src + 4 * e);
+                for (int e = tid; e < BLOCK / 4; e += kThreads) copy16(to + b * PIECE + 4 * e, src + 4 * e);
                 if (tid < kCols) {                           // four tokens' values of the CTA's columns; beyond the last token: that one's
                     const int t = min(t0 + 4 * c + tid / 4, t1 - 1);
-                    dr_cp16(to + b * PIECE + BLOCK + 4 * tid, vv + (size_t) t * HV + h * V + cb * kCols + 4 * (tid % 4));
+                    copy16(to + b * PIECE + BLOCK + 4 * tid, vv + (size_t) t * HV + h * V + cb * kCols + 4 * (tid % 4));
                 }
             }
         }
@@ -845,8 +826,8 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
                     const ulonglong2 e = *reinterpret_cast<const ulonglong2 *>(vec + v * D + 4 * lane + 4 * kPairLanes * i);
 #pragma unroll
                     for (int x = 0; x < 2; x++) {
-                        acc[x][v] = dr_fma2(e.x, S[x][2 * i], acc[x][v]);
-                        acc[x][v] = dr_fma2(e.y, S[x][2 * i + 1], acc[x][v]);
+                        acc[x][v] = fma2(e.x, S[x][2 * i], acc[x][v]);
+                        acc[x][v] = fma2(e.y, S[x][2 * i + 1], acc[x][v]);
                     }
                 }
             }
@@ -886,15 +867,15 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
                 const int at = 4 * lane + 4 * kPairLanes * i;
                 ulonglong2 e = *reinterpret_cast<const ulonglong2 *>(vec + 12 * D + at);
 #pragma unroll
-                for (int x = 0; x < 2; x++) { S[x][2 * i] = dr_mul2(e.x, S[x][2 * i]); S[x][2 * i + 1] = dr_mul2(e.y, S[x][2 * i + 1]); }
+                for (int x = 0; x < 2; x++) { S[x][2 * i] = mul2(e.x, S[x][2 * i]); S[x][2 * i + 1] = mul2(e.y, S[x][2 * i + 1]); }
 #pragma unroll
                 for (int t = 0; t < 4; t++) {
                     e = *reinterpret_cast<const ulonglong2 *>(vec + (8 + t) * D + at);
 #pragma unroll
                     for (int x = 0; x < 2; x++) {
-                        const unsigned long long w = dr_twice(u[x][t]);
-                        S[x][2 * i] = dr_fma2(e.x, w, S[x][2 * i]);
-                        S[x][2 * i + 1] = dr_fma2(e.y, w, S[x][2 * i + 1]);
+                        const unsigned long long w = pack2(u[x][t], u[x][t]);
+                        S[x][2 * i] = fma2(e.x, w, S[x][2 * i]);
+                        S[x][2 * i + 1] = fma2(e.y, w, S[x][2 * i + 1]);
                     }
                 }
             }
@@ -954,7 +935,6 @@ IIAN_API int iian_delta_block_scan(const float * qn, const float * kn, const flo
     }
     return IIAN_OK;
 }
-
 
 // Floats of a slot's state: S [H, V, D], then the tail [taps - 1, 2 G D + H V].
 IIAN_API long long iian_delta_state_floats(int H, int G, int D, int V, int n_taps) {

@@ -10,6 +10,7 @@
 // K products in the order k = 0, 1, 2, ..., so a row's result does not depend on how many other
 // rows the batch has.
 #include "common.cuh"
+#include "packed.cuh"
 
 namespace iian {
 
@@ -63,29 +64,6 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const TX * __restrict__ 
             if (m < M) out[(size_t) n * M + m] = from_f32<TO>(acc[i][j]);
         }
     }
-}
-
-__device__ __forceinline__ void gs_cp16(float * dst, const float * src, bool valid) {
-    const unsigned d = (unsigned) __cvta_generic_to_shared(dst);
-    const int n = valid ? 16 : 0;                            // src-size 0: zeros are written, nothing is read
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n));
-}
-
-// Two independent float32 multiply-adds in one instruction, each rounded as fmaf rounds.
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ unsigned long long twice(float v) {
-    unsigned long long d;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(v));
-    return d;
-}
-__device__ __forceinline__ float2 halves(unsigned long long v) {
-    float2 f;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
-    return f;
 }
 
 // Tiles of TILE_N rows x TILE_M columns, a thread TN x TM of them (in blocks of 4 x 4), operands through two stages of shared
@@ -162,7 +140,7 @@ gemm_tile_kernel(const float * __restrict__ x, const float * __restrict__ w, TO 
                     *reinterpret_cast<const ulonglong2 *>(&ws[cur][k][(j * (TILE_M / (TM / 4)) + tx * 4) ^ flip]);
 #pragma unroll
             for (int i = 0; i < TN; i++) {
-                const unsigned long long v = twice(a[i]);
+                const unsigned long long v = pack2(a[i], a[i]);
 #pragma unroll
                 for (int j = 0; j < TM / 2; j++) acc[i][j] = fma2(v, b[j], acc[i][j]);
             }
@@ -182,7 +160,7 @@ gemm_tile_kernel(const float * __restrict__ x, const float * __restrict__ w, TO 
 #pragma unroll
         for (int j = 0; j < TM / 2; j++) {
             const int m = m0 + (j / 2) * (TILE_M / (TM / 4)) + tx * 4 + (j % 2) * 2;
-            const float2 v = halves(acc[i][j]);
+            const float2 v = unpack2(acc[i][j]);
             if (m < M) out[(size_t) n * M + m] = from_f32<TO>(v.x);
             if (m + 1 < M) out[(size_t) n * M + m + 1] = from_f32<TO>(v.y);
         }
@@ -213,7 +191,7 @@ gemm_rows_kernel(const float * __restrict__ x, const float * __restrict__ w, TO 
                 const bool is_w = r < TILE_M;
                 const bool in = k < K && (!is_w || m0 + r < M);
                 const float * from = is_w ? w + (size_t) (m0 + r) * K + k : x + (size_t) (r - TILE_M) * K + k;
-                gs_cp16(to + r * LD + (k - k0), in ? from : x, in);
+                copy16(to + r * LD + (k - k0), in ? from : x, in);
             }
         }
         asm volatile("cp.async.commit_group;");

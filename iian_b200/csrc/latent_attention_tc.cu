@@ -294,31 +294,31 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(
                 moved = true;
             }
             const float neg = m_run == -INFINITY ? 0.0f : m_run * sl;
-            const unsigned long long sl2 = at_pack2(sl, sl), neg2 = at_pack2(-neg, -neg);
+            const unsigned long long sl2 = pack2(sl, sl), neg2 = pack2(-neg, -neg);
             unsigned long long sum2[2] = {0ull, 0ull};
 #pragma unroll
             for (int j = 0; j < LT_HALF; j += 4)
 #pragma unroll
                 for (int e = 0; e < 2; e++) {
-                    const unsigned long long t = at_fma2(at_pack2(__uint_as_float(v[j + 2 * e]), __uint_as_float(v[j + 2 * e + 1])), sl2, neg2);
+                    const unsigned long long t = fma2(pack2(__uint_as_float(v[j + 2 * e]), __uint_as_float(v[j + 2 * e + 1])), sl2, neg2);
                     float t0, t1;
-                    at_unpack2(t, t0, t1);
+                    unpack2(t, t0, t1);
                     __nv_bfloat162 h = __floats2bfloat162_rn(at_exp2(t0), at_exp2(t1));
                     const unsigned w = *reinterpret_cast<unsigned *>(&h);
                     // the weights as they are multiplied, so that their rounding weighs on both sides of the quotient
-                    sum2[e] = at_add2(sum2[e], at_pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)));
+                    sum2[e] = add2(sum2[e], pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)));
                     v[(j >> 1) + e] = w;
                 }
             float s0, s1, s2, s3;
-            at_unpack2(sum2[0], s0, s1);
-            at_unpack2(sum2[1], s2, s3);
+            unpack2(sum2[0], s0, s1);
+            unpack2(sum2[1], s2, s3);
             l_run = l_run * corr + ((s0 + s1) + (s2 + s3));
             lt_st16(tS + (unsigned) (half * (LT_HALF / 2)), v);    // P as bf16 pairs into the columns S came from (32 of its 64)
             if (i > 0 && __any_sync(0xffffffffu, moved)) {
                 if (!failed && !at_wait(at_smem(&own_free[(i - 1) & 1]), (unsigned) ((i - 1) >> 1) & 1u)) { status[0] = 9; status[1] = i; failed = true; }
                 __syncwarp();
                 at_fence_after();
-                const unsigned long long corr2 = at_pack2(corr, corr);
+                const unsigned long long corr2 = pack2(corr, corr);
 #pragma unroll 1
                 for (int c0 = 0; c0 < LT_SHARE / 2; c0 += 64) {
                     unsigned o[64];
@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(
 #pragma unroll
                     for (int j = 0; j < 64; j += 2) {
                         float a, b;
-                        at_unpack2(at_mul2(at_pack2(__uint_as_float(o[j]), __uint_as_float(o[j + 1])), corr2), a, b);
+                        unpack2(mul2(pack2(__uint_as_float(o[j]), __uint_as_float(o[j + 1])), corr2), a, b);
                         o[j] = __float_as_uint(a);
                         o[j + 1] = __float_as_uint(b);
                     }

@@ -28,19 +28,6 @@ __device__ __forceinline__ unsigned order_key(float f) {
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
-__device__ __forceinline__ int block_sum_int(int v, int * scratch) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if (lane == 0) scratch[warp] = v;
-    __syncthreads();
-    int t = lane < (blockDim.x >> 5) ? scratch[lane] : 0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    return t;
-}
-
 // (max value, lowest index holding it) over a row
 __device__ __forceinline__ void block_argmax(const float * row, int V, float scale, float & best, int & best_idx,
                                              float * fs, int * is) {

@@ -1,9 +1,10 @@
-// What the tcgen05 attention kernels share: barriers, copies, products, tensor memory, packed float32 arithmetic, and the order in which
+// What the tcgen05 attention kernels share: barriers, copies, products, tensor memory, and the order in which
 // the row tiles of a step's requests are taken.
 #pragma once
 #include <cuda.h>
 
 #include "common.cuh"
+#include "packed.cuh"
 
 namespace iian {
 
@@ -71,25 +72,6 @@ __device__ __forceinline__ void at_st32(unsigned taddr, const unsigned * r) {
 }
 __device__ __forceinline__ void at_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void at_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// packed pairs of float32 (one instruction for two values) and the maximum of three
-__device__ __forceinline__ unsigned long long at_pack2(float a, float b) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void at_unpack2(unsigned long long v, float & a, float & b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long at_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ unsigned long long at_mul2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 __device__ __forceinline__ float at_min3(float a, float b, float c) {
     float r;
     asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
@@ -100,11 +82,6 @@ __device__ __forceinline__ float at_tanh(float x) {      // 1 - 2 / (1 + e^2x), 
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * 2.8853900817779268f));
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
     return fmaf(-2.0f, r, 1.0f);
-}
-__device__ __forceinline__ unsigned long long at_add2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
 }
 __device__ __forceinline__ float at_max3(float a, float b, float c) {
     float r;
