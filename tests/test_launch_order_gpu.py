@@ -43,9 +43,11 @@ def check(out, want, bound):
     assert bool(((out.double() - want).abs() <= (2.0 ** -7 + 2e-4) * bound).all())
 
 
+@pytest.mark.parametrize("contexts", [lambda i: 1 + (i * 131) % 700 if i % 5 else 333, lambda i: 40, lambda i: 3000 if i == 7 else 1 + i % 3,
+                                      lambda i: 1 << (i % 11)])
 @pytest.mark.parametrize("S,nkv", [(37, 8), (38, 8), (56, 8), (64, 8), (256, 2), (257, 2), (130, 4)])
-def test_decode_in_falling_order_of_contexts(S, nkv):
-    ctx = [1 + (i * 131) % 700 if i % 5 else 333 for i in range(S)]
+def test_decode_in_falling_order_of_contexts(S, nkv, contexts):
+    ctx = [contexts(i) for i in range(S)]
     q, k, v, meta, want, bound = case(ctx, [1] * S, 2 * nkv, nkv)
     out = torch.full((S, 2 * nkv * 128), 7.0, device="cuda", dtype=torch.bfloat16)
     CudaKernels().paged_attention_mma(q, k, v, out, meta, num_heads=2 * nkv, num_kv_heads=nkv, head_dim=128, scale=128 ** -0.5, window=None,
@@ -54,7 +56,9 @@ def test_decode_in_falling_order_of_contexts(S, nkv):
 
 
 @pytest.mark.parametrize("cached,news", [([0], [300]), ([500, 0, 3], [33, 260, 1]), ([64] * 33, [64] * 33),
-                                         ([(i * 37) % 300 for i in range(90)], [1 + (i * 53) % 70 for i in range(90)])])
+                                         ([(i * 37) % 300 for i in range(90)], [1 + (i * 53) % 70 for i in range(90)]),
+                                         ([2000, 0] + [(i * 97) % 900 for i in range(150)], [65, 200] + [1 + (i * 53) % 70 for i in range(150)]),
+                                         ([7] * 40, [65 + i % 2 for i in range(40)]), ([(i * 211) % 1500 for i in range(140)], [1] * 139 + [129])])
 def test_portions_in_falling_order_of_their_keys(cached, news):
     q, k, v, meta, want, bound = case([c + n for c, n in zip(cached, news)], news, 8, 2)
     K, out = CudaKernels(), torch.full((sum(news), 8 * 128), 7.0, device="cuda", dtype=torch.bfloat16)
