@@ -279,15 +279,16 @@ delta_prep_tile_kernel(const A * __restrict__ proj, long long ld, int col_off, i
 }
 
 // The same preparation for steps of many tokens of bfloat16 models with heads of 128 and four taps: a warp takes one unit of 128 channels
-// (a query/key head's q and k, 128 values, a head's decays) over kWideTokens neighbouring rows, a lane four neighbouring channels.  The
-// convolution's window slides through registers, so every input is read once, eight bytes a lane, four tokens ahead; nothing is staged
-// and no lane waits for another but in the three sums of a query/key head.  What bounds it: instruction issue (the exponentials and
-// logarithms of silu and softplus) and the latency of a window's loads.  1,500 tokens, 16 heads of 128 with a decay per channel: 37 us
-// for 66 of the tiled kernel (the inputs and results are 74 MB, 11 us).  (The sums over a head run over a lane's four channels, then the
-// lanes: another order than the kernels above keep between them for the 32-bit path, which stays with those.)
-constexpr int kWideTokens = 16, kWideWarps = 4;
+// (a query/key head's q and k, 128 values, a head's decays) over a few neighbouring rows, a lane four channels.  The
+// convolution's window slides through registers, so every input is read once, four tokens ahead; nothing is staged
+// and no lane waits for another but in the three sums of a query/key head.  There a lane has the channels lane, lane + 32, ... of the kernels
+// above, so that the sums are taken in their order and the results are the same bits; values and decays go four neighbours a lane.
+// What bounds it: instruction issue (the exponentials and
+// logarithms of silu and softplus) and the latency of a window's loads.  1,500 tokens, 16 heads of 128 with a decay per channel: 35 us
+// for 54 of the tiled kernel (replayed, the inputs in the L2; they and the results are 74 MB, 11 us).
+constexpr int kWideWarps = 4;
 
-template <bool HEAD>
+template <bool HEAD, int kWideTokens>
 __global__ void __launch_bounds__(kWideWarps * 32)
 delta_prep_wide_kernel(const __nv_bfloat16 * __restrict__ proj, long long ld, int col_off, int b_off, const float * __restrict__ b_pre,
                        const float * __restrict__ z, long long ld_z, const float * __restrict__ taps,
@@ -333,20 +334,26 @@ delta_prep_wide_kernel(const __nv_bfloat16 * __restrict__ proj, long long ld, in
         return;
     }
     const bool is_qk = u < G;
-    // this lane's channels: four of q and four of k, or four values
-    const int c[2] = {is_qk ? u * D + 4 * lane : 2 * GD + (u - G) * 128 + 4 * lane, GD + u * D + 4 * lane};
-    const int parts = is_qk ? 2 : 1;
+    // this lane's channels, `apart` from one another: four of q and four of k, or four values
+    const int c[2] = {is_qk ? u * D + lane : 2 * GD + (u - G) * 128 + 4 * lane, GD + u * D + lane};
+    const int parts = is_qk ? 2 : 1, apart = is_qk ? 32 : 1;
     float w[2][4][TAPS], x[2][TAPS][4];          // filters; the last four inputs, the current one last
 #pragma unroll
     for (int p = 0; p < 2; p++)
         if (p < parts)
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                const float4 f = *reinterpret_cast<const float4 *>(taps + (size_t) (c[p] + e) * TAPS);
+                const float4 f = *reinterpret_cast<const float4 *>(taps + (size_t) (c[p] + e * apart) * TAPS);
                 w[p][e][0] = f.x; w[p][e][1] = f.y; w[p][e][2] = f.z; w[p][e][3] = f.w;
             }
     auto input = [&](int p, long long r, float * to) {
-        const uint2 raw = *reinterpret_cast<const uint2 *>(proj + (size_t) r * ld + col_off + c[p]);
+        const __nv_bfloat16 * from = proj + (size_t) r * ld + col_off + c[p];
+        if (is_qk) {
+#pragma unroll
+            for (int e = 0; e < 4; e++) to[e] = __bfloat162float(from[32 * e]);
+            return;
+        }
+        const uint2 raw = *reinterpret_cast<const uint2 *>(from);
         const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.x));
         const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.y));
         to[0] = a.x; to[1] = a.y; to[2] = b.x; to[3] = b.y;
@@ -379,7 +386,7 @@ delta_prep_wide_kernel(const __nv_bfloat16 * __restrict__ proj, long long ld, in
                         else {
                             const int idx = (int) (r - first) + TAPS - 1;
 #pragma unroll
-                            for (int e = 0; e < 4; e++) x[p][j][e] = tail != nullptr && idx >= 0 ? tail[(size_t) idx * C + c[p] + e] : 0.0f;
+                            for (int e = 0; e < 4; e++) x[p][j][e] = tail != nullptr && idx >= 0 ? tail[(size_t) idx * C + c[p] + e * apart] : 0.0f;
                         }
                     }
                 }
@@ -411,8 +418,11 @@ delta_prep_wide_kernel(const __nv_bfloat16 * __restrict__ proj, long long ld, in
             s_k = warp_sum(s_k);
             dot = warp_sum(dot);
             const float iq = q_scale / sqrtf(s_q + 1e-6f), ik = 1.0f / sqrtf(s_k + 1e-6f);
-            *reinterpret_cast<float4 *>(qn + (size_t) t * GD + c[0]) = make_float4(a[0][0] * iq, a[0][1] * iq, a[0][2] * iq, a[0][3] * iq);
-            *reinterpret_cast<float4 *>(kn + (size_t) t * GD + c[0]) = make_float4(a[1][0] * ik, a[1][1] * ik, a[1][2] * ik, a[1][3] * ik);
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                qn[(size_t) t * GD + c[0] + 32 * e] = a[0][e] * iq;
+                kn[(size_t) t * GD + c[0] + 32 * e] = a[1][e] * ik;
+            }
             if (lane == 0) qk[(size_t) t * G + u] = dot * iq * ik;
         }
     }
@@ -954,9 +964,18 @@ static int launch_prep(const A * proj, long long ld, int col_off, int b_off, con
                            (((uintptr_t) taps | (uintptr_t) dt_bias | (uintptr_t) qn | (uintptr_t) kn | (uintptr_t) vv | (uintptr_t) decay) & 15) == 0;
         if (N >= kPrepTileFrom && D == 128 && V % 128 == 0 && n_taps == 4 && whole) {
             const int units = G + H * V / 128 + H;
-            return iian_launch(delta_prep_wide_kernel<HEAD>, dim3((N + kWideTokens - 1) / kWideTokens, (units + kWideWarps - 1) / kWideWarps),
-                               dim3(kWideWarps * 32), 0, stream, proj, ld, col_off, b_off, b_pre, z, ld_z, taps, a_log, dt_bias, state, state_stride,
-                               tail_off, seq_of_token, cu_q, state_slots, qn, kn, vv, beta, decay, qk, N, H, G, V, q_scale);
+            // rows a warp walks: the more the fewer windows are begun, but the grid should be two rounds of CTAs (three an SM): 16 heads with a
+            // decay per channel, 4, 8 and 16 rows: 256 tokens 8.6, 13.4, 23.2 us (tiles 13.8), 768 20.5, 19.3, 25.1 (29.7), 1,500 37.3, 35.5,
+            // 34.8 (54.2)
+            auto ctas = [&](int T) { return (long long) ((N + T - 1) / T) * ((units + kWideWarps - 1) / kWideWarps); };
+            auto go = [&](auto tokens) {
+                constexpr int T = decltype(tokens)::value;
+                return iian_launch(delta_prep_wide_kernel<HEAD, T>, dim3((N + T - 1) / T, (units + kWideWarps - 1) / kWideWarps),
+                                   dim3(kWideWarps * 32), 0, stream, proj, ld, col_off, b_off, b_pre, z, ld_z, taps, a_log, dt_bias, state, state_stride,
+                                   tail_off, seq_of_token, cu_q, state_slots, qn, kn, vv, beta, decay, qk, N, H, G, V, q_scale);
+            };
+            if (ctas(16) >= 6 * 148) return go(std::integral_constant<int, 16>());
+            return ctas(8) >= 6 * 148 ? go(std::integral_constant<int, 8>()) : go(std::integral_constant<int, 4>());
         }
     }
     // many tokens: tiles of T rows through shared memory; few: a CTA per token and unit, so that they spread over the GPU

@@ -1,5 +1,6 @@
-"""The delta rule's scan over portions of prompts, four tokens at a time, against the scan token by token: lengths around multiples
-of four and of a stage, sequences of a single token and padding between long ones, states that go on, the step whole and in segments."""
+"""The delta rule over portions of prompts in bfloat16 models.  The scan four tokens at a time against the scan token by token: lengths around
+multiples of four and of a stage, sequences of a single token and padding between long ones, states that go on, the step whole and in
+segments.  The preparation of steps of many tokens against steps of few, bit for bit."""
 from types import SimpleNamespace
 
 import pytest
@@ -54,3 +55,41 @@ def test_four_tokens_at_a_time(lens, H, G, D, V, per_head):
         # both are 32-bit sums of the same terms in another order: D of them in a dot product, the sequence's tokens in the state
         for a, b in ((got, want), (state, want_state)):
             assert (a - b).norm() <= 1e-5 * b.norm() and (a - b).abs().max() <= 1e-4 * b.abs().max()
+
+
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("given", [False, True])
+@pytest.mark.parametrize("H,G,V", [(4, 2, 128), (2, 2, 256), (3, 1, 128)])
+def test_preparation_of_many_tokens_gives_the_bits_of_few(H, G, V, given, per_head):
+    """Sequences that begin inside a tile of 16 rows, states and convolution tails that are not zero, padding in between, write strengths out
+    of the projections or given: one step of 475 tokens against steps of 100 at most, one sequence each."""
+    K, D, off = CudaKernels(), 128, 8
+    K.DELTA_BLOCKS = False
+    g = torch.Generator("cuda").manual_seed(H + V)
+    lens, slots, C = [5, 300, 3, 37, 130], [3, 0, -1, 1, 2], 2 * G * D + H * V
+    n, zw = sum(lens), H if per_head else H * D
+    state0 = torch.randn(4, K.delta_state_floats(H, G, D, V, 4), device="cuda", generator=g)
+    proj = torch.randn(n, off + C + H + (-(C + H)) % 8, device="cuda", generator=g).bfloat16()
+    both = torch.randn(n, zw + H + (-(zw + H)) % 4, device="cuda", generator=g)
+    taps = torch.randn(C, 4, device="cuda", generator=g) * 0.4
+    a_log, dt_bias = torch.rand(H, device="cuda", generator=g) * 2.5, torch.randn(zw, device="cuda", generator=g) - 2.0
+
+    def step(rows, cu, seq, which, state, out):
+        i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+        bufs = {}
+        ctx = SimpleNamespace(cu_q=i32(cu), seq_of_token=i32(seq), state_slots=i32(which), max_q_len=max(b - a for a, b in zip(cu, cu[1:])),
+                              buf=lambda name, shape, dt: bufs.setdefault(name, torch.full(shape, float("nan"), dtype=dt, device="cuda")))
+        K.delta_rule(proj[rows], off, off + C, both[rows, :zw], taps, a_log, dt_bias, state, ctx, out[rows], num_heads=H, num_kv_heads=G, dim=D,
+                     v_dim=V, b_pre=both[rows, zw: zw + H] if given else None)
+
+    cu = [0]
+    for m in lens:
+        cu.append(cu[-1] + m)
+    whole, few = state0.clone(), state0.clone()
+    a, b = torch.full((n, H * V), 7.0, device="cuda"), torch.zeros(n, H * V, device="cuda")
+    step(slice(0, n), cu, [i if slots[i] >= 0 else -1 for i, m in enumerate(lens) for _ in range(m)], slots, whole, a)
+    for i, m in enumerate(lens):
+        for lo in range(0, m if slots[i] >= 0 else 0, 100):
+            k = min(100, m - lo)
+            step(slice(cu[i] + lo, cu[i] + lo + k), [0, k], [0] * k, [slots[i]], few, b)
+    assert torch.equal(whole, few) and torch.equal(a, b)
