@@ -444,17 +444,15 @@ template <int N> __device__ __forceinline__ void dr_wait() { asm volatile("cp.as
 // 16 bytes at a time (E a multiple of 4); else entry d = lane + kLanes * i, word by word.  The tokens of a sequence pass
 // through two stages of shared memory, `chunk` tokens each: while one is worked through, cp.async fills the other.
 // HEAD: one decay per (token, head), decay [N, H]; it sits beside the write strength and q . k of its token.
+__host__ __device__ constexpr int scan_floats(bool head, int Dp, int chunk) { return 2 * chunk * ((head ? 2 : 3) * Dp + kCols + 4); }      // of shared memory
+
 template <int E, bool VEC, bool HEAD, typename A>
-__global__ void __launch_bounds__(kCols * kLanes)
-delta_scan_kernel(const float * __restrict__ qn, const float * __restrict__ kn, const float * __restrict__ vv,
+__device__ __forceinline__ void delta_scan(float * sm, const float * __restrict__ qn, const float * __restrict__ kn, const float * __restrict__ vv,
                   const float * __restrict__ beta, const float * __restrict__ decay, const float * __restrict__ qk,
                   float * __restrict__ state, long long state_stride, long long tail_off,
                   const A * __restrict__ proj, long long ld, int col_off, int n_taps,
                   const int * __restrict__ cu_q, const int * __restrict__ state_slots, float * __restrict__ out,
                   int H, int G, int D, int V, int chunk) {
-    pdl_wait();
-    pdl_launch_dependents();
-    extern __shared__ __align__(16) float sm[];
     const int Dp = (D + 3) & ~3;                             // rows start on 16-byte boundaries
     const int stage_floats = chunk * ((HEAD ? 2 : 3) * Dp + kCols + 4);      // q | k | decay (not HEAD) | v | beta, q . k, decay (HEAD), -
     const int cb = blockIdx.x, h = blockIdx.y, s = blockIdx.z;
@@ -640,6 +638,21 @@ delta_scan_kernel(const float * __restrict__ qn, const float * __restrict__ kn, 
     }
 }
 
+template <int E, bool VEC, bool HEAD, typename A>
+__global__ void __launch_bounds__(kCols * kLanes)
+delta_scan_kernel(const float * __restrict__ qn, const float * __restrict__ kn, const float * __restrict__ vv,
+                  const float * __restrict__ beta, const float * __restrict__ decay, const float * __restrict__ qk,
+                  float * __restrict__ state, long long state_stride, long long tail_off,
+                  const A * __restrict__ proj, long long ld, int col_off, int n_taps,
+                  const int * __restrict__ cu_q, const int * __restrict__ state_slots, float * __restrict__ out,
+                  int H, int G, int D, int V, int chunk) {
+    pdl_wait();
+    pdl_launch_dependents();
+    extern __shared__ __align__(16) float sm[];
+    delta_scan<E, VEC, HEAD, A>(sm, qn, kn, vv, beta, decay, qk, state, state_stride, tail_off, proj, ld, col_off, n_taps, cu_q, state_slots, out,
+                                H, G, D, V, chunk);
+}
+
 // ---- portions of prompts, four tokens at a time ------------------------------------------------------------------
 // Over four tokens the recurrence is a product with the state before them and small sums among themselves.  With G_t the decays'
 // product from the first of the four to token t and G_ts that from the token behind s to t (both per key channel):
@@ -671,7 +684,7 @@ __device__ __forceinline__ size_t first_piece(const int * __restrict__ cu_q, int
 __global__ void __launch_bounds__(128)
 delta_block_kernel(const float * __restrict__ qn, const float * __restrict__ kn, const float * __restrict__ beta,
                    const float * __restrict__ decay, int per_head, const int * __restrict__ cu_q, const int * __restrict__ state_slots,
-                   float * __restrict__ blocks, int from, int pieces, int S, int H, int G, int D) {
+                   float * __restrict__ blocks, int from, int pieces, int at_least, int S, int H, int G, int D) {
     const int h = blockIdx.y, g = h / (H / G);
     int s = blockIdx.z, c = blockIdx.x;
     if (pieces == 0) {                           // the last sequence that begins at or before this piece
@@ -685,7 +698,7 @@ delta_block_kernel(const float * __restrict__ qn, const float * __restrict__ kn,
     }
     const long long t0 = (long long) cu_q[s] + from + 4 * c;
     const int n = (int) min(4ll, cu_q[s + 1] - t0);
-    if (n <= 0 || state_slots[s] < 0) return;
+    if (n <= 0 || state_slots[s] < 0 || cu_q[s + 1] - cu_q[s] < at_least) return;
     float * b = blocks + ((first_piece(cu_q, s, pieces) + c) * H + h) * (13 * D + kBlockNumbers);
     __shared__ float red[4][16];
     const int d = threadIdx.x, lane = d & 31, warp = d >> 5;
@@ -743,14 +756,19 @@ delta_block_kernel(const float * __restrict__ qn, const float * __restrict__ kn,
 // is what shared memory delivers to registers); 32 lanes for two columns, two warps per scheduler, 240 us, but 565 against 500 us for four
 // sequences of 2,048; a warp per eighth of D and a lane per column, the sums through shared memory, 241 and 523 us.
 // V a multiple of kCols; state and values on 16-byte boundaries.
+// Sequences with fewer than at_least tokens are walked token by token as in the scan above, in the same launch: a piece costs more than a
+// token, and a launch of their own would wait for the long ones' chain (a portion of 100 tokens beside 100
+// decoded ones, 16 heads with a decay per channel, through the mixer: 142 us, in two launches 166).
 constexpr int kPairLanes = 16;
 
-template <int E, typename A>
+template <int E, bool HEAD, typename A>
 __global__ void __launch_bounds__(kCols / 2 * kPairLanes)
-delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restrict__ vv, float * __restrict__ state, long long state_stride,
+delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restrict__ qn, const float * __restrict__ kn,
+                        const float * __restrict__ vv, const float * __restrict__ beta, const float * __restrict__ decay,
+                        const float * __restrict__ qk, float * __restrict__ state, long long state_stride,
                         long long tail_off, const A * __restrict__ proj, long long ld, int col_off, int n_taps,
                         const int * __restrict__ cu_q, const int * __restrict__ state_slots, float * __restrict__ out,
-                        int from, int pieces, int H, int G, int V) {
+                        int from, int pieces, int at_least, int H, int G, int V) {
     constexpr int D = E * kPairLanes, BLOCK = 13 * D + kBlockNumbers, PIECE = BLOCK + 4 * kCols, STAGE = kBlocksPerStage * PIECE;
     constexpr int kThreads = kCols / 2 * kPairLanes;
     extern __shared__ __align__(16) float sm[];
@@ -758,6 +776,13 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
     const int tid = threadIdx.x, pair = tid / kPairLanes, lane = tid % kPairLanes, j = cb * kCols + 2 * pair;
     const int q0 = cu_q[s], q1 = cu_q[s + 1], slot = state_slots[s], HV = H * V;
     const int t0 = q0 + from, t1 = pieces > 0 ? min(q1, t0 + 4 * pieces) : q1;
+    if (q1 - q0 < at_least) {
+        static_assert(kCols / 2 * kPairLanes == kCols * kLanes && scan_floats(HEAD, D, 16) <= kBlockStages * STAGE, "both walks fit one launch");
+        if (from == 0)
+            delta_scan<D / kLanes, true, HEAD, A>(sm, qn, kn, vv, beta, decay, qk, state, state_stride, tail_off, proj, ld, col_off, n_taps, cu_q,
+                                                  state_slots, out, H, G, D, V, 16);
+        return;
+    }
     if (t0 >= t1) return;
     if (slot < 0) {
         for (int t = t0; t < t1; t++)
@@ -916,30 +941,33 @@ using namespace iian;
 // Floats of one four-token piece (all heads) of iian_delta_block_scan's scratch.
 IIAN_API long long iian_delta_block_floats(int H, int D) { return (long long) H * (13 * D + kBlockNumbers); }
 
-// The scan of iian_delta_scan for bfloat16 models and portions of many tokens, four tokens at a time.  blocks: scratch for N / 4 + S
+// The scan of iian_delta_scan for bfloat16 models, portions of at_least tokens and more four tokens at a time.  blocks: scratch for N / 4 + S
 // pieces with `pieces` 0, else for S * pieces: the step is then walked in segments of 4 * pieces tokens of every sequence, max_q_len the
 // most tokens a sequence has.  D 64 or 128, V a multiple of 16.
 IIAN_API int iian_delta_block_scan(const float * qn, const float * kn, const float * vv, const float * beta, const float * decay,
-                                   float * blocks, int pieces, float * state, long long state_stride, const void * proj, long long ld,
+                                   const float * qk, float * blocks, int pieces, float * state, long long state_stride, const void * proj, long long ld,
                                    int col_off, int n_taps, const int * cu_q, const int * state_slots, float * out, int N, int S, int H,
-                                   int G, int D, int V, int max_q_len, int per_head, cudaStream_t stream) {
+                                   int G, int D, int V, int max_q_len, int at_least, int per_head, cudaStream_t stream) {
     if (N <= 0 || S <= 0 || max_q_len <= 0) return IIAN_OK;
     if (H <= 0 || G <= 0 || H % G || (D != 64 && D != 128) || V <= 0 || V % kCols || n_taps < 1 || n_taps > kMaxTaps || pieces < 0 || S > 65535 ||
         H > 65535) return IIAN_ERR_SHAPE;
-    if (state_stride % 4 || (((uintptr_t) blocks | (uintptr_t) vv | (uintptr_t) state) & 15)) return IIAN_ERR_ALIGN;
+    if (state_stride % 4 || (((uintptr_t) blocks | (uintptr_t) qn | (uintptr_t) kn | (uintptr_t) vv | (uintptr_t) decay | (uintptr_t) state) & 15))
+        return IIAN_ERR_ALIGN;
     typedef __nv_bfloat16 bf;
     const size_t smem = (size_t) kBlockStages * kBlocksPerStage * (13 * D + kBlockNumbers + 4 * kCols) * sizeof(float);
-    auto scan = D == 128 ? delta_block_scan_kernel<8, bf> : delta_block_scan_kernel<4, bf>;
+    auto scan = D == 128 ? (per_head ? delta_block_scan_kernel<8, true, bf> : delta_block_scan_kernel<8, false, bf>)
+                         : (per_head ? delta_block_scan_kernel<4, true, bf> : delta_block_scan_kernel<4, false, bf>);
     const cudaError_t e = cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
     if (e != cudaSuccess) return 1000 + (int) e;
     const int step = pieces > 0 ? 4 * pieces : max_q_len;
     for (int from = 0; from < max_q_len; from += step) {
         const dim3 grid = pieces > 0 ? dim3(min(pieces, (max_q_len - from + 3) / 4), H, S) : dim3(N / 4 + S, H);
-        delta_block_kernel<<<grid, 128, 0, stream>>>(qn, kn, beta, decay, per_head, cu_q, state_slots, blocks, from, pieces, S, H, G, D);
+        delta_block_kernel<<<grid, 128, 0, stream>>>(qn, kn, beta, decay, per_head, cu_q, state_slots, blocks, from, pieces, at_least, S, H, G, D);
         int rc = iian_launch_status();
         if (rc != IIAN_OK) return rc;
-        scan<<<dim3(V / kCols, H, S), kCols / 2 * kPairLanes, smem, stream>>>(blocks, vv, state, state_stride, (long long) H * V * D, (const bf *) proj, ld,
-                                                                      col_off, n_taps, cu_q, state_slots, out, from, pieces, H, G, V);
+        scan<<<dim3(V / kCols, H, S), kCols / 2 * kPairLanes, smem, stream>>>(blocks, qn, kn, vv, beta, decay, qk, state, state_stride, (long long) H * V * D,
+                                                                      (const bf *) proj, ld, col_off, n_taps, cu_q, state_slots, out, from, pieces,
+                                                                      at_least, H, G, V);
         rc = iian_launch_status();
         if (rc != IIAN_OK) return rc;
     }
@@ -1026,7 +1054,7 @@ static int launch_scan(const float * qn, const float * kn, const float * vv, con
     const int Dp = (D + 3) & ~3;
     int chunk = D <= 256 ? 16 : 8;             // tokens per stage of shared memory
     if (max_q_len > 0 && max_q_len < chunk) chunk = max_q_len;         // single tokens: small stages, more CTAs per SM
-    const size_t smem = (size_t) 2 * chunk * ((HEAD ? 2 : 3) * Dp + kCols + 4) * sizeof(float);
+    const size_t smem = (size_t) scan_floats(HEAD, Dp, chunk) * sizeof(float);
     if (smem > 200 * 1024) return IIAN_ERR_LIMIT;
     const dim3 grid((V + kCols - 1) / kCols, H, S);
     if constexpr (E % 4 == 0) if (vec) {

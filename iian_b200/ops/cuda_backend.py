@@ -1148,7 +1148,8 @@ class CudaKernels:
         if parts > 1:
             LAUNCHES[0] += 1
 
-    # portions of prompts and, from 32 heads on, decoded tokens on tcgen05 (csrc/latent_attention_tc.cu): bfloat16, rank 256 / 512, rows of up to 576 values in chunks of 64
+    # portions of prompts and, from 32 heads on, decoded tokens on tcgen05 (csrc/latent_attention_tc.cu): bfloat16, rank 256 / 512, rows of up to
+    # 576 values in chunks of 64
     LATENT_TC = os.environ.get("IIAN_LATENT_TC", "1") not in ("0", "false", "off")
     # (row, key) pairs of a step, times the shares of the rank, from which it is used: 48 tokens of 16 heads behind 600 cached ones take 23 us
     # for 25 on mma.sync, 32 of them 24 for 21, 16 behind 4,000 25 for 38; rank 256: 64 behind 600 22 for 19, 128 of them 23 for 28
@@ -1265,8 +1266,8 @@ class CudaKernels:
                   c_void_p, c_int, c_void_p])
         epilogue = (1 if activation == "silu" else 4) if gated else 3 if relu2 else 0
         _check(fn(_cuda(x, "moe rows"), _cuda(w, "expert weights"), _cuda(out, "moe out"), BF16, m, n, e, k, epilogue,
-                  self.ACTIVATIONS[activation], limit, 64 if tile_rows <= 64 else 256, status, _cuda(tiles, "tiles", torch.int32), _cuda(offsets, "offsets", torch.int32), (tiles.numel() - 1) // 2,
-                  _stream()), "gemm_tcgen05_grouped")
+                  self.ACTIVATIONS[activation], limit, 64 if tile_rows <= 64 else 256, status, _cuda(tiles, "tiles", torch.int32),
+                  _cuda(offsets, "offsets", torch.int32), (tiles.numel() - 1) // 2, _stream()), "gemm_tcgen05_grouped")
 
     def moe_route(self, logits: torch.Tensor, top: int, ids: torch.Tensor, weights: torch.Tensor) -> None:
         """Router logits (float32, may be a column slice) -> the ``top`` experts of each token by sigmoid score, and the scores."""
@@ -2087,13 +2088,23 @@ class CudaKernels:
     # the delta rule's scan over portions of prompts, four tokens at a time (bfloat16 models); IIAN_DELTA_BLOCKS=0: token by token.
     # The 32-bit path stays token by token: there a token's bits must not depend on how its prompt was cut.
     DELTA_BLOCKS = os.environ.get("IIAN_DELTA_BLOCKS", "1") not in ("0", "false", "off")
-    DELTA_BLOCK_MIN_TOKENS = 32            # of the longest portion (16 tokens 148 -> 150 us a layer, 100 tokens 156 -> 152, 1,500 tokens 585 -> 457)
+    # tokens of a portion from which it is walked so, whatever else is in the step (16 tokens 148 -> 150 us a layer, 100 tokens 156 -> 152,
+    # 1,500 tokens 585 -> 457)
+    DELTA_BLOCK_MIN_TOKENS = 32
     DELTA_BLOCK_BYTES = 192 << 20          # of scratch for the pieces; a step that needs more is walked in segments
+    # pieces a sequence has in a segment, at least: each is two launches and a pass over the states (a portion of 2,048 tokens beside a
+    # hundred of 16, 32 heads, in segments of 8 pieces 3,204 us, token by token 1,769)
+    DELTA_SEGMENT_MIN_PIECES = 64
+    _delta_floats = {}
 
     def _delta_block_floats(self, h: int, d: int) -> int:
-        fn = _build.load("delta_rule").iian_delta_block_floats
-        fn.restype = c_longlong
-        return int(fn(c_int(h), c_int(d)))
+        """Floats of a piece of four tokens, all heads."""
+        n = self._delta_floats.get((h, d))
+        if n is None:
+            fn = _build.load("delta_rule").iian_delta_block_floats
+            fn.restype = c_longlong
+            n = self._delta_floats[(h, d)] = int(fn(c_int(h), c_int(d)))
+        return n
 
     def _delta_pieces(self, code: int, n: int, s: int, h: int, d: int, v: int, max_q_len: int, state: torch.Tensor) -> Optional[int]:
         """None: the scan token by token; 0: in pieces of four tokens, the whole step at once; else that many pieces of every sequence
@@ -2104,7 +2115,7 @@ class CudaKernels:
         most = self.DELTA_BLOCK_BYTES // (4 * self._delta_block_floats(h, d))
         if n // 4 + s <= most:
             return 0
-        return 1 << ((most // s).bit_length() - 1) if most // s >= 8 else None
+        return 1 << ((most // s).bit_length() - 1) if most // s >= self.DELTA_SEGMENT_MIN_PIECES else None
 
     def delta_rule(self, proj: torch.Tensor, col_off: int, b_off: int, z: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor,
                    dt_bias: torch.Tensor, state: torch.Tensor, ctx, out: torch.Tensor, *, num_heads: int, num_kv_heads: int, dim: int,
@@ -2113,8 +2124,8 @@ class CudaKernels:
         column ``col_off`` and the write strengths' pre-activations at ``b_off`` (or ``b_pre`` float32 [N, heads] holds them);
         ``z`` float32 [N, heads * dim] (a decay per key channel) or [N, heads] (one per head) the decays' pre-activations
         without bias; ``z`` and ``b_pre`` may be column slices of one matrix; ``taps`` float32 [channels, taps]; ``state`` float32 [slots, state floats];
-        ``out`` float32 [N, heads * v_dim] receives ``S^T q`` per head.  Two launches: per-token preparation, then the scan; portions of
-        prompts in bfloat16 models walk the scan four tokens at a time (``_delta_pieces``)."""
+        ``out`` float32 [N, heads * v_dim] receives ``S^T q`` per head.  Per-token preparation, then the scan; in bfloat16 models the
+        portions of DELTA_BLOCK_MIN_TOKENS tokens and more are walked four tokens at a time (``_delta_pieces``)."""
         n = proj.shape[0]
         h, g, d, v = num_heads, num_kv_heads, dim, v_dim
         channels = 2 * g * d + h * v
@@ -2153,11 +2164,12 @@ class CudaKernels:
             count = n // 4 + s if pieces == 0 else s * pieces
             blocks = ctx.buf("delta_blocks", (count * self._delta_block_floats(h, d),), f32)
             fn = _fn("delta_rule", "iian_delta_block_scan",
-                     [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_int,
-                      c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
-            _check(fn(qn.data_ptr(), kn.data_ptr(), vv.data_ptr(), beta.data_ptr(), decay.data_ptr(), blocks.data_ptr(), pieces,
+                     [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_longlong,
+                      c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
+            _check(fn(qn.data_ptr(), kn.data_ptr(), vv.data_ptr(), beta.data_ptr(), decay.data_ptr(), qk.data_ptr(), blocks.data_ptr(), pieces,
                       state.data_ptr(), state.shape[1], pp, ld, col_off, n_taps, ctx.cu_q.data_ptr(), ctx.state_slots.data_ptr(),
-                      _cuda(out, "delta out", f32), n, s, h, g, d, v, max_q_len, 1 if per_head else 0, _stream()), "delta_block_scan")
+                      _cuda(out, "delta out", f32), n, s, h, g, d, v, max_q_len, self.DELTA_BLOCK_MIN_TOKENS, 1 if per_head else 0, _stream()),
+                   "delta_block_scan")
             LAUNCHES[0] += 2 * (1 if pieces == 0 else -(-max_q_len // (4 * pieces))) - 1
             return
         fn = _fn("delta_rule", "iian_delta_scan",

@@ -11,8 +11,10 @@ from iian_b200.ops.cuda_backend import CudaKernels
 pytestmark = pytest.mark.gpu
 
 
-def walk(blocks, scratch, lens, H, G, D, V, per_head):
-    K = CudaKernels()
+def walk(blocks, scratch, lens, H, G, D, V, per_head, told=False):
+    """(outputs of two steps, states, what ``_delta_pieces`` chose); ``told``: the lengths are known on the host too."""
+    K, chosen = CudaKernels(), []
+    K._delta_pieces = lambda *a: chosen.append(CudaKernels._delta_pieces(K, *a)) or chosen[-1]
     g = torch.Generator("cuda").manual_seed(sum(lens) + D + H)
     C = 2 * G * D + H * V
     state = torch.randn(len(lens) + 1, K.delta_state_floats(H, G, D, V, 4), device="cuda", generator=g)
@@ -30,31 +32,41 @@ def walk(blocks, scratch, lens, H, G, D, V, per_head):
             cu.append(cu[-1] + x)
         seq = torch.tensor([i if slots[i] >= 0 else -1 for i, x in enumerate(lens) for _ in range(x)], dtype=torch.int32, device="cuda")
         ctx = SimpleNamespace(cu_q=torch.tensor(cu, dtype=torch.int32, device="cuda"), seq_of_token=seq, max_q_len=max(lens),
-                              state_slots=torch.tensor(slots, dtype=torch.int32, device="cuda"),
+                              state_slots=torch.tensor(slots, dtype=torch.int32, device="cuda"), h_q_len=list(lens) if told else [],
                               buf=lambda name, shape, dt: bufs.setdefault((name, tuple(shape)), torch.zeros(shape, dtype=dt, device="cuda")))
         out = torch.full((n, H * V), 7.0, device="cuda")
-        was = CudaKernels.DELTA_BLOCKS, CudaKernels.DELTA_BLOCK_BYTES
-        CudaKernels.DELTA_BLOCKS, CudaKernels.DELTA_BLOCK_BYTES = blocks, scratch
-        try:
-            K.delta_rule(proj, 0, C, z, taps, a_log, dt_bias, state, ctx, out, num_heads=H, num_kv_heads=G, dim=D, v_dim=V)
-        finally:
-            CudaKernels.DELTA_BLOCKS, CudaKernels.DELTA_BLOCK_BYTES = was
+        K.DELTA_BLOCKS, K.DELTA_BLOCK_BYTES, K.DELTA_SEGMENT_MIN_PIECES = blocks, scratch, 8
+        K.delta_rule(proj, 0, C, z, taps, a_log, dt_bias, state, ctx, out, num_heads=H, num_kv_heads=G, dim=D, v_dim=V)
         outs.append(out)
-    assert not blocks or any(name == "delta_blocks" for name, _ in bufs)
-    return torch.cat(outs), state
+    return outs, state, set(chosen)
 
 
 @pytest.mark.parametrize("per_head", [False, True])
 @pytest.mark.parametrize("H,G,D,V", [(4, 2, 128, 128), (3, 3, 64, 48), (2, 1, 128, 16)])
-@pytest.mark.parametrize("lens", [[32], [33, 3, 1], [1, 2, 47, 1, 64], [35, 1, 130]])
+@pytest.mark.parametrize("lens", [[32], [33, 3, 1], [1, 2, 47, 1, 64], [35, 1, 130], [132], [133, 3, 1], [1, 2, 147, 1, 64], [40, 33, 70]])
 def test_four_tokens_at_a_time(lens, H, G, D, V, per_head):
-    want, want_state = walk(False, 0, lens, H, G, D, V, per_head)
+    want, want_state, none = walk(False, 0, lens, H, G, D, V, per_head)
+    assert none == {None}
     piece = 4 * H * (13 * D + 28)
-    for scratch in (192 << 20, piece * 8 * len(lens)):            # the whole step at once, and in segments of eight pieces
-        got, state = walk(True, scratch, lens, H, G, D, V, per_head)
+    cut = sum(lens) // 4 + len(lens) > 8 * len(lens)              # more pieces than eight per sequence
+    for scratch, pieces, told in ((192 << 20, 0, False), (192 << 20, 0, True), (piece * 8 * len(lens), 8 if cut else 0, False)):
+        got, state, chosen = walk(True, scratch, lens, H, G, D, V, per_head, told)
+        assert chosen == {pieces}                                 # the whole step at once, and in segments of eight pieces
         # both are 32-bit sums of the same terms in another order: D of them in a dot product, the sequence's tokens in the state
-        for a, b in ((got, want), (state, want_state)):
+        for a, b in ((torch.cat(got), torch.cat(want)), (state, want_state)):
             assert (a - b).norm() <= 1e-5 * b.norm() and (a - b).abs().max() <= 1e-4 * b.abs().max()
+        at = 0
+        for i, n in enumerate(lens):                              # short portions are walked token by token beside long ones too
+            if n < CudaKernels.DELTA_BLOCK_MIN_TOKENS:
+                assert all(torch.equal(a[at: at + n], b[at: at + n]) for a, b in zip(got, want)) and torch.equal(state[i], want_state[i])
+            at += n
+
+
+def test_short_segments_are_walked_token_by_token():
+    K, state = CudaKernels(), torch.zeros(1, 4, device="cuda")
+    K.DELTA_BLOCK_BYTES = 4 * K._delta_block_floats(32, 128) * 900
+    choose = lambda n, s: K._delta_pieces(1, n, s, 32, 128, 128, 2048, state)
+    assert [choose(3000, 10), choose(3800, 1), choose(4096, 4), choose(3648, 101)] == [0, 512, 128, None]
 
 
 @pytest.mark.parametrize("per_head", [False, True])
