@@ -374,7 +374,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_grouped_kernel(
     int act, float limit) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char * smem = (unsigned char *) (((uintptr_t) smem_raw + 1023) & ~(uintptr_t) 1023);
-    constexpr int W_BYTES = TC_BM * TC_BK * 2, BOX_ROWS = 32, BOX_BYTES = BOX_ROWS * TC_BK * 2, X_BYTES = COLS * TC_BK * 2, STAGE_BYTES = KPS * (W_BYTES + X_BYTES);
+    constexpr int W_BYTES = TC_BM * TC_BK * 2, BOX_ROWS = 32, BOX_BYTES = BOX_ROWS * TC_BK * 2, X_BYTES = COLS * TC_BK * 2;
+    constexpr int STAGE_BYTES = KPS * (W_BYTES + X_BYTES);
     constexpr unsigned TMEM_COLS = 2 * COLS;
     __shared__ __align__(8) unsigned long long full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
     __shared__ unsigned tmem_base_s;

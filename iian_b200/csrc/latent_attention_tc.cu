@@ -433,14 +433,15 @@ IIAN_API int iian_latent_attention_tc_ok(int rank, int width, int H, int page_si
 // parts (1..32): into how many parts the keys are cut; with more than one part_o [N * H, parts, rank] and part_ml [N * H, parts, 2] are needed.
 // status: two ints on the device, zero before the launch; non-zero afterwards means a wait gave up and the output is not valid.
 IIAN_API int iian_latent_attention_tc(const void * q, const void * cache, void * out, float * part_o, float * part_ml, const float * sink,
-                                      const int * cu_q, const int * ctx_len, const int * seq_of_token, const int * block_table, int max_blocks, int N, int S, int max_q_len, int H,
-                                      int rank, int width, int page_size, int num_pages, float scale, int window, int parts,
+                                      const int * cu_q, const int * ctx_len, const int * seq_of_token, const int * block_table, int max_blocks,
+                                      int N, int S, int max_q_len, int H, int rank, int width, int page_size, int num_pages, float scale, int window, int parts,
                                       int * status, cudaStream_t stream) {
     if (N <= 0 || S <= 0) return IIAN_OK;
     const int code = iian_latent_attention_tc_ok(rank, width, H, page_size);
     if (code != IIAN_OK) return code;
     if (!(scale > 0.0f) || status == nullptr || num_pages <= 0 || (long long) N * H < LT_ROWS) return IIAN_ERR_SHAPE;
-    if (parts < 1 || parts > 32 || (parts > 1 && (part_o == nullptr || part_ml == nullptr || ((uintptr_t) part_o & 15) || ((uintptr_t) part_ml & 7)))) return IIAN_ERR_SHAPE;
+    if (parts < 1 || parts > 32) return IIAN_ERR_SHAPE;
+    if (parts > 1 && (part_o == nullptr || part_ml == nullptr || ((uintptr_t) part_o & 15) || ((uintptr_t) part_ml & 7))) return IIAN_ERR_SHAPE;
     if (((uintptr_t) q & 15) || ((uintptr_t) cache & 15) || ((uintptr_t) out & 15)) return IIAN_ERR_ALIGN;
     // a row number is a signed 32-bit coordinate of a copy
     if ((long long) N * H + LT_ROWS > 2147483647LL || (long long) (num_pages + 1) * page_size > 2147483647LL) return IIAN_ERR_LIMIT;
@@ -450,7 +451,8 @@ IIAN_API int iian_latent_attention_tc(const void * q, const void * cache, void *
     rc = lt_make_map(&mk, cache, (long long) num_pages * page_size, width, page_size);
     if (rc != IIAN_OK) return rc;
     LatentTcParams p;
-    p.out = (__nv_bfloat16 *) out; p.q = (const __nv_bfloat16 *) q; p.part_o = part_o; p.part_ml = part_ml; p.scale = scale; p.cu_q = cu_q; p.ctx_len = ctx_len; p.block_table = block_table; p.sink = sink; p.status = status;
+    p.out = (__nv_bfloat16 *) out; p.q = (const __nv_bfloat16 *) q; p.part_o = part_o; p.part_ml = part_ml; p.scale = scale;
+    p.cu_q = cu_q; p.ctx_len = ctx_len; p.block_table = block_table; p.sink = sink; p.status = status;
     p.num_seqs = S; p.max_blocks = max_blocks; p.H = H; p.rank = rank; p.width = width; p.page_size = page_size; p.num_pages = num_pages;
     p.window = window;
     p.scale_log2 = scale * 1.4426950408889634f;
