@@ -59,7 +59,7 @@ struct TcAttnParams {
     const int * ctx_len;            // [S]
     const int * block_table;        // [S, max_blocks]
     int max_blocks, nh, nkv, page_size, num_pages, window, num_seqs;
-    int single;                     // no request has more than one row tile
+    int single;                     // as at_row_tile has it
     float scale_log2;               // scale * log2(e)
     int * status;                   // {code, where}; zero before the launch
     // a sink per head: a logit without key and value that joins the softmax's denominator once, not scaled
@@ -159,12 +159,12 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
     // one warp's work, beside the barriers' and tensor memory's set-up.
     __shared__ AtPlace place;                                // (s < 0: none left)
     __shared__ int span_s[3];
-    const bool search = p.num_seqs > 1 && p.single == 0;
+    const bool search = p.num_seqs > 1 && p.single != 1;
     AtPlace at;
     at.s = -1;
     int tile_lo = 0, k_hi_a = 0, k_hi = 0;                   // first key tile; last key of the first group of rows, of all
     if (!search || warp == 2) {
-        const bool mine = at_row_tile<AT_BN>(p.cu_q, p.ctx_len, p.num_seqs, p.single != 0, G, CTA_ROWS, (int) (blockIdx.z * kAtUnits + blockIdx.y), at);
+        const bool mine = at_row_tile<AT_BN>(p.cu_q, p.ctx_len, p.num_seqs, p.single, G, CTA_ROWS, (int) (blockIdx.z * kAtUnits + blockIdx.y), at);
         if (!mine && !search) return;
         if (mine) {
             const int pos0 = at.ctx - at.q_len, row0 = at.tile * CTA_ROWS, last = at.q_len * G - 1, first = pos0 + row0 / G;
@@ -774,7 +774,7 @@ IIAN_API int iian_attention_tc_kept(const void * q, long long ld_q, const void *
         configured[kept ? 1 : 0] = true;
     }
     const dim3 grid = at_grid(N, S, max_q_len, nh, nkv, AT_ROWS);
-    p.single = at_tiles(max_q_len, nh / nkv, AT_ROWS) <= 1;
+    p.single = at_single(N, S, max_q_len, nh / nkv, AT_ROWS, nkv);
     if (kept) attention_tc_kernel<AT_KEPT><<<grid, AT_THREADS, smem, stream>>>(mk, mv, p);
     else attention_tc_kernel<AT_PLAIN><<<grid, AT_THREADS, smem, stream>>>(mk, mv, p);
     return iian_launch_status();
@@ -816,7 +816,7 @@ IIAN_API int iian_attention_tc_capped(const void * q, long long ld_q, const void
         configured = true;
     }
     const dim3 grid = at_grid(N, S, max_q_len, nh, nkv, AT_ROWS);
-    p.single = at_tiles(max_q_len, nh / nkv, AT_ROWS) <= 1;
+    p.single = at_single(N, S, max_q_len, nh / nkv, AT_ROWS, nkv);
     attention_tc_kernel<AT_CAP><<<grid, AT_THREADS, smem, stream>>>(mk, mv, p);
     return iian_launch_status();
 }
@@ -854,7 +854,7 @@ IIAN_API int iian_attention_tc_difference(const void * q, const void * k_cache, 
         configured = true;
     }
     const dim3 grid = at_grid(N, S, max_q_len, nh, nkv, AT_BM);
-    p.single = at_tiles(max_q_len, nh / nkv, AT_BM) <= 1;
+    p.single = at_single(N, S, max_q_len, nh / nkv, AT_BM, nkv);
     attention_tc_kernel<AT_DIFF><<<grid, AT_THREADS, smem, stream>>>(mk, mv, p);
     return iian_launch_status();
 }

@@ -47,7 +47,7 @@ struct LatentTcParams {
     const float * sink;             // [H] or null
     int * status;                   // {code, where}; zero before the launch
     int num_seqs, max_blocks, H, rank, width, page_size, num_pages, window;
-    int single;                     // no request has more than one row tile
+    int single;                     // as at_row_tile has it
     float scale, scale_log2, sink_to_raw;
 };
 
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(
     const int shares = p.rank / LT_SHARE;
     const int H = p.H;
     AtPlace at;
-    if (!at_row_tile<LT_KEYS>(p.cu_q, p.ctx_len, p.num_seqs, p.single != 0, H, LT_ROWS, (int) blockIdx.x / shares, at)) return;
+    if (!at_row_tile<LT_KEYS>(p.cu_q, p.ctx_len, p.num_seqs, p.single, H, LT_ROWS, (int) blockIdx.x / shares, at)) return;
     const int s = at.s, row_tile = at.tile;
     const int part = (int) blockIdx.x % shares;                    // this CTA's share of the values: chunks own .. own + LT_OWN - 1
     const int own = part * LT_OWN;
@@ -457,7 +457,7 @@ IIAN_API int iian_latent_attention_tc(const void * q, const void * cache, void *
     p.window = window;
     p.scale_log2 = scale * 1.4426950408889634f;
     p.sink_to_raw = 1.0f / scale;
-    p.single = at_tiles(max_q_len, H, LT_ROWS) <= 1;
+    p.single = at_single(N, S, max_q_len, H, LT_ROWS, (rank / LT_SHARE) * parts);
     const dim3 grid((unsigned) (at_units(N, S, max_q_len, H, LT_ROWS) * (rank / LT_SHARE)), (unsigned) parts);
     int rc2 = IIAN_OK;
     switch (width / LT_CHUNK - LT_OWN) {

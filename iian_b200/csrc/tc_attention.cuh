@@ -121,21 +121,24 @@ struct AtPlace { int s, tile, q0, q_len, ctx; };
 // behind 200 to 6,000 cached ones, heads of 128).  A row tile of `rows` rows sees ceil((pos0 + last token + 1) / KEYS) key tiles, which
 // grows with its number; the number of row tiles of a request that see L key tiles or more is a closed form, and a warp finds the L of the
 // unit by bisection with its lanes over the requests -- to an eighth of the longest walk, which balances as well and takes three
-// steps of some hundred cycles.  `single`: no request has more than one row tile; then the order of the batch, which needs no search, is
-// kept (68 portions of 30 tokens 37.6 us, ranked 41.8).  A whole warp calls it.
+// steps of some hundred cycles.  Where no request has more than one row tile the order of the batch, which needs no search, is kept if all
+// CTAs fit at once (`single` 1) or the longest walk is no 1.75 times the mean (`single` 2; 68 portions of 30 tokens 37.9 us,
+// ranked 43; 100 of them behind 0 to 4,000 tokens 256, in the batch's order 272).  A whole warp
+// calls it.
 template <int KEYS>
-__device__ __forceinline__ bool at_row_tile(const int * __restrict__ cu_q, const int * __restrict__ ctx_len, int num_seqs, bool single, int G,
+__device__ __forceinline__ bool at_row_tile(const int * __restrict__ cu_q, const int * __restrict__ ctx_len, int num_seqs, int single, int G,
                                             int rows, int unit, AtPlace & at) {
     auto place = [&](int s, int q0, int q_len, int ctx, int tile) {
         at.s = s; at.q0 = q0; at.q_len = q_len; at.ctx = ctx; at.tile = tile;
         return tile >= 0;
     };
-    if (num_seqs == 1 || single) {
-        const int s = num_seqs == 1 ? 0 : unit;
+    auto in_order = [&](int s, int before) {
         if (s >= num_seqs) return false;
         const int q0 = cu_q[s], q_len = cu_q[s + 1] - q0, ctx = ctx_len[s];
-        return place(s, q0, q_len, ctx, (q_len * G + rows - 1) / rows - 1 - (num_seqs == 1 ? unit : 0));
-    }
+        return place(s, q0, q_len, ctx, (q_len * G + rows - 1) / rows - 1 - before);
+    };
+    if (num_seqs == 1) return in_order(0, unit);
+    if (single == 1) return in_order(unit, 0);
     const int lane = threadIdx.x & 31;
     constexpr int HELD = 4;                                  // requests a lane holds: lane, lane + 32, ...; further ones are read again
     auto request = [&](int i, int & len, int & pos0) {
@@ -147,10 +150,11 @@ __device__ __forceinline__ bool at_row_tile(const int * __restrict__ cu_q, const
         if (x <= 0) return n;
         return x < len ? n - x * G / rows : 0;               // the first of them holds row x * G
     };
-    int len[HELD], pos0[HELD], all = 0, most = 0;
+    int len[HELD], pos0[HELD], all = 0, most = 0, sum = 0;
     auto add = [&](int q, int p) {
         all += tiles_from(q, p, 1);
         most = max(most, q > 0 ? p + q : 0);
+        sum += p + q;
     };
 #pragma unroll
     for (int h = 0; h < HELD; h++) request(lane + 32 * h, len[h], pos0[h]);
@@ -164,6 +168,10 @@ __device__ __forceinline__ bool at_row_tile(const int * __restrict__ cu_q, const
     }
     all = __reduce_add_sync(0xffffffffu, all);
     most = __reduce_max_sync(0xffffffffu, most);
+    if (single == 2) {
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        if ((float) most * (float) (4 * num_seqs) < 7.0f * (float) sum) return in_order(unit, 0);
+    }
     if (all <= unit) return false;
     const int step = (most + 8 * KEYS - 1) / (8 * KEYS);     // key tiles to an eighth
     int lo = 0, above = 0;                                   // row tiles that see 1 + step * lo or more > unit >= those of a higher eighth = above
@@ -212,6 +220,11 @@ static inline long long at_tiles(int max_q_len, int G, int rows) { return ((long
 static inline long long at_units(int N, int S, int max_q_len, int G, int rows) {
     const long long each = at_tiles(max_q_len, G, rows) * S, all = (long long) N * G / rows + S;
     return each < all ? each : all;
+}
+// `single` of at_row_tile for a step whose row tiles are `copies` CTAs each, one CTA an SM
+static inline int at_single(int N, int S, int max_q_len, int G, int rows, int copies) {
+    if (at_tiles(max_q_len, G, rows) > 1) return 0;
+    return at_units(N, S, max_q_len, G, rows) * copies <= 148 ? 1 : 2;
 }
 
 typedef CUresult (*AtEncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
