@@ -664,9 +664,9 @@ delta_scan_kernel(const float * __restrict__ qn, const float * __restrict__ kn, 
 // Everything is float32; the decays' products are of at most four factors, taken as such (no logarithms), and only ever shrink.
 //   delta_block  per four tokens and head: the 13 vectors G_t k_t, G_t q_t, G_3t k_t, G_3 and the 28 numbers beta, A, B, one piece of
 //                memory (tokens beyond a sequence's last count as k = q = 0, decay 1, beta 0: nothing changes).
-//   delta_block_scan  the recurrence: the pieces come through a ring of shared memory, kBlocksPerStage at a time.
+//   delta_block_scan  the recurrence: the pieces come through a ring of four stages in shared memory, PER at a time.
 constexpr int kBlockNumbers = 28;               // beta [4], A (1,0) (2,0) (2,1) (3,0) (3,1) (3,2) 0 0, B [4][4] (zero above the diagonal)
-constexpr int kBlocksPerStage = 2, kBlockStages = 4;
+constexpr int kBlockStages = 4;
 
 __device__ __forceinline__ float dr_both(unsigned long long v) {
     const float2 f = unpack2(v);
@@ -758,10 +758,11 @@ delta_block_kernel(const float * __restrict__ qn, const float * __restrict__ kn,
 // V a multiple of kCols; state and values on 16-byte boundaries.
 // Sequences with fewer than at_least tokens are walked token by token as in the scan above, in the same launch: a piece costs more than a
 // token, and a launch of their own would wait for the long ones' chain (a portion of 100 tokens beside 100
-// decoded ones, 16 heads with a decay per channel, through the mixer: 142 us, in two launches 166).
+// decoded ones, 16 heads with a decay per channel, through the mixer: 131 us, in two launches 166).  PER: pieces of a stage, 2 where the long
+// walks decide, 1 where many short ones do, so that seven CTAs share an SM and not four (the same 131 us for 142, but 1,500 tokens 386 for 363).
 constexpr int kPairLanes = 16;
 
-template <int E, bool HEAD, typename A>
+template <int E, int PER, bool HEAD, typename A>
 __global__ void __launch_bounds__(kCols / 2 * kPairLanes)
 delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restrict__ qn, const float * __restrict__ kn,
                         const float * __restrict__ vv, const float * __restrict__ beta, const float * __restrict__ decay,
@@ -769,7 +770,7 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
                         long long tail_off, const A * __restrict__ proj, long long ld, int col_off, int n_taps,
                         const int * __restrict__ cu_q, const int * __restrict__ state_slots, float * __restrict__ out,
                         int from, int pieces, int at_least, int H, int G, int V) {
-    constexpr int D = E * kPairLanes, BLOCK = 13 * D + kBlockNumbers, PIECE = BLOCK + 4 * kCols, STAGE = kBlocksPerStage * PIECE;
+    constexpr int D = E * kPairLanes, BLOCK = 13 * D + kBlockNumbers, PIECE = BLOCK + 4 * kCols, STAGE = PER * PIECE;
     constexpr int kThreads = kCols / 2 * kPairLanes;
     extern __shared__ __align__(16) float sm[];
     const int cb = blockIdx.x, h = blockIdx.y, s = blockIdx.z;
@@ -777,10 +778,11 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
     const int q0 = cu_q[s], q1 = cu_q[s + 1], slot = state_slots[s], HV = H * V;
     const int t0 = q0 + from, t1 = pieces > 0 ? min(q1, t0 + 4 * pieces) : q1;
     if (q1 - q0 < at_least) {
-        static_assert(kCols / 2 * kPairLanes == kCols * kLanes && scan_floats(HEAD, D, 16) <= kBlockStages * STAGE, "both walks fit one launch");
+        constexpr int CHUNK = scan_floats(HEAD, D, 16) <= kBlockStages * STAGE ? 16 : 8;
+        static_assert(kCols / 2 * kPairLanes == kCols * kLanes && scan_floats(HEAD, D, CHUNK) <= kBlockStages * STAGE, "both walks fit one launch");
         if (from == 0)
             delta_scan<D / kLanes, true, HEAD, A>(sm, qn, kn, vv, beta, decay, qk, state, state_stride, tail_off, proj, ld, col_off, n_taps, cu_q,
-                                                  state_slots, out, H, G, D, V, 16);
+                                                  state_slots, out, H, G, D, V, CHUNK);
         return;
     }
     if (t0 >= t1) return;
@@ -790,14 +792,14 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
         return;
     }
     float * st = state + (size_t) slot * state_stride;
-    const int n_blocks = (t1 - t0 + 3) / 4, turns = (n_blocks + kBlocksPerStage - 1) / kBlocksPerStage;
+    const int n_blocks = (t1 - t0 + 3) / 4, turns = (n_blocks + PER - 1) / PER;
     const float * mine = blocks + (first_piece(cu_q, s, pieces) * H + h) * BLOCK;
     auto fill = [&](int turn) {
         if (turn < turns) {
             float * to = sm + (turn % kBlockStages) * STAGE;
 #pragma unroll
-            for (int b = 0; b < kBlocksPerStage; b++) {
-                const int c = turn * kBlocksPerStage + b;
+            for (int b = 0; b < PER; b++) {
+                const int c = turn * PER + b;
                 if (c >= n_blocks) break;
                 const float * src = mine + (size_t) c * H * BLOCK;
                 for (int e = tid; e < BLOCK / 4; e += kThreads) copy16(to + b * PIECE + 4 * e, src + 4 * e);
@@ -846,8 +848,8 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
         fill(turn + kBlockStages - 1);
         const float * stage = sm + (turn % kBlockStages) * STAGE;
 #pragma unroll
-        for (int b = 0; b < kBlocksPerStage; b++) {
-            const int c = turn * kBlocksPerStage + b;
+        for (int b = 0; b < PER; b++) {
+            const int c = turn * PER + b;
             if (c >= n_blocks) break;
             const float * vec = stage + b * PIECE;
             const float * num = vec + 13 * D;
@@ -954,9 +956,14 @@ IIAN_API int iian_delta_block_scan(const float * qn, const float * kn, const flo
     if (state_stride % 4 || (((uintptr_t) blocks | (uintptr_t) qn | (uintptr_t) kn | (uintptr_t) vv | (uintptr_t) decay | (uintptr_t) state) & 15))
         return IIAN_ERR_ALIGN;
     typedef __nv_bfloat16 bf;
-    const size_t smem = (size_t) kBlockStages * kBlocksPerStage * (13 * D + kBlockNumbers + 4 * kCols) * sizeof(float);
-    auto scan = D == 128 ? (per_head ? delta_block_scan_kernel<8, true, bf> : delta_block_scan_kernel<8, false, bf>)
-                         : (per_head ? delta_block_scan_kernel<4, true, bf> : delta_block_scan_kernel<4, false, bf>);
+    const int per = max_q_len < 4 * S ? 1 : 2;
+    const size_t smem = (size_t) kBlockStages * per * (13 * D + kBlockNumbers + 4 * kCols) * sizeof(float);
+    auto by_head = [&](auto depth, auto each) {
+        constexpr int E = decltype(depth)::value, PER = decltype(each)::value;
+        return per_head ? delta_block_scan_kernel<E, PER, true, bf> : delta_block_scan_kernel<E, PER, false, bf>;
+    };
+    auto by_depth = [&](auto each) { return D == 128 ? by_head(std::integral_constant<int, 8>(), each) : by_head(std::integral_constant<int, 4>(), each); };
+    auto scan = per == 2 ? by_depth(std::integral_constant<int, 2>()) : by_depth(std::integral_constant<int, 1>());
     const cudaError_t e = cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
     if (e != cudaSuccess) return 1000 + (int) e;
     const int step = pieces > 0 ? 4 * pieces : max_q_len;
