@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(128, STAGES == 2 ? 3 : 2) attention_decode_ker
     const int split = blockIdx.z % p.n_split;
     int s = blockIdx.z / p.n_split;
     int q0 = p.cu_q[s], q_end = p.cu_q[s + 1], ctx = p.ctx_len[s];       // (on their way while the ranking waits for its own loads)
-    if (p.longest_first) {
+    if (!CLUSTER && p.longest_first) {                       // (a cluster's CTAs are the parts of split keys: nothing to rank)
         const int t = longest_first(p.ctx_len, gridDim.z, s, p.longest_first);
         if (t != s) { s = t; q0 = p.cu_q[s]; q_end = p.cu_q[s + 1]; ctx = p.ctx_len[s]; }
     }
