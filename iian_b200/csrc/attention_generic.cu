@@ -212,6 +212,9 @@ paged_attention_tile_kernel(
             k_lo = min(k_lo, window > 0 ? max(0, p - window + 1) : 0);
         }
         first = end;
+        int last[8];                                   // the items' last keys in this run, -1: the item is another run's
+#pragma unroll
+        for (int i = 0; i < 8; i++) last[i] = tok[i] >= begin && tok[i] < end ? hi[i] : -1;
         const int * bt = block_table + (size_t) s * max_blocks;
         const int kb0 = (k_lo / 32) * 32;
         auto fill = [&](int kb, int stage) {           // four lanes a key
@@ -247,7 +250,7 @@ paged_attention_tile_kernel(
             const int j = kb + lane;
             bool any = false;
 #pragma unroll
-            for (int i = 0; i < 8; i++) any |= tok[i] >= begin && tok[i] < end && kb <= hi[i] && kb + 31 >= lo[i];
+            for (int i = 0; i < 8; i++) any |= kb <= last[i] && kb + 31 >= lo[i];
             if (any) {                                 // the same for all lanes: an item's numbers are the warp's
                 unsigned long long dot[4] = {0ull, 0ull, 0ull, 0ull};
                 const float * kr = ks + lane * kTileLd;
@@ -270,7 +273,7 @@ paged_attention_tile_kernel(
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
                     const float2 two = unpack2(dot[i >> 1]);
-                    const bool valid = here && tok[i] >= begin && tok[i] < end && j >= lo[i] && j <= hi[i];
+                    const bool valid = here && j >= lo[i] && j <= last[i];
                     const float sc = valid ? ((i & 1) ? two.y : two.x) * scale : -INFINITY;
                     const float tile_max = warp_max(sc);
                     float pj = 0.0f;
