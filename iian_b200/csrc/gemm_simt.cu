@@ -1,14 +1,17 @@
 // out[n, m] = sum_k x[n, k] * w[m, k]: the plain matrix product of the 32-bit path, and the
 // fallback for element-type combinations the tensor-core kernels do not take.
 //
-// Three forms with the same bits: tiles of register blocks for steps of many rows and a form that streams the weights for steps of
-// few (both: float32 operands with rows of whole 16-byte pieces), and the plain one for everything else.
+// Four forms with the same bits: tiles of register blocks for steps of many rows, smaller tiles fed by a ring for a few hundred, a form
+// that streams the weights for steps of few (all three: float32 operands with rows of whole 16-byte pieces), and the plain one for
+// everything else.
 //
 // Weights are row-major [out_features, in_features] exactly as the file stores them, which is
 // also the reference's layout (ggml_mul_mat(W, x) = W x, src/iian/graph.cpp:121-160).  Products
 // and sums are float32 FMAs (no reduced-precision matrix mode); every output element adds its
 // K products in the order k = 0, 1, 2, ..., so a row's result does not depend on how many other
 // rows the batch has.
+#include <algorithm>
+
 #include "common.cuh"
 #include "packed.cuh"
 
@@ -167,6 +170,88 @@ gemm_tile_kernel(const float * __restrict__ x, const float * __restrict__ w, TO 
     }
 }
 
+// Small tiles for steps whose large ones would leave SMs idle: a warp covers 4 TN rows x 8 TM columns, a CTA WY x WX warps.  Operands lie
+// in shared memory as they do in memory, along k, so that they come by cp.async through a ring and nothing is turned around; a
+// thread reads four k of a row at once.  The multiply-adds are single ones: packed ones want neighbours of one k side by side.
+// Lanes are dealt so that neighbours share a row of one operand or of the other (bits 0 and 4 pick the row of x, bits 1 to 3 that of w):
+// 16-byte reads then take 2 clocks a warp, 4 where equal addresses lie 8 lanes apart.  What bounds it: one warp a scheduler leaves
+// the 4-clock chain and the reads' latency bare, more of them the dispatch of three-operand multiply-adds (41 clocks for 32).
+template <int TN, int TM, int WY, int WX, int STAGES, int DEPTH, typename TO>
+__global__ void __launch_bounds__(WY * WX * 32)
+gemm_ring_kernel(const float * __restrict__ x, const float * __restrict__ w, TO * __restrict__ out, int N, int M, int K) {
+    constexpr int TILE_N = 4 * TN * WY, TILE_M = 8 * TM * WX, THREADS = WY * WX * 32, LD = DEPTH + 4, PIECES = DEPTH / 4;
+    constexpr int LOADS = (TILE_N + TILE_M) * PIECES / THREADS;
+    static_assert(LOADS * THREADS == (TILE_N + TILE_M) * PIECES && THREADS % PIECES == 0, "whole pieces per thread");
+    extern __shared__ __align__(16) float ring[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n0 = blockIdx.y * TILE_N, m0 = blockIdx.x * TILE_M;
+    const int turns = (K + DEPTH - 1) / DEPTH;
+    auto fill = [&](int s) {
+        if (s < turns) {
+            const int at = tid % PIECES * 4, k = s * DEPTH + at; // K is a multiple of 4: a piece lies inside or outside as a whole
+            float * to = ring + (s % STAGES) * (TILE_N + TILE_M) * LD + at;
+#pragma unroll
+            for (int i = 0; i < LOADS; i++) {
+                const int r = (tid + i * THREADS) / PIECES;
+                const bool is_x = r < TILE_N;
+                const int g = is_x ? n0 + r : m0 + r - TILE_N;
+                const bool in = k < K && g < (is_x ? N : M);
+                copy16(to + r * LD, in ? (is_x ? x : w) + (size_t) g * K + k : x, in);
+            }
+        }
+        asm volatile("cp.async.commit_group;");
+    };
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; s++) fill(s);
+    float acc[TN][TM];
+#pragma unroll
+    for (int i = 0; i < TN; i++)
+#pragma unroll
+        for (int j = 0; j < TM; j++) acc[i][j] = 0.0f;
+    const int row = warp / WX * 4 * TN + ((lane & 1) | (lane >> 4) << 1), col = warp % WX * 8 * TM + ((lane >> 1) & 7);
+    for (int s = 0; s < turns; s++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2));
+        __syncthreads();                                     // this stage has landed for everyone; the one before has been read by everyone
+        fill(s + STAGES - 1);
+        const float * xr = ring + ((s % STAGES) * (TILE_N + TILE_M) + row) * LD;
+        const float * wr = ring + ((s % STAGES) * (TILE_N + TILE_M) + TILE_N + col) * LD;
+#pragma unroll
+        for (int k = 0; k < DEPTH; k += 4) {
+            float4 a[TN], b[TM];
+#pragma unroll
+            for (int i = 0; i < TN; i++) a[i] = *reinterpret_cast<const float4 *>(xr + i * 4 * LD + k);
+#pragma unroll
+            for (int j = 0; j < TM; j++) b[j] = *reinterpret_cast<const float4 *>(wr + j * 8 * LD + k);
+#pragma unroll
+            for (int i = 0; i < TN; i++)
+#pragma unroll
+                for (int j = 0; j < TM; j++) acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < TN; i++)
+#pragma unroll
+                for (int j = 0; j < TM; j++) acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < TN; i++)
+#pragma unroll
+                for (int j = 0; j < TM; j++) acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < TN; i++)
+#pragma unroll
+                for (int j = 0; j < TM; j++) acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < TN; i++) {
+        const int n = n0 + row + 4 * i;
+        if (n >= N) continue;
+#pragma unroll
+        for (int j = 0; j < TM; j++) {
+            const int m = m0 + col + 8 * j;
+            if (m < M) out[(size_t) n * M + m] = from_f32<TO>(acc[i][j]);
+        }
+    }
+}
+
 // Steps of few rows: the weights stream through a ring of shared-memory stages (cp.async, 128 of K per stage), TILE_M weight
 // rows per CTA; a thread owns one weight row and every (128 / TILE_M)-th row of x, so that an output stays one chain over k.
 // What bounds it: HBM where there are many weight rows (32 per CTA: four CTAs an SM hold some 130 KB in flight); with few (8 per
@@ -237,6 +322,18 @@ static int launch_tile(const float * x, const float * w, TO * out, int N, int M,
     return iian_launch_status();
 }
 
+template <int TN, int TM, int STAGES, int DEPTH, typename TO>
+static int launch_ring(const float * x, const float * w, TO * out, int N, int M, int K, cudaStream_t stream) {
+    constexpr int TILE_N = 8 * TN, TILE_M = 16 * TM;         // two by two warps
+    constexpr size_t smem = (size_t) STAGES * (TILE_N + TILE_M) * (DEPTH + 4) * sizeof(float);
+    auto kernel = gemm_ring_kernel<TN, TM, 2, 2, STAGES, DEPTH, TO>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    if (e != cudaSuccess) return 1000 + (int) e;
+    const dim3 grid((M + TILE_M - 1) / TILE_M, (N + TILE_N - 1) / TILE_N);
+    kernel<<<grid, 128, smem, stream>>>(x, w, out, N, M, K);
+    return iian_launch_status();
+}
+
 template <int TILE_M, int STAGES, int PER, typename TO>
 static int launch_rows(const float * x, const float * w, TO * out, int N, int M, int K, cudaStream_t stream) {
     const size_t smem = (size_t) STAGES * (TILE_M + N) * (kRowsK + 4) * sizeof(float);
@@ -252,12 +349,16 @@ static int launch_rows(const float * x, const float * w, TO * out, int N, int M,
 // Up to kRowsMax rows the streaming form; its CTAs own 32 weight rows where there are enough of them for every SM, 8 below
 // (us: 2 x 6,144 x 1,024 14.3 against 16.5; 16 x 4,096 x 4,096 67 against 96; but 4 x 4,096 x 12,288 113 against 76, 12 x 1,024 x 1,024
 // 18.7 against 10.8).  Above, the tile that makes the fullest SM finish first; us:
-//   rows x columns x K     64 x 128   64 x 64 (8 x 4)   32 x 64 (4 x 4)   the plain form
-//   301 x 4,096 x 1,024       108            87               103              156
-//   301 x 1,024 x 2,048       127            76                83              157
-//   17 x 4,096 x 1,024         65            39                31               74
-//   1,024 x 4,096 x 4,096     775           727             1,017            1,548
-//   2,048 x 6,144 x 4,096   2,023         2,107             3,017            3,996
+//   rows x columns x K     64 x 128   64 x 64 (8 x 4)   ring: 32 x 64   32 x 32   16 x 32   the plain form
+//   301 x 4,096 x 1,024       108            87               78            82        99         156
+//   301 x 1,024 x 2,048       127            76               76            56        58         157
+//   301 x 6,144 x 1,024       109           119              105           115       136
+//   301 x 1,024 x 3,072       185           129              111            82        84
+//   17 x 4,096 x 1,024         65            39               25            15        16          74
+//   17 x 1,024 x 2,048        130            78               50            28        23
+//   120 x 1,024 x 2,048       130            78               52            29        31
+//   1,024 x 4,096 x 4,096     775           727              781           930     1,070       1,548
+//   2,048 x 6,144 x 4,096   2,023         2,107                                                3,996
 template <typename TO>
 static int launch_f32(const float * x, const float * w, TO * out, int N, int M, int K, cudaStream_t stream) {
     if (N <= kRowsMax) {
@@ -265,15 +366,20 @@ static int launch_f32(const float * x, const float * w, TO * out, int N, int M, 
         if (N <= 4) return launch_rows<32, 3, 1, TO>(x, w, out, N, M, K, stream);
         return N <= 8 ? launch_rows<32, 3, 2, TO>(x, w, out, N, M, K, stream) : launch_rows<32, 3, 4, TO>(x, w, out, N, M, K, stream);
     }
-    // us per 1,024 of K: `alone` for the first tile of an SM, `more` for each further one (they run side by side)
-    auto cost = [&](int tn, int tm, double alone, double more) {
-        const long long tiles = (long long) ((N + tn - 1) / tn) * ((M + tm - 1) / tm);
-        return alone + more * (double) ((tiles - 1) / 148);
+    // us per 1,024 of K: `alone` for the first tile of an SM, `more` for each further one that runs beside it (up to `beside`), `then` for
+    // those that wait for one of them to end
+    auto cost = [&](int tn, int tm, double alone, double more, int beside, double then) {
+        const long long tiles = (long long) ((N + tn - 1) / tn) * ((M + tm - 1) / tm), further = (tiles - 1) / 148;
+        return alone + more * (double) std::min<long long>(further, beside) + then * (double) std::max<long long>(further - beside, 0);
     };
-    const double wide = cost(64, 128, 65.0, 43.0), even = cost(64, 64, 40.0, 24.0), small = cost(32, 64, 31.0, 17.5);
-    if (wide <= even && wide <= small) return launch_tile<64, 128, 8, 8, 1, TO>(x, w, out, N, M, K, stream);
-    if (even <= small) return launch_tile<64, 64, 8, 4, 3, TO>(x, w, out, N, M, K, stream);
-    return launch_tile<32, 64, 4, 4, 6, TO>(x, w, out, N, M, K, stream);
+    const double wide = cost(64, 128, 65.0, 43.0, 1, 43.0), even = cost(64, 64, 40.0, 24.0, 1, 24.0);
+    const double half = cost(32, 64, 24.0, 13.3, 4, 13.3), small = cost(32, 32, 14.5, 6.8, 2, 9.2), least = cost(16, 32, 12.3, 4.3, 4, 5.4);
+    const double best = std::min({wide, even, half, small, least});
+    if (wide == best) return launch_tile<64, 128, 8, 8, 1, TO>(x, w, out, N, M, K, stream);
+    if (even == best) return launch_tile<64, 64, 8, 4, 3, TO>(x, w, out, N, M, K, stream);
+    if (half == best) return launch_ring<4, 4, 3, 32, TO>(x, w, out, N, M, K, stream);
+    if (small == best) return launch_ring<4, 2, 4, 64, TO>(x, w, out, N, M, K, stream);
+    return launch_ring<2, 2, 4, 32, TO>(x, w, out, N, M, K, stream);
 }
 
 template <typename TX, typename TW, typename TO>

@@ -588,6 +588,18 @@ def test_gemm_simt_forms_give_the_same_bits(od, N, M, K_):
     assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("N,M", [(120, 4100), (100, 1030), (31, 4099), (17, 1)])
+@pytest.mark.parametrize("K_", [4, 36, 64, 196, 260])
+def test_gemm_simt_small_tiles_give_the_same_bits(N, M, K_):
+    """The three sizes of tile that a ring feeds (by the fullest SM: 32 x 64, 32 x 32, 16 x 32), K ending inside a stage and with one."""
+    x, w = rnd(N, K_, seed=42), rnd(M, K_, seed=43)
+    odd = torch.empty(N * K_ + 1, dtype=torch.float32, device="cuda")[1:].view(N, K_).copy_(x)
+    a, b = (torch.full((N, M), float("nan"), device="cuda") for _ in range(2))
+    K().gemm_simt(x, w, a)
+    K().gemm_simt(odd, w, b)
+    assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("window", [0, 19])
 @pytest.mark.parametrize("ctx_lens,q_lens", [([8], [8]), ([45], [40]), ([75, 266], [75, 226]), ([23, 101, 20], [20, 1, 13]),
                                              ([13, 22, 39, 41, 67], [3, 2, 9, 1, 17]), ([2, 3, 4, 5, 6, 7, 36], [2, 2, 2, 2, 2, 2, 30])])
