@@ -152,18 +152,21 @@ __global__ void paged_attention_generic_kernel(
     }
 }
 
-// The same attention in float32 for neighbouring tokens: a CTA owns 32 (token, head) items of one KV head, eight a warp, and its key
+// The same attention in float32 for neighbouring tokens: a CTA owns 32 (token, head) items of one KV head, four a warp, and its key
 // tiles -- the same 32 keys from the same multiples of 32 -- come once through two stages of shared memory for all of them.  Every
 // item's arithmetic is the kernel's above term by term (a lane is a key in the scores and four output entries in the sum; packed
 // multiply-adds of two items, or of two entries, round as single ones do), so an item has the same bits whichever kernel it falls to.
-// What bounds it: reads of shared memory (a tile's keys and values per warp against eight items' multiply-adds).  2 requests,
-// 301 tokens x 16 heads of 128: 487 -> 77 us; 2,048 tokens 19.6 -> 1.2 ms (a warp per item, each reading its keys row by row from
-// global memory).
+// What bounds it: reads of shared memory.  A warp's 16-byte read of one key row a lane takes 4 clocks, of one address for all lanes 2: a
+// tile's scores are 3,072 clocks of an SM, its sums 1,536 (measured 3,100 and about 1,600, copies 1,300, the softmax 1,300 with its
+// shuffles for four items side by side).  Eight warps of four items, so that a scheduler has two to choose from, and a page looked up
+// a tile before its copy.  2 requests, 301 tokens x 16 heads of 128: 44 us (four warps of eight items, an item's softmax after
+// another's: 72; a warp per item, each reading its keys row by row from global memory: 487).
 constexpr int kTileHeadDim = 128;
+constexpr int kTileWarps = 8, kWarpItems = kTileItems / kTileWarps;
 constexpr int kTileLd = kTileHeadDim + 4;
-constexpr size_t kTileSmem = (size_t) (2 * 2 * 32 * kTileLd + kTileItems * kTileHeadDim + kGenWarps * 8 * 64) * sizeof(float);
+constexpr size_t kTileSmem = (size_t) (2 * 2 * 32 * kTileLd + kTileItems * kTileHeadDim + kTileItems * 32) * sizeof(float);
 
-__global__ void __launch_bounds__(kGenWarps * 32)
+__global__ void __launch_bounds__(kTileWarps * 32)
 paged_attention_tile_kernel(
     const float * __restrict__ q, const float * __restrict__ k_cache, const float * __restrict__ v_cache,
     float * __restrict__ out, const int * __restrict__ positions, const int * __restrict__ seq_of_token,
@@ -174,23 +177,37 @@ paged_attention_tile_kernel(
     float * stages = sm;                               // [2][keys | values][32][kTileLd]
     float * qs = sm + 2 * 2 * 32 * kTileLd;            // [16 pairs of items][hd][2]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    float * ps = qs + kTileItems * kTileHeadDim + warp * 8 * 64;       // [8 items][32 keys][2]: probabilities, each twice
-    __shared__ unsigned good[2];                       // keys of a stage whose page exists
+    float * ps = qs + kTileItems * kTileHeadDim + warp * kWarpItems * 32;       // [items of a warp][32 keys]: probabilities
+    __shared__ unsigned char good[2][kTileWarps];      // keys of a stage whose page exists, four a warp
     const int G = nh / nkv, tokens = kTileItems / G;
     const int t0 = blockIdx.x * tokens, kvh = blockIdx.y;
     if (!tile_is_shared(seq_of_token, t0, tokens, N)) return;
     const int n_tok = min(tokens, N - t0), n_items = n_tok * G;
-    for (int e = tid; e < kTileItems * hd; e += kGenWarps * 32) {
-        const int item = e / hd, d = e % hd;
-        const float v = item < n_items ? q[((size_t) (t0 + item / G) * nh + kvh * G + item % G) * hd + d] : 0.0f;
-        qs[((item >> 1) * hd + d) * 2 + (item & 1)] = v;
-    }
-    unsigned long long acc[8][2];
-    float m[8], l[8];
-    int lo[8], hi[8], tok[8];                          // first and last key; the token, -1: no item
+    {                                                  // eight threads an item
+        const int item = tid >> 3;
+        const float * from = q + ((size_t) (t0 + item / G) * nh + kvh * G + item % G) * hd;
+        float * to = qs + (item >> 1) * hd * 2 + (item & 1);
+        float4 v[kTileHeadDim / 32];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const int item = warp * 8 + i, t = t0 + item / G;
+        for (int u = 0; u < kTileHeadDim / 32; u++) {
+            const int d = ((tid & 7) + 8 * u) * 4;
+            v[u] = item < n_items && d < hd ? __ldg(reinterpret_cast<const float4 *>(from + d)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int u = 0; u < kTileHeadDim / 32; u++) {
+            const int d = ((tid & 7) + 8 * u) * 4;
+            if (d < hd) {
+                to[d * 2] = v[u].x; to[d * 2 + 2] = v[u].y;
+                to[d * 2 + 4] = v[u].z; to[d * 2 + 6] = v[u].w;
+            }
+        }
+    }
+    unsigned long long acc[kWarpItems][2];
+    float m[kWarpItems], l[kWarpItems];
+    int lo[kWarpItems], hi[kWarpItems], tok[kWarpItems];                          // first and last key; the token, -1: no item
+#pragma unroll
+    for (int i = 0; i < kWarpItems; i++) {
+        const int item = warp * kWarpItems + i, t = t0 + item / G;
         const bool real = item < n_items;
         const float sk = sink != nullptr ? sink[kvh * G + item % G] : -INFINITY;
         m[i] = sk;
@@ -202,39 +219,39 @@ paged_attention_tile_kernel(
         acc[i][0] = acc[i][1] = 0ull;
     }
     const int pieces = hd / 4;
+    // a lane per token: its request, last key and first key, so that a run's are found without a walk through memory
+    const int my_seq = lane < n_tok ? seq_of_token[t0 + lane] : -1;
+    int my_hi = lane < n_tok ? positions[t0 + lane] : -1;
+    const int my_lo = lane < n_tok && window > 0 ? max(0, my_hi - window + 1) : 0;
+    if (lane < n_tok && ctx_len != nullptr) my_hi = min(my_hi, ctx_len[my_seq] - 1);
     int first = t0;
     while (first < t0 + n_tok) {                       // run after run of one request's tokens; an item walks the keys in its own run alone
-        const int s = seq_of_token[first], begin = first;
-        int end = first, k_lo = 0x7fffffff, k_hi = -1;
-        for (; end < t0 + n_tok && seq_of_token[end] == s; end++) {
-            const int p = positions[end];
-            k_hi = max(k_hi, ctx_len != nullptr ? min(p, ctx_len[s] - 1) : p);
-            k_lo = min(k_lo, window > 0 ? max(0, p - window + 1) : 0);
-        }
+        const int begin = first, s = __shfl_sync(0xffffffffu, my_seq, begin - t0);
+        const unsigned others = __ballot_sync(0xffffffffu, lane < n_tok && my_seq != s) & (0xffffffffu << (begin - t0));
+        const int end = others ? t0 + __ffs(others) - 1 : t0 + n_tok;
+        const bool mine = lane >= begin - t0 && lane < end - t0;
+        const int k_hi = __reduce_max_sync(0xffffffffu, mine ? my_hi : -1), k_lo = __reduce_min_sync(0xffffffffu, mine ? my_lo : 0x7fffffff);
         first = end;
-        int last[8];                                   // the items' last keys in this run, -1: the item is another run's
+        int last[kWarpItems];                                   // the items' last keys in this run, -1: the item is another run's
 #pragma unroll
-        for (int i = 0; i < 8; i++) last[i] = tok[i] >= begin && tok[i] < end ? hi[i] : -1;
+        for (int i = 0; i < kWarpItems; i++) last[i] = tok[i] >= begin && tok[i] < end ? hi[i] : -1;
         const int * bt = block_table + (size_t) s * max_blocks;
         const int kb0 = (k_lo / 32) * 32;
-        auto fill = [&](int kb, int stage) {           // four lanes a key
+        auto page_of = [&](int j) { return j <= k_hi ? bt[j / page_size] : -1; };
+        int next_page = page_of(kb0 + (tid >> 3));     // looked up a tile ahead of its copy
+        auto fill = [&](int kb, int stage) {           // eight lanes a key
             if (kb <= k_hi) {
-                const int r = tid >> 2, j = kb + r;
-                int page = -1;
-                if (j <= k_hi) page = bt[j / page_size];
+                const int r = tid >> 3, j = kb + r, page = next_page;
+                next_page = page_of(kb + 32 + r);
                 const bool ok = page >= 0 && page < num_pages;
                 const size_t cell = ok ? (((size_t) page * nkv + kvh) * page_size + (j % page_size)) * hd : 0;
                 float * to = stages + (size_t) stage * 2 * 32 * kTileLd + r * kTileLd;
-                for (int c = tid & 3; c < pieces; c += 4) {
+                for (int c = tid & 7; c < pieces; c += 8) {
                     copy16(to + c * 4, k_cache + cell + c * 4, ok);
                     copy16(to + 32 * kTileLd + c * 4, v_cache + cell + c * 4, ok);
                 }
-                const unsigned b = __ballot_sync(0xffffffffu, ok);       // this warp's eight keys, four bits each
-                if (lane == 0) {
-                    unsigned mine = 0;
-                    for (int e = 0; e < 8; e++) mine |= ((b >> (4 * e)) & 1u) << e;
-                    reinterpret_cast<unsigned char *>(&good[stage])[warp] = (unsigned char) mine;
-                }
+                const unsigned b = __ballot_sync(0xffffffffu, ok);       // this warp's four keys, eight bits each
+                if (lane == 0) good[stage][warp] = (unsigned char) ((b & 1u) | (b >> 7 & 2u) | (b >> 14 & 4u) | (b >> 21 & 8u));
             }
             asm volatile("cp.async.commit_group;");
         };
@@ -246,21 +263,23 @@ paged_attention_tile_kernel(
             __syncthreads();
             const float * ks = stages + (size_t) stage * 2 * 32 * kTileLd;
             const float * vs = ks + 32 * kTileLd;
-            const bool here = (good[stage] >> lane) & 1u;
+            const bool here = good[stage][lane >> 2] >> (lane & 3) & 1;
             const int j = kb + lane;
             bool any = false;
 #pragma unroll
-            for (int i = 0; i < 8; i++) any |= kb <= last[i] && kb + 31 >= lo[i];
+            for (int i = 0; i < kWarpItems; i++) any |= kb <= last[i] && kb + 31 >= lo[i];
             if (any) {                                 // the same for all lanes: an item's numbers are the warp's
-                unsigned long long dot[4] = {0ull, 0ull, 0ull, 0ull};
+                unsigned long long dot[kWarpItems / 2];
+#pragma unroll
+                for (int pr = 0; pr < kWarpItems / 2; pr++) dot[pr] = 0ull;
                 const float * kr = ks + lane * kTileLd;
-                const float * qw = qs + (size_t) warp * 4 * hd * 2;
+                const float * qw = qs + (size_t) warp * kWarpItems * hd;
 #pragma unroll 4
                 for (int d = 0; d < hd; d += 4) {
                     const float4 k4 = *reinterpret_cast<const float4 *>(kr + d);
                     const unsigned long long k0 = pack2(k4.x, k4.x), k1 = pack2(k4.y, k4.y), k2 = pack2(k4.z, k4.z), k3 = pack2(k4.w, k4.w);
 #pragma unroll
-                    for (int pr = 0; pr < 4; pr++) {
+                    for (int pr = 0; pr < kWarpItems / 2; pr++) {
                         const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(qw + (pr * hd + d) * 2);
                         const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(qw + (pr * hd + d + 2) * 2);
                         dot[pr] = fma2(a.x, k0, dot[pr]);
@@ -270,54 +289,79 @@ paged_attention_tile_kernel(
                     }
                 }
                 bool full = true;                      // every item weighs every key of the tile: no term is left out below
+                float sc[kWarpItems], tile_max[kWarpItems], pj[kWarpItems], sum[kWarpItems], corr[kWarpItems];
+                // step by step for all items, so that one's shuffles run in the shadow of another's; an item without a key here keeps
+                // its maximum, and a factor of one and a sum of zero leave its numbers as they are
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
+                for (int i = 0; i < kWarpItems; i++) {
                     const float2 two = unpack2(dot[i >> 1]);
                     const bool valid = here && j >= lo[i] && j <= last[i];
-                    const float sc = valid ? ((i & 1) ? two.y : two.x) * scale : -INFINITY;
-                    const float tile_max = warp_max(sc);
-                    float pj = 0.0f;
-                    if (tile_max != -INFINITY) {
-                        const float m_new = fmaxf(m[i], tile_max);
-                        pj = valid ? expf(sc - m_new) : 0.0f;
-                        const float corr = (m[i] == -INFINITY) ? 0.0f : expf(m[i] - m_new);
-                        l[i] = l[i] * corr + warp_sum(pj);
+                    tile_max[i] = sc[i] = valid ? ((i & 1) ? two.y : two.x) * scale : -INFINITY;
+                }
 #pragma unroll
-                        for (int e = 0; e < 2; e++) {
-                            const float2 v = unpack2(acc[i][e]);
-                            acc[i][e] = pack2(v.x * corr, v.y * corr);
-                        }
-                        m[i] = m_new;
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int i = 0; i < kWarpItems; i++) tile_max[i] = fmaxf(tile_max[i], __shfl_xor_sync(0xffffffffu, tile_max[i], o));
+#pragma unroll
+                for (int i = 0; i < kWarpItems; i++) {
+                    const bool valid = here && j >= lo[i] && j <= last[i], some = tile_max[i] != -INFINITY;
+                    const float m_new = fmaxf(m[i], tile_max[i]);
+                    sum[i] = pj[i] = some && valid ? expf(sc[i] - m_new) : 0.0f;
+                    corr[i] = !some ? 1.0f : m[i] == -INFINITY ? 0.0f : expf(m[i] - m_new);
+                    if (some) m[i] = m_new;
+                    full &= pj[i] != 0.0f;
+                    ps[i * 32 + lane] = pj[i];
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int i = 0; i < kWarpItems; i++) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], o);
+#pragma unroll
+                for (int i = 0; i < kWarpItems; i++) {
+                    l[i] = l[i] * corr[i] + sum[i];
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        const float2 v = unpack2(acc[i][e]);
+                        acc[i][e] = pack2(v.x * corr[i], v.y * corr[i]);
                     }
-                    full &= pj != 0.0f;
-                    *reinterpret_cast<float2 *>(ps + (i * 32 + lane) * 2) = make_float2(pj, pj);
                 }
                 full = __all_sync(0xffffffffu, full);
                 __syncwarp();
                 if (full && lane < pieces) {
-#pragma unroll 4
-                    for (int jj = 0; jj < 32; jj += 2) {
-                        const ulonglong2 v0 = *reinterpret_cast<const ulonglong2 *>(vs + jj * kTileLd + lane * 4);
-                        const ulonglong2 v1 = *reinterpret_cast<const ulonglong2 *>(vs + (jj + 1) * kTileLd + lane * 4);
+#pragma unroll 2
+                    for (int jj = 0; jj < 32; jj += 4) {
+                        ulonglong2 v[4];
 #pragma unroll
-                        for (int i = 0; i < 8; i++) {
-                            const ulonglong2 p2 = *reinterpret_cast<const ulonglong2 *>(ps + (i * 32 + jj) * 2);
-                            acc[i][0] = fma2(p2.x, v0.x, acc[i][0]);
-                            acc[i][1] = fma2(p2.x, v0.y, acc[i][1]);
-                            acc[i][0] = fma2(p2.y, v1.x, acc[i][0]);
-                            acc[i][1] = fma2(p2.y, v1.y, acc[i][1]);
+                        for (int u = 0; u < 4; u++) v[u] = *reinterpret_cast<const ulonglong2 *>(vs + (jj + u) * kTileLd + lane * 4);
+#pragma unroll
+                        for (int i = 0; i < kWarpItems; i++) {
+                            const float4 p4 = *reinterpret_cast<const float4 *>(ps + i * 32 + jj);
+                            const float p[4] = {p4.x, p4.y, p4.z, p4.w};
+#pragma unroll
+                            for (int u = 0; u < 4; u++) {
+                                const unsigned long long pp = pack2(p[u], p[u]);
+                                acc[i][0] = fma2(pp, v[u].x, acc[i][0]);
+                                acc[i][1] = fma2(pp, v[u].y, acc[i][1]);
+                            }
                         }
                     }
                 } else if (lane < pieces) {
-#pragma unroll 4
-                    for (int jj = 0; jj < 32; jj += 2) {
-                        const ulonglong2 v0 = *reinterpret_cast<const ulonglong2 *>(vs + jj * kTileLd + lane * 4);
-                        const ulonglong2 v1 = *reinterpret_cast<const ulonglong2 *>(vs + (jj + 1) * kTileLd + lane * 4);
+#pragma unroll 2
+                    for (int jj = 0; jj < 32; jj += 4) {
+                        ulonglong2 v[4];
 #pragma unroll
-                        for (int i = 0; i < 8; i++) {
-                            const ulonglong2 p2 = *reinterpret_cast<const ulonglong2 *>(ps + (i * 32 + jj) * 2);
-                            if (unpack2(p2.x).x != 0.0f) { acc[i][0] = fma2(p2.x, v0.x, acc[i][0]); acc[i][1] = fma2(p2.x, v0.y, acc[i][1]); }
-                            if (unpack2(p2.y).x != 0.0f) { acc[i][0] = fma2(p2.y, v1.x, acc[i][0]); acc[i][1] = fma2(p2.y, v1.y, acc[i][1]); }
+                        for (int u = 0; u < 4; u++) v[u] = *reinterpret_cast<const ulonglong2 *>(vs + (jj + u) * kTileLd + lane * 4);
+#pragma unroll
+                        for (int i = 0; i < kWarpItems; i++) {
+                            const float4 p4 = *reinterpret_cast<const float4 *>(ps + i * 32 + jj);
+                            const float p[4] = {p4.x, p4.y, p4.z, p4.w};
+#pragma unroll
+                            for (int u = 0; u < 4; u++)
+                                if (p[u] != 0.0f) {
+                                    const unsigned long long pp = pack2(p[u], p[u]);
+                                    acc[i][0] = fma2(pp, v[u].x, acc[i][0]);
+                                    acc[i][1] = fma2(pp, v[u].y, acc[i][1]);
+                                }
                         }
                     }
                 }
@@ -329,8 +373,8 @@ paged_attention_tile_kernel(
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const int item = warp * 8 + i;
+    for (int i = 0; i < kWarpItems; i++) {
+        const int item = warp * kWarpItems + i;
         if (item >= n_items || lane >= pieces) continue;
         const int t = t0 + item / G, h = kvh * G + item % G;
         const float inv = l[i] > 0.0f ? 1.0f / l[i] : 0.0f;
@@ -400,7 +444,7 @@ IIAN_API int iian_paged_attention_sink(
         tile_tokens = kTileItems / group;
         const cudaError_t e = cudaFuncSetAttribute(paged_attention_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kTileSmem);
         if (e != cudaSuccess) return 1000 + (int) e;
-        paged_attention_tile_kernel<<<dim3((N + tile_tokens - 1) / tile_tokens, nkv), kGenWarps * 32, kTileSmem, stream>>>(
+        paged_attention_tile_kernel<<<dim3((N + tile_tokens - 1) / tile_tokens, nkv), kTileWarps * 32, kTileSmem, stream>>>(
             (const float *) q, (const float *) k_cache, (const float *) v_cache, (float *) out, positions, seq_of_token, block_table,
             max_blocks, ctx_len, N, nh, nkv, hd, page_size, num_pages, scale, window, sink, (const float *) gate, ld_gate);
         const int rc = iian_launch_status();
