@@ -133,20 +133,34 @@ __global__ void argmax_final_kernel(const float * __restrict__ part_val, const i
 // ---- temperature sampling ------------------------------------------------------------------------------------------
 // A row is worked on by a thread-block cluster: each CTA keeps a slice of the row in shared memory as ordered integer keys,
 // so the row is read from global memory once (V > 8 x kStagedMax: read again per pass) and a row of 150,000 entries has up
-// to 8 SMs.  The k-th largest value and the top-p cut are found exactly by narrowing an interval of keys eight ways per pass:
-// a pass counts (and for top-p adds the probability of) the keys at or above seven borders inside the interval, looking
-// only at keys inside it -- what lies above is known --, and the CTAs swap their numbers through each other's shared
-// memory behind one cluster barrier.  A search ends when one key is left inside.
-// Every sum has an order fixed by V alone (entries of a thread, lanes, warps, CTAs): the same row gives the same token
+// to 8 SMs.  The k-th largest value and the top-p cut are found exactly.
+//  * top-k up to half the cluster's warps: the entries not below the k-th largest of the warps' largest values are listed -- a few more
+//    than k --, every CTA takes over all lists, sorts and draws from them, and the row is not scanned again (draw_from_list).
+//  * Else the candidates fall into bins by their distance from the largest value (counts, or for top-p masses as integers, so that no
+//    order of adding matters), the CTAs add the cluster's bins up, and the entries of the bin that holds the cut are listed (cut_by_bins).
+//  * Where more than kListMax entries would be listed (many equal logits), or the cut lies in the last, open bin, an interval of keys is
+//    narrowed eight ways per pass: a pass counts (and for top-p adds the probability of) the keys at or above seven borders inside the
+//    interval, and the CTAs swap their numbers through each other's shared memory behind one cluster barrier.
+// Every sum has an order fixed by V alone (entries of a thread, lanes, warps, CTAs), or is one of integers: the same row gives the same token
 // whatever else is in the batch.
-// What bounds it: latency of the passes (a scan of a slice, two block barriers, a cluster barrier: about 1 us, some 20 of them),
-// not the bytes.  Rows of 151,936, the usual mix of settings: 48 rows 131 us, 8 rows 82 us, one row with top-k and top-p 51 us (one
-// block per row with 32 one-bit passes per search over the L2: 2,208 us for 48 rows).
+// What bounds it: latency -- the row's way in (4 us), three scans of a slice (bins 6.5, list 3, draw 4.5 us) and the barriers between them --
+// and two waves of CTAs from 38 rows on.  Rows of 151,936, the usual mix of settings: 48 rows 49 us, 8 rows 35 us, one row with top-k and
+// top-p 16 us (by narrowing alone, some 20 passes: 123, 82 and 51 us).
 constexpr int kDrawThreads = 512;
 constexpr int kDrawWarps = kDrawThreads / 32;
 constexpr int kDrawCluster = 8;                  // CTAs per row, at most
+static_assert(kDrawWarps == 16, "lists are merged by two warps for each CTA");
+constexpr int kSliceGoal = 13000;                // entries of a slice before a row gets more CTAs
 constexpr int kStagedMax = 50 * 1024;            // entries of a slice that shared memory holds (200 KB)
 constexpr int kBorders = 7;
+constexpr int kBins = kDrawThreads;              // a thread per bin, the last one open
+constexpr int kListMax = 1024;                   // entries that are sorted, two a thread
+
+// Bins by the distance from the largest value, 16 to a halving of the mass.  Masses of a bin are whole multiples of 2^-bin_bits: a mass lies
+// above half of 2^-(bin / 16) (up to rounding), so its last bit is worth at least 2^-bin_bits times two, and the multiple is at most 2^25.  What
+// falls into the last, open bin is cut off below that.
+constexpr float kBinsPerUnit = 16.0f * 1.4426950409f;
+__device__ __forceinline__ int bin_bits(int bin) { return 25 + (bin >> 4); }
 
 // NaN: below every key that is looked at; the two zeros are equal values and get one key
 __device__ __forceinline__ unsigned draw_key(float z) { return z != z ? 0u : order_key(z + 0.0f); }
@@ -160,6 +174,16 @@ struct DrawShared {
     double warp_d[kDrawWarps];
     int warp_i[kDrawWarps];
     int pick;
+    int n_list, found[2], n_span;
+    double m_above;
+    unsigned long long warp_q[kDrawWarps];
+    unsigned lo_key, hi_key;
+    float tops[kDrawCluster * kDrawWarps];       // the largest value of every warp of the cluster
+    unsigned long long list[kListMax];           // this CTA's entries that take part in the sort: key, then ~id
+    union {                                      // the bins have been read by all before any CTA sorts
+        struct { int count[kBins]; unsigned low[kBins], high[kBins]; } bins;     // the masses' last 13 bits and the rest
+        unsigned long long sorted[kListMax];
+    };
 };
 
 template <bool STAGED>
@@ -309,6 +333,289 @@ struct Draw {
     }
 };
 
+// Sums from the first thread to this one (inclusive), in an order fixed by the block: `total` is everyone's.
+__device__ __forceinline__ void block_scan(DrawShared & sh, int & c, double & m, int & c_total, double & m_total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int cv = __shfl_up_sync(0xffffffffu, c, o);
+        const double mv = __shfl_up_sync(0xffffffffu, m, o);
+        if (lane >= o) { c += cv; m += mv; }
+    }
+    __syncthreads();
+    if (lane == 31) { sh.warp_i[warp] = c; sh.warp_d[warp] = m; }
+    __syncthreads();
+    int c_before = 0;
+    double m_before = 0.0;
+    c_total = 0;
+    m_total = 0.0;
+    for (int w = 0; w < kDrawWarps; w++) {
+        if (w == warp) { c_before = c_total; m_before = m_total; }
+        c_total += sh.warp_i[w];
+        m_total += sh.warp_d[w];
+    }
+    c += c_before;
+    m += m_before;
+}
+
+// sh.sorted[0, n) in falling order, no two alike: an entry's place is the number of larger ones, which costs less than a sort for the
+// few dozen that are left as a rule (a bitonic one of 30 entries 4,800 clocks, of 500 15,000).
+__device__ __forceinline__ void block_sort(DrawShared & sh, int n) {
+    unsigned long long v[2];
+    int place[2] = {0, 0};
+#pragma unroll
+    for (int e = 0; e < 2; e++) v[e] = (int) threadIdx.x + e * kDrawThreads < n ? sh.sorted[threadIdx.x + e * kDrawThreads] : 0ull;
+    if (threadIdx.x < n) {
+#pragma unroll 4
+        for (int i = 0; i < n; i++) {
+            const unsigned long long other = sh.sorted[i];
+            place[0] += other > v[0];
+            place[1] += other > v[1];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 2; e++)
+        if ((int) threadIdx.x + e * kDrawThreads < n) sh.sorted[place[e]] = v[e];
+    __syncthreads();
+}
+
+// The lists of all CTAs, in no order, in every CTA's sh.sorted.  Returns how many; above kListMax nothing is there.
+template <bool STAGED>
+__device__ __forceinline__ int merge_lists(const Draw<STAGED> & d) {
+    cg::cluster_group cl = cg::this_cluster();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    cl.sync();
+    // counts: a lane per CTA; entries: two warps per CTA (kDrawWarps = 2 x kDrawCluster)
+    const int own = lane < d.ctas ? cl.map_shared_rank(&d.sh, lane)->n_list : 0;
+    const int n = __reduce_add_sync(0xffffffffu, own);
+    if (n > kListMax) return n;
+    const int r = warp >> 1, of_r = __shfl_sync(0xffffffffu, own, r), at = __reduce_add_sync(0xffffffffu, lane < r ? own : 0);
+    if (r < d.ctas) {
+        const DrawShared * from = cl.map_shared_rank(&d.sh, r);
+        for (int i = (warp & 1) * 32 + lane; i < of_r; i += 64) d.sh.sorted[at + i] = from->list[i];
+    }
+    __syncthreads();
+    return n;
+}
+
+// The shortest run of the sorted list that reaches `share` of its first `limit` entries' mass.
+template <bool STAGED>
+__device__ __forceinline__ int shortest_run(const Draw<STAGED> & d, int limit, float share) {
+    DrawShared & sh = d.sh;
+    const int tid = threadIdx.x;
+    double own[2], run, in_list;
+#pragma unroll
+    for (int e = 0; e < 2; e++) own[e] = 2 * tid + e < limit ? (double) d.mass((unsigned) (sh.sorted[2 * tid + e] >> 32)) : 0.0;
+    run = own[0] + own[1];
+    int none = 0, none_total;
+    block_scan(sh, none, run, none_total, in_list);
+    const double goal = (double) share * in_list;
+    if (tid == 0) sh.found[1] = limit;
+    __syncthreads();
+    if (2 * tid + 1 < limit && run >= goal) atomicMin(&sh.found[1], 2 * tid + 2);
+    if (2 * tid < limit && run - own[1] >= goal) atomicMin(&sh.found[1], 2 * tid + 1);
+    __syncthreads();
+    return sh.found[1];
+}
+
+// A row with top-k of which few entries are left: they are listed, sorted and drawn from, without another scan.  What bounds the list
+// from below is the k-th largest of the warps' largest values: k entries at least are as large.  False: too many, nothing drawn.
+template <bool STAGED>
+__device__ __forceinline__ bool draw_from_list(const Draw<STAGED> & d, int begin, int k, float P, unsigned cut, float uniform, int & token) {
+    DrawShared & sh = d.sh;
+    const int tid = threadIdx.x, tops = d.ctas * kDrawWarps;
+    if (tid == 0) { sh.n_list = 0; sh.found[0] = kListMax; }
+    __syncthreads();
+    if (tid < tops) {                            // this warp's rank among them, equal ones by place
+        const float own = sh.tops[tid];
+        int rank = 0;
+#pragma unroll 8
+        for (int i = 0; i < tops; i++) rank += sh.tops[i] > own || (sh.tops[i] == own && i < tid);
+        if (rank == k - 1) sh.n_span = (int) draw_key(own);
+    }
+    __syncthreads();
+    const unsigned least = max(cut, (unsigned) sh.n_span);
+#pragma unroll 4
+    for (int i = tid; i < d.n; i += kDrawThreads) {
+        const unsigned key = d.key(i);
+        if (key < least) continue;
+        const int at = atomicAdd(&sh.n_list, 1);
+        if (at < kListMax) sh.list[at] = ((unsigned long long) key << 32) | (0xffffffffu - (unsigned) (begin + i));
+    }
+    const int n = merge_lists(d);
+    if (n > kListMax) return false;
+    block_sort(sh, n);                           // largest first, equal values by id
+    int kept = min(k, n);
+    if (P < 1.0f) kept = shortest_run(d, kept, P);
+    unsigned long long mine[2];                  // in the vocabulary's order
+#pragma unroll
+    for (int e = 0; e < 2; e++) mine[e] = 2 * tid + e < kept ? sh.sorted[2 * tid + e] : 0ull;
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 2; e++)
+        if (2 * tid + e < kept) sh.sorted[2 * tid + e] = mine[e] << 32 | mine[e] >> 32;
+    __syncthreads();
+    block_sort(sh, kept);
+    double own[2], run, total;
+#pragma unroll
+    for (int e = 0; e < 2; e++) own[e] = 2 * tid + e < kept ? (double) d.mass((unsigned) sh.sorted[2 * tid + e]) : 0.0;
+    run = own[0] + own[1];
+    int none = 0, none_total;
+    if (tid == 0) sh.found[1] = 0;
+    block_scan(sh, none, run, none_total, total);
+    const double u = (double) uniform * total;
+    if (own[0] > 0.0) { if (run - own[1] > u) atomicMin(&sh.found[0], 2 * tid); atomicMax(&sh.found[1], 2 * tid); }
+    if (own[1] > 0.0) { if (run > u) atomicMin(&sh.found[0], 2 * tid + 1); atomicMax(&sh.found[1], 2 * tid + 1); }
+    __syncthreads();
+    token = (int) (0xffffffffu - (unsigned) (sh.sorted[sh.found[0] < kListMax ? sh.found[0] : sh.found[1]] >> 32));   // else (rounding) the last
+    return true;
+}
+
+// The cut of top-k (0: none) and top-p (>= 1: none) among the keys at or above `cut`, by bins and a sorted list: candidates are the keys
+// above the new cut and the first n_tie entries equal to it.  False, and nothing changed: not found this way.
+template <bool STAGED>
+__device__ __forceinline__ bool cut_by_bins(const Draw<STAGED> & d, int begin, int V, int k, float P, unsigned & cut, int & n_tie) {
+    DrawShared & sh = d.sh;
+    cg::cluster_group cl = cg::this_cluster();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool by_k = k > 0;                     // then only counts: the list's own masses are enough for top-p
+    // the bins reach as far as the cut may lie: beyond log(V / (1 - P)) all entries together weigh less than 1 - P of the largest one
+    const int open = by_k ? kBins - 1 : (int) fminf((logf((float) V) - logf(1.0f - P) + 0.5f) * kBinsPerUnit, (float) (kBins - 1));
+    sh.bins.count[tid] = 0;
+    sh.bins.low[tid] = sh.bins.high[tid] = 0u;
+    if (tid == 0) sh.found[0] = kBins;
+    __syncthreads();
+    int open_c = 0;                              // the open bin is kept in registers: most of a peaked row falls into it
+    unsigned long long open_m = 0ull;
+    for (int i0 = tid; i0 < d.n; i0 += 4 * kDrawThreads) {   // four entries side by side: their bins before the first is counted
+        int bin[4];
+        unsigned q[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int i = i0 + u * kDrawThreads;
+            const unsigned key = i < d.n ? d.key(i) : 0u;
+            const float z = key_value(max(key, cut));
+            bin[u] = (int) fminf((d.zmax - z) * kBinsPerUnit, (float) open);
+            if (!by_k) q[u] = (unsigned) (expf(z - d.zmax) * __int_as_float((127 + bin_bits(bin[u])) << 23));
+            if (key < cut) bin[u] = -1;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (bin[u] == open) {
+                open_c++;
+                if (!by_k) open_m += q[u];
+            } else if (bin[u] >= 0) {
+                if (by_k) atomicAdd(&sh.bins.count[bin[u]], 1);
+                else { atomicAdd(&sh.bins.low[bin[u]], q[u] & 8191u); atomicAdd(&sh.bins.high[bin[u]], q[u] >> 13); }
+            }
+        }
+    }
+    if (open_c > 0) {
+        atomicAdd(&sh.bins.count[open], open_c);
+        atomicAdd(&sh.bins.low[open], (unsigned) (open_m & 8191u));
+        atomicAdd(&sh.bins.high[open], (unsigned) (open_m >> 13));
+    }
+    cl.sync();                                   // what the CTAs listed before, if they did, has been read too
+    if (tid == 0) sh.n_list = 0;
+    int c = 0;
+    unsigned long long low = 0ull, high = 0ull;
+#pragma unroll
+    for (int r = 0; r < kDrawCluster; r++) {
+        if (r >= d.ctas) break;
+        const DrawShared * from = cl.map_shared_rank(&sh, r);
+        if (by_k) c += from->bins.count[tid];
+        else { low += from->bins.low[tid]; high += from->bins.high[tid]; }
+    }
+    double m = (double) (low + (high << 13)) * __longlong_as_double((long long) (1023 - bin_bits(tid)) << 52), mass;
+    const int own_c = c;
+    int count;
+    block_scan(sh, c, m, count, mass);           // from the largest values down to this bin
+    const double target = (double) P * mass;
+    if (by_k ? c >= k && c - own_c < k : m >= target) atomicMin(&sh.found[0], tid);
+    __syncthreads();
+    const int last = sh.found[0];                // the bin that holds the cut (with both: the one of top-k)
+    if (last >= open) return false;              // top-k of no effect, or a cut in the open bin
+    if (tid == last - 1) sh.m_above = m;
+    __syncthreads();
+    const int first = by_k ? 0 : last;           // with top-k the list begins at the top
+    const double m_above = by_k || last == 0 ? 0.0 : sh.m_above;
+    for (int i0 = tid; i0 < d.n; i0 += 4 * kDrawThreads) {
+        unsigned key[4];
+        bool in[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int i = i0 + u * kDrawThreads;
+            key[u] = i < d.n ? d.key(i) : 0u;
+            const float place = (d.zmax - key_value(max(key[u], cut))) * kBinsPerUnit;
+            in[u] = key[u] >= cut && place >= (float) first && place < (float) (last + 1);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (in[u]) {
+                const int at = atomicAdd(&sh.n_list, 1);
+                if (at < kListMax) sh.list[at] = ((unsigned long long) key[u] << 32) | (0xffffffffu - (unsigned) (begin + i0 + u * kDrawThreads));
+            }
+    }
+    const int n = merge_lists(d);
+    if (n > kListMax) return false;
+    if (by_k) {
+        block_sort(sh, n);
+        const int kept = P < 1.0f ? shortest_run(d, k, P) : k;
+        const unsigned at_cut = (unsigned) (sh.sorted[kept - 1] >> 32);
+        cut = at_cut;
+        __syncthreads();                         // found[1] has been read
+        for (int i = tid; i < n; i += kDrawThreads) {
+            if ((unsigned) (sh.sorted[i] >> 32) != at_cut) continue;
+            if (i == 0 || (unsigned) (sh.sorted[i - 1] >> 32) != at_cut) sh.found[0] = i;
+            if (i == n - 1 || (unsigned) (sh.sorted[i + 1] >> 32) != at_cut) sh.found[1] = i;
+        }
+        __syncthreads();
+        n_tie = kept == sh.found[1] + 1 ? 0x7fffffff : kept - sh.found[0];       // all of them, or the first few
+        return true;
+    }
+    // The largest key whose list entries from there on weigh what is still to reach, in the bin's own whole multiples: every warp weighs
+    // one border a pass, and an interval of keys shrinks to a sixteenth.
+    const float unit = __int_as_float((127 + bin_bits(last)) << 23);
+    const unsigned long long need = (unsigned long long) fmax(ceil((target - m_above) * (double) unit), 1.0);
+    if (tid == 0) { sh.lo_key = 0xffffffffu; sh.hi_key = 0u; }
+    __syncthreads();
+    for (int i = tid; i < n; i += kDrawThreads) {            // (key, ~id) -> (key, weight)
+        const unsigned key = (unsigned) (sh.sorted[i] >> 32);
+        sh.sorted[i] = ((unsigned long long) key << 32) | (unsigned) (d.mass(key) * unit);
+        atomicMin(&sh.lo_key, key);
+        atomicMax(&sh.hi_key, key);
+    }
+    __syncthreads();
+    unsigned lo = sh.lo_key, hi = sh.hi_key + 1u;
+    unsigned long long q_hi = 0ull;              // what the keys from hi on weigh: less than `need`; from lo on all do (or rounding has it so)
+    while (hi - lo > 1u) {
+        const unsigned long long span = hi - lo;
+        const unsigned border = lo + (unsigned) ((span * (unsigned) (warp + 1)) >> 4);   // the last warp's is hi
+        unsigned part = 0u;                      // at most 32 weights of 2^25 a lane
+        for (int i = lane; i < n; i += 32) {
+            const unsigned long long x = sh.sorted[i];
+            part += (unsigned) (x >> 32) >= border ? (unsigned) x : 0u;
+        }
+        const unsigned q_low = __reduce_add_sync(0xffffffffu, part & 0xffffu), q_high = __reduce_add_sync(0xffffffffu, part >> 16);
+        if (lane == 0) sh.warp_q[warp] = ((unsigned long long) q_high << 16) + q_low;
+        __syncthreads();
+        const unsigned ok = __ballot_sync(0xffffffffu, lane < kDrawWarps - 1 && sh.warp_q[lane & (kDrawWarps - 1)] >= need);
+        const int reached = __popc(ok);          // the borders rise: the first of them reach
+        if (reached < kDrawWarps - 1) { q_hi = sh.warp_q[reached]; hi = lo + (unsigned) ((span * (unsigned) (reached + 1)) >> 4); }
+        lo += (unsigned) ((span * (unsigned) reached) >> 4);
+        __syncthreads();
+    }
+    int ties = 0;
+    for (int i = lane; i < n; i += 32) ties += (unsigned) (sh.sorted[i] >> 32) == lo;
+    ties = __reduce_add_sync(0xffffffffu, ties);
+    const unsigned long long each = (unsigned long long) (d.mass(lo) * unit);
+    const unsigned long long some = each > 0ull && need > q_hi ? (need - q_hi + each - 1ull) / each : 1ull;
+    cut = lo;
+    n_tie = some >= (unsigned long long) ties ? 0x7fffffff : (int) some;         // all of them, or the first few
+    return true;
+}
+
 template <bool STAGED>
 __global__ void __launch_bounds__(kDrawThreads) sample_kernel(
     const float * __restrict__ logits, int V, size_t stride, int slice, const float * __restrict__ temperature,
@@ -330,7 +637,7 @@ __global__ void __launch_bounds__(kDrawThreads) sample_kernel(
     // the slice into shared memory; the row's largest value and the lowest id that holds it
     float best = -INFINITY;
     int best_i = 0x7fffffff;
-#pragma unroll 8
+#pragma unroll 16
     for (int i = tid; i < n; i += kDrawThreads) {
         const float z = src[i] * inv_t;
         if (STAGED) staged[i] = draw_key(z);
@@ -355,6 +662,8 @@ __global__ void __launch_bounds__(kDrawThreads) sample_kernel(
             const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
             better(ob, oi);
         }
+        if (STAGED && lane < kDrawWarps)         // the warps' largest values too
+            for (int r = 0; r < ctas; r++) cl.map_shared_rank(&sh, r)->tops[rank * kDrawWarps + lane] = fs[lane];
         d.send(lane, 0, (double) best, best_i);
     }
     d.swap();
@@ -374,12 +683,22 @@ __global__ void __launch_bounds__(kDrawThreads) sample_kernel(
     }
     const unsigned top = draw_key(best) + 1;     // above every key
     // candidates: keys above `cut`, and the first n_tie entries (by id) whose key is `cut`
-    unsigned cut = 1u;
+    unsigned cut = order_key(-INFINITY) + 1u;    // entries without mass change nothing
     int n_tie = 0x7fffffff;
     const float mp = min_p[row];
-    if (mp > 0.0f) cut = order_key(best + logf(mp));
+    if (mp > 0.0f) cut = max(cut, order_key(best + logf(mp)));
     const int k = top_k[row];
-    if (k > 0 && cut < top) {
+    const bool cuts = cut < top && (k > 0 || P < 1.0f);
+    if (STAGED && cuts && k > 0 && k <= ctas * kDrawWarps / 2) {
+        int token;
+        if (draw_from_list(d, begin, k, P, cut, uniform[row], token)) {
+            if (rank == 0 && tid == 0) out[row] = token;
+            cl.sync();                           // the lists of this CTA have been read
+            return;
+        }
+    }
+    const bool found = STAGED && cuts && cut_by_bins(d, begin, V, k, P, cut, n_tie);
+    if (cuts && !found && k > 0) {
         int c;
         double m;
         d.template pass<false>(cut, cut, top, c, m);
@@ -390,7 +709,7 @@ __global__ void __launch_bounds__(kDrawThreads) sample_kernel(
             n_tie = k - above;
         }
     }
-    if (P < 1.0f && cut < top) {
+    if (cuts && !found && P < 1.0f) {
         // borders: cut in lane 0, cut + 1 in the others (entries equal to the cut: the difference of the counts)
         int c;
         double m;
@@ -421,28 +740,31 @@ __global__ void __launch_bounds__(kDrawThreads) sample_kernel(
     // inverse CDF in vocabulary order: thread t owns `per` neighbouring entries (an odd number: no two lanes in one bank)
     const int per = ((n + kDrawThreads - 1) / kDrawThreads) | 1;
     const int i0 = (int) min((long long) n, (long long) tid * per), i1 = min(n, i0 + per);
-    int ties = 0;
-    for (int i = i0; i < i1; i++) ties += d.key(i) == cut;
-    int tie_rank = ties;                         // inclusive scan over the CTA, then the CTAs before
+    int ties = 0, tie_rank = 0;
+    if (n_tie != 0x7fffffff) {                   // else every entry equal to the cut stays
+        for (int i = i0; i < i1; i++) ties += d.key(i) == cut;
+        tie_rank = ties;                         // inclusive scan over the CTA, then the CTAs before
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, tie_rank, o);
-        if (lane >= o) tie_rank += v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, tie_rank, o);
+            if (lane >= o) tie_rank += v;
+        }
+        __syncthreads();                             // sh.warp_i may still be read from the search
+        if (lane == 31) sh.warp_i[warp] = tie_rank;
+        __syncthreads();
+        if (warp == 0) {
+            const int w = lane < kDrawWarps ? sh.warp_i[lane] : 0;
+            d.send(lane, 0, 0.0, __reduce_add_sync(0xffffffffu, w));
+        }
+        d.swap();
+        tie_rank -= ties;
+        for (int w = 0; w < warp; w++) tie_rank += sh.warp_i[w];
+        for (int r = 0; r < rank; r++) tie_rank += sh.inbox_c[d.turn][r][0];
+        d.turn ^= 1;
     }
-    __syncthreads();                             // sh.warp_i may still be read from the search
-    if (lane == 31) sh.warp_i[warp] = tie_rank;
-    __syncthreads();
-    if (warp == 0) {
-        const int w = lane < kDrawWarps ? sh.warp_i[lane] : 0;
-        d.send(lane, 0, 0.0, __reduce_add_sync(0xffffffffu, w));
-    }
-    d.swap();
-    tie_rank -= ties;
-    for (int w = 0; w < warp; w++) tie_rank += sh.warp_i[w];
-    for (int r = 0; r < rank; r++) tie_rank += sh.inbox_c[d.turn][r][0];
-    d.turn ^= 1;
     double cm = 0.0;
     int tr = tie_rank;
+#pragma unroll 4
     for (int i = i0; i < i1; i++) {
         const unsigned kk = d.key(i);
         if (kk > cut) cm += (double) d.mass(kk);
@@ -627,20 +949,20 @@ IIAN_API int iian_argmax_wide(const float * logits, int R, int V, long long stri
     return iian_launch(argmax_final_kernel, dim3(R), dim3(32), 0, stream, (const float *) pv, (const int *) pi, parts, out);
 }
 
-// CTAs per row: slices of 4,096 entries and more, up to 8 CTAs (a smaller slice is scanned in less time than the cluster's
-// barrier takes).
+// CTAs per row: slices of up to 13,000 entries, up to 8 CTAs.  Less of a slice is no faster for a few rows and a wave more for many: 48 rows
+// of 32,768 with 8 CTAs 31 us, with 4 22, with 2 27; of 50,257 with 8 35, with 4 29; 16 CTAs of a row of 151,936 72 for 49 with 8.
 IIAN_API int iian_sample(const float * logits, int R, int V, long long stride, const float * temperature,
                          const int * top_k, const float * top_p, const float * min_p, const float * uniform,
                          int * out, cudaStream_t stream) {
     if (R <= 0) return IIAN_OK;
     if (V <= 0) return IIAN_ERR_SHAPE;
     int ctas = 1;
-    while (ctas < kDrawCluster && V > ctas * 4096) ctas *= 2;
+    while (ctas < kDrawCluster && V > ctas * kSliceGoal) ctas *= 2;
     const int slice = (V - 1) / ctas + 1;
     const bool staged = slice <= kStagedMax;
     const size_t smem = staged ? (size_t) slice * sizeof(unsigned) : 0;
     auto kernel = staged ? sample_kernel<true> : sample_kernel<false>;
-    if (smem > 40 * 1024) {
+    if (smem > 24 * 1024) {                      // with the 20 KB of static memory above what a launch may ask for by itself
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
         if (e != cudaSuccess) return 1000 + (int) e;
     }

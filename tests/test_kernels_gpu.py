@@ -313,6 +313,35 @@ def test_sample_matches_the_plain_walk(V, params):
         assert lo - slack <= target <= hi + slack, f"row {r}: u*total={target} not in [{lo}, {hi}]"
 
 
+@pytest.mark.parametrize("V", [1, 37, 13001, 50257, 60000])
+@pytest.mark.parametrize("top_k,top_p,min_p", [(20, 0.8, 0.0), (1, 1.0, 0.0), (60, 1.0, 0.0), (3, 0.5, 0.0), (900, 0.97, 0.0), (1500, 0.9, 0.0), (60000, 0.6, 0.0),
+                                               (0, 0.9, 0.0), (0, 0.2, 0.0), (0, 0.9999999, 0.0), (40, 0.9, 0.02), (0, 0.7, 0.3)])
+def test_sample_cuts(V, top_k, top_p, min_p):
+    """Rows on which the cut is found in different ways: a bell, ties around the cut, all equal, a few far above the rest (the cut in the
+    bin without an end), most of the row masked, one entry left."""
+    g = torch.Generator().manual_seed(V + top_k)
+    bell = torch.randn(V, generator=g) * 2.5
+    peaked = bell - 60.0
+    peaked[:: max(1, V // 5)] += 60.0
+    masked = torch.where(torch.rand(V, generator=g) < 0.9, torch.tensor(float("-inf")), bell)
+    masked[V // 2] = 1.0
+    one = torch.full((V,), float("-inf"))
+    one[V // 3] = -3.0
+    rows = torch.stack([bell, (bell * 2).round() / 2, torch.zeros(V), peaked, masked, one])
+    u = torch.rand(len(rows), generator=g)
+    out = torch.empty(len(rows), dtype=torch.int32).cuda()
+    f = lambda v, dt: torch.full((len(rows),), v, dtype=dt).cuda()
+    K().sample(rows.cuda(), f(0.9, torch.float32), f(top_k, torch.int32), f(top_p, torch.float32), f(min_p, torch.float32), u.cuda(), out)
+    for r, got in enumerate(out.tolist()):
+        probs = plain.candidate_probs(rows[r], 0.9, top_k, top_p, min_p)
+        cum = torch.cumsum(probs.double(), 0)
+        total, target = cum[-1].item(), u[r].item() * cum[-1].item()
+        # a cut within the float32 rounding of its mass may fall one entry further, where every entry has the same share
+        slack = 1e-5 * total + (probs.max().item() if r in (1, 2) else 0.0)
+        assert probs[got] > 0 or r in (1, 2), f"row {r}: token {got} is outside the candidate set"
+        assert cum[got].item() - probs[got].item() - slack <= target <= cum[got].item() + slack, f"row {r}"
+
+
 @pytest.mark.parametrize("od", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("B,M,K_", [(1, 70, 64), (3, 16, 32), (8, 257, 96), (9, 100, 160), (17, 48, 4096), (33, 130, 320),
                                     (64, 1000, 1024), (2, 4096, 12288)])
