@@ -37,9 +37,17 @@
 // taken of the raw scores and capped alone, and the polynomial's last step x * P(x^2) is the multiply-add that takes the maximum off:
 // the cap costs four packed operations for two scores.
 //
+// The split form: the key tiles of a row tile in `parts` equal runs, one CTA of a thread-block cluster each, where the row tiles would
+// leave SMs idle (iian_attention_tc_choose has the rule).  Every CTA ends with its own maximum, sum and O per row;
+// behind a cluster barrier (no CTA reads its K and V stages any more) a row goes to the CTA that finishes it, through distributed
+// shared memory into those stages, and behind a second one each CTA adds up 256 / parts rows.
+//
 // Every wait on an mbarrier is bounded: after kSpinLimit polls the waiter records where it gave up in
 // `status`, and every role falls through to the common exit, where tensor memory is freed.
 #include <cuda.h>
+
+#include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
 #include "tc_attention.cuh"
@@ -60,6 +68,7 @@ struct TcAttnParams {
     const int * block_table;        // [S, max_blocks]
     int max_blocks, nh, nkv, page_size, num_pages, window, num_seqs;
     int single;                     // as at_row_tile has it
+    int parts = 1;                  // split form: CTAs of a row tile
     float scale_log2;               // scale * log2(e)
     int * status;                   // {code, where}; zero before the launch
     // a sink per head: a logit without key and value that joins the softmax's denominator once, not scaled
@@ -107,8 +116,17 @@ template <int N> __device__ __forceinline__ unsigned long long at_cap_two(unsign
 }
 
 // The form with kept first keys and a gate per head (AT_KEPT), the difference form (AT_DIFF) and the capped form (AT_CAP) are
-// instances of their own, so that the plain one stays as it was
-enum { AT_PLAIN = 0, AT_KEPT = 1, AT_DIFF = 2, AT_CAP = 3 };
+// instances of their own, so that the plain one stays as it was; so is the split form (AT_SPLIT, no gate)
+enum { AT_PLAIN = 0, AT_KEPT = 1, AT_DIFF = 2, AT_CAP = 3, AT_SPLIT = 4 };
+
+__device__ __forceinline__ void at_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ unsigned at_peer(unsigned addr, unsigned rank) {      // the same place in the shared memory of CTA `rank`
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
 
 // probabilities of a row's 128 scores in v against the maximum -neg, capped by the polynomial of N coefficients: bf16 pairs into
 // v[0 .. 63], the sums in two packed pairs
@@ -132,6 +150,8 @@ template <int N> __device__ __forceinline__ void at_capped_row(unsigned * v, con
     }
 }
 
+constexpr int kAtParts = 8;               // CTAs of a row tile, at most
+
 // A step's grid: the KV heads, then the row tiles as `unit` counts them (no division in front of a CTA's first load).
 constexpr int kAtUnits = 32768;
 static inline dim3 at_grid(int N, int S, int max_q_len, int nh, int nkv, int rows) {
@@ -142,7 +162,7 @@ static inline dim3 at_grid(int N, int S, int max_q_len, int nh, int nkv, int row
 template <int FORM>
 __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
     const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const TcAttnParams p) {
-    constexpr bool KEPT = FORM == AT_KEPT, DIFF = FORM == AT_DIFF, CAP = FORM == AT_CAP;
+    constexpr bool KEPT = FORM == AT_KEPT, DIFF = FORM == AT_DIFF, CAP = FORM == AT_CAP, SPLIT = FORM == AT_SPLIT;
     constexpr int CTA_ROWS = DIFF ? AT_BM : AT_ROWS;
     extern __shared__ __align__(1024) unsigned char at_smem_raw[];
     unsigned char * smem = (unsigned char *) (((uintptr_t) at_smem_raw + 1023) & ~(uintptr_t) 1023);
@@ -154,7 +174,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = p.nh / p.nkv;
-    const int kvh = blockIdx.x;
+    const int kvh = SPLIT ? (int) blockIdx.x / p.parts : (int) blockIdx.x, part = SPLIT ? (int) blockIdx.x % p.parts : 0;
     // Which rows are this CTA's.  Where it takes a search (some hundred instructions, which ten warps would issue in half a microsecond) it is
     // one warp's work, beside the barriers' and tensor memory's set-up.
     __shared__ AtPlace place;                                // (s < 0: none left)
@@ -171,6 +191,12 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
             tile_lo = (p.window > 0 ? max(0, first - p.window + 1) : p.chunk > 0 ? first - first % p.chunk : 0) / AT_BN;
             k_hi_a = pos0 + min(last, row0 + AT_BM - 1) / G;
             k_hi = pos0 + min(last, row0 + CTA_ROWS - 1) / G;
+            if constexpr (SPLIT) {                           // this part's run of the tiles (it may be empty)
+                const int tiles = k_hi / AT_BN - tile_lo + 1;
+                k_hi = min(k_hi, (tile_lo + tiles * (part + 1) / p.parts) * AT_BN - 1);
+                k_hi_a = min(k_hi_a, k_hi);
+                tile_lo += tiles * part / p.parts;
+            }
             if (warp == (search ? 2 : 0)) {                  // the producer's first reads of the block table
                 const int j0 = tile_lo * AT_BN + lane * p.page_size;
                 if (lane < AT_BN / p.page_size && j0 <= k_hi)
@@ -209,11 +235,11 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
 
     // two groups of 128 rows (A, B) share every K/V tile; B may be empty, and A may need a tile less than B
     const bool has_b = DIFF || row0 + AT_BM < rows_total;
-    const int tile_hi = k_hi / AT_BN;
+    const int tile_hi = SPLIT ? (k_hi + AT_BN) / AT_BN - 1 : k_hi / AT_BN;
     const int n_keep = (KEPT && p.keep_first > 0 && p.window > 0) ? min((p.keep_first + AT_BN - 1) / AT_BN, tile_lo) : 0;
     auto phys = [&](int i) { return KEPT && i < n_keep ? i : tile_lo + i - n_keep; };        // the cache tile of the i-th tile walked
     const int n_tiles = tile_hi - tile_lo + 1 + n_keep;
-    const int n_grp[2] = {k_hi_a / AT_BN - tile_lo + 1 + n_keep, has_b ? n_tiles : 0};
+    const int n_grp[2] = {SPLIT ? max(0, (k_hi_a + AT_BN) / AT_BN - tile_lo) : k_hi_a / AT_BN - tile_lo + 1 + n_keep, has_b ? n_tiles : 0};
     const int * bt = p.block_table + (size_t) s * p.max_blocks;
     int * status = p.status;
 
@@ -332,6 +358,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
             }
             at_commit(at_smem(&s_full[g]));
         };
+        if (SPLIT && n_tiles <= 0) goto done;
         if (!at_wait(at_smem(&q_full), 0u)) { status[0] = 4; status[1] = 0; goto done; }
         if (!at_wait(at_smem(&k_full[0]), 0u)) { status[0] = 3; status[1] = 0; goto done; }
         at_fence_after();
@@ -369,7 +396,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
         const unsigned tS = tmem_base + (unsigned) (g * 128), tO = tmem_base + 256u + (unsigned) (g * 128);
         const int n_mine = n_grp[g];
         float m_run = -INFINITY, l_run = 0.0f;
-        if (p.sink != nullptr && row_ok) {      // the running softmax starts at the sink: maximum sink, sum 1, nothing in O
+        if (p.sink != nullptr && row_ok && (!SPLIT || part == 0)) {      // the running softmax starts at the sink: maximum sink, sum 1, nothing in O
             m_run = p.sink[kvh * G + R % G] * p.sink_to_raw;
             l_run = 1.0f;
         }
@@ -581,6 +608,74 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
                 }
             }
         } else
+        if constexpr (SPLIT) {
+            // ---- this part's maximum, sum and O of every row to the CTA that finishes the row -----------------------
+            if (n_mine > 0 && !failed && !at_wait(at_smem(&pv_done[g]), (unsigned) (n_mine - 1) & 1u)) {
+                if (lane == 0) { status[0] = 9; status[1] = n_mine; }
+                failed = true;
+            }
+            at_cluster_sync();
+            __syncwarp();
+            at_fence_after();
+            const int each = AT_ROWS / p.parts, row = g * AT_BM + r, local = row % each;
+            const unsigned to = (unsigned) (row / each);
+            const bool any = n_mine > 0 && !failed;
+            const unsigned cell = at_peer(at_smem(sK), to) + (unsigned) ((part * each + local) * AT_HD * 4);
+#pragma unroll
+            for (int c0 = 0; c0 < AT_HD; c0 += 32) {
+                unsigned o[32];
+                at_ld32(tO + lane_addr + (unsigned) c0, o);
+                at_wait_ld();
+#pragma unroll
+                for (int j = 0; j < 8; j++) {         // 16-byte pieces in an order of the row's own: a warp's rows fall into all banks
+                    const unsigned at_piece = cell + (unsigned) (((c0 / 4 + j) ^ (local & 31)) << 4);
+                    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at_piece), "r"(any ? o[4 * j] : 0u), "r"(any ? o[4 * j + 1] : 0u),
+                                 "r"(any ? o[4 * j + 2] : 0u), "r"(any ? o[4 * j + 3] : 0u) : "memory");
+                }
+            }
+            asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(at_peer(at_smem(sQ), to) + (unsigned) ((part * each + local) * 8)), "f"(m_run), "f"(l_run)
+                         : "memory");
+            at_cluster_sync();
+            // ---- 256 / parts rows, `parts` threads a row with 128 / parts columns each
+            const int t = g * AT_BM + r, my = t % each, Rm = row0 + part * each + my, cols = AT_HD / p.parts;
+            if (Rm < rows_total) {
+                const float2 * ml = reinterpret_cast<const float2 *>(sQ);
+                float M = -INFINITY, L = 0.0f, w[kAtParts];
+#pragma unroll
+                for (int j = 0; j < kAtParts; j++)
+                    if (j < p.parts) M = fmaxf(M, ml[j * each + my].x);
+#pragma unroll
+                for (int j = 0; j < kAtParts; j++) {
+                    w[j] = 0.0f;
+                    if (j < p.parts) {
+                        const float2 x = ml[j * each + my];
+                        if (x.x != -INFINITY) w[j] = at_exp2((x.x - M) * sl);
+                        L = fmaf(x.y, w[j], L);
+                    }
+                }
+                const float inv = L > 0.0f ? 1.0f / L : 0.0f;
+                __nv_bfloat16 * dst = p.out + ((size_t) (q0 + Rm / G) * p.nh + kvh * G + Rm % G) * AT_HD;
+                for (int c = t / each * cols; c < (t / each + 1) * cols; c += 8) {
+                    float sum[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                    for (int j = 0; j < kAtParts; j++)
+                        if (j < p.parts) {
+                            const float4 * cells = reinterpret_cast<const float4 *>(sK) + (j * each + my) * (AT_HD / 4);
+                            const float4 a = cells[(c / 4) ^ (my & 31)], b = cells[(c / 4 + 1) ^ (my & 31)];
+                            sum[0] = fmaf(a.x, w[j], sum[0]); sum[1] = fmaf(a.y, w[j], sum[1]); sum[2] = fmaf(a.z, w[j], sum[2]); sum[3] = fmaf(a.w, w[j], sum[3]);
+                            sum[4] = fmaf(b.x, w[j], sum[4]); sum[5] = fmaf(b.y, w[j], sum[5]); sum[6] = fmaf(b.z, w[j], sum[6]); sum[7] = fmaf(b.w, w[j], sum[7]);
+                        }
+                    uint4 pk;
+                    unsigned * words = reinterpret_cast<unsigned *>(&pk);
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        __nv_bfloat162 h = __floats2bfloat162_rn(sum[2 * e] * inv, sum[2 * e + 1] * inv);
+                        words[e] = *reinterpret_cast<unsigned *>(&h);
+                    }
+                    *reinterpret_cast<uint4 *>(dst + c) = pk;
+                }
+            }
+        } else
         // ---- O / sum -> out ---------------------------------------------------------------------------
         if (n_mine > 0 && !failed) {
             if (at_wait(at_smem(&pv_done[g]), (unsigned) (n_mine - 1) & 1u)) {
@@ -629,12 +724,42 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_tc_kernel(
         }
     }
 done:
+    if (SPLIT && warp < 2) {              // the softmax warps have passed both barriers above
+        at_cluster_sync();
+        at_cluster_sync();
+    }
     at_fence_before();
     __syncthreads();
     if (warp == 1) {
         at_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }
+}
+
+// Clusters of `parts` CTAs that the GPU holds at once, asked once (an SM holds one CTA, and a cluster stays inside one GPC).
+static int at_clusters(int parts, size_t smem) {
+    static std::atomic<int> known[4];
+    std::atomic<int> & slot = known[parts >= 8 ? 3 : parts >= 4 ? 2 : 1];
+    int n = slot.load(std::memory_order_relaxed);
+    if (n == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned) parts);
+        cfg.blockDim = dim3(AT_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned) parts;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaFuncSetAttribute(attention_tc_kernel<AT_SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, attention_tc_kernel<AT_SPLIT>, &cfg) != cudaSuccess || n <= 0) {
+            cudaGetLastError();
+            n = -1;                                          // not to be had: no split of this size
+        }
+        slot.store(n, std::memory_order_relaxed);
+    }
+    return n;
 }
 
 // a cache [num_pages, nkv, page_size, 128] bf16; boxes of one page and half a head: [page_size rows, 64 values]
@@ -691,6 +816,101 @@ IIAN_API int iian_attention_tc(const void * q, const void * k_cache, const void 
                                float scale, int window, int * status, cudaStream_t stream) {
     return iian_attention_tc_sink(q, k_cache, v_cache, out, cu_q, ctx_len, block_table, max_blocks, N, S, max_q_len, nh, nkv, hd,
                                   page_size, num_pages, scale, window, status, nullptr, stream);
+}
+
+// CTAs that should share each row tile's keys, from the step's host numbers (cu_q [S + 1], ctx_len [S]).  us of a launch, as measured: 12 + 2.3 a
+// key tile of the longest walk, or of an SM's share of all of them with 4 tiles' time for every further CTA; split, 19 + 2.3 a tile of a
+// part (set-up and merge), 7 tiles' time for a CTA of a further wave.  Clusters of four and eight only where all fit at once.
+//   tokens behind cached ones, 32 heads on 8     one CTA    2      4      8 a row tile
+//   40 behind 3,000                                 67      47     34     27
+//   100 behind 7,000                               144      87     54     69 (a second wave)
+//   512 behind 3,000                                76      52     70    132
+//   150 + 450 behind 1,200 and 6,000               130      86    120    184
+//   1,024 behind 3,000                              87      99    138    240
+//   151, 756 and 454 behind 200, 3,100, 6,000      143     167    216    360
+IIAN_API int iian_attention_tc_choose(const int * cu_q, const int * ctx_len, int S, int nh, int nkv, int window) {
+    if (S <= 0 || nkv <= 0 || nh % nkv != 0) return 1;
+    const int G = nh / nkv;
+    if ((long long) (cu_q[S] - cu_q[0]) * G / AT_ROWS * nkv >= 2 * 148) return 1;    // enough CTAs as it is
+    long long units = 0, work = 0, longest = 0;
+    for (int s = 0; s < S; s++) {
+        const int q = cu_q[s + 1] - cu_q[s], pos0 = ctx_len[s] - q, n = (q * G + AT_ROWS - 1) / AT_ROWS;
+        units += n;
+        for (int t = 0; t < n; t++) {
+            const int last = pos0 + std::min(q * G - 1, t * AT_ROWS + AT_ROWS - 1) / G, first = pos0 + t * AT_ROWS / G;
+            const long long tiles = last / AT_BN - (window > 0 ? std::max(0, first - window + 1) / AT_BN : 0) + 1;
+            work += tiles;
+            longest = std::max(longest, tiles);
+        }
+    }
+    units *= nkv;
+    work *= nkv;
+    const size_t smem = (size_t) 6 * AT_TILE_BYTES + 1024;
+    int best = 1;
+    double least = 12.0 + 2.3 * std::max((double) longest, (double) (work + 4 * units) / 148.0);
+    for (int parts = 2; parts <= kAtParts && parts <= longest; parts *= 2) {
+        const int clusters = at_clusters(parts, smem);
+        if (clusters < 0 || (parts > 2 && units > clusters)) break;
+        double tiles = (double) ((longest + parts - 1) / parts);
+        if (units > clusters) tiles = std::max(tiles, (double) (work + 7 * units * parts) / 148.0);
+        const double us = 19.0 + 2.3 * tiles;
+        if (us < 0.95 * least) { least = us; best = parts; }
+    }
+    return best;
+}
+
+// The same with a sink per head (f32 [nh], or null; needs scale > 0), and with the keys of a row tile shared by `parts` CTAs (1, 2, 4 or 8).
+IIAN_API int iian_attention_tc_parts(const void * q, const void * k_cache, const void * v_cache, void * out,
+                                     const int * cu_q, const int * ctx_len, const int * block_table, int max_blocks,
+                                     int N, int S, int max_q_len, int nh, int nkv, int hd, int page_size, int num_pages,
+                                     float scale, int window, int * status, const float * sink, int parts, cudaStream_t stream) {
+    if (N <= 0 || S <= 0) return IIAN_OK;
+    if (parts < 1 || parts > kAtParts || (parts & (parts - 1))) return IIAN_ERR_SHAPE;
+    if (parts == 1)
+        return iian_attention_tc_sink(q, k_cache, v_cache, out, cu_q, ctx_len, block_table, max_blocks, N, S, max_q_len, nh, nkv, hd,
+                                      page_size, num_pages, scale, window, status, sink, stream);
+    if (sink != nullptr && !(scale > 0.0f)) return IIAN_ERR_SHAPE;
+    if (hd != AT_HD || nkv <= 0 || nh % nkv != 0) return IIAN_ERR_SHAPE;
+    if (page_size != 8 && page_size != 16 && page_size != 32 && page_size != 64 && page_size != 128) return IIAN_ERR_SHAPE;
+    if (status == nullptr) return IIAN_ERR_SHAPE;
+    if (((uintptr_t) q & 15) || ((uintptr_t) k_cache & 15) || ((uintptr_t) v_cache & 15) || ((uintptr_t) out & 15)) return IIAN_ERR_ALIGN;
+    if (S > 65535 || nkv > 65535) return IIAN_ERR_LIMIT;
+    CUtensorMap mk, mv;
+    int rc = at_make_map(&mk, k_cache, num_pages, nkv, page_size);
+    if (rc != IIAN_OK) return rc;
+    rc = at_make_map(&mv, v_cache, num_pages, nkv, page_size);
+    if (rc != IIAN_OK) return rc;
+    TcAttnParams p;
+    p.q = (const __nv_bfloat16 *) q; p.out = (__nv_bfloat16 *) out; p.cu_q = cu_q; p.ctx_len = ctx_len; p.block_table = block_table;
+    p.max_blocks = max_blocks; p.nh = nh; p.nkv = nkv; p.num_seqs = S; p.page_size = page_size; p.num_pages = num_pages; p.window = window;
+    p.scale_log2 = scale * 1.4426950408889634f;
+    p.status = status;
+    p.sink = sink;
+    p.sink_to_raw = sink != nullptr ? 1.0f / scale : 0.0f;
+    p.ld_q = (long long) nh * hd;
+    p.parts = parts;
+    p.single = at_single(N, S, max_q_len, nh / nkv, AT_ROWS, nkv * parts);
+    const size_t smem = (size_t) 6 * AT_TILE_BYTES + 1024;
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel<AT_SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+        if (e != cudaSuccess) return 1000 + (int) e;
+        configured = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = at_grid(N, S, max_q_len, nh, nkv, AT_ROWS);
+    cfg.gridDim.x *= (unsigned) parts;
+    cfg.blockDim = dim3(AT_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned) parts;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, attention_tc_kernel<AT_SPLIT>, mk, mv, p);
+    return e == cudaSuccess ? iian_launch_status() : 1000 + (int) e;
 }
 
 // The same with a sink per head in the softmax's denominator (sink: f32 [nh], or null; needs scale > 0).

@@ -60,7 +60,8 @@ struct Kernels {
     int (*gemm_tcgen05_fused)(const void *, const void *, void *, int, int, int, int, int, int, int *, const float *, int, float,
                               float, float *, const float *, float *, S) = nullptr;
     int (*attention_tc)(const void *, const void *, const void *, void *, const int *, const int *, const int *, int, int, int,
-                        int, int, int, int, int, int, float, int, int *, S) = nullptr;
+                        int, int, int, int, int, int, float, int, int *, const float *, int, S) = nullptr;
+    int (*attention_tc_choose)(const int *, const int *, int, int, int, int) = nullptr;
     int (*attention_mma)(const void *, const void *, const void *, void *, float *, float *, int *, const int *, const int *,
                          const int *, int, int, int, int, int, int, int, int, int, float, int, int, int, int *, S) = nullptr;
     int (*attention_decode_fused)(const void *, void *, void *, void *, float *, float *, int *, const int *, const int *,
@@ -113,6 +114,7 @@ struct StepInts {
     int N = 0, S = 0, R = 0;
     int max_q_len = 0, max_ctx = 0;
     bool decode_only = false, rows_identity = false;
+    const int * h_cu_q = nullptr, * h_ctx_len = nullptr;       // cu_q and ctx_len on the host, until the next step is staged
     const int * tokens = nullptr, * positions = nullptr, * seq_of_token = nullptr, * cu_q = nullptr, * ctx_len = nullptr,
               * state_slots = nullptr, * out_rows = nullptr;
     std::vector<const int *> slots, block_table;      // per group
@@ -451,14 +453,16 @@ struct NativeRunner::Impl {
                                       nh, nkv, hd, ps, c.num_pages, L.scale, L.window, n_split, cluster ? 2 : 1, decode_status(),
                                       mixed_stream), "attention_mma");
                 check(k.attention_tc(q, c.k_cache, c.v_cache, out, si.cu_q + Sd, si.ctx_len + Sd, bt + (size_t) Sd * mb, mb, si.N,
-                                     si.S - Sd, si.max_q_len, nh, nkv, hd, ps, c.num_pages, L.scale, L.window, tc_status, stream),
+                                     si.S - Sd, si.max_q_len, nh, nkv, hd, ps, c.num_pages, L.scale, L.window, tc_status, nullptr,
+                                     k.attention_tc_choose(si.h_cu_q + Sd, si.h_ctx_len + Sd, si.S - Sd, nh, nkv, L.window), stream),
                       "attention_tc");
                 cuda_ok(cudaEventRecord(mixed_join, mixed_stream), "cudaEventRecord");
                 cuda_ok(cudaStreamWaitEvent(stream, mixed_join, 0), "cudaStreamWaitEvent");
                 return;
             }
             check(k.attention_tc(q, c.k_cache, c.v_cache, out, si.cu_q, si.ctx_len, bt, mb, si.N, si.S, si.max_q_len, nh, nkv, hd, ps,
-                                 c.num_pages, L.scale, L.window, tc_status, stream), "attention_tc");
+                                 c.num_pages, L.scale, L.window, tc_status, nullptr,
+                                 k.attention_tc_choose(si.h_cu_q, si.h_ctx_len, si.S, nh, nkv, L.window), stream), "attention_tc");
             return;
         }
         if (bf16_mode() && (hd == 64 || hd == 128)) {
@@ -753,6 +757,7 @@ struct NativeRunner::Impl {
         si.state_slots = dev + o_state; si.out_rows = dev + o_rows;
         for (int g = 0; g < G; g++) { si.slots.push_back(dev + o_slots[g]); si.block_table.push_back(dev + o_bt[g]); }
         si.max_blocks = max_blocks;
+        si.h_cu_q = host + o_cu; si.h_ctx_len = host + o_ctx;
         si.max_q_len = max_q; si.max_ctx = max_ctx;
         if (slot != nullptr) { si.max_q_len = 1; si.max_ctx = slot->ctx_bucket; si.n_split = slot->n_split; }
         si.decode_only = si.max_q_len == 1;
@@ -926,8 +931,10 @@ NativeRunner::NativeRunner(const ModelDesc & model, const KernelLibraries & libs
             bind(h, "iian_gemm_tcgen05", k.gemm_tcgen05, libs.gemm_tcgen05);
             bind(h, "iian_gemm_tcgen05_fused", k.gemm_tcgen05_fused, libs.gemm_tcgen05);
         } else fail("the gemm_tcgen05 kernel library is required for bfloat16");
-        if (void * h = open(libs.attention_tc)) bind(h, "iian_attention_tc", k.attention_tc, libs.attention_tc);
-        else fail("the attention_tc kernel library is required for bfloat16");
+        if (void * h = open(libs.attention_tc)) {
+            bind(h, "iian_attention_tc_parts", k.attention_tc, libs.attention_tc);
+            bind(h, "iian_attention_tc_choose", k.attention_tc_choose, libs.attention_tc);
+        } else fail("the attention_tc kernel library is required for bfloat16");
         if (void * h = open(libs.attention_mma)) {
             bind(h, "iian_attention_mma", k.attention_mma, libs.attention_mma);
             bind(h, "iian_attention_decode_fused", k.attention_decode_fused, libs.attention_mma);

@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import itertools
 import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
 from types import SimpleNamespace
@@ -672,9 +673,10 @@ class CudaKernels:
                 and meta.max_q_len * (nh // nkv) >= self.TC_ATTENTION_MIN_ROWS)
 
     def paged_attention_tc(self, q, k_cache, v_cache, out, meta, *, num_heads, num_kv_heads, head_dim, scale, window,
-                           sink: Optional[torch.Tensor] = None) -> None:
+                           sink: Optional[torch.Tensor] = None, parts: int = 0) -> None:
         """Prefill attention on tcgen05 + TMA: head size 128, bfloat16, pages of 8 to 128 tokens.  ``sink``: float32 [heads],
-        a logit per head that joins the softmax's denominator (needs ``scale`` > 0)."""
+        a logit per head that joins the softmax's denominator (needs ``scale`` > 0).  ``parts``: CTAs that share a row tile's
+        keys (1, 2, 4, 8; 0: chosen by the step's sizes)."""
         n = q.shape[0]
         if k_cache.dtype != torch.bfloat16 or q.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
             raise KernelError("paged_attention_tc: bfloat16 only")
@@ -685,14 +687,27 @@ class CudaKernels:
         bt = meta.block_table
         if sink is not None and sink.numel() != num_heads:
             raise KernelError("paged_attention_tc: one sink per head")
-        fn = _fn("attention_tc", "iian_attention_tc_sink",
+        if parts == 0:
+            parts = self.attention_tc_parts(meta, num_heads, num_kv_heads, window)
+        fn = _fn("attention_tc", "iian_attention_tc_parts",
                  [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
-                  c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_void_p])
+                  c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_int, c_void_p])
         _check(fn(_cuda(q, "q"), _cuda(k_cache, "k cache"), _cuda(v_cache, "v cache"), _cuda(out, "attention out"),
                   _cuda(meta.cu_q, "cu_q", torch.int32), _cuda(meta.ctx_len, "ctx_len", torch.int32),
                   _cuda(bt, "block table", torch.int32), bt.shape[1], n, meta.num_seqs, meta.max_q_len, num_heads,
                   num_kv_heads, head_dim, k_cache.shape[2], k_cache.shape[0], scale, window or 0,
-                  status.data_ptr(), _cuda(sink, "sink", torch.float32), _stream()), "attention_tc")
+                  status.data_ptr(), _cuda(sink, "sink", torch.float32), parts, _stream()), "attention_tc")
+
+    def attention_tc_parts(self, meta, num_heads: int, num_kv_heads: int, window) -> int:
+        """How many CTAs of the prefill kernel should share each row tile's keys, from the step's lengths as the host knows them (1
+        where it does not)."""
+        lens, ctxs = getattr(meta, "h_q_len", ()), getattr(meta, "h_ctx_len", ())
+        s = meta.num_seqs
+        if len(lens) != s or len(ctxs) != s or max(ctxs) <= 6 * 128 or sum(lens) * num_heads >= 2 * 148 * 256:     # no gain there
+            return 1
+        cu = (c_int * (s + 1))(0, *itertools.accumulate(lens))
+        return _fn("attention_tc", "iian_attention_tc_choose", [c_void_p, c_void_p, c_int, c_int, c_int, c_int])(
+            cu, (c_int * s)(*ctxs), s, num_heads, num_kv_heads, window or 0)
 
     def _attention_dispatch(self, q, k_cache, v_cache, out, meta, nh, nkv, hd, scale, window, n_split=None) -> None:
         if self._attention_tc_ok(q, k_cache, meta, nh, nkv, hd):

@@ -604,6 +604,23 @@ def test_paged_attention_mma(case, standout, mode):
     assert err < tol(dtype, max(1.0, want.abs().max().item())), err
 
 
+@pytest.mark.parametrize("parts", [2, 4, 8])
+@pytest.mark.parametrize("window", [0, 150])
+@pytest.mark.parametrize("ctx_lens,q_lens", [([700], [300]), ([1100, 129, 40], [33, 129, 40]), ([128], [128]), ([1500], [16])])
+@pytest.mark.parametrize("nh,nkv,ps", [(8, 2, 16), (2, 2, 64)])
+def test_prefill_attention_shared_by_ctas(nh, nkv, ps, ctx_lens, q_lens, window, parts):
+    """A row tile's keys in several runs, some of them empty: against the oracle, and against one CTA's result, from which it differs by the
+    rounding of P to bfloat16 (2^-9 of a value of order one, whichever maximum it is taken against) and of the result."""
+    q, kc, vc, m, want, scale = attention_case(torch.bfloat16, nh, nkv, 128, ps, ctx_lens, q_lens, window, seed=3)
+    one, out = (torch.full((q.shape[0], nh * 128), float("nan"), dtype=torch.bfloat16).cuda() for _ in range(2))
+    kw = dict(num_heads=nh, num_kv_heads=nkv, head_dim=128, scale=scale, window=window)
+    K().paged_attention_tc(q, kc, vc, one, m, parts=1, **kw)
+    K().paged_attention_tc(q, kc, vc, out, m, parts=parts, **kw)
+    K().tcgen05_check(q.device)
+    assert (out.double().cpu() - want).abs().max() < tol(torch.bfloat16, max(1.0, want.abs().max().item()))
+    assert (out.double() - one.double()).abs().max() < 2 ** -7 * max(1.0, want.abs().max().item())
+
+
 @pytest.mark.parametrize("od", DT)
 @pytest.mark.parametrize("N", [1, 2, 4, 5, 8, 9, 16, 17, 33, 64, 65, 130])
 @pytest.mark.parametrize("M,K_", [(1, 4), (33, 132), (130, 260), (257, 1000), (6151, 48)])
