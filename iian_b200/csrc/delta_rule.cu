@@ -430,6 +430,7 @@ delta_prep_wide_kernel(const __nv_bfloat16 * __restrict__ proj, long long ld, in
 
 constexpr int kCols = 16;        // columns of S a CTA owns
 constexpr int kLanes = 8;        // lanes that share a column
+constexpr int kScanThreads = kCols * kLanes;
 
 __device__ __forceinline__ void dr_cp4(float * dst, const float * src, bool valid) {
     const unsigned d = (unsigned) __cvta_generic_to_shared(dst);
@@ -479,7 +480,7 @@ __device__ __forceinline__ void delta_scan(float * sm, const float * __restrict_
         float * s_b = s_v + chunk * kCols;
         if (VEC) {
             const int per = D >> 2;
-            for (int e = threadIdx.x; e < nt * per; e += blockDim.x) {
+            for (int e = threadIdx.x; e < nt * per; e += kScanThreads) {
                 const int tt = e / per, d = (e - tt * per) << 2;
                 const size_t t = c0 + tt;
                 copy16(s_q + tt * Dp + d, qn + t * GD + g * D + d);
@@ -487,7 +488,7 @@ __device__ __forceinline__ void delta_scan(float * sm, const float * __restrict_
                 if (!HEAD) copy16(s_g + tt * Dp + d, decay + t * HD + h * D + d);
             }
         } else {
-            for (int e = threadIdx.x; e < nt * D; e += blockDim.x) {
+            for (int e = threadIdx.x; e < nt * D; e += kScanThreads) {
                 const int tt = e / D, d = e - tt * D;
                 const size_t t = c0 + tt;
                 dr_cp4(s_q + tt * Dp + d, qn + t * GD + g * D + d, true);
@@ -495,12 +496,12 @@ __device__ __forceinline__ void delta_scan(float * sm, const float * __restrict_
                 if (!HEAD) dr_cp4(s_g + tt * Dp + d, decay + t * HD + h * D + d, true);
             }
         }
-        for (int e = threadIdx.x; e < nt * kCols; e += blockDim.x) {
+        for (int e = threadIdx.x; e < nt * kCols; e += kScanThreads) {
             const int tt = e / kCols, c = e - tt * kCols;
             const int jj = cb * kCols + c;
             dr_cp4(s_v + e, vv + (size_t) (c0 + tt) * HV + h * V + (jj < V ? jj : 0), jj < V);
         }
-        for (int e = threadIdx.x; e < nt; e += blockDim.x) {
+        for (int e = threadIdx.x; e < nt; e += kScanThreads) {
             dr_cp4(s_b + kPer * e, beta + (size_t) (c0 + e) * H + h, true);
             dr_cp4(s_b + kPer * e + 1, qk + (size_t) (c0 + e) * G + g, true);
             if (HEAD) dr_cp4(s_b + kPer * e + 2, decay + (size_t) (c0 + e) * H + h, true);
@@ -514,7 +515,7 @@ __device__ __forceinline__ void delta_scan(float * sm, const float * __restrict_
         const int C = 2 * GD + HV, back = n_taps - 1, L = t1 - t0;
         float * tail = st + tail_off;
         const int part = h * gridDim.x + cb, parts = gridDim.x * gridDim.y;
-        for (int c = part * blockDim.x + threadIdx.x; c < C; c += parts * blockDim.x) {
+        for (int c = part * kScanThreads + threadIdx.x; c < C; c += parts * kScanThreads) {
             float keep[kMaxTaps];
 #pragma unroll
             for (int i = 0; i < kMaxTaps - 1; i++) {
@@ -750,11 +751,15 @@ delta_block_kernel(const float * __restrict__ qn, const float * __restrict__ kn,
 }
 
 // A CTA owns kCols columns of one (sequence, head); 16 lanes share two columns, E = D / 16 entries of each a lane (groups of four
-// neighbours, d = 4 lane + 64 i): a vector that is read serves both.  Where the time goes: some 260 instructions a warp and piece, 5 clocks
-// each with one warp per scheduler, their chain (reduction over the lanes, four writes, update) uncovered.  1,500 tokens x 16 heads: 256 us
-// (token by token 399 us).  Measured against it: eight lanes a column, each column reading every vector for itself, 300 us (128 bytes a clock
-// is what shared memory delivers to registers); 32 lanes for two columns, two warps per scheduler, 240 us, but 565 against 500 us for four
-// sequences of 2,048; a warp per eighth of D and a lane per column, the sums through shared memory, 241 and 523 us.
+// neighbours, d = 4 lane + 64 i): a vector that is read serves both.  Where the time goes: some 260 instructions a warp and piece with one
+// warp per scheduler; of 920 clocks the eight dot products take 400, their reduction over the lanes 180, the four writes 170, the update 170,
+// and shared memory's reads and shuffles fill 530 of them.
+// AHEAD, where every CTA has an SM to itself: a fifth warp copies the pieces (350 clocks of a piece where every warp copied its share in its
+// own chain), and their vectors are read into registers a step before they are needed; that takes 200 registers a thread, one CTA an SM, so
+// it is not the form for more CTAs (32 heads, 2,048 tokens: 485 us in two rounds, 440 side by side).  1,500 tokens x 16 heads: 181 us (243
+// without, with equal addresses 16 lanes apart; token by token 399).  Measured against the sixteen lanes: eight lanes a column, each
+// column reading every vector for itself, 300 us (128 bytes a clock is what shared memory delivers to registers); 32 lanes for two columns, two
+// warps per scheduler, 240 for then 256; a warp per eighth of D and a lane per column, the sums through shared memory, 241.
 // V a multiple of kCols; state and values on 16-byte boundaries.
 // Sequences with fewer than at_least tokens are walked token by token as in the scan above, in the same launch: a piece costs more than a
 // token, and a launch of their own would wait for the long ones' chain (a portion of 100 tokens beside 100
@@ -762,8 +767,8 @@ delta_block_kernel(const float * __restrict__ qn, const float * __restrict__ kn,
 // walks decide, 1 where many short ones do, so that seven CTAs share an SM and not four (the same 131 us for 142, but 1,500 tokens 386 for 363).
 constexpr int kPairLanes = 16;
 
-template <int E, int PER, bool HEAD, typename A>
-__global__ void __launch_bounds__(kCols / 2 * kPairLanes)
+template <int E, int PER, bool AHEAD, bool HEAD, typename A>
+__global__ void __launch_bounds__(kCols / 2 * kPairLanes + (AHEAD ? 32 : 0))
 delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restrict__ qn, const float * __restrict__ kn,
                         const float * __restrict__ vv, const float * __restrict__ beta, const float * __restrict__ decay,
                         const float * __restrict__ qk, float * __restrict__ state, long long state_stride,
@@ -771,16 +776,17 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
                         const int * __restrict__ cu_q, const int * __restrict__ state_slots, float * __restrict__ out,
                         int from, int pieces, int at_least, int H, int G, int V) {
     constexpr int D = E * kPairLanes, BLOCK = 13 * D + kBlockNumbers, PIECE = BLOCK + 4 * kCols, STAGE = PER * PIECE;
-    constexpr int kThreads = kCols / 2 * kPairLanes;
+    constexpr int kThreads = kCols / 2 * kPairLanes;         // with AHEAD and a warp that copies
     extern __shared__ __align__(16) float sm[];
     const int cb = blockIdx.x, h = blockIdx.y, s = blockIdx.z;
-    const int tid = threadIdx.x, pair = tid / kPairLanes, lane = tid % kPairLanes, j = cb * kCols + 2 * pair;
+    // neighbouring threads have the same entries of two pairs of columns: a 16-byte read then takes 2 clocks a warp, 4 where they lie 16 apart
+    const int tid = threadIdx.x, pair = tid / 32 * 2 + (tid & 1), lane = tid % 32 >> 1, j = cb * kCols + 2 * pair;
     const int q0 = cu_q[s], q1 = cu_q[s + 1], slot = state_slots[s], HV = H * V;
     const int t0 = q0 + from, t1 = pieces > 0 ? min(q1, t0 + 4 * pieces) : q1;
     if (q1 - q0 < at_least) {
         constexpr int CHUNK = scan_floats(HEAD, D, 16) <= kBlockStages * STAGE ? 16 : 8;
         static_assert(kCols / 2 * kPairLanes == kCols * kLanes && scan_floats(HEAD, D, CHUNK) <= kBlockStages * STAGE, "both walks fit one launch");
-        if (from == 0)
+        if (from == 0 && tid < kThreads)
             delta_scan<D / kLanes, true, HEAD, A>(sm, qn, kn, vv, beta, decay, qk, state, state_stride, tail_off, proj, ld, col_off, n_taps, cu_q,
                                                   state_slots, out, H, G, D, V, CHUNK);
         return;
@@ -788,13 +794,14 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
     if (t0 >= t1) return;
     if (slot < 0) {
         for (int t = t0; t < t1; t++)
-            if (lane < 2) out[(size_t) t * HV + h * V + j + lane] = 0.0f;
+            if (lane < 2 && tid < kThreads) out[(size_t) t * HV + h * V + j + lane] = 0.0f;
         return;
     }
     float * st = state + (size_t) slot * state_stride;
     const int n_blocks = (t1 - t0 + 3) / 4, turns = (n_blocks + PER - 1) / PER;
     const float * mine = blocks + (first_piece(cu_q, s, pieces) * H + h) * BLOCK;
-    auto fill = [&](int turn) {
+    auto fill = [&](int turn, int me, auto threads) {
+        constexpr int kCopiers = decltype(threads)::value;
         if (turn < turns) {
             float * to = sm + (turn % kBlockStages) * STAGE;
 #pragma unroll
@@ -802,17 +809,33 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
                 const int c = turn * PER + b;
                 if (c >= n_blocks) break;
                 const float * src = mine + (size_t) c * H * BLOCK;
-                for (int e = tid; e < BLOCK / 4; e += kThreads) copy16(to + b * PIECE + 4 * e, src + 4 * e);
-                if (tid < kCols) {                           // four tokens' values of the CTA's columns; beyond the last token: that one's
-                    const int t = min(t0 + 4 * c + tid / 4, t1 - 1);
-                    copy16(to + b * PIECE + BLOCK + 4 * tid, vv + (size_t) t * HV + h * V + cb * kCols + 4 * (tid % 4));
+#pragma unroll (kCopiers == 32 ? 4 : 1)
+                for (int e = me; e < BLOCK / 4; e += kCopiers) copy16(to + b * PIECE + 4 * e, src + 4 * e);
+                if (me < kCols) {                            // four tokens' values of the CTA's columns; beyond the last token: that one's
+                    const int t = min(t0 + 4 * c + me / 4, t1 - 1);
+                    copy16(to + b * PIECE + BLOCK + 4 * me, vv + (size_t) t * HV + h * V + cb * kCols + 4 * (me % 4));
                 }
             }
         }
         dr_commit();
     };
+    if constexpr (AHEAD) if (tid >= kThreads) {
+        // The copying warp: every turn it waits for what is read next, and fills the stage that has been read by everyone.
+        const std::integral_constant<int, 32> one_warp;
 #pragma unroll
-    for (int i = 0; i < kBlockStages - 1; i++) fill(i);
+        for (int i = 0; i < kBlockStages - 1; i++) fill(i, tid - kThreads, one_warp);
+        for (int turn = 0; turn < turns; turn++) {
+            dr_wait<kBlockStages - 3>();
+            __syncthreads();
+            fill(turn + kBlockStages - 1, tid - kThreads, one_warp);
+        }
+        return;
+    }
+    const std::integral_constant<int, kThreads> all_warps;
+    if constexpr (!AHEAD) {
+#pragma unroll
+        for (int i = 0; i < kBlockStages - 1; i++) fill(i, tid, all_warps);
+    }
 
     if (from == 0 && n_taps > 1) {             // the convolution's tail moves on, as in the scan above
         const int C = 2 * G * D + HV, back = n_taps - 1, L = q1 - q0;
@@ -842,16 +865,34 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
             const ulonglong2 e = *reinterpret_cast<const ulonglong2 *>(scol + x * D + 4 * lane + 4 * kPairLanes * i);
             S[x][2 * i] = e.x; S[x][2 * i + 1] = e.y;
         }
+    // AHEAD: a piece's vectors for the dot products are read while the piece before is reduced and written, from a stage that has landed a turn
+    // early, and those for the update before the reduction, so that no read of shared memory stands in the chain.
+    ulonglong2 dv[E / 4][8], uv[E / 4][5];
+    float * to_out = out + (size_t) t0 * HV + h * V + j + (lane >> 3);
+    auto piece = [&](int c) { return sm + (c / PER % kBlockStages) * STAGE + c % PER * PIECE; };
+    auto at = [&](const float * vec, int v, int i) { return *reinterpret_cast<const ulonglong2 *>(vec + v * D + 4 * lane + 4 * kPairLanes * i); };
+    auto read_dots = [&](const float * vec) {
+#pragma unroll
+        for (int i = 0; i < E / 4; i++)
+#pragma unroll
+            for (int v = 0; v < 8; v++) dv[i][v] = at(vec, v, i);
+    };
+    auto read_update = [&](const float * vec) {
+#pragma unroll
+        for (int i = 0; i < E / 4; i++)
+#pragma unroll
+            for (int v = 0; v < 5; v++) uv[i][v] = at(vec, 8 + v, i);
+    };
     for (int turn = 0; turn < turns; turn++) {
-        dr_wait<kBlockStages - 2>();
-        __syncthreads();                       // this turn's pieces have landed; the stage filled next was read by everyone
-        fill(turn + kBlockStages - 1);
-        const float * stage = sm + (turn % kBlockStages) * STAGE;
+        if (!AHEAD) dr_wait<kBlockStages - 2>();
+        __syncthreads();                       // this turn's pieces have landed (and the next one's); the stage filled next was read by everyone
+        if constexpr (!AHEAD) fill(turn + kBlockStages - 1, tid, all_warps);
+        if (AHEAD && turn == 0) read_dots(piece(0));
 #pragma unroll
         for (int b = 0; b < PER; b++) {
             const int c = turn * PER + b;
             if (c >= n_blocks) break;
-            const float * vec = stage + b * PIECE;
+            const float * vec = piece(c);
             const float * num = vec + 13 * D;
             unsigned long long acc[2][8];
 #pragma unroll
@@ -860,13 +901,24 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
             for (int i = 0; i < E / 4; i++) {
 #pragma unroll
                 for (int v = 0; v < 8; v++) {
-                    const ulonglong2 e = *reinterpret_cast<const ulonglong2 *>(vec + v * D + 4 * lane + 4 * kPairLanes * i);
+                    const ulonglong2 e = AHEAD ? dv[i][v] : at(vec, v, i);
 #pragma unroll
                     for (int x = 0; x < 2; x++) {
                         acc[x][v] = fma2(e.x, S[x][2 * i], acc[x][v]);
                         acc[x][v] = fma2(e.y, S[x][2 * i + 1], acc[x][v]);
                     }
                 }
+            }
+            const float4 be = *reinterpret_cast<const float4 *>(num), A0 = *reinterpret_cast<const float4 *>(num + 4);
+            const float2 A1 = *reinterpret_cast<const float2 *>(num + 8);
+            const float4 B = *reinterpret_cast<const float4 *>(num + 12 + 4 * (lane & 3));
+            const float * val = vec + BLOCK + 2 * pair;
+            float2 v[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) v[t] = *reinterpret_cast<const float2 *>(val + t * kCols);
+            if (AHEAD) {
+                read_update(vec);
+                if (c + 1 < n_blocks) read_dots(piece(c + 1));
             }
             float a[16];
 #pragma unroll
@@ -879,21 +931,15 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
 #pragma unroll
                 for (int i = 0; i < half; i++) {
                     const float give = up ? a[i] : a[i + half], keep = up ? a[i + half] : a[i];
-                    a[i] = keep + __shfl_xor_sync(0xffffffffu, give, half);
+                    a[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * half);
                 }
             }
-            const float4 be = *reinterpret_cast<const float4 *>(num), A0 = *reinterpret_cast<const float4 *>(num + 4);
-            const float2 A1 = *reinterpret_cast<const float2 *>(num + 8);
-            const float * val = vec + BLOCK + 2 * pair;
-            float2 v[4];
-#pragma unroll
-            for (int t = 0; t < 4; t++) v[t] = *reinterpret_cast<const float2 *>(val + t * kCols);
             float u[2][4];
 #pragma unroll
             for (int x = 0; x < 2; x++) {
                 float p[4];
 #pragma unroll
-                for (int t = 0; t < 4; t++) p[t] = (x ? v[t].y : v[t].x) - __shfl_sync(0xffffffffu, a[0], 8 * x + t, kPairLanes);
+                for (int t = 0; t < 4; t++) p[t] = (x ? v[t].y : v[t].x) - __shfl_sync(0xffffffffu, a[0], 2 * (8 * x + t) + (tid & 1));
                 u[x][0] = be.x * p[0];
                 u[x][1] = be.y * (p[1] - A0.x * u[x][0]);
                 u[x][2] = be.z * (p[2] - (A0.y * u[x][0] + A0.z * u[x][1]));
@@ -901,13 +947,12 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
             }
 #pragma unroll
             for (int i = 0; i < E / 4; i++) {
-                const int at = 4 * lane + 4 * kPairLanes * i;
-                ulonglong2 e = *reinterpret_cast<const ulonglong2 *>(vec + 12 * D + at);
+                ulonglong2 e = AHEAD ? uv[i][4] : at(vec, 12, i);
 #pragma unroll
                 for (int x = 0; x < 2; x++) { S[x][2 * i] = mul2(e.x, S[x][2 * i]); S[x][2 * i + 1] = mul2(e.y, S[x][2 * i + 1]); }
 #pragma unroll
                 for (int t = 0; t < 4; t++) {
-                    e = *reinterpret_cast<const ulonglong2 *>(vec + (8 + t) * D + at);
+                    e = AHEAD ? uv[i][t] : at(vec, 8 + t, i);
 #pragma unroll
                     for (int x = 0; x < 2; x++) {
                         const unsigned long long w = pack2(u[x][t], u[x][t]);
@@ -916,14 +961,13 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
                     }
                 }
             }
-            const int t = t0 + 4 * c + (lane & 7) - 4;
-            if ((lane & 4) && t < t1) {
-                const float4 B = *reinterpret_cast<const float4 *>(num + 12 + 4 * (lane & 3));
-                const bool second = lane & 8;
-                const float u0 = second ? u[1][0] : u[0][0], u1 = second ? u[1][1] : u[0][1], u2 = second ? u[1][2] : u[0][2];
-                const float u3 = second ? u[1][3] : u[0][3];
-                out[(size_t) t * HV + h * V + j + (second ? 1 : 0)] = a[0] + (B.x * u0 + B.y * u1 + B.z * u2 + B.w * u3);
-            }
+            // every lane's sum, so that only the store is under a condition
+            const int t = 4 * c + (lane & 7) - 4;
+            const bool second = lane & 8;
+            const float u0 = second ? u[1][0] : u[0][0], u1 = second ? u[1][1] : u[0][1], u2 = second ? u[1][2] : u[0][2];
+            const float u3 = second ? u[1][3] : u[0][3];
+            const float o = a[0] + (B.x * u0 + B.y * u1 + B.z * u2 + B.w * u3);
+            if ((lane & 4) && t < t1 - t0) to_out[(long long) t * HV] = o;
         }
     }
 #pragma unroll
@@ -956,14 +1000,20 @@ IIAN_API int iian_delta_block_scan(const float * qn, const float * kn, const flo
     if (state_stride % 4 || (((uintptr_t) blocks | (uintptr_t) qn | (uintptr_t) kn | (uintptr_t) vv | (uintptr_t) decay | (uintptr_t) state) & 15))
         return IIAN_ERR_ALIGN;
     typedef __nv_bfloat16 bf;
+    const bool ahead = (long long) (V / kCols) * H * S <= 148;
     const int per = max_q_len < 4 * S ? 1 : 2;
-    const size_t smem = (size_t) kBlockStages * per * (13 * D + kBlockNumbers + 4 * kCols) * sizeof(float);
-    auto by_head = [&](auto depth, auto each) {
+    const size_t smem = (size_t) kBlockStages * (ahead ? 2 : per) * (13 * D + kBlockNumbers + 4 * kCols) * sizeof(float);
+    auto by_head = [&](auto depth, auto each, auto first) {
         constexpr int E = decltype(depth)::value, PER = decltype(each)::value;
-        return per_head ? delta_block_scan_kernel<E, PER, true, bf> : delta_block_scan_kernel<E, PER, false, bf>;
+        constexpr bool AHEAD = decltype(first)::value;
+        return per_head ? delta_block_scan_kernel<E, PER, AHEAD, true, bf> : delta_block_scan_kernel<E, PER, AHEAD, false, bf>;
     };
-    auto by_depth = [&](auto each) { return D == 128 ? by_head(std::integral_constant<int, 8>(), each) : by_head(std::integral_constant<int, 4>(), each); };
-    auto scan = per == 2 ? by_depth(std::integral_constant<int, 2>()) : by_depth(std::integral_constant<int, 1>());
+    auto by_depth = [&](auto each, auto first) {
+        return D == 128 ? by_head(std::integral_constant<int, 8>(), each, first) : by_head(std::integral_constant<int, 4>(), each, first);
+    };
+    auto scan = ahead ? by_depth(std::integral_constant<int, 2>(), std::true_type())
+              : per == 2 ? by_depth(std::integral_constant<int, 2>(), std::false_type()) : by_depth(std::integral_constant<int, 1>(), std::false_type());
+    const unsigned threads = kCols / 2 * kPairLanes + (ahead ? 32 : 0);
     const cudaError_t e = cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
     if (e != cudaSuccess) return 1000 + (int) e;
     const int step = pieces > 0 ? 4 * pieces : max_q_len;
@@ -972,7 +1022,7 @@ IIAN_API int iian_delta_block_scan(const float * qn, const float * kn, const flo
         delta_block_kernel<<<grid, 128, 0, stream>>>(qn, kn, beta, decay, per_head, cu_q, state_slots, blocks, from, pieces, at_least, S, H, G, D);
         int rc = iian_launch_status();
         if (rc != IIAN_OK) return rc;
-        scan<<<dim3(V / kCols, H, S), kCols / 2 * kPairLanes, smem, stream>>>(blocks, qn, kn, vv, beta, decay, qk, state, state_stride, (long long) H * V * D,
+        scan<<<dim3(V / kCols, H, S), threads, smem, stream>>>(blocks, qn, kn, vv, beta, decay, qk, state, state_stride, (long long) H * V * D,
                                                                       (const bf *) proj, ld, col_off, n_taps, cu_q, state_slots, out, from, pieces,
                                                                       at_least, H, G, V);
         rc = iian_launch_status();
