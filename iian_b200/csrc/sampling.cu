@@ -616,11 +616,30 @@ __device__ __forceinline__ bool cut_by_bins(const Draw<STAGED> & d, int begin, i
     return true;
 }
 
-template <bool STAGED>
+// A row's settings: from arrays on the device, or from the launch's own parameters (no copy in front of it).
+struct SettingArrays {
+    const float * temperature_, * top_p_, * min_p_, * uniform_;
+    const int * top_k_;
+    __device__ __forceinline__ float temperature(int r) const { return temperature_[r]; }
+    __device__ __forceinline__ float top_p(int r) const { return top_p_[r]; }
+    __device__ __forceinline__ float min_p(int r) const { return min_p_[r]; }
+    __device__ __forceinline__ float uniform(int r) const { return uniform_[r]; }
+    __device__ __forceinline__ int top_k(int r) const { return top_k_[r]; }
+};
+constexpr int kRowsAtOnce = 128;                 // rows of a launch whose settings are parameters: 2.5 of 4 KB
+struct SettingRows {
+    float temperature_[kRowsAtOnce], top_p_[kRowsAtOnce], min_p_[kRowsAtOnce], uniform_[kRowsAtOnce];
+    int top_k_[kRowsAtOnce];
+    __device__ __forceinline__ float temperature(int r) const { return temperature_[r]; }
+    __device__ __forceinline__ float top_p(int r) const { return top_p_[r]; }
+    __device__ __forceinline__ float min_p(int r) const { return min_p_[r]; }
+    __device__ __forceinline__ float uniform(int r) const { return uniform_[r]; }
+    __device__ __forceinline__ int top_k(int r) const { return top_k_[r]; }
+};
+
+template <bool STAGED, typename Settings>
 __global__ void __launch_bounds__(kDrawThreads) sample_kernel(
-    const float * __restrict__ logits, int V, size_t stride, int slice, const float * __restrict__ temperature,
-    const int * __restrict__ top_k, const float * __restrict__ top_p, const float * __restrict__ min_p,
-    const float * __restrict__ uniform, int * __restrict__ out) {
+    const float * __restrict__ logits, int V, size_t stride, int slice, const __grid_constant__ Settings set, int * __restrict__ out) {
     extern __shared__ unsigned staged[];
     __shared__ DrawShared sh;
     __shared__ float fs[32];
@@ -630,7 +649,7 @@ __global__ void __launch_bounds__(kDrawThreads) sample_kernel(
     const int ctas = (int) cl.num_blocks(), rank = (int) cl.block_rank(), row = blockIdx.x / ctas;
     const int begin = (int) min((long long) V, (long long) rank * slice), n = (int) min((long long) V, (long long) begin + slice) - begin;
     const float * src = logits + (size_t) row * stride + begin;
-    const float T = temperature[row];
+    const float T = set.temperature(row);
     const bool greedy = T < 1e-5f;
     const float inv_t = greedy ? 1.0f : 1.0f / T;
 
@@ -673,7 +692,7 @@ __global__ void __launch_bounds__(kDrawThreads) sample_kernel(
     d.turn ^= 1;
     const int imax = best_i == 0x7fffffff ? 0 : best_i;
     d.zmax = best;
-    const float P = top_p[row];
+    const float P = set.top_p(row);
     // nothing to draw from: a greedy row, an infinite or missing largest value, or a share of the mass that keeps none (these
     // tests see the same numbers in every CTA, so a cluster leaves together; what was sent has been read by its receiver only
     // after the barrier above, and nothing is sent after it)
@@ -685,13 +704,13 @@ __global__ void __launch_bounds__(kDrawThreads) sample_kernel(
     // candidates: keys above `cut`, and the first n_tie entries (by id) whose key is `cut`
     unsigned cut = order_key(-INFINITY) + 1u;    // entries without mass change nothing
     int n_tie = 0x7fffffff;
-    const float mp = min_p[row];
+    const float mp = set.min_p(row);
     if (mp > 0.0f) cut = max(cut, order_key(best + logf(mp)));
-    const int k = top_k[row];
+    const int k = set.top_k(row);
     const bool cuts = cut < top && (k > 0 || P < 1.0f);
     if (STAGED && cuts && k > 0 && k <= ctas * kDrawWarps / 2) {
         int token;
-        if (draw_from_list(d, begin, k, P, cut, uniform[row], token)) {
+        if (draw_from_list(d, begin, k, P, cut, set.uniform(row), token)) {
             if (rank == 0 && tid == 0) out[row] = token;
             cl.sync();                           // the lists of this CTA have been read
             return;
@@ -788,7 +807,7 @@ __global__ void __launch_bounds__(kDrawThreads) sample_kernel(
     d.swap();
     double total = 0.0;
     for (int r = 0; r < ctas; r++) total += sh.inbox_m[d.turn][r][0];
-    const double u = (double) uniform[row] * total;
+    const double u = (double) set.uniform(row) * total;
     // the CTA the draw falls into: the first whose running sum passes it, else (rounding) the last that holds mass
     int owner = -1;
     double run = 0.0, ahead = 0.0;
@@ -951,17 +970,14 @@ IIAN_API int iian_argmax_wide(const float * logits, int R, int V, long long stri
 
 // CTAs per row: slices of up to 13,000 entries, up to 8 CTAs.  Less of a slice is no faster for a few rows and a wave more for many: 48 rows
 // of 32,768 with 8 CTAs 31 us, with 4 22, with 2 27; of 50,257 with 8 35, with 4 29; 16 CTAs of a row of 151,936 72 for 49 with 8.
-IIAN_API int iian_sample(const float * logits, int R, int V, long long stride, const float * temperature,
-                         const int * top_k, const float * top_p, const float * min_p, const float * uniform,
-                         int * out, cudaStream_t stream) {
-    if (R <= 0) return IIAN_OK;
-    if (V <= 0) return IIAN_ERR_SHAPE;
+template <typename Settings>
+static int launch_sample(const float * logits, int R, int V, long long stride, const Settings & set, int * out, cudaStream_t stream) {
     int ctas = 1;
     while (ctas < kDrawCluster && V > ctas * kSliceGoal) ctas *= 2;
     const int slice = (V - 1) / ctas + 1;
     const bool staged = slice <= kStagedMax;
     const size_t smem = staged ? (size_t) slice * sizeof(unsigned) : 0;
-    auto kernel = staged ? sample_kernel<true> : sample_kernel<false>;
+    auto kernel = staged ? sample_kernel<true, Settings> : sample_kernel<false, Settings>;
     if (smem > 24 * 1024) {                      // with the 20 KB of static memory above what a launch may ask for by itself
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
         if (e != cudaSuccess) return 1000 + (int) e;
@@ -977,9 +993,47 @@ IIAN_API int iian_sample(const float * logits, int R, int V, long long stride, c
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cfg.gridDim = dim3((unsigned) R * (unsigned) ctas);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, logits, V, (size_t) stride, slice, temperature, top_k, top_p, min_p,
-                                             uniform, out);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, logits, V, (size_t) stride, slice, set, out);
     return e == cudaSuccess ? IIAN_OK : 1000 + (int) e;
+}
+
+IIAN_API int iian_sample(const float * logits, int R, int V, long long stride, const float * temperature,
+                         const int * top_k, const float * top_p, const float * min_p, const float * uniform,
+                         int * out, cudaStream_t stream) {
+    if (R <= 0) return IIAN_OK;
+    if (V <= 0) return IIAN_ERR_SHAPE;
+    return launch_sample(logits, R, V, stride, SettingArrays{temperature, top_p, min_p, uniform, top_k}, out, stream);
+}
+
+static inline unsigned long long splitmix64(unsigned long long x) {
+    x += 0x9E3779B97F4A7C15ull;
+    x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
+    x = (x ^ (x >> 27)) * 0x94D049BB133111EBull;
+    return x ^ (x >> 31);
+}
+
+// The same with the rows' settings on the host: (temperature, top_p, min_p) a row, top_k, and number `index` of the row's stream of uniform
+// numbers, a hash of (seed, index).  They travel as launch parameters, kRowsAtOnce rows a launch.  out may be pinned host memory: it
+// holds the tokens once the stream has been waited for.
+IIAN_API int iian_sample_rows(const float * logits, int R, int V, long long stride, const float * settings, const int * top_k,
+                              const unsigned long long * seeds, const unsigned long long * indices, int * out, cudaStream_t stream) {
+    if (R <= 0) return IIAN_OK;
+    if (V <= 0 || settings == nullptr || top_k == nullptr || seeds == nullptr || indices == nullptr) return IIAN_ERR_SHAPE;
+    for (int r0 = 0; r0 < R; r0 += kRowsAtOnce) {
+        const int n = R - r0 < kRowsAtOnce ? R - r0 : kRowsAtOnce;
+        SettingRows set;
+        for (int r = 0; r < n; r++) {
+            set.temperature_[r] = settings[3 * (r0 + r)];
+            set.top_p_[r] = settings[3 * (r0 + r) + 1];
+            set.min_p_[r] = settings[3 * (r0 + r) + 2];
+            set.top_k_[r] = top_k[r0 + r];
+            const unsigned long long h = splitmix64(splitmix64(seeds[r0 + r]) ^ (indices[r0 + r] * 0xD1B54A32D192ED03ull));
+            set.uniform_[r] = (float) (h >> 40) * 5.9604644775390625e-8f;                      // 2^-24: 24 bits, exact
+        }
+        const int rc = launch_sample(logits + (size_t) r0 * stride, n, V, stride, set, out + r0, stream);
+        if (rc != IIAN_OK) return rc;
+    }
+    return IIAN_OK;
 }
 
 // logits [R, V] float32, changed in place.  allow_off / edit_off: [R + 1] int32 prefix sums; a token may appear in

@@ -2270,6 +2270,25 @@ class CudaKernels:
                   _cuda(min_p, "min_p", torch.float32), _cuda(uniform, "uniform", torch.float32),
                   _cuda(out, "sample out", torch.int32), _stream()), "sample")
 
+    def sample_rows(self, logits: torch.Tensor, settings, top_k, seeds, indices) -> list:
+        """The tokens of all rows, waited for.  The rows' settings are host arrays (``array.array``): ``settings`` floats (temperature,
+        top_p, min_p) a row, ``top_k`` ints, ``seeds`` and ``indices`` unsigned 64-bit; they travel with the launch, and the tokens
+        come back through pinned memory, so that no copy stands on either side of the kernel."""
+        r, v = logits.shape
+        if not logits.is_cuda or logits.dtype != torch.float32 or logits.stride(1) != 1:
+            raise KernelError("sample: logits must be float32 on CUDA with contiguous rows")
+        if (settings.typecode, top_k.typecode, seeds.typecode, indices.typecode) != ("f", "i", "Q", "Q") or \
+                (len(settings), len(top_k), len(seeds), len(indices)) != (3 * r, r, r, r):
+            raise KernelError("sample: three floats, an int and two unsigned 64-bit numbers a row")
+        fn = _fn("sampling", "iian_sample_rows", [c_void_p, c_int, c_int, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p])
+        out = torch.empty(r, dtype=torch.int32, pin_memory=True)
+        with torch.cuda.device(logits.device):
+            stream = torch.cuda.current_stream()
+            _check(fn(logits.data_ptr(), r, v, logits.stride(0), settings.buffer_info()[0], top_k.buffer_info()[0], seeds.buffer_info()[0],
+                      indices.buffer_info()[0], out.data_ptr(), stream.cuda_stream), "sample")
+            stream.synchronize()
+        return out.tolist()
+
 
 class WeightPrefetcher:
     """Keeps HBM busy between the weight-streaming products of a captured decode step.

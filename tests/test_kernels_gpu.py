@@ -342,6 +342,24 @@ def test_sample_cuts(V, top_k, top_p, min_p):
         assert cum[got].item() - probs[got].item() - slack <= target <= cum[got].item() + slack, f"row {r}"
 
 
+@pytest.mark.parametrize("R", [1, 128, 131])
+def test_sample_rows_with_settings_from_the_host(R):
+    """Settings that travel with the launch (128 rows at once) against the same settings in device arrays: the same tokens."""
+    from array import array
+
+    from iian_b200.sampling.sampler import uniforms
+    g = torch.Generator().manual_seed(R)
+    logits = (torch.randn(R, 997, generator=g) * 2.5).cuda()
+    T, p, m = (0.3 + torch.rand(R, generator=g)).tolist(), (0.5 + 0.5 * torch.rand(R, generator=g)).tolist(), [0.05 * (r % 3 == 0) for r in range(R)]
+    T[-1], k = 0.0 if R > 1 else 0.7, [(7 * r) % 30 for r in range(R)]
+    seeds, at = [(r * 0x9E3779B97F4A7C15 + 5) & (2 ** 64 - 1) for r in range(R)], [3 * r for r in range(R)]
+    got = K().sample_rows(logits, array("f", [x for r in range(R) for x in (T[r], p[r], m[r])]), array("i", k), array("Q", seeds), array("Q", at))
+    f = lambda v, dt=torch.float32: torch.tensor(v, dtype=dt).cuda()
+    out = torch.empty(R, dtype=torch.int32).cuda()
+    K().sample(logits, f(T), f(k, torch.int32), f(p), f(m), f(uniforms(seeds, at).tolist()), out)
+    assert got == out.tolist()
+
+
 @pytest.mark.parametrize("od", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("B,M,K_", [(1, 70, 64), (3, 16, 32), (8, 257, 96), (9, 100, 160), (17, 48, 4096), (33, 130, 320),
                                     (64, 1000, 1024), (2, 4096, 12288)])
