@@ -395,6 +395,431 @@ done:
     }
 }
 
+// ---- decoded tokens: the keys as the rows of the products ---------------------------------------------------------------
+// A decoded token has its heads for rows, 16 or fewer, and would leave most of a row tile empty.  Here a tile of 128 keys is the M operand:
+// S^T = K Q^T (128 keys x 16 heads), and with P^T [16 heads][128 keys] in shared memory O^T = V^T P^T, the rank in blocks of 128 rows,
+// V^T the same chunks read MN-major.  Every cached row passes shared memory once, for all heads.
+// The tiles of all sequences lie end to end, and the CTAs, one an SM, take equal stretches of that line: a stretch may end inside a sequence
+// (its part goes to scratch memory, slot sequence + CTA) and go on into the next ones.  latent_line_merge_kernel puts the parts together.
+// Roles: warps 0..3 the softmax (a thread a key, all heads), warp 4 lane 0 the products, warps 5.. the copies: one for each pair of the
+// latent's chunks of 64 values (a ring of five pairs), one for the rotated chunk and Q.  The first pair's and the rotated chunk's share of a
+// tile's scores is formed in the shadow of the softmax in front of it.
+// What bounds it: 68 products a tile of rank 512, some 100 cycles each however few the heads (128 rows of A from shared memory), and the
+// softmax between them, 5 us for the 3.3 a tile takes to arrive; tiles ahead fetched into the L2 make it slower.  16 heads, rank 512, us
+// with the merge, on mma.sync and here: 48 tokens behind 800 to 4,000 cached 78 and 62, 64 behind 4,000 114 and 96, 128 behind 4,000 212 and
+// 164 (rank 256: 55 and 38, 83 and 62, 153 and 105); the CTA's set-up, its first tile and the merge are 20, so that fewer keys stay with
+// mma.sync (32 behind 4,000 57 and 62, 64 behind 1,500 49 and 52).  With 32 heads the kernel above is faster.
+constexpr int LL_KEYS = 128, LL_HEADS = 16, LL_SLOTS = 5;
+constexpr int LL_CHUNK_BYTES = LL_KEYS * 128, LL_PAIR_BYTES = 2 * LL_CHUNK_BYTES;
+constexpr unsigned LL_O = 64u;                  // tensor-memory columns: two S^T from 0 on, the blocks of O^T behind
+constexpr int kLineCtas = 148;
+
+struct LatentLineParams {
+    __nv_bfloat16 * out;            // [N, H, rank]
+    float * part_o, * part_ml;      // [S + CTAs, H, rank] unnormalised, [S + CTAs, H, 2] maximum and sum
+    const int * cu_q, * ctx_len, * seq_of_token, * block_table;
+    const float * sink;             // [H] or null
+    int * status;
+    int num_seqs, max_blocks, H, rank, page_size, num_pages, window;
+    float scale, scale_log2, sink_to_raw;
+};
+
+// Key tiles of a sequence's one token (0: no token, or padding), its row of q and its first tile.
+__device__ __forceinline__ int ll_tiles(const LatentLineParams & p, int s, int & q0, int & ctx, int & tile_lo) {
+    q0 = p.cu_q[s];
+    ctx = p.ctx_len[s];
+    tile_lo = 0;
+    if (p.cu_q[s + 1] <= q0 || ctx <= 0 || p.seq_of_token[q0] < 0) return 0;
+    tile_lo = (p.window > 0 ? max(0, ctx - p.window) : 0) / LL_KEYS;
+    return (ctx - 1) / LL_KEYS - tile_lo + 1;
+}
+// All tiles, and those in front of sequence `before`.  A whole warp calls it.
+__device__ __forceinline__ int ll_total(const LatentLineParams & p, int before, int & ahead) {
+    int all = 0, q0, ctx, lo;
+    ahead = 0;
+    for (int s = threadIdx.x & 31; s < p.num_seqs; s += 32) {
+        const int n = ll_tiles(p, s, q0, ctx, lo);
+        all += n;
+        if (s < before) ahead += n;
+    }
+    ahead = __reduce_add_sync(0xffffffffu, ahead);
+    return __reduce_add_sync(0xffffffffu, all);
+}
+__device__ __forceinline__ int ll_border(int total, int cta, int ctas) { return ctas > 0 ? (int) ((long long) total * cta / ctas) : 0; }
+__device__ __forceinline__ int ll_cta_of(int total, int tile, int ctas) { return (int) (((long long) (tile + 1) * ctas - 1) / total); }
+
+__device__ __forceinline__ void ll_ld16(unsigned taddr, unsigned * r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
+}
+// Sixteen values over the 32 lanes, reduced: the values a lane carries are halved with every exchange; lane l ends with value l >> 1.
+template <typename F> __device__ __forceinline__ float ll_reduce(float * a, F f) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int half = LL_HEADS / 2, o = 16; half >= 1; half >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int j = 0; j < half; j++) {
+            const float give = up ? a[j] : a[j + half], keep = up ? a[j + half] : a[j];
+            a[j] = f(keep, __shfl_xor_sync(0xffffffffu, give, o));
+        }
+    }
+    return f(a[0], __shfl_xor_sync(0xffffffffu, a[0], 1));
+}
+
+template <int PAIRS>
+__global__ void __launch_bounds__(32 * (6 + PAIRS), 1) latent_line_kernel(
+    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const LatentLineParams p) {
+    constexpr int N = LL_HEADS, CHUNKS = 2 * PAIRS + 1, ROPES = 2, Q_BYTES = N * 128;
+    extern __shared__ __align__(1024) unsigned char lt_smem_raw[];
+    unsigned char * sK = (unsigned char *) (((uintptr_t) lt_smem_raw + 1023) & ~(uintptr_t) 1023);     // [LL_SLOTS][2 chunks][128 keys][128 B]
+    unsigned char * sR = sK + LL_SLOTS * LL_PAIR_BYTES;            // [ROPES][128 keys][128 B]
+    unsigned char * sQ = sR + ROPES * LL_CHUNK_BYTES;              // [CHUNKS][N heads][128 B]
+    unsigned char * sP = sQ + CHUNKS * Q_BYTES;                    // [2][N heads][64 keys]
+    __shared__ __align__(8) unsigned long long pair_full[LL_SLOTS], pair_free[LL_SLOTS], rope_full[ROPES], rope_free[ROPES], q_full, q_free, s_full, p_full, o_done;
+    __shared__ unsigned tmem_base_s;
+    __shared__ __align__(16) float wm[2][4][N], wl[4][N];
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // this CTA's stretch of the line: from tile `off` of sequence s on, `left` tiles
+    int s = 0, off = 0, left;
+    {
+        int none;
+        const int total = ll_total(p, 0, none), ctas = min((int) gridDim.x, total), g0 = ll_border(total, blockIdx.x, ctas);
+        if ((int) blockIdx.x >= ctas) return;                      // (with fewer tiles than CTAs, one each)
+        left = ll_border(total, blockIdx.x + 1, ctas) - g0;
+        int run = 0;
+        for (int base = 0; base < p.num_seqs; base += 32) {
+            int q0, ctx, lo, n = base + lane < p.num_seqs ? ll_tiles(p, base + lane, q0, ctx, lo) : 0, upto = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += v;
+            }
+            const unsigned here = __ballot_sync(0xffffffffu, run + upto > g0);
+            if (here != 0) {
+                const int l = __ffs(here) - 1;
+                s = base + l;
+                off = g0 - (run + __shfl_sync(0xffffffffu, upto - n, l));
+                break;
+            }
+            run += __shfl_sync(0xffffffffu, upto, 31);
+        }
+    }
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < LL_SLOTS; b++) { at_mbar_init(at_smem(&pair_full[b]), 1); at_mbar_init(at_smem(&pair_free[b]), 1); }
+        for (int b = 0; b < ROPES; b++) { at_mbar_init(at_smem(&rope_full[b]), 1); at_mbar_init(at_smem(&rope_free[b]), 1); }
+        at_mbar_init(at_smem(&q_full), 1); at_mbar_init(at_smem(&q_free), 1);
+        at_mbar_init(at_smem(&s_full), 1); at_mbar_init(at_smem(&p_full), 4); at_mbar_init(at_smem(&o_done), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 4) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at_smem(&tmem_base_s)), "r"(256u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    at_fence_before();
+    __syncthreads();
+    at_fence_after();
+    const unsigned tmem_base = tmem_base_s;
+    int * status = p.status;
+
+    // the stretch, sequence by sequence: body(segment, sequence, its row of q, context, first key tile of it here, tiles here, tiles in all)
+    auto walk = [&](auto body) {
+        int s_ = s, off_ = off, left_ = left;
+        for (int seg = 0; left_ > 0 && s_ < p.num_seqs; s_++) {
+            int q0, ctx, lo;
+            const int all = ll_tiles(p, s_, q0, ctx, lo);
+            if (all <= off_) { off_ = 0; continue; }
+            const int n = min(all - off_, left_);
+            if (!body(seg, s_, q0, ctx, lo + off_, n, all, off_)) return;
+            seg++;
+            left_ -= n;
+            off_ = 0;
+        }
+    };
+
+    if (warp >= 5) {
+        // ---- copies: a lane a page of the tile (of a pair: one for each chunk), the block table read a tile ahead -----------------
+        const int ps = p.page_size, pages = LL_KEYS / ps, pr = warp - 5;
+        const bool pair = pr < PAIRS;
+        const int per = pair ? 2 : 1, pg = lane % pages, half = lane / pages;
+        const bool mine = lane < per * pages;
+        int it = 0;                                                // tiles of this CTA so far
+        walk([&](int seg, int s_, int q0, int ctx, int tile0, int n, int, int) {
+            const int * bt = p.block_table + (size_t) s_ * p.max_blocks;
+            auto page_of = [&](int t) {
+                const int j0 = (tile0 + t) * LL_KEYS + pg * ps;
+                return t < n && mine && j0 < ctx ? __ldg(bt + j0 / ps) : -1;
+            };
+            int page = page_of(0), good = 1;
+            if (!pair) {                                           // Q of this sequence, once the scores of the one before are formed
+                if (lane == 0) {
+                    if (seg > 0) good = at_wait(at_smem(&q_free), (unsigned) (seg - 1) & 1u) ? 1 : 0;
+                    if (good) {
+                        at_expect_tx(at_smem(&q_full), (unsigned) (CHUNKS * Q_BYTES));
+                        for (int c = 0; c < CHUNKS; c++) lt_tma_2d(at_smem(sQ + c * Q_BYTES), &map_q, c * 64, q0 * p.H, at_smem(&q_full));
+                    } else { status[0] = 31; status[1] = seg; }
+                }
+                if (!__all_sync(0xffffffffu, good)) return false;
+            }
+            for (int t = 0; t < n; t++, it++) {
+                const int page_next = page_of(t + 1);
+                const int k = pair ? it * PAIRS + pr : it, ring = pair ? LL_SLOTS : ROPES, slot = k % ring, round = k / ring;
+                const unsigned full = at_smem(pair ? &pair_full[slot] : &rope_full[slot]);
+                if (lane == 0) {
+                    if (round > 0) good = at_wait(at_smem(pair ? &pair_free[slot] : &rope_free[slot]), (unsigned) (round - 1) & 1u) ? 1 : 0;
+                    if (good) at_expect_tx(full, (unsigned) (pair ? LL_PAIR_BYTES : LL_CHUNK_BYTES));
+                    else { status[0] = 32; status[1] = it; }
+                }
+                if (!__all_sync(0xffffffffu, good)) return false;
+                if (mine) {
+                    const int y = (page >= 0 && page < p.num_pages ? page : p.num_pages) * ps;         // out of range: filled with zeros
+                    unsigned char * to = (pair ? sK + slot * LL_PAIR_BYTES + half * LL_CHUNK_BYTES : sR + slot * LL_CHUNK_BYTES) + pg * ps * 128;
+                    lt_tma_2d(at_smem(to), &map_k, (pair ? 2 * pr + half : 2 * PAIRS) * 64, y, full);
+                }
+                page = page_next;
+            }
+            return true;
+        });
+    } else if (warp == 4) {
+        if (lane == 0) {
+            // ---- products ------------------------------------------------------------------------------------------------------
+            constexpr unsigned idesc_s = at_idesc(LL_KEYS, N, false), idesc_o = at_idesc(128, N, false) | (1u << 15);      // V^T: A is MN-major
+            const unsigned long long dk = at_desc(at_smem(sK), 16, 1024), dr = at_desc(at_smem(sR), 16, 1024), dq = at_desc(at_smem(sQ), 16, 1024);
+            const unsigned long long dv = at_desc(at_smem(sK), LL_CHUNK_BYTES, 1024), dp = at_desc(at_smem(sP), 16, 1024);
+            int it = 0;
+            walk([&](int seg, int, int, int, int, int n, int, int) {
+                if (!at_wait(at_smem(&q_full), (unsigned) seg & 1u)) { status[0] = 33; status[1] = seg; return false; }
+                // the scores of tile i: one pair of chunks, the rotated chunk
+                auto pair_scores = [&](int i, int pr, bool opens) {
+                    const int k_ = i * PAIRS + pr, slot = k_ % LL_SLOTS;
+                    if (!at_wait(at_smem(&pair_full[slot]), (unsigned) (k_ / LL_SLOTS) & 1u)) { status[0] = 34; status[1] = i; return false; }
+                    at_fence_after();
+#pragma unroll
+                    for (int k = 0; k < 8; k++)                    // 16 values per step: 32 bytes inside the swizzle atom
+                        at_mma(tmem_base + (unsigned) ((i & 1) * N), dk + (unsigned long long) (slot * (LL_PAIR_BYTES >> 4) + (k >> 2) * (LL_CHUNK_BYTES >> 4) + (k & 3) * 2),
+                               dq + (unsigned long long) ((2 * pr + (k >> 2)) * (Q_BYTES >> 4) + (k & 3) * 2), idesc_s, !opens || k > 0 ? 1u : 0u);
+                    return true;
+                };
+                auto rope_scores = [&](int i) {
+                    const int rs = i % ROPES;
+                    if (!at_wait(at_smem(&rope_full[rs]), (unsigned) (i / ROPES) & 1u)) { status[0] = 35; status[1] = i; return false; }
+                    at_fence_after();
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        at_mma(tmem_base + (unsigned) ((i & 1) * N), dr + (unsigned long long) (rs * (LL_CHUNK_BYTES >> 4) + k * 2),
+                               dq + (unsigned long long) (2 * PAIRS * (Q_BYTES >> 4) + k * 2), idesc_s, 1u);
+                    at_commit(at_smem(&rope_free[rs]));
+                    return true;
+                };
+                // what of a tile is there before the tile in front of it has been let go: the first pair and the rotated chunk
+                auto early = [&](int i) { return pair_scores(i, 0, true) && rope_scores(i); };
+                if (!early(it)) return false;
+                for (int t = 0; t < n; t++, it++) {
+#pragma unroll 1
+                    for (int pr = 1; pr < PAIRS; pr++)
+                        if (!pair_scores(it, pr, false)) return false;
+                    if (t == n - 1) at_commit(at_smem(&q_free));
+                    at_commit(at_smem(&s_full));
+                    if (t + 1 < n && !early(it + 1)) return false;          // in the shadow of this tile's softmax
+                    if (!at_wait(at_smem(&p_full), (unsigned) it & 1u)) { status[0] = 36; status[1] = it; return false; }
+                    at_fence_after();
+#pragma unroll 1
+                    for (int pr = 0; pr < PAIRS; pr++) {           // 16 keys per step: 16 rows of V, 32 bytes of P
+                        const int slot = (it * PAIRS + pr) % LL_SLOTS;
+#pragma unroll
+                        for (int k = 0; k < 8; k++)
+                            at_mma(tmem_base + LL_O + (unsigned) (pr * N), dv + (unsigned long long) (slot * (LL_PAIR_BYTES >> 4) + k * 128),
+                                   dp + (unsigned long long) ((k >> 2) * (Q_BYTES >> 4) + (k & 3) * 2), idesc_o, t > 0 || k > 0 ? 1u : 0u);
+                        at_commit(at_smem(&pair_free[slot]));
+                    }
+                    if (t == n - 1) at_commit(at_smem(&o_done));
+                }
+                return true;
+            });
+        }
+    } else {
+        // ---- softmax: a thread a key, all heads ------------------------------------------------------------------------------
+        const int r = threadIdx.x;
+        const unsigned lane_addr = (unsigned) (warp * 32) << 16, tS = tmem_base + lane_addr, tO = tS + LL_O;
+        const float sl = p.scale_log2;
+        auto group_sync = [&]() { asm volatile("bar.sync 1, 128;" ::: "memory"); };
+        auto larger = [](float a, float b) { return fmaxf(a, b); };
+        auto sum = [](float a, float b) { return a + b; };
+        bool failed = false;                                       // a wait that gave up is recorded and the walk goes on
+        int it = 0;
+        walk([&](int seg, int s_, int q0, int ctx, int tile0, int n, int all, int first) {
+            float m_run[N], l_run[N];                              // the maximum of all keys, the sum of the thread's own
+#pragma unroll
+            for (int h = 0; h < N; h++) {
+                const bool with = p.sink != nullptr && first == 0 && h < p.H;          // the sink counts once
+                m_run[h] = with ? p.sink[h] * p.sink_to_raw : -INFINITY;
+                l_run[h] = with && r == 0 ? 1.0f : 0.0f;
+            }
+            const int lo = p.window > 0 ? ctx - p.window : 0;
+            for (int t = 0; t < n; t++, it++) {
+                const int key0 = (tile0 + t) * LL_KEYS, j = key0 + r;
+                if (!failed && !at_wait(at_smem(&s_full), (unsigned) it & 1u)) { status[0] = 37; status[1] = it; failed = true; }
+                __syncwarp();
+                at_fence_after();
+                unsigned v[N];
+                ll_ld16(tS + (unsigned) ((it & 1) * N), v);
+                at_wait_ld();
+                const bool seen = j < ctx && j >= lo;
+                float a[N];
+#pragma unroll
+                for (int h = 0; h < N; h++) {
+                    if (!seen) v[h] = 0xff800000u;                 // -inf
+                    a[h] = __uint_as_float(v[h]);
+                }
+                const float mx = ll_reduce(a, larger);
+                if ((lane & 1) == 0) wm[it & 1][warp][lane >> 1] = mx;
+                // rows behind the newest key: whatever they hold must not meet P's zeros (pages without a key came as zeros)
+                const int past = ctx - key0;
+                if (past < LL_KEYS && r >= past) {
+                    for (int pr = 0; pr < PAIRS; pr++) {
+                        unsigned char * row = sK + (it * PAIRS + pr) % LL_SLOTS * LL_PAIR_BYTES + r * 128;
+#pragma unroll
+                        for (int e = 0; e < 8; e++) {
+                            reinterpret_cast<uint4 *>(row)[e] = make_uint4(0u, 0u, 0u, 0u);
+                            reinterpret_cast<uint4 *>(row + LL_CHUNK_BYTES)[e] = make_uint4(0u, 0u, 0u, 0u);
+                        }
+                    }
+                }
+                group_sync();
+                // the exact running maximum, as above: the largest weight is 1 and not rounded
+                bool moved = false;
+                float corr[N];
+#pragma unroll
+                for (int h = 0; h < N; h += 4) {
+                    const float4 a0 = *reinterpret_cast<const float4 *>(&wm[it & 1][0][h]), a1 = *reinterpret_cast<const float4 *>(&wm[it & 1][1][h]);
+                    const float4 a2 = *reinterpret_cast<const float4 *>(&wm[it & 1][2][h]), a3 = *reinterpret_cast<const float4 *>(&wm[it & 1][3][h]);
+                    const float top[4] = {fmaxf(at_max3(a0.x, a1.x, a2.x), a3.x), fmaxf(at_max3(a0.y, a1.y, a2.y), a3.y),
+                                          fmaxf(at_max3(a0.z, a1.z, a2.z), a3.z), fmaxf(at_max3(a0.w, a1.w, a2.w), a3.w)};
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        corr[h + e] = 1.0f;
+                        if (top[e] > m_run[h + e]) {
+                            corr[h + e] = m_run[h + e] == -INFINITY ? 0.0f : at_exp2((m_run[h + e] - top[e]) * sl);
+                            m_run[h + e] = top[e];
+                            moved = true;
+                        }
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < N; h += 2) {
+                    unsigned w[2];
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        const float neg = m_run[h + e] == -INFINITY ? 0.0f : m_run[h + e] * sl;
+                        const float x = at_exp2(fmaf(__uint_as_float(v[h + e]), sl, -neg));
+                        w[e] = (unsigned) __bfloat16_as_ushort(__float2bfloat16_rn(x));
+                        // the weights as they are multiplied, so that their rounding weighs on both sides of the quotient
+                        l_run[h + e] = fmaf(l_run[h + e], corr[h + e], __uint_as_float(w[e] << 16));
+                    }
+                    // two neighbouring keys in a word: the even lane takes head h, the odd one head h + 1
+                    const bool odd = lane & 1;
+                    const unsigned got = __shfl_xor_sync(0xffffffffu, odd ? w[0] : w[1], 1), word = odd ? got | w[1] << 16 : w[0] | got << 16;
+                    const int head = h + (odd ? 1 : 0), key = r & 62;
+                    *reinterpret_cast<unsigned *>(sP + (r >> 6) * Q_BYTES + head * 128 + (((key >> 3) ^ (head & 7)) << 4) + (key & 7) * 2) = word;
+                }
+                if (t > 0 && moved) {                              // (the scores of this tile followed the products of the one before)
+#pragma unroll 1
+                    for (int pr = 0; pr < PAIRS; pr++) {
+                        unsigned o[N];
+                        ll_ld16(tO + (unsigned) (pr * N), o);
+                        at_wait_ld();
+#pragma unroll
+                        for (int h = 0; h < N; h++) o[h] = __float_as_uint(__uint_as_float(o[h]) * corr[h]);
+                        lt_st16(tO + (unsigned) (pr * N), o);
+                    }
+                    at_wait_st();
+                }
+                at_fence_async_smem();
+                at_fence_before();
+                __syncwarp();
+                if (lane == 0) at_arrive(at_smem(&p_full));
+            }
+            // ---- this sequence's part ----------------------------------------------------------------------------------------
+            const float mine = ll_reduce(l_run, sum);
+            if ((lane & 1) == 0) wl[warp][lane >> 1] = mine;
+            group_sync();
+            if (!failed && !at_wait(at_smem(&o_done), (unsigned) seg & 1u)) { status[0] = 38; status[1] = it; failed = true; }
+            __syncwarp();
+            at_fence_after();
+            const bool whole = n == all;
+            const size_t slot = (size_t) s_ + blockIdx.x;
+            float inv[N];
+#pragma unroll
+            for (int h = 0; h < N; h++) {
+                const float l = (wl[0][h] + wl[1][h]) + (wl[2][h] + wl[3][h]);
+                inv[h] = l > 0.0f ? 1.0f / l : 0.0f;
+                if (!whole && r == 0 && h < p.H)
+                    *reinterpret_cast<float2 *>(p.part_ml + (slot * p.H + h) * 2) = make_float2(m_run[h] * p.scale, l);
+            }
+#pragma unroll 1
+            for (int pr = 0; pr < PAIRS; pr++) {
+                unsigned o[N];
+                ll_ld16(tO + (unsigned) (pr * N), o);
+                at_wait_ld();
+#pragma unroll
+                for (int h = 0; h < N; h++) {
+                    if (h >= p.H) continue;
+                    if (whole) p.out[((size_t) q0 * p.H + h) * p.rank + pr * 128 + r] = __float2bfloat16_rn(__uint_as_float(o[h]) * inv[h]);
+                    else p.part_o[(slot * p.H + h) * p.rank + pr * 128 + r] = __uint_as_float(o[h]);
+                }
+            }
+            group_sync();                                          // wl has been read
+            return true;
+        });
+    }
+    at_fence_before();
+    __syncthreads();
+    if (warp == 4) {
+        at_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(256u) : "memory");
+    }
+}
+
+// Grid (S, H): the parts of a sequence that several CTAs walked; zeros for a token of no sequence.
+__global__ void __launch_bounds__(128) latent_line_merge_kernel(const LatentLineParams p, int ctas) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int s = blockIdx.x, h = blockIdx.y;
+    int q0, ctx, lo, ahead;
+    const int n = ll_tiles(p, s, q0, ctx, lo);
+    if (p.cu_q[s + 1] <= q0) return;
+    __nv_bfloat16 * out = p.out + ((size_t) q0 * p.H + h) * p.rank;
+    if (n == 0) {
+        for (int c = threadIdx.x; c < p.rank; c += 128) out[c] = __float2bfloat16_rn(0.0f);
+        return;
+    }
+    const int total = ll_total(p, s, ahead);
+    ctas = min(ctas, total);
+    const int first = ll_cta_of(total, ahead, ctas), last = ll_cta_of(total, ahead + n - 1, ctas);
+    if (first == last) return;                                     // written whole
+    const size_t slot = (size_t) s + first;
+    float m = -INFINITY, l = 0.0f;
+#pragma unroll 4
+    for (int z = 0; z <= last - first; z++) m = fmaxf(m, p.part_ml[((slot + z) * p.H + h) * 2]);
+    float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    const int c = threadIdx.x * 4;
+#pragma unroll 4
+    for (int z = 0; z <= last - first; z++) {
+        const float2 ml = *reinterpret_cast<const float2 *>(p.part_ml + ((slot + z) * p.H + h) * 2);
+        const float w = ml.x == -INFINITY ? 0.0f : __expf(ml.x - m);
+        l = fmaf(ml.y, w, l);
+        if (c < p.rank) {
+            const float4 x = *reinterpret_cast<const float4 *>(p.part_o + ((slot + z) * p.H + h) * p.rank + c);
+            a[0] = fmaf(x.x, w, a[0]); a[1] = fmaf(x.y, w, a[1]); a[2] = fmaf(x.z, w, a[2]); a[3] = fmaf(x.w, w, a[3]);
+        }
+    }
+    const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+    if (c < p.rank) *reinterpret_cast<uint2 *>(out + c) = make_uint2(pack_bf16(a[0] * inv, a[1] * inv), pack_bf16(a[2] * inv, a[3] * inv));
+}
+
 // [rows, width] bf16, boxes of 64 columns x box_rows, 128-byte swizzle, zeros outside
 static int lt_make_map(CUtensorMap * map, const void * base, long long rows, int width, int box_rows) {
     AtEncodeFn fn = at_encode_fn();
@@ -415,6 +840,15 @@ static int lt_launch(const CUtensorMap & mq, const CUtensorMap & mk, const Laten
     const cudaError_t e = cudaFuncSetAttribute(latent_attention_tc_kernel<REST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
     if (e != cudaSuccess) return 1000 + (int) e;
     latent_attention_tc_kernel<REST><<<grid, LT_THREADS, smem, stream>>>(mq, mk, p);
+    return iian_launch_status();
+}
+
+template <int PAIRS>
+static int ll_launch(const CUtensorMap & mq, const CUtensorMap & mk, const LatentLineParams & p, cudaStream_t stream) {
+    const size_t smem = (size_t) LL_SLOTS * LL_PAIR_BYTES + 2 * LL_CHUNK_BYTES + (size_t) (2 * PAIRS + 3) * LL_HEADS * 128 + 1024;
+    const cudaError_t e = cudaFuncSetAttribute(latent_line_kernel<PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    if (e != cudaSuccess) return 1000 + (int) e;
+    latent_line_kernel<PAIRS><<<kLineCtas, 32 * (6 + PAIRS), smem, stream>>>(mq, mk, p);
     return iian_launch_status();
 }
 
@@ -470,4 +904,40 @@ IIAN_API int iian_latent_attention_tc(const void * q, const void * cache, void *
     }
     if (rc2 != IIAN_OK || parts == 1) return rc2;
     return latent_merge(part_o, part_ml, out, seq_of_token, N, H, parts, rank, stream);
+}
+
+// Decoded tokens (every sequence has one token at most), the keys as the rows of the products.  0 if the sizes are ones it takes: rank 256 or
+// 512 with a rotated part of 64 values, 1 to 16 heads, pages of 8 to 128 tokens.
+IIAN_API int iian_latent_line_ok(int rank, int width, int H, int page_size) {
+    if ((rank != 256 && rank != 512) || width != rank + LT_CHUNK || H < 1 || H > LL_HEADS) return IIAN_ERR_SHAPE;
+    return page_size == 8 || page_size == 16 || page_size == 32 || page_size == 64 || page_size == 128 ? IIAN_OK : IIAN_ERR_SHAPE;
+}
+// Floats of scratch for a step of S sequences.
+IIAN_API long long iian_latent_line_scratch(int S, int H, int rank) { return (long long) (S + kLineCtas) * H * (rank + 2); }
+
+// As iian_latent_attention_tc; scratch: iian_latent_line_scratch floats on a 16-byte boundary.
+IIAN_API int iian_latent_line(const void * q, const void * cache, void * out, float * scratch, const float * sink, const int * cu_q, const int * ctx_len,
+                              const int * seq_of_token, const int * block_table, int max_blocks, int N, int S, int H, int rank, int width,
+                              int page_size, int num_pages, float scale, int window, int * status, cudaStream_t stream) {
+    if (N <= 0 || S <= 0) return IIAN_OK;
+    const int code = iian_latent_line_ok(rank, width, H, page_size);
+    if (code != IIAN_OK) return code;
+    if (!(scale > 0.0f) || status == nullptr || num_pages <= 0 || scratch == nullptr) return IIAN_ERR_SHAPE;
+    if (((uintptr_t) q & 15) || ((uintptr_t) cache & 15) || ((uintptr_t) out & 15) || ((uintptr_t) scratch & 15)) return IIAN_ERR_ALIGN;
+    if (S > 65535 || (long long) N * H + 64 > 2147483647LL || (long long) (num_pages + 1) * page_size > 2147483647LL) return IIAN_ERR_LIMIT;
+    if ((long long) N * H < LL_HEADS) return IIAN_ERR_SHAPE;           // a box of Q
+    CUtensorMap mq, mk;
+    int rc = lt_make_map(&mq, q, (long long) N * H, width, LL_HEADS);
+    if (rc != IIAN_OK) return rc;
+    rc = lt_make_map(&mk, cache, (long long) num_pages * page_size, width, page_size);
+    if (rc != IIAN_OK) return rc;
+    LatentLineParams p;
+    p.out = (__nv_bfloat16 *) out;
+    p.part_o = scratch; p.part_ml = scratch + (size_t) (S + kLineCtas) * H * rank;
+    p.cu_q = cu_q; p.ctx_len = ctx_len; p.seq_of_token = seq_of_token; p.block_table = block_table; p.sink = sink; p.status = status;
+    p.num_seqs = S; p.max_blocks = max_blocks; p.H = H; p.rank = rank; p.page_size = page_size; p.num_pages = num_pages; p.window = window;
+    p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.sink_to_raw = 1.0f / scale;
+    rc = rank == 512 ? ll_launch<4>(mq, mk, p, stream) : ll_launch<2>(mq, mk, p, stream);
+    if (rc != IIAN_OK) return rc;
+    return iian_launch(latent_line_merge_kernel, dim3((unsigned) S, (unsigned) H), dim3(128), 0, stream, p, kLineCtas);
 }

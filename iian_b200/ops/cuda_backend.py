@@ -1233,6 +1233,45 @@ class CudaKernels:
         if parts > 1:
             LAUNCHES[0] += 1
 
+    # decoded tokens with the keys as the rows of the products (csrc/latent_attention_tc.cu): bfloat16, rank 256 / 512 with 64 rotated values, up to
+    # 16 heads.  Keys of a step (tokens times the longest context) from which it is used: 48 tokens behind 800 to 4,000 cached 78 us on
+    # mma.sync, 62 here, 128 behind 1,500 88 and 84, but 32 behind 4,000 57 and 62 (rank 256 40 and 40), 64 behind 1,500 49 and 52
+    LATENT_LINE_MIN_KEYS = 180_000
+
+    def latent_line_pays(self, num_seqs: int, max_q_len: int, num_heads: int, max_ctx: int, window: Optional[int]) -> bool:
+        return max_q_len == 1 and num_heads <= 16 and num_seqs * (min(max_ctx, window + 1) if window else max_ctx) >= self.LATENT_LINE_MIN_KEYS
+
+    def latent_line_ok(self, q_cat: torch.Tensor, cache_rows: torch.Tensor, rank: int, scale: float) -> bool:
+        """Whether that kernel takes these operands at all."""
+        if not (self.LATENT_MMA and self.LATENT_TC) or not scale > 0 or q_cat.dtype != torch.bfloat16 or cache_rows.dtype != torch.bfloat16:
+            return False
+        n, h, width = q_cat.shape
+        fn = _fn("latent_attention_tc", "iian_latent_line_ok", [c_int, c_int, c_int, c_int])
+        return n * h >= 16 and fn(rank, width, h, cache_rows.shape[1]) == 0
+
+    def latent_line(self, q_cat: torch.Tensor, cache_rows: torch.Tensor, out: torch.Tensor, sink: Optional[torch.Tensor],
+                    meta, *, num_heads: int, rank: int, scale: float, window: Optional[int]) -> None:
+        """Attention over the cached latent of a step in which every sequence has one token."""
+        n, h, width = q_cat.shape
+        if h != num_heads or cache_rows.shape[-1] != width or out.shape != (n, h, rank) or q_cat.dtype != torch.bfloat16 \
+                or cache_rows.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or (sink is not None and sink.numel() != h) or meta.max_q_len != 1:
+            raise KernelError(f"latent_line: q {tuple(q_cat.shape)}, cache {tuple(cache_rows.shape)}, out {tuple(out.shape)} do not fit")
+        status = self.tcgen05_status_buffer(q_cat.device)
+        CudaKernels._tc_used = True
+        floats = _fn("latent_attention_tc", "iian_latent_line_scratch", [c_int, c_int, c_int])
+        floats.restype = c_longlong
+        scratch = self.attention_scratch(q_cat.device, floats(meta.num_seqs, h, rank))
+        bt = meta.block_table
+        fn = _fn("latent_attention_tc", "iian_latent_line",
+                 [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
+                  c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p])
+        _check(fn(_cuda(q_cat, "q_cat"), _cuda(cache_rows, "latent cache"), _cuda(out, "attention out"), scratch.data_ptr(),
+                  _cuda(sink, "sink", torch.float32), _cuda(meta.cu_q, "cu_q", torch.int32), _cuda(meta.ctx_len, "ctx_len", torch.int32),
+                  _cuda(meta.seq_of_token, "seq_of_token", torch.int32), _cuda(bt, "block table", torch.int32), bt.shape[1], n,
+                  meta.num_seqs, h, rank, width, cache_rows.shape[1], cache_rows.shape[0], scale, window or 0, status.data_ptr(), _stream()),
+               "latent_line")
+        LAUNCHES[0] += 1
+
     # ---- routed experts (csrc/moe.cu) -----------------------------------------------------------------------------
     _moe_tile_rows = None
 

@@ -77,3 +77,42 @@ def test_tokens_without_a_key_give_zeros(rank, rot, heads, parts):
     p = torch.softmax(torch.cat([z, sink.double()[None, :, None].expand(33, -1, 1)], 2), 2)[..., :-1]
     # as above
     assert bool(((out[157:190].double() - p @ keys[:, :rank]).abs() <= (2.0 ** -7 + 2e-4) * (p @ keys[:, :rank].abs())).all())
+
+
+@pytest.mark.parametrize("rank,heads,page", [(512, 16, 16), (512, 8, 64), (512, 13, 8), (256, 16, 128), (256, 5, 16), (256, 16, 32)])
+@pytest.mark.parametrize("contexts,window", [([64, 1, 128, 129], 0), ([300] * 40, 0), ([40 + 97 * i for i in range(33)], 0), ([5000, 17, 3, 900], 0),
+                                             ([700, 130, 20, 128, 4000], 128), ([1 + 61 * i for i in range(170)], 1000)])
+def test_decoded_tokens_with_keys_as_rows(rank, heads, page, contexts, window):
+    """The line of key tiles over the CTAs: sequences of one tile and of many, cut by a CTA's border or not, padding and a request without
+    context among them, the last page NaN behind the newest key."""
+    g = torch.Generator("cuda").manual_seed(rank + heads + len(contexts))
+    width, n = rank + 64, len(contexts) + 2                        # a request without context and a padding token at the end
+    blocks = [-(-c // page) for c in contexts]
+    order = torch.randperm(sum(blocks) + 1, generator=torch.Generator().manual_seed(7)).tolist()
+    rows = torch.full((sum(blocks) + 1, page, width), float("nan"), device="cuda", dtype=torch.bfloat16)
+    bt = torch.full((n, max(blocks)), -1, dtype=torch.int32)
+    q = (2 * torch.randn(n, heads, width, device="cuda", generator=g)).bfloat16()
+    sink = torch.randn(heads, device="cuda", generator=g)
+    scale, want, bound = width ** -0.5, [], []
+    for i, c in enumerate(contexts):
+        keys = torch.randn(c, width, device="cuda", generator=g).bfloat16()
+        for b in range(blocks[i]):
+            bt[i, b] = order.pop()
+            part = keys[b * page: (b + 1) * page]
+            rows[int(bt[i, b]), : len(part)] = part
+        z = (q[i].double() @ keys.double().T) * scale
+        if window:
+            z[:, : max(0, c - window)] = float("-inf")
+        p = torch.softmax(torch.cat([z, sink.double()[:, None]], 1), 1)[:, :-1]
+        want.append(p @ keys[:, :rank].double())
+        bound.append(p @ keys[:, :rank].double().abs())
+    cuda = lambda x: torch.as_tensor(x, dtype=torch.int32).cuda()
+    meta = SimpleNamespace(cu_q=cuda(list(range(n + 1))), ctx_len=cuda(contexts + [0, 1]), block_table=bt.cuda(), num_seqs=n, max_q_len=1,
+                           seq_of_token=cuda(list(range(n - 1)) + [-1]))
+    K, out = CudaKernels(), torch.full((n, heads, rank), 7.0, device="cuda", dtype=torch.bfloat16)
+    assert K.latent_line_ok(q, rows, rank, scale)
+    K.latent_line(q, rows, out, sink, meta, num_heads=heads, rank=rank, scale=scale, window=window or None)
+    K.tcgen05_check(q.device)
+    assert not out[-2:].any()
+    # as above
+    assert bool(((out[:-2].double() - torch.stack(want)).abs() <= (2.0 ** -7 + 2e-4) * torch.stack(bound)).all())
