@@ -113,18 +113,6 @@ __global__ void __launch_bounds__(GS_THREADS) gemm_stream_kernel(
     // the grid before to complete.  The grid after this one may be launched as soon as SMs become free.
     pdl_launch_dependents();
     const bool scaled = ex.in_partial != nullptr;
-    if (warp < GS_WARPS) {
-        pdl_wait();
-        if (scaled) {                           // row n's factor: one warp adds its partial sums in a fixed order
-            for (int n = warp; n < B; n += GS_WARPS) {
-                float a = 0.0f;
-                for (int i = lane; i < ex.in_tiles; i += 32) a += ex.in_partial[(size_t) n * ex.in_tiles + i];
-                a = warp_sum(a);
-                if (lane == 0) s_rs[n] = rsqrtf(a * ex.inv_width + ex.eps);
-            }
-        }
-        gs_consumer_sync();
-    }
     volatile int * failed = &s_failed;
 
     if (warp == GS_WARPS) {
@@ -174,6 +162,7 @@ __global__ void __launch_bounds__(GS_THREADS) gemm_stream_kernel(
     constexpr int PER_STAGE = GS_KC / 32 / GS_WARPS;      // chunks of a stage per warp
     constexpr int XR = XREG > 0 ? XREG : 1;
     uint4 xb[XR];
+    pdl_wait();
     if (XREG > 0) {
 #pragma unroll
         for (int i = 0; i < XR; i++) {
@@ -181,6 +170,18 @@ __global__ void __launch_bounds__(GS_THREADS) gemm_stream_kernel(
             xb[i] = c < nchunks ? __ldg(xr + (size_t) c * 4) : make_uint4(0u, 0u, 0u, 0u);
         }
     }
+    // row n's factor: one warp adds its partial sums in a fixed order, while the activations are on their way.  A product of a decode step is some
+    // 4 us, most of it trips to memory in a row, so what it needs is asked for at once: a request behind 90 tokens, 8 layers of 2 products with
+    // a factor and 2 with a residual (below), 272 us with each in its place, 258 so (8b shape, eight requests, 4 layers: 548 and 541)
+    if (scaled) {
+        for (int n = warp; n < B; n += GS_WARPS) {
+            float a = 0.0f;
+            for (int i = lane; i < ex.in_tiles; i += 32) a += ex.in_partial[(size_t) n * ex.in_tiles + i];
+            a = warp_sum(a);
+            if (lane == 0) s_rs[n] = rsqrtf(a * ex.inv_width + ex.eps);
+        }
+    }
+    gs_consumer_sync();
     auto fetch = [&](int s_, uint4 * dst) {                // the activations of stage s_ (of any row block) for this warp
 #pragma unroll
         for (int i = 0; i < PER_STAGE; i++) {
@@ -209,6 +210,14 @@ __global__ void __launch_bounds__(GS_THREADS) gemm_stream_kernel(
         }
         __syncwarp();
         if (lane == 0) gs_arrive(gs_smem(&empty[slot]));
+    };
+    // what the residual epilogue of row block b reads, asked for before the block is multiplied
+    float res_r = 0.0f, norm_r = 0.0f;
+    auto ask_block = [&](int b) {
+        if (EPI == 2) {
+            const int n = (int) threadIdx.x / GS_ROWS, m = b * GS_ROWS + (int) threadIdx.x % GS_ROWS;
+            if ((int) threadIdx.x < GS_ROWS * 8 && n < B && m < M) { res_r = ex.res[(size_t) n * M + m]; norm_r = ex.norm_w[m]; }
+        }
     };
     // the eight warps' sums of row block b, in a fixed order; then the epilogue; the sums start again at zero
     auto finish_block = [&](int b, float * acc) {
@@ -247,9 +256,9 @@ __global__ void __launch_bounds__(GS_THREADS) gemm_stream_kernel(
                 float rn = 0.0f;
                 if (n < B && m < M) {
                     const size_t at = (size_t) n * M + m;
-                    rn = ex.res[at] + __bfloat162float(__float2bfloat16_rn(sum));
+                    rn = res_r + __bfloat162float(__float2bfloat16_rn(sum));
                     ex.res[at] = rn;
-                    out[at] = from_f32<OutT>(rn * ex.norm_w[m]);
+                    out[at] = from_f32<OutT>(rn * norm_r);
                 }
                 float sq = rn * rn;
 #pragma unroll
@@ -275,6 +284,7 @@ __global__ void __launch_bounds__(GS_THREADS) gemm_stream_kernel(
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     if (XREG > 0) {
         for (int b = blockIdx.x; b < n_blocks; b += gridDim.x) {
+            ask_block(b);
 #pragma unroll
             for (int s_ = 0; s_ < XR / PER_STAGE; s_++)
                 if (s_ < n_st) { stage(it, s_, acc, xb + s_ * PER_STAGE); it++; }
@@ -285,14 +295,15 @@ __global__ void __launch_bounds__(GS_THREADS) gemm_stream_kernel(
         uint4 pa[PER_STAGE], pb[PER_STAGE];
         int b = blockIdx.x, s_ = 0;
         if (b >= n_blocks) return;
+        ask_block(b);
         fetch(0, pa);
         for (;;) {
             fetch(s_ + 1 == n_st ? 0 : s_ + 1, pb);
             stage(it++, s_, acc, pa);
-            if (++s_ == n_st) { finish_block(b, acc); s_ = 0; b += gridDim.x; if (b >= n_blocks) break; }
+            if (++s_ == n_st) { finish_block(b, acc); s_ = 0; b += gridDim.x; if (b >= n_blocks) break; ask_block(b); }
             fetch(s_ + 1 == n_st ? 0 : s_ + 1, pa);
             stage(it++, s_, acc, pb);
-            if (++s_ == n_st) { finish_block(b, acc); s_ = 0; b += gridDim.x; if (b >= n_blocks) break; }
+            if (++s_ == n_st) { finish_block(b, acc); s_ = 0; b += gridDim.x; if (b >= n_blocks) break; ask_block(b); }
         }
     }
 }
