@@ -438,7 +438,8 @@ IIAN_API int iian_paged_attention_sink(
     // side, as when decoding) goes to the kernel with a warp per item, which leaves the others out (8 heads of 64 on one KV head, eight
     // requests behind 1,500: 244 us, 848 when a tile walks its four requests in turn; 16 on 2 of 128: 734 and 1,027)
     const int group = nh / nkv;
-    const uintptr_t all = (uintptr_t) k_cache | (uintptr_t) v_cache | (uintptr_t) out;
+    // the tiled kernel moves 16 bytes at once on all four sides; the other one reads q and writes out an entry at a time
+    const uintptr_t all = (uintptr_t) q | (uintptr_t) k_cache | (uintptr_t) v_cache | (uintptr_t) out;
     int tile_tokens = 0;
     if (N >= kTileMinTokens && group <= 8 && kTileItems % group == 0 && hd <= kTileHeadDim && hd % 4 == 0 && all % 16 == 0 && nkv <= 65535) {
         tile_tokens = kTileItems / group;

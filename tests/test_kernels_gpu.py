@@ -707,3 +707,15 @@ def test_paged_attention_generic_takes_a_requests_tokens_in_several_runs(G, runs
         one = torch.empty(1, nkv * G * hd).cuda()
         call(q[t:t + 1].contiguous(), One, one)
         assert torch.equal(one[0], out[i]), (i, t)
+
+
+@pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 16), (16, 8, 128), (8, 1, 64)])
+def test_paged_attention_generic_takes_q_at_any_offset(nh, nkv, hd):
+    """Neighbouring tokens whose q does not start on 16 bytes: the same bits as from a copy that does."""
+    q, kc, vc, m, _, scale = attention_case(torch.float32, nh, nkv, hd, 16, [75, 60], [70, 41], 0, seed=14)
+    outs = []
+    for skip in (0, 1, 3):
+        at = torch.empty(q.numel() + skip, device="cuda")[skip:].view(q.shape).copy_(q)
+        outs.append(torch.full((q.shape[0], nh * hd), float("nan")).cuda())
+        K().paged_attention_generic(at, kc, vc, outs[-1], m, num_heads=nh, num_kv_heads=nkv, head_dim=hd, scale=scale, window=0)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
