@@ -399,6 +399,9 @@ done:
 // A decoded token has its heads for rows, 16 or fewer, and would leave most of a row tile empty.  Here a tile of 128 keys is the M operand:
 // S^T = K Q^T (128 keys x 16 heads), and with P^T [16 heads][128 keys] in shared memory O^T = V^T P^T, the rank in blocks of 128 rows,
 // V^T the same chunks read MN-major.  Every cached row passes shared memory once, for all heads.
+// P is held as two bfloat16 parts, the upper 16 bits of a weight and what they leave, which are 32 columns of one product where 16 would
+// take as long.  With one part the outputs were further from 64 bits than those of mma.sync, whose parts of the keys have a largest
+// weight of 1, and so an exact one, each (rank 512, 48 tokens behind 800 to 4,000: 0.00192 for 0.00189, of which 0.00166 are the result's own rounding).
 // The tiles of all sequences lie end to end, and the CTAs, one an SM, take equal stretches of that line: a stretch may end inside a sequence
 // (its part goes to scratch memory, slot sequence + CTA) and go on into the next ones.  latent_line_merge_kernel puts the parts together.
 // Roles: warps 0..3 the softmax (a thread a key, all heads), warp 4 lane 0 the products, warps 5.. the copies: one for each pair of the
@@ -472,12 +475,12 @@ template <typename F> __device__ __forceinline__ float ll_reduce(float * a, F f)
 template <int PAIRS>
 __global__ void __launch_bounds__(32 * (6 + PAIRS), 1) latent_line_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const LatentLineParams p) {
-    constexpr int N = LL_HEADS, CHUNKS = 2 * PAIRS + 1, ROPES = 2, Q_BYTES = N * 128;
+    constexpr int N = LL_HEADS, CHUNKS = 2 * PAIRS + 1, ROPES = 2, Q_BYTES = N * 128, P_BYTES = 2 * N * 128;
     extern __shared__ __align__(1024) unsigned char lt_smem_raw[];
     unsigned char * sK = (unsigned char *) (((uintptr_t) lt_smem_raw + 1023) & ~(uintptr_t) 1023);     // [LL_SLOTS][2 chunks][128 keys][128 B]
     unsigned char * sR = sK + LL_SLOTS * LL_PAIR_BYTES;            // [ROPES][128 keys][128 B]
     unsigned char * sQ = sR + ROPES * LL_CHUNK_BYTES;              // [CHUNKS][N heads][128 B]
-    unsigned char * sP = sQ + CHUNKS * Q_BYTES;                    // [2][N heads][64 keys]
+    unsigned char * sP = sQ + CHUNKS * Q_BYTES;                    // [2][high parts, low parts][N heads][64 keys]
     __shared__ __align__(8) unsigned long long pair_full[LL_SLOTS], pair_free[LL_SLOTS], rope_full[ROPES], rope_free[ROPES], q_full, q_free, s_full, p_full, o_done;
     __shared__ unsigned tmem_base_s;
     __shared__ __align__(16) float wm[2][4][N], wl[4][N];
@@ -586,7 +589,7 @@ __global__ void __launch_bounds__(32 * (6 + PAIRS), 1) latent_line_kernel(
     } else if (warp == 4) {
         if (lane == 0) {
             // ---- products ------------------------------------------------------------------------------------------------------
-            constexpr unsigned idesc_s = at_idesc(LL_KEYS, N, false), idesc_o = at_idesc(128, N, false) | (1u << 15);      // V^T: A is MN-major
+            constexpr unsigned idesc_s = at_idesc(LL_KEYS, N, false), idesc_o = at_idesc(128, 2 * N, false) | (1u << 15);      // V^T: A is MN-major
             const unsigned long long dk = at_desc(at_smem(sK), 16, 1024), dr = at_desc(at_smem(sR), 16, 1024), dq = at_desc(at_smem(sQ), 16, 1024);
             const unsigned long long dv = at_desc(at_smem(sK), LL_CHUNK_BYTES, 1024), dp = at_desc(at_smem(sP), 16, 1024);
             int it = 0;
@@ -631,8 +634,8 @@ __global__ void __launch_bounds__(32 * (6 + PAIRS), 1) latent_line_kernel(
                         const int slot = (it * PAIRS + pr) % LL_SLOTS;
 #pragma unroll
                         for (int k = 0; k < 8; k++)
-                            at_mma(tmem_base + LL_O + (unsigned) (pr * N), dv + (unsigned long long) (slot * (LL_PAIR_BYTES >> 4) + k * 128),
-                                   dp + (unsigned long long) ((k >> 2) * (Q_BYTES >> 4) + (k & 3) * 2), idesc_o, t > 0 || k > 0 ? 1u : 0u);
+                            at_mma(tmem_base + LL_O + (unsigned) (pr * 2 * N), dv + (unsigned long long) (slot * (LL_PAIR_BYTES >> 4) + k * 128),
+                                   dp + (unsigned long long) ((k >> 2) * (P_BYTES >> 4) + (k & 3) * 2), idesc_o, t > 0 || k > 0 ? 1u : 0u);
                         at_commit(at_smem(&pair_free[slot]));
                     }
                     if (t == n - 1) at_commit(at_smem(&o_done));
@@ -689,7 +692,7 @@ __global__ void __launch_bounds__(32 * (6 + PAIRS), 1) latent_line_kernel(
                     }
                 }
                 group_sync();
-                // the exact running maximum, as above: the largest weight is 1 and not rounded
+                // the exact running maximum, as above
                 bool moved = false;
                 float corr[N];
 #pragma unroll
@@ -710,30 +713,32 @@ __global__ void __launch_bounds__(32 * (6 + PAIRS), 1) latent_line_kernel(
                 }
 #pragma unroll
                 for (int h = 0; h < N; h += 2) {
-                    unsigned w[2];
+                    float x[2];
 #pragma unroll
                     for (int e = 0; e < 2; e++) {
                         const float neg = m_run[h + e] == -INFINITY ? 0.0f : m_run[h + e] * sl;
-                        const float x = at_exp2(fmaf(__uint_as_float(v[h + e]), sl, -neg));
-                        w[e] = (unsigned) __bfloat16_as_ushort(__float2bfloat16_rn(x));
-                        // the weights as they are multiplied, so that their rounding weighs on both sides of the quotient
-                        l_run[h + e] = fmaf(l_run[h + e], corr[h + e], __uint_as_float(w[e] << 16));
+                        x[e] = at_exp2(fmaf(__uint_as_float(v[h + e]), sl, -neg));
+                        l_run[h + e] = fmaf(l_run[h + e], corr[h + e], x[e]);
                     }
                     // two neighbouring keys in a word: the even lane takes head h, the odd one head h + 1
                     const bool odd = lane & 1;
-                    const unsigned got = __shfl_xor_sync(0xffffffffu, odd ? w[0] : w[1], 1), word = odd ? got | w[1] << 16 : w[0] | got << 16;
+                    const float got = __shfl_xor_sync(0xffffffffu, odd ? x[0] : x[1], 1), first_key = odd ? got : x[0], next_key = odd ? x[1] : got;
+                    const unsigned b0 = __float_as_uint(first_key), b1 = __float_as_uint(next_key);
                     const int head = h + (odd ? 1 : 0), key = r & 62;
-                    *reinterpret_cast<unsigned *>(sP + (r >> 6) * Q_BYTES + head * 128 + (((key >> 3) ^ (head & 7)) << 4) + (key & 7) * 2) = word;
+                    unsigned char * to = sP + (r >> 6) * P_BYTES + head * 128 + (((key >> 3) ^ (head & 7)) << 4) + (key & 7) * 2;
+                    *reinterpret_cast<unsigned *>(to) = __byte_perm(b0, b1, 0x7632);
+                    *reinterpret_cast<unsigned *>(to + N * 128) =
+                        pack_bf16(first_key - __uint_as_float(b0 & 0xffff0000u), next_key - __uint_as_float(b1 & 0xffff0000u));
                 }
                 if (t > 0 && moved) {                              // (the scores of this tile followed the products of the one before)
 #pragma unroll 1
                     for (int pr = 0; pr < PAIRS; pr++) {
-                        unsigned o[N];
-                        ll_ld16(tO + (unsigned) (pr * N), o);
+                        unsigned o[2 * N];
+                        at_ld32(tO + (unsigned) (pr * 2 * N), o);
                         at_wait_ld();
 #pragma unroll
-                        for (int h = 0; h < N; h++) o[h] = __float_as_uint(__uint_as_float(o[h]) * corr[h]);
-                        lt_st16(tO + (unsigned) (pr * N), o);
+                        for (int h = 0; h < 2 * N; h++) o[h] = __float_as_uint(__uint_as_float(o[h]) * corr[h % N]);
+                        at_st32(tO + (unsigned) (pr * 2 * N), o);
                     }
                     at_wait_st();
                 }
@@ -761,14 +766,15 @@ __global__ void __launch_bounds__(32 * (6 + PAIRS), 1) latent_line_kernel(
             }
 #pragma unroll 1
             for (int pr = 0; pr < PAIRS; pr++) {
-                unsigned o[N];
-                ll_ld16(tO + (unsigned) (pr * N), o);
+                unsigned o[2 * N];
+                at_ld32(tO + (unsigned) (pr * 2 * N), o);
                 at_wait_ld();
 #pragma unroll
                 for (int h = 0; h < N; h++) {
                     if (h >= p.H) continue;
-                    if (whole) p.out[((size_t) q0 * p.H + h) * p.rank + pr * 128 + r] = __float2bfloat16_rn(__uint_as_float(o[h]) * inv[h]);
-                    else p.part_o[(slot * p.H + h) * p.rank + pr * 128 + r] = __uint_as_float(o[h]);
+                    const float both = __uint_as_float(o[h]) + __uint_as_float(o[h + N]);
+                    if (whole) p.out[((size_t) q0 * p.H + h) * p.rank + pr * 128 + r] = __float2bfloat16_rn(both * inv[h]);
+                    else p.part_o[(slot * p.H + h) * p.rank + pr * 128 + r] = both;
                 }
             }
             group_sync();                                          // wl has been read
@@ -845,7 +851,7 @@ static int lt_launch(const CUtensorMap & mq, const CUtensorMap & mk, const Laten
 
 template <int PAIRS>
 static int ll_launch(const CUtensorMap & mq, const CUtensorMap & mk, const LatentLineParams & p, cudaStream_t stream) {
-    const size_t smem = (size_t) LL_SLOTS * LL_PAIR_BYTES + 2 * LL_CHUNK_BYTES + (size_t) (2 * PAIRS + 3) * LL_HEADS * 128 + 1024;
+    const size_t smem = (size_t) LL_SLOTS * LL_PAIR_BYTES + 2 * LL_CHUNK_BYTES + (size_t) (2 * PAIRS + 5) * LL_HEADS * 128 + 1024;
     const cudaError_t e = cudaFuncSetAttribute(latent_line_kernel<PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
     if (e != cudaSuccess) return 1000 + (int) e;
     latent_line_kernel<PAIRS><<<kLineCtas, 32 * (6 + PAIRS), smem, stream>>>(mq, mk, p);

@@ -116,3 +116,28 @@ def test_decoded_tokens_with_keys_as_rows(rank, heads, page, contexts, window):
     assert not out[-2:].any()
     # as above
     assert bool(((out[:-2].double() - torch.stack(want)).abs() <= (2.0 ** -7 + 2e-4) * torch.stack(bound)).all())
+
+
+@pytest.mark.parametrize("rank,heads,contexts", [(512, 16, [800, 2400, 1600]), (256, 16, [3000, 900]), (512, 3, [130, 64, 2000, 5000, 257, 31])])
+def test_decoded_tokens_weights_keep_more_than_16_bits(rank, heads, contexts):
+    """The error against 64 bits is the result's own rounding to bfloat16 and little more: weights in two parts are good to 2^-17, sums of
+    products to 2^-20 or so, against 2^-9.  One bfloat16 part each would add 2^-9 / sqrt(3) of the root mean square, some 15 percent here."""
+    g = torch.Generator("cuda").manual_seed(rank + heads)
+    width, n, page = rank + 64, len(contexts), 16
+    rows = torch.randn(sum(-(-c // page) for c in contexts), page, width, device="cuda", generator=g).bfloat16()
+    bt, at, want = torch.full((n, -(-max(contexts) // page)), -1, dtype=torch.int32), 0, []
+    q = torch.randn(n, heads, width, device="cuda", generator=g).bfloat16()
+    for i, c in enumerate(contexts):
+        pages = -(-c // page)
+        bt[i, :pages] = torch.arange(at, at + pages)
+        keys = rows[at: at + pages].view(-1, width)[:c].double()
+        at += pages
+        want.append(torch.softmax(q[i].double() @ keys.T * width ** -0.5, 1) @ keys[:, :rank])
+    want = torch.stack(want)
+    cuda = lambda x: torch.as_tensor(x, dtype=torch.int32).cuda()
+    meta = SimpleNamespace(cu_q=cuda(list(range(n + 1))), ctx_len=cuda(contexts), block_table=bt.cuda(), num_seqs=n, max_q_len=1,
+                           seq_of_token=cuda(list(range(n))))
+    K, out = CudaKernels(), torch.empty(n, heads, rank, device="cuda", dtype=torch.bfloat16)
+    K.latent_line(q, rows, out, None, meta, num_heads=heads, rank=rank, scale=width ** -0.5, window=None)
+    K.tcgen05_check(q.device)
+    assert (out.double() - want).norm() < 1.02 * (want.bfloat16().double() - want).norm()
