@@ -1234,12 +1234,27 @@ class CudaKernels:
             LAUNCHES[0] += 1
 
     # decoded tokens with the keys as the rows of the products (csrc/latent_attention_tc.cu): bfloat16, rank 256 / 512 with 64 rotated values, up to
-    # 16 heads.  Keys of a step (tokens times the longest context) from which it is used: 48 tokens behind 800 to 4,000 cached 78 us on
-    # mma.sync, 62 here, 128 behind 1,500 88 and 84, but 32 behind 4,000 57 and 62 (rank 256 40 and 40), 64 behind 1,500 49 and 52
-    LATENT_LINE_MIN_KEYS = 180_000
+    # 16 heads.  us of a step as measured with the L2 cold.  That kernel: a + b a thousand keys, whole tiles of all sequences.  On mma.sync:
+    # c + d a thousand keys of the longest walk + e of the mean one, which shares its SM.  Sequences x context, rank 512 (rank 256), there
+    # and here: 44 x 2,100 54 and 64 (42 and 44), 48 x 3,000 73 and 79 (54 and 52), 24 x 8,000 87 and 93 (64 and 58), 64 x 4,000 124 and 110 (91
+    # and 67), 128 x 4,000 222 and 179 (161 and 106), 48 x 800 to 4,000 85 and 73 (64 and 50), 6 x 30,000 120 and 93 (87 and 60)
+    LATENT_LINE_US = {512: (39.3, 0.2725, 16.0, 68.0, 38.0), 256: (29.5, 0.147, 16.8, 56.0, 16.0)}
 
-    def latent_line_pays(self, num_seqs: int, max_q_len: int, num_heads: int, max_ctx: int, window: Optional[int]) -> bool:
-        return max_q_len == 1 and num_heads <= 16 and num_seqs * (min(max_ctx, window + 1) if window else max_ctx) >= self.LATENT_LINE_MIN_KEYS
+    def latent_line_pays(self, num_seqs: int, max_q_len: int, num_heads: int, rank: int, max_ctx: int, window: Optional[int], ctxs=()) -> bool:
+        """``ctxs``: the sequences' contexts where the host has them.  Else (a captured graph) ``max_ctx`` is a bucket that they fill by half
+        at least: all of them at that half, where mma.sync does best against this kernel, so that no replay is slower for it."""
+        if max_q_len != 1 or num_heads > 16 or rank not in self.LATENT_LINE_US:
+            return False
+        a, b, c, d, e = self.LATENT_LINE_US[rank]
+        parts = self.latent_attention_parts(num_seqs, 1, num_heads, max_ctx, window)
+        if len(ctxs) != num_seqs:
+            longest = mean = min(max_ctx / 2, window or max_ctx)
+        else:
+            longest = max(ctxs)
+            if window and longest > window:
+                longest, ctxs = window, [min(x, window) for x in ctxs]
+            mean = sum(ctxs) / num_seqs
+        return a + b * num_seqs * (mean + 64) / 1000 < c + (d * longest + e * mean) / (1000 * parts)
 
     def latent_line_ok(self, q_cat: torch.Tensor, cache_rows: torch.Tensor, rank: int, scale: float) -> bool:
         """Whether that kernel takes these operands at all."""

@@ -125,7 +125,7 @@ class LatentAttention(Mixer):
             return None
         return {"parts": k.latent_attention_parts(num_seqs, 1, self.nh, max_ctx, self.window),
                 "tc": k.latent_attention_tc_parts(num_seqs, num_seqs, 1, self.nh, self.rank, max_ctx, self.window),
-                "line": hasattr(k, "latent_line_pays") and k.latent_line_pays(num_seqs, 1, self.nh, max_ctx, self.window)}
+                "line": hasattr(k, "latent_line_pays") and k.latent_line_pays(num_seqs, 1, self.nh, self.rank, max_ctx, self.window)}
 
     def forward(self, x, ctx, cache, writes_cache: bool, with_extra: bool = False):
         """``x`` [N, hidden] in the activation dtype.  Returns the mixer's output [N, hidden], or with ``with_extra`` the
@@ -157,12 +157,14 @@ class LatentAttention(Mixer):
                       q_cat.view(n, self.nh * self.width), 0, self.width, num_heads=self.nh, n_in=self.dim, n_out=self.rank)
         lat = ctx.buf("latent_ctx", (n, self.nh, self.rank), self.dtype)
         plan, tc, line = ctx.graph_plan(self), 0, False
-        if hasattr(k, "latent_attention_tc_parts"):
+        if hasattr(k, "latent_line_pays"):
+            line = plan["line"] if plan else k.latent_line_pays(meta.num_seqs, meta.max_q_len, self.nh, self.rank, meta.max_ctx, self.window,
+                                                                getattr(meta, "h_ctx_len", ()))
+        line = line and k.latent_line_ok(q_cat, cache.rows, self.rank, self.scale)
+        if not line and hasattr(k, "latent_attention_tc_parts"):
             tc = plan["tc"] if plan else k.latent_attention_tc_parts(n, meta.num_seqs, meta.max_q_len, self.nh, self.rank, meta.max_ctx,
                                                                      self.window)
-        if hasattr(k, "latent_line_pays"):
-            line = plan["line"] if plan else k.latent_line_pays(meta.num_seqs, meta.max_q_len, self.nh, meta.max_ctx, self.window)
-        if line and k.latent_line_ok(q_cat, cache.rows, self.rank, self.scale):
+        if line:
             k.latent_line(q_cat, cache.rows, lat, self.sink, meta, num_heads=self.nh, rank=self.rank, scale=self.scale, window=self.window)
         elif tc and k.latent_attention_tc_ok(q_cat, cache.rows, self.rank, self.scale):
             k.latent_attention_tc(q_cat, cache.rows, lat, self.sink, meta, num_heads=self.nh, rank=self.rank, scale=self.scale,
