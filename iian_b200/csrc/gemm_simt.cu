@@ -369,6 +369,7 @@ static int launch_f32(const float * x, const float * w, TO * out, int N, int M, 
     // us per 1,024 of K: `alone` for the first tile of an SM, `more` for each further one that runs beside it (up to `beside`), `then` for
     // those that wait for one of them to end
     auto cost = [&](int tn, int tm, double alone, double more, int beside, double then) {
+        if ((N + tn - 1) / tn > 65535) return 1e30;          // more row tiles than a grid has (of 64 rows a call that comes here has not)
         const long long tiles = (long long) ((N + tn - 1) / tn) * ((M + tm - 1) / tm), further = (tiles - 1) / 148;
         return alone + more * (double) std::min<long long>(further, beside) + then * (double) std::max<long long>(further - beside, 0);
     };

@@ -652,7 +652,8 @@ def test_gemm_simt_forms_give_the_same_bits(od, N, M, K_):
     assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("N,M", [(120, 4100), (100, 1030), (31, 4099), (17, 1)])
+# 98 x 6,130, 137 x 2,813 and 137 x 1,000 take the three by 10, 24 and 28 percent of the estimate
+@pytest.mark.parametrize("N,M", [(120, 4100), (100, 1030), (31, 4099), (17, 1), (98, 6130), (137, 2813), (137, 1000)])
 @pytest.mark.parametrize("K_", [4, 36, 64, 196, 260])
 def test_gemm_simt_small_tiles_give_the_same_bits(N, M, K_):
     """The three sizes of tile that a ring feeds (by the fullest SM: 32 x 64, 32 x 32, 16 x 32), K ending inside a stage and with one."""
@@ -662,6 +663,16 @@ def test_gemm_simt_small_tiles_give_the_same_bits(N, M, K_):
     K().gemm_simt(x, w, a)
     K().gemm_simt(odd, w, b)
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("N,M", [(32 * 65535 + 1, 3), (64 * 65535, 1)])
+def test_gemm_simt_takes_rows_up_to_its_limit(N, M):
+    """More row tiles of 32 than a grid's second dimension has; sums of four whole numbers, which float32 holds exactly."""
+    x = torch.randint(-9, 10, (N, 4), generator=torch.Generator("cuda").manual_seed(5), device="cuda").float()
+    w = torch.tensor([[1.0, -2.0, 3.0, 5.0], [0.0, 7.0, 1.0, -1.0], [2.0, 2.0, -4.0, 1.0]], device="cuda")[:M].contiguous()
+    out = torch.full((N, M), float("nan"), device="cuda")
+    K().gemm_simt(x, w, out)
+    assert torch.equal(out.double(), x.double() @ w.double().T)
 
 
 @pytest.mark.parametrize("window", [0, 19])
