@@ -818,7 +818,8 @@ IIAN_API int iian_attention_tc(const void * q, const void * k_cache, const void 
                                   page_size, num_pages, scale, window, status, nullptr, stream);
 }
 
-// CTAs that should share each row tile's keys, from the step's host numbers (cu_q [S + 1], ctx_len [S]).  us of a launch, as measured: 12 + 2.3 a
+// CTAs that should share each row tile's keys, from the step's host numbers (cu_q [S + 1], ctx_len [S]): the one rule, which every caller
+// asks, so that all step functions launch the same form.  us of a launch, as measured: 12 + 2.3 a
 // key tile of the longest walk, or of an SM's share of all of them with 4 tiles' time for every further CTA; split, 19 + 2.3 a tile of a
 // part (set-up and merge), 7 tiles' time for a CTA of a further wave.  Clusters of four and eight only where all fit at once.
 //   tokens behind cached ones, 32 heads on 8     one CTA    2      4      8 a row tile
@@ -831,7 +832,8 @@ IIAN_API int iian_attention_tc(const void * q, const void * k_cache, const void 
 IIAN_API int iian_attention_tc_choose(const int * cu_q, const int * ctx_len, int S, int nh, int nkv, int window) {
     if (S <= 0 || nkv <= 0 || nh % nkv != 0) return 1;
     const int G = nh / nkv;
-    if ((long long) (cu_q[S] - cu_q[0]) * G / AT_ROWS * nkv >= 2 * 148) return 1;    // enough CTAs as it is
+    // enough CTAs as they are, or walks of six key tiles at most, where a split saves less than its set-up and merge take
+    if ((long long) (cu_q[S] - cu_q[0]) * nh >= 2LL * 148 * AT_ROWS || *std::max_element(ctx_len, ctx_len + S) <= 6 * AT_BN) return 1;
     long long units = 0, work = 0, longest = 0;
     for (int s = 0; s < S; s++) {
         const int q = cu_q[s + 1] - cu_q[s], pos0 = ctx_len[s] - q, n = (q * G + AT_ROWS - 1) / AT_ROWS;

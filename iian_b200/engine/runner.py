@@ -94,6 +94,7 @@ class PageMeta:
     decode_only: bool
     h_q_len: Sequence[int] = ()
     h_ctx_len: Sequence[int] = ()
+    host_lens: Optional[tuple] = None      # (cu_q, ctx_len) of the step as C arrays, for the rules that the libraries hold: made once, on demand
 
 
 AttentionMeta = PageMeta

@@ -700,14 +700,18 @@ class CudaKernels:
 
     def attention_tc_parts(self, meta, num_heads: int, num_kv_heads: int, window) -> int:
         """How many CTAs of the prefill kernel should share each row tile's keys, from the step's lengths as the host knows them (1
-        where it does not)."""
+        where it does not).  The rule is the library's, which the native step function asks as well."""
         lens, ctxs = getattr(meta, "h_q_len", ()), getattr(meta, "h_ctx_len", ())
         s = meta.num_seqs
-        if len(lens) != s or len(ctxs) != s or max(ctxs) <= 6 * 128 or sum(lens) * num_heads >= 2 * 148 * 256:     # no gain there
+        if s == 0 or len(lens) != s or len(ctxs) != s:
             return 1
-        cu = (c_int * (s + 1))(0, *itertools.accumulate(lens))
+        arrays = getattr(meta, "host_lens", None)
+        if arrays is None:
+            arrays = (c_int * (s + 1))(0, *itertools.accumulate(lens)), (c_int * s)(*ctxs)
+            if hasattr(meta, "host_lens"):
+                meta.host_lens = arrays
         return _fn("attention_tc", "iian_attention_tc_choose", [c_void_p, c_void_p, c_int, c_int, c_int, c_int])(
-            cu, (c_int * s)(*ctxs), s, num_heads, num_kv_heads, window or 0)
+            *arrays, s, num_heads, num_kv_heads, window or 0)
 
     def _attention_dispatch(self, q, k_cache, v_cache, out, meta, nh, nkv, hd, scale, window, n_split=None) -> None:
         if self._attention_tc_ok(q, k_cache, meta, nh, nkv, hd):

@@ -639,6 +639,22 @@ def test_prefill_attention_shared_by_ctas(nh, nkv, ps, ctx_lens, q_lens, window,
     assert (out.double() - one.double()).abs().max() < 2 ** -7 * max(1.0, want.abs().max().item())
 
 
+def test_rule_of_shared_row_tiles():
+    """By the step's lengths alone: the same where cu_q does not begin at zero, as the portions' of a mixed step; one CTA a row tile for contexts
+    of 768, for a step that fills the GPU, and where the host does not know the lengths."""
+    from ctypes import c_int
+    from iian_b200.ops.cuda_backend import _fn
+    choose = lambda cu, ctx, nh=32, nkv=8: _fn("attention_tc", "iian_attention_tc_choose", None)((c_int * len(cu))(*cu), (c_int * len(ctx))(*ctx), len(ctx), nh, nkv, 0)
+    m = Meta()
+    m.num_seqs, m.h_q_len, m.h_ctx_len = 2, [40, 30], [3000, 1500]
+    parts = K().attention_tc_parts(m, 32, 8, None)
+    assert parts > 1 and choose([0, 40, 70], [3000, 1500]) == parts and choose([5, 45, 75], [3000, 1500]) == parts
+    assert choose([0, 40], [768]) == 1 and choose([0, 40], [641]) == 1 and choose([0, 40], [3000]) > 1
+    assert choose([0, 2368], [9000]) == 1 and choose([0, 18, 2372], [9000, 2354]) == 1                 # 296 CTAs of 256 rows
+    m.h_ctx_len = [3000]
+    assert K().attention_tc_parts(m, 32, 8, None) == 1
+
+
 @pytest.mark.parametrize("od", DT)
 @pytest.mark.parametrize("N", [1, 2, 4, 5, 8, 9, 16, 17, 33, 64, 65, 130])
 @pytest.mark.parametrize("M,K_", [(1, 4), (33, 132), (130, 260), (257, 1000), (6151, 48)])

@@ -68,6 +68,42 @@ def test_native_and_python_step_functions_give_the_same_bits(folders, name, dtyp
         assert worst == 0.0, f"{name} {dtype} {mode}: native and Python logits differ by {worst}"
 
 
+@pytest.mark.parametrize("split_mixed", [False, True])
+def test_step_functions_share_long_contexts_alike(folders, tmp_path, split_mixed, monkeypatch):
+    """Portions behind contexts of 600 to 1,600 tokens, where the rule shares a row tile's keys among CTAs or does not (730 tokens: not),
+    and one beside a decoded token: the step functions' logits are the same bits.  The products (128 rows and more) stay out of the library.  Where
+    the native one sends the decoded token to another kernel, the portion is a step of its own to the rule: there to rounding."""
+    from iian_b200.config.registry import get_architecture
+    from iian_b200.engine.replay import TraceReplayer
+    from iian_b200.models.qwen3 import qwen3_config_from_dict
+    from iian_b200.ops import cuda_backend
+    from iian_b200.weights.random_init import write_model_folder
+    for flag, value in (("TCGEN05_MIN_TILES", 0), ("SPLIT_MIXED", split_mixed)):
+        monkeypatch.setattr(cuda_backend.CudaKernels, flag, value)
+    d = os.path.join(str(tmp_path), "long")
+    cfg = dict(TINY["D"], num_attention_heads=32, num_key_value_heads=8, num_hidden_layers=1, max_position_embeddings=2048, use_sliding_window=False)
+    write_model_folder(d, get_architecture("Qwen3ForCausalLM"), qwen3_config_from_dict(cfg), seed=9, store_dtype=torch.bfloat16)
+    entry = lambda rid, t, a, b: {"id": rid, "tokens": t[a:b], "want": [b - a - 1]}
+    r = {f"r{i}": random_tokens(cfg["vocab_size"], n, 500 + i) for i, n in enumerate([1640, 770, 900])}
+    steps = [[entry("r0", r["r0"], 0, 1200)], [entry("r1", r["r1"], 0, 600)], [entry("r0", r["r0"], 1200, 1360)], [entry("r1", r["r1"], 600, 730)],
+             [entry("r0", r["r0"], 1360, 1500), entry("r1", r["r1"], 730, 770)], [entry("r2", r["r2"], 0, 700)],
+             [entry("r0", r["r0"], 1500, 1501), entry("r2", r["r2"], 700, 900)], [entry("r0", r["r0"], 1501, 1640)]]
+    out, asked = [], []
+    choose = cuda_backend.CudaKernels.attention_tc_parts
+    monkeypatch.setattr(cuda_backend.CudaKernels, "attention_tc_parts", lambda self, *a: asked.append(choose(self, *a)) or asked[-1])
+    for native in (False, True):
+        rp = TraceReplayer.from_folder(d, "bfloat16", 4096, 16, 4, native=native)
+        rp.runner.cuda_graphs = False
+        out.append(replay_and_collect(rp, [{"step": i, "entries": e, "end": []} for i, e in enumerate(steps)]))
+        rp.runner.check_device_status()
+    assert asked[3] == 1 and max(asked) > 1
+    for key, a in out[0].items():
+        if split_mixed and key in (("r0", 1500), ("r2", 899)):
+            assert (a - out[1][key]).abs().max() <= 1e-2 * a.abs().max(), key
+        else:
+            assert torch.equal(a, out[1][key]), key
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("name", ["B", "D"])
 def test_native_engine_produces_the_python_engines_tokens(folders, name, dtype):
