@@ -1244,6 +1244,8 @@ class CudaKernels:
     # and 67), 128 x 4,000 222 and 179 (161 and 106), 48 x 800 to 4,000 85 and 73 (64 and 50), 6 x 30,000 120 and 93 (87 and 60)
     LATENT_LINE_US = {512: (39.3, 0.2725, 16.0, 68.0, 38.0), 256: (29.5, 0.147, 16.8, 56.0, 16.0)}
 
+    _line_floats = {}
+
     def latent_line_pays(self, num_seqs: int, max_q_len: int, num_heads: int, rank: int, max_ctx: int, window: Optional[int], ctxs=()) -> bool:
         """``ctxs``: the sequences' contexts where the host has them.  Else (a captured graph) ``max_ctx`` is a bucket that they fill by half
         at least: all of them at that half, where mma.sync does best against this kernel, so that no replay is slower for it."""
@@ -1261,12 +1263,10 @@ class CudaKernels:
         return a + b * num_seqs * (mean + 64) / 1000 < c + (d * longest + e * mean) / (1000 * parts)
 
     def latent_line_ok(self, q_cat: torch.Tensor, cache_rows: torch.Tensor, rank: int, scale: float) -> bool:
-        """Whether that kernel takes these operands at all."""
-        if not (self.LATENT_MMA and self.LATENT_TC) or not scale > 0 or q_cat.dtype != torch.bfloat16 or cache_rows.dtype != torch.bfloat16:
-            return False
+        """Whether that kernel takes these operands at all (``iian_latent_line_ok`` and the box of 16 rows of q, asked without a call)."""
         n, h, width = q_cat.shape
-        fn = _fn("latent_attention_tc", "iian_latent_line_ok", [c_int, c_int, c_int, c_int])
-        return n * h >= 16 and fn(rank, width, h, cache_rows.shape[1]) == 0
+        return (self.LATENT_MMA and self.LATENT_TC and scale > 0 and q_cat.dtype == cache_rows.dtype == torch.bfloat16 and rank in (256, 512)
+                and width == rank + 64 and 1 <= h <= 16 <= n * h and cache_rows.shape[1] in (8, 16, 32, 64, 128))
 
     def latent_line(self, q_cat: torch.Tensor, cache_rows: torch.Tensor, out: torch.Tensor, sink: Optional[torch.Tensor],
                     meta, *, num_heads: int, rank: int, scale: float, window: Optional[int]) -> None:
@@ -1277,9 +1277,12 @@ class CudaKernels:
             raise KernelError(f"latent_line: q {tuple(q_cat.shape)}, cache {tuple(cache_rows.shape)}, out {tuple(out.shape)} do not fit")
         status = self.tcgen05_status_buffer(q_cat.device)
         CudaKernels._tc_used = True
-        floats = _fn("latent_attention_tc", "iian_latent_line_scratch", [c_int, c_int, c_int])
-        floats.restype = c_longlong
-        scratch = self.attention_scratch(q_cat.device, floats(meta.num_seqs, h, rank))
+        size = (meta.num_seqs, h, rank)
+        if size not in self._line_floats:
+            floats = _fn("latent_attention_tc", "iian_latent_line_scratch", [c_int, c_int, c_int])
+            floats.restype = c_longlong
+            self._line_floats[size] = floats(*size)
+        scratch = self.attention_scratch(q_cat.device, self._line_floats[size])
         bt = meta.block_table
         fn = _fn("latent_attention_tc", "iian_latent_line",
                  [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
