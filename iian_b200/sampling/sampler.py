@@ -147,9 +147,10 @@ class Sampler:
             k.argmax(logits, out)
             return out.tolist()
         # plain arrays, which the launch carries along: 48 rows take some 20 us of host time (by numpy and one upload 85, filled element by element
-        # through torch 700)
+        # through torch 700).  A list of one stands for all rows, and a top_k need not be an int, as when numpy took them.
+        params, seeds, indices = (x if len(x) != 1 else list(x) * r for x in (params, seeds, indices))
         settings = array("f", [x for p in params for x in (p.temperature, p.top_p, p.min_p)])
-        top_k = array("i", [min(max(p.top_k, 0), 0x7FFFFFFF) for p in params])
+        top_k = array("i", [int(min(max(p.top_k, 0), 0x7FFFFFFF)) for p in params])
         return k.sample_rows(logits, settings, top_k, array("Q", [s & _MASK for s in seeds]), array("Q", [i & _MASK for i in indices]))
 
     def logprobs(self, raw_logits: torch.Tensor, tokens: Sequence[int], params: Sequence[SamplingParams]):

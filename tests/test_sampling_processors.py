@@ -184,3 +184,23 @@ def test_uniform_streams_of_a_step_are_the_requests_own():
     seeds = [rng.getrandbits(64) for _ in range(200)] + [0, -3, 2 ** 64 - 1, 2 ** 70]
     indices = [rng.randrange(1 << 20) for _ in range(200)] + [0, 1, 2, 3]
     assert uniforms(seeds, indices).tolist() == [uniform(s, i) for s, i in zip(seeds, indices)]
+
+
+def test_sampler_takes_settings_as_numpy_did():
+    """A top_k that is no int counts as its whole part, and a list of one stands for all rows; anything else of another length is refused."""
+    from iian_b200 import ops
+    from iian_b200.sampling.sampler import Sampler
+
+    class Kernels:
+        def sample_rows(self, logits, settings, top_k, seeds, indices):
+            if not len(settings) / 3 == len(top_k) == len(seeds) == len(indices) == logits.shape[0]:
+                raise ValueError("lengths")
+            return list(zip(settings[::3], top_k, seeds, indices))
+
+    one = lambda k: SamplingParams(temperature=0.5, top_k=k)
+    with ops.use_kernels(Kernels()):
+        sample, logits = Sampler("cpu").sample, torch.zeros(3, 9)
+        assert sample(logits, [one(20.0), one(float("inf")), one(7.9)], [1, 2, 3], [0, 1, 2]) == [(0.5, 20, 1, 0), (0.5, 0x7FFFFFFF, 2, 1), (0.5, 7, 3, 2)]
+        assert sample(logits, [one(4)], [-1], [0, 1, 2]) == [(0.5, 4, 2 ** 64 - 1, i) for i in range(3)]
+        with pytest.raises(ValueError):
+            sample(logits, [one(4)] * 2, [1], [0])
