@@ -138,9 +138,10 @@ __global__ void argmax_final_kernel(const float * __restrict__ part_val, const i
 //    than k --, every CTA takes over all lists, sorts and draws from them, and the row is not scanned again (draw_from_list).
 //  * Else the candidates fall into bins by their distance from the largest value (counts, or for top-p masses as integers, so that no
 //    order of adding matters), the CTAs add the cluster's bins up, and the entries of the bin that holds the cut are listed (cut_by_bins).
-//  * Where more than kListMax entries would be listed (many equal logits), or the cut lies in the last, open bin, an interval of keys is
-//    narrowed eight ways per pass: a pass counts (and for top-p adds the probability of) the keys at or above seven borders inside the
-//    interval, and the CTAs swap their numbers through each other's shared memory behind one cluster barrier.
+//  * Where more than kListMax entries would be listed (a row of 151,936 with T = 1.0 and top-p 0.95 does that as a rule, and so do many equal
+//    logits), the interval of keys that belongs to the cut's bin is narrowed eight ways per pass, and all keys' where the cut lies in the last, open
+//    bin: a pass counts (and for top-p adds the probability of) the keys at or above seven borders inside the interval, and the CTAs swap their
+//    numbers through each other's shared memory behind one cluster barrier.
 // Every sum has an order fixed by V alone (entries of a thread, lanes, warps, CTAs), or is one of integers: the same row gives the same token
 // whatever else is in the batch.
 // What bounds it: latency -- the row's way in (4 us), three scans of a slice (bins 6.5, list 3, draw 4.5 us) and the barriers between them --
@@ -174,8 +175,8 @@ struct DrawShared {
     double warp_d[kDrawWarps];
     int warp_i[kDrawWarps];
     int pick;
-    int n_list, found[2], n_span;
-    double m_above;
+    int n_list, found[2], n_span, c_above, c_at;
+    double m_above, m_at, target;                // with found[0], the cut's bin: masses and counts in front of it and with it, the mass to reach
     unsigned long long warp_q[kDrawWarps];
     unsigned lo_key, hi_key;
     float tops[kDrawCluster * kDrawWarps];       // the largest value of every warp of the cluster
@@ -285,11 +286,10 @@ struct Draw {
     __device__ __forceinline__ void swap() { cg::this_cluster().sync(); }
 
     // The largest key K in [lo, hi) whose count (or mass) of keys at or above it reaches the goal; it does at lo and does not at hi.
-    // In: the aggregates at lo and hi.  Out: lo = K and the aggregates of the keys at or above it and above it.
+    // In: the aggregates at lo and hi; whether the interval may be all keys.  Out: lo = K and the aggregates of the keys at or above it and above it.
     template <bool MASS>
-    __device__ __forceinline__ void search(unsigned & lo, unsigned hi, int & c_lo, int & c_hi, double & m_hi, double goal) {
+    __device__ __forceinline__ void search(unsigned & lo, unsigned hi, int & c_lo, int & c_hi, double & m_hi, double goal, bool first) {
         const int lane = threadIdx.x & 31;
-        bool first = true;
         while (hi - lo > 1) {
             if (c_lo - c_hi == 1) {              // one key left inside: it is K
                 unsigned found = 0;
@@ -472,10 +472,26 @@ __device__ __forceinline__ bool draw_from_list(const Draw<STAGED> & d, int begin
     return true;
 }
 
-// The cut of top-k (0: none) and top-p (>= 1: none) among the keys at or above `cut`, by bins and a sorted list: candidates are the keys
-// above the new cut and the first n_tie entries equal to it.  False, and nothing changed: not found this way.
+// The smallest key in front of bin b.  A whole warp calls it: seven rounds of 32 borders.
 template <bool STAGED>
-__device__ __forceinline__ bool cut_by_bins(const Draw<STAGED> & d, int begin, int V, int k, float P, unsigned & cut, int & n_tie) {
+__device__ __forceinline__ unsigned bin_border(const Draw<STAGED> & d, int b) {
+    unsigned lo = order_key(-INFINITY), hi = draw_key(d.zmax) + 1u;          // in a later bin, and as if in front of the first
+    while (hi - lo > 1u) {
+        const unsigned long long span = hi - lo;
+        const unsigned border = lo + (unsigned) (span * (unsigned) ((threadIdx.x & 31) + 1) >> 5);       // the last lane's is hi
+        const bool before = border == hi || (d.zmax - key_value(border)) * kBinsPerUnit < (float) b;
+        const int first = __ffs(__ballot_sync(0xffffffffu, before)) - 1;     // borders rise, so that all from here on are
+        hi = lo + (unsigned) (span * (unsigned) (first + 1) >> 5);
+        lo += (unsigned) (span * (unsigned) first >> 5);
+    }
+    return hi;
+}
+
+// The cut of top-k (0: none) and top-p (>= 1: none) among the keys at or above `cut`, by bins and a sorted list.  1: candidates are the keys
+// above the new cut and the first n_tie entries equal to it.  0: not found this way.  2: more entries share the cut's bin than are listed;
+// what is known of the bin is in shared memory.  With 0 and 2 cut and n_tie are as before.
+template <bool STAGED>
+__device__ __forceinline__ int cut_by_bins(const Draw<STAGED> & d, int begin, int V, int k, float P, unsigned & cut, int & n_tie) {
     DrawShared & sh = d.sh;
     cg::cluster_group cl = cg::this_cluster();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -535,11 +551,14 @@ __device__ __forceinline__ bool cut_by_bins(const Draw<STAGED> & d, int begin, i
     if (by_k ? c >= k && c - own_c < k : m >= target) atomicMin(&sh.found[0], tid);
     __syncthreads();
     const int last = sh.found[0];                // the bin that holds the cut (with both: the one of top-k)
-    if (last >= open) return false;              // top-k of no effect, or a cut in the open bin
-    if (tid == last - 1) sh.m_above = m;
+    if (last >= open) return 0;                  // top-k of no effect, or a cut in the open bin
+    if (tid == last - 1) { sh.m_above = m; sh.c_above = c; }
+    if (tid == last) { sh.m_at = m; sh.c_at = c; sh.target = target; }
     __syncthreads();
     const int first = by_k ? 0 : last;           // with top-k the list begins at the top
     const double m_above = by_k || last == 0 ? 0.0 : sh.m_above;
+    // entries to list: counted, or of a bin's mass at the most that one of its entries weighs (up to 4 percent too few)
+    if (by_k ? sh.c_at > kListMax : (sh.m_at - m_above) * (double) exp2f((float) last * 0.0625f) > (double) kListMax) return 2;
     for (int i0 = tid; i0 < d.n; i0 += 4 * kDrawThreads) {
         unsigned key[4];
         bool in[4];
@@ -558,7 +577,7 @@ __device__ __forceinline__ bool cut_by_bins(const Draw<STAGED> & d, int begin, i
             }
     }
     const int n = merge_lists(d);
-    if (n > kListMax) return false;
+    if (n > kListMax) return 2;
     if (by_k) {
         block_sort(sh, n);
         const int kept = P < 1.0f ? shortest_run(d, k, P) : k;
@@ -572,7 +591,7 @@ __device__ __forceinline__ bool cut_by_bins(const Draw<STAGED> & d, int begin, i
         }
         __syncthreads();
         n_tie = kept == sh.found[1] + 1 ? 0x7fffffff : kept - sh.found[0];       // all of them, or the first few
-        return true;
+        return 1;
     }
     // The largest key whose list entries from there on weigh what is still to reach, in the bin's own whole multiples: every warp weighs
     // one border a pass, and an interval of keys shrinks to a sixteenth.
@@ -613,7 +632,79 @@ __device__ __forceinline__ bool cut_by_bins(const Draw<STAGED> & d, int begin, i
     const unsigned long long some = each > 0ull && need > q_hi ? (need - q_hi + each - 1ull) / each : 1ull;
     cut = lo;
     n_tie = some >= (unsigned long long) ties ? 0x7fffffff : (int) some;         // all of them, or the first few
-    return true;
+    return 1;
+}
+
+// What bins and lists have not found: an interval of keys is narrowed, all from `cut` to `top` or (near) those of the cut's bin alone, some 2^16 and
+// half the passes.  Rows of 151,936, T = 1.0, top-p 0.95 (1,258 entries in the bin): 48 rows 115 us, one 52; from all keys 190 and 80.
+// Out of line: the common rows' path loses 10 percent where the compiler has to find registers for this one, too.
+struct Cut { unsigned key; int n_tie, turn; };
+template <bool STAGED>
+__device__ __noinline__ Cut cut_by_passes(Draw<STAGED> d, int begin, int V, int k, float P, unsigned top, unsigned cut, int n_tie, bool near) {
+    const int lane = threadIdx.x & 31;
+    if (k > 0) {
+        unsigned lo = cut, hi = top;
+        int count, above = 0;
+        if (near) {
+            const int bin = d.sh.found[0];
+            lo = max(cut, bin_border(d, bin + 1));
+            hi = bin_border(d, bin);
+            count = d.sh.c_at;
+            above = bin > 0 ? d.sh.c_above : 0;
+        }
+        else {
+            int c;
+            double m;
+            d.template pass<false>(cut, cut, top, c, m);
+            count = __shfl_sync(0xffffffffu, c, 0);
+        }
+        double none = 0.0;
+        if (near || k < count) {
+            d.template search<false>(lo, hi, count, above, none, (double) k, !near);
+            cut = lo;
+            n_tie = k - above;
+        }
+        const bool whole = near && count - above == n_tie;   // no entry equal to the cut was left out: bins serve for top-p
+        near = false;
+        if (whole && P < 1.0f) {
+            cg::this_cluster().sync();           // the bins of this CTA have been read
+            const int how = cut_by_bins(d, begin, V, 0, P, cut, n_tie);
+            if (how == 1) return {cut, n_tie, d.turn};
+            near = how == 2;
+        }
+    }
+    if (P < 1.0f) {
+        // the cut moves up to the largest key whose mass from there on reaches the target
+        auto move_up = [&](unsigned K, unsigned hi, int c_gt, int c_above, double m_above, double target, bool wide) {
+            d.template search<true>(K, hi, c_gt, c_above, m_above, target, wide);
+            const int tie_p = c_gt - c_above;
+            const float pe = d.mass(K);
+            const int need = pe > 0.0f ? (int) fmin(ceil((target - m_above) / (double) pe), 2147483647.0) : tie_p;
+            cut = K;
+            n_tie = max(1, min(need, tie_p));
+        };
+        if (near) {                              // (of the counts only those of a pass are needed)
+            const int bin = d.sh.found[0];
+            move_up(max(cut, bin_border(d, bin + 1)), bin_border(d, bin), 0x7fffffff, 0, bin > 0 ? d.sh.m_above : 0.0, d.sh.target, false);
+        } else {
+            // borders: cut in lane 0, cut + 1 in the others (entries equal to the cut: the difference of the counts)
+            int c;
+            double m;
+            d.template pass<true>(cut + (lane > 0 ? 1u : 0u), cut, top, c, m);
+            const int c_all = __shfl_sync(0xffffffffu, c, 0), c_gt = __shfl_sync(0xffffffffu, c, 1);
+            const double m_gt = __shfl_sync(0xffffffffu, m, 1);
+            const int ties_in = min(c_all - c_gt, n_tie);
+            const float pe_cut = ties_in > 0 ? d.mass(cut) : 0.0f;
+            const double target = (double) P * (m_gt + (double) ties_in * (double) pe_cut);
+            if (target > 0.0 && m_gt >= target) move_up(cut + 1, top, c_gt, 0, 0.0, target, true);
+            else if (ties_in > 0 && pe_cut > 0.0f) {
+                const int need = (int) fmin(ceil((target - m_gt) / (double) pe_cut), 2147483647.0);
+                n_tie = max(m_gt >= target ? 0 : 1, min(need, ties_in));
+                if (m_gt <= 0.0) n_tie = max(n_tie, 1);
+            }
+        }
+    }
+    return {cut, n_tie, d.turn};
 }
 
 // A row's settings: from arrays on the device, or from the launch's own parameters (no copy in front of it).
@@ -638,7 +729,7 @@ struct SettingRows {
 };
 
 template <bool STAGED, typename Settings>
-__global__ void __launch_bounds__(kDrawThreads) sample_kernel(
+__global__ void __launch_bounds__(kDrawThreads, 2) sample_kernel(
     const float * __restrict__ logits, int V, size_t stride, int slice, const __grid_constant__ Settings set, int * __restrict__ out) {
     extern __shared__ unsigned staged[];
     __shared__ DrawShared sh;
@@ -716,44 +807,12 @@ __global__ void __launch_bounds__(kDrawThreads) sample_kernel(
             return;
         }
     }
-    const bool found = STAGED && cuts && cut_by_bins(d, begin, V, k, P, cut, n_tie);
-    if (cuts && !found && k > 0) {
-        int c;
-        double m;
-        d.template pass<false>(cut, cut, top, c, m);
-        int count = __shfl_sync(0xffffffffu, c, 0), above = 0;
-        double none = 0.0;
-        if (k < count) {
-            d.template search<false>(cut, top, count, above, none, (double) k);
-            n_tie = k - above;
-        }
-    }
-    if (cuts && !found && P < 1.0f) {
-        // borders: cut in lane 0, cut + 1 in the others (entries equal to the cut: the difference of the counts)
-        int c;
-        double m;
-        d.template pass<true>(cut + (lane > 0 ? 1u : 0u), cut, top, c, m);
-        const int c_all = __shfl_sync(0xffffffffu, c, 0);
-        int c_gt = __shfl_sync(0xffffffffu, c, 1);
-        const double m_gt = __shfl_sync(0xffffffffu, m, 1);
-        const int ties_in = min(c_all - c_gt, n_tie);
-        const float pe_cut = ties_in > 0 ? d.mass(cut) : 0.0f;
-        const double target = (double) P * (m_gt + (double) ties_in * (double) pe_cut);
-        if (target > 0.0 && m_gt >= target) {    // the cut moves up: the largest key whose mass from there on reaches the target
-            unsigned K = cut + 1;
-            int c_above = 0;
-            double m_above = 0.0;
-            d.template search<true>(K, top, c_gt, c_above, m_above, target);
-            const int tie_p = c_gt - c_above;
-            const float pe = d.mass(K);
-            const int need = pe > 0.0f ? (int) fmin(ceil((target - m_above) / (double) pe), 2147483647.0) : tie_p;
-            cut = K;
-            n_tie = max(1, min(need, tie_p));
-        } else if (ties_in > 0 && pe_cut > 0.0f) {
-            const int need = (int) fmin(ceil((target - m_gt) / (double) pe_cut), 2147483647.0);
-            n_tie = max(m_gt >= target ? 0 : 1, min(need, ties_in));
-            if (m_gt <= 0.0) n_tie = max(n_tie, 1);
-        }
+    const int how = STAGED && cuts ? cut_by_bins(d, begin, V, k, P, cut, n_tie) : 0;
+    if (cuts && how != 1) {
+        const Cut now = cut_by_passes(d, begin, V, k, P, top, cut, n_tie, how == 2);
+        cut = now.key;
+        n_tie = now.n_tie;
+        d.turn = now.turn;
     }
 
     // inverse CDF in vocabulary order: thread t owns `per` neighbouring entries (an odd number: no two lanes in one bank)

@@ -342,6 +342,35 @@ def test_sample_cuts(V, top_k, top_p, min_p):
         assert cum[got].item() - probs[got].item() - slack <= target <= cum[got].item() + slack, f"row {r}"
 
 
+@pytest.mark.parametrize("V", [60000, 151936])
+@pytest.mark.parametrize("top_k,top_p", [(0, 0.3), (0, 0.6), (0, 0.74), (0, 0.95), (1024, 1.0), (1100, 1.0), (5000, 0.9), (30000, 1.0), (30000, 0.97)])
+def test_sample_cuts_among_many_entries_of_alike_value(V, top_k, top_p):
+    """More entries share the cut's bin than are listed: distinct values on both sides of zero, values far from zero, hundreds of equal ones."""
+    g = torch.Generator().manual_seed(V + top_k)
+    flat = torch.randn(V, generator=g)
+    rows = torch.stack([flat, flat + 20.0, (flat * 16).round() / 16 - 3.0, torch.full((V,), -2.5)])
+    u = torch.rand(len(rows), generator=g)
+    out = torch.empty(len(rows), dtype=torch.int32).cuda()
+    f = lambda v, dt: torch.full((len(rows),), v, dtype=dt).cuda()
+    K().sample(rows.cuda(), f(0.9, torch.float32), f(top_k, torch.int32), f(top_p, torch.float32), f(0.0, torch.float32), u.cuda(), out)
+    for r, got in enumerate(out.tolist()):
+        z = (rows[r] * (torch.tensor(1.0) / 0.9)).double()                     # as the kernel scales, in float32
+        order = torch.sort(z, descending=True, stable=True).indices            # equal values by id
+        mass = torch.exp(z[order] - z.max())[: top_k or None]
+        run = torch.cumsum(mass, 0)
+        # the float32 masses of the kernel are good to 1e-6: its shortest run that reaches top_p may end that share of the mass further
+        kept = [int(torch.searchsorted(run, top_p * run[-1] * (1 + e))) + 1 if top_p < 1 else len(mass) for e in (-2e-6, 2e-6)]
+        found = False
+        for n in {kept[0], min(kept[1], len(mass)), min((kept[0] + kept[1]) // 2, len(mass))}:
+            ids = order[:n].sort().values
+            cum = torch.cumsum(torch.exp(z[ids] - z.max()), 0)
+            at = torch.searchsorted(ids, got)
+            if at < n and ids[at] == got:
+                slack, target = 4e-6 * float(cum[-1]), float(u[r]) * float(cum[-1])
+                found |= float(cum[at - 1]) * int(at > 0) - slack <= target <= float(cum[at]) + slack
+        assert found, f"row {r}: token {got}"
+
+
 @pytest.mark.parametrize("R", [1, 128, 131])
 def test_sample_rows_with_settings_from_the_host(R):
     """Settings that travel with the launch (128 rows at once) against the same settings in device arrays: the same tokens."""
