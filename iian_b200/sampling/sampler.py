@@ -150,7 +150,11 @@ class Sampler:
         # through torch 700).  A list of one stands for all rows, and a top_k need not be an int, as when numpy took them.
         params, seeds, indices = (x if len(x) != 1 else list(x) * r for x in (params, seeds, indices))
         settings = array("f", [x for p in params for x in (p.temperature, p.top_p, p.min_p)])
-        top_k = array("i", [int(min(max(p.top_k, 0), 0x7FFFFFFF)) for p in params])
+        top_k = [min(max(p.top_k, 0), 0x7FFFFFFF) for p in params]
+        try:
+            top_k = array("i", top_k)
+        except TypeError:
+            top_k = array("i", map(int, top_k))
         return k.sample_rows(logits, settings, top_k, array("Q", [s & _MASK for s in seeds]), array("Q", [i & _MASK for i in indices]))
 
     def logprobs(self, raw_logits: torch.Tensor, tokens: Sequence[int], params: Sequence[SamplingParams]):
