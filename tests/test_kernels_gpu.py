@@ -334,12 +334,19 @@ def test_sample_cuts(V, top_k, top_p, min_p):
     K().sample(rows.cuda(), f(0.9, torch.float32), f(top_k, torch.int32), f(top_p, torch.float32), f(min_p, torch.float32), u.cuda(), out)
     for r, got in enumerate(out.tolist()):
         probs = plain.candidate_probs(rows[r], 0.9, top_k, top_p, min_p)
-        cum = torch.cumsum(probs.double(), 0)
-        total, target = cum[-1].item(), u[r].item() * cum[-1].item()
-        # a cut within the float32 rounding of its mass may fall one entry further, where every entry has the same share
-        slack = 1e-5 * total + (probs.max().item() if r in (1, 2) else 0.0)
-        assert probs[got] > 0 or r in (1, 2), f"row {r}: token {got} is outside the candidate set"
-        assert cum[got].item() - probs[got].item() - slack <= target <= cum[got].item() + slack, f"row {r}"
+        z = rows[r] * (torch.tensor(1.0) / 0.9)
+        n, order, good = int((probs > 0).sum()), torch.sort(z, descending=True, stable=True).indices, False
+        # the float32 rounding of masses may take the cut of top-p one entry further, in the order of values and ids, or one less; that of
+        # top-k and min-p is exact
+        for m in (n, n + 1, n - 1) if top_p < 1 else (n,):
+            kept = torch.zeros(V, dtype=torch.float64)
+            kept[order[:m]] = torch.exp(z[order[:m]].double() - z.max().double())
+            cum = torch.cumsum(kept, 0)
+            total, target = cum[-1].item(), u[r].item() * cum[-1].item()
+            good |= kept[got].item() > 0 and cum[got].item() - kept[got].item() - 1e-5 * total <= target <= cum[got].item() + 1e-5 * total
+        assert good, f"row {r}: token {got}"
+        if top_k == 1:
+            assert got == plain.argmax(rows[r])
 
 
 @pytest.mark.parametrize("V", [60000, 151936])
@@ -666,6 +673,33 @@ def test_prefill_attention_shared_by_ctas(nh, nkv, ps, ctx_lens, q_lens, window,
     K().tcgen05_check(q.device)
     assert (out.double().cpu() - want).abs().max() < tol(torch.bfloat16, max(1.0, want.abs().max().item()))
     assert (out.double() - one.double()).abs().max() < 2 ** -7 * max(1.0, want.abs().max().item())
+
+
+@pytest.mark.parametrize("parts", [0, 1, 2, 4, 8])
+@pytest.mark.parametrize("window", [0, 150])
+def test_shared_row_tiles_count_the_sink_once(window, parts):
+    """Sinks of a visible share of the denominator, in row tiles whose first part has many keys, few, or none that a row sees; parts 0: as the
+    rule has it, which shares this step without a window."""
+    nh, nkv, ctx_lens, q_lens = 8, 2, [2100, 129, 40], [33, 129, 40]
+    q, kc, vc, m, _, scale = attention_case(torch.bfloat16, nh, nkv, 128, 16, ctx_lens, q_lens, window, seed=21)
+    sink = (5.0 + 2.0 * torch.randn(nh, generator=torch.Generator().manual_seed(22))).cuda()
+    want, at = [], 0
+    for s, (c, n) in enumerate(zip(ctx_lens, q_lens)):
+        pages = m.block_table[s, : -(-c // 16)].long()
+        k, v = (t[pages].transpose(1, 2).reshape(-1, nkv, 128)[:c].double().repeat_interleave(nh // nkv, 1) for t in (kc, vc))
+        z = torch.einsum("thd,chd->thc", q[at: at + n].view(n, nh, 128).double(), k) * scale
+        row, key = torch.arange(c - n, c, device="cuda")[:, None, None], torch.arange(c, device="cuda")
+        z = z.masked_fill((key > row) | (key <= row - (window or c)), float("-inf"))
+        p = torch.softmax(torch.cat([z, sink.double()[None, :, None].expand(n, -1, 1)], 2), 2)
+        assert 0.02 < p[..., -1].mean() < 0.98
+        want.append(torch.einsum("thc,chd->thd", p[..., :-1], v).reshape(n, nh * 128))
+        at += n
+    want, out = torch.cat(want), torch.full((at, nh * 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+    if parts == 0 and not window:
+        assert K().attention_tc_parts(m, nh, nkv, window) > 1
+    K().paged_attention_tc(q, kc, vc, out, m, num_heads=nh, num_kv_heads=nkv, head_dim=128, scale=scale, window=window, sink=sink, parts=parts)
+    K().tcgen05_check(q.device)
+    assert (out.double() - want).abs().max() < tol(torch.bfloat16, max(1.0, want.abs().max().item()))
 
 
 def test_rule_of_shared_row_tiles():
