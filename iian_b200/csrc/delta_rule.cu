@@ -430,7 +430,6 @@ delta_prep_wide_kernel(const __nv_bfloat16 * __restrict__ proj, long long ld, in
 
 constexpr int kCols = 16;        // columns of S a CTA owns
 constexpr int kLanes = 8;        // lanes that share a column
-constexpr int kScanThreads = kCols * kLanes;
 
 __device__ __forceinline__ void dr_cp4(float * dst, const float * src, bool valid) {
     const unsigned d = (unsigned) __cvta_generic_to_shared(dst);
@@ -445,6 +444,7 @@ template <int N> __device__ __forceinline__ void dr_wait() { asm volatile("cp.as
 // 16 bytes at a time (E a multiple of 4); else entry d = lane + kLanes * i, word by word.  The tokens of a sequence pass
 // through two stages of shared memory, `chunk` tokens each: while one is worked through, cp.async fills the other.
 // HEAD: one decay per (token, head), decay [N, H]; it sits beside the write strength and q . k of its token.
+// threads: those that call it (a constant only where the CTA has more: written in as one, short portions take 2 to 4 percent longer).
 __host__ __device__ constexpr int scan_floats(bool head, int Dp, int chunk) { return 2 * chunk * ((head ? 2 : 3) * Dp + kCols + 4); }      // of shared memory
 
 template <int E, bool VEC, bool HEAD, typename A>
@@ -453,7 +453,7 @@ __device__ __forceinline__ void delta_scan(float * sm, const float * __restrict_
                   float * __restrict__ state, long long state_stride, long long tail_off,
                   const A * __restrict__ proj, long long ld, int col_off, int n_taps,
                   const int * __restrict__ cu_q, const int * __restrict__ state_slots, float * __restrict__ out,
-                  int H, int G, int D, int V, int chunk) {
+                  int H, int G, int D, int V, int chunk, unsigned threads) {
     const int Dp = (D + 3) & ~3;                             // rows start on 16-byte boundaries
     const int stage_floats = chunk * ((HEAD ? 2 : 3) * Dp + kCols + 4);      // q | k | decay (not HEAD) | v | beta, q . k, decay (HEAD), -
     const int cb = blockIdx.x, h = blockIdx.y, s = blockIdx.z;
@@ -480,7 +480,7 @@ __device__ __forceinline__ void delta_scan(float * sm, const float * __restrict_
         float * s_b = s_v + chunk * kCols;
         if (VEC) {
             const int per = D >> 2;
-            for (int e = threadIdx.x; e < nt * per; e += kScanThreads) {
+            for (int e = threadIdx.x; e < nt * per; e += threads) {
                 const int tt = e / per, d = (e - tt * per) << 2;
                 const size_t t = c0 + tt;
                 copy16(s_q + tt * Dp + d, qn + t * GD + g * D + d);
@@ -488,7 +488,7 @@ __device__ __forceinline__ void delta_scan(float * sm, const float * __restrict_
                 if (!HEAD) copy16(s_g + tt * Dp + d, decay + t * HD + h * D + d);
             }
         } else {
-            for (int e = threadIdx.x; e < nt * D; e += kScanThreads) {
+            for (int e = threadIdx.x; e < nt * D; e += threads) {
                 const int tt = e / D, d = e - tt * D;
                 const size_t t = c0 + tt;
                 dr_cp4(s_q + tt * Dp + d, qn + t * GD + g * D + d, true);
@@ -496,12 +496,12 @@ __device__ __forceinline__ void delta_scan(float * sm, const float * __restrict_
                 if (!HEAD) dr_cp4(s_g + tt * Dp + d, decay + t * HD + h * D + d, true);
             }
         }
-        for (int e = threadIdx.x; e < nt * kCols; e += kScanThreads) {
+        for (int e = threadIdx.x; e < nt * kCols; e += threads) {
             const int tt = e / kCols, c = e - tt * kCols;
             const int jj = cb * kCols + c;
             dr_cp4(s_v + e, vv + (size_t) (c0 + tt) * HV + h * V + (jj < V ? jj : 0), jj < V);
         }
-        for (int e = threadIdx.x; e < nt; e += kScanThreads) {
+        for (int e = threadIdx.x; e < nt; e += threads) {
             dr_cp4(s_b + kPer * e, beta + (size_t) (c0 + e) * H + h, true);
             dr_cp4(s_b + kPer * e + 1, qk + (size_t) (c0 + e) * G + g, true);
             if (HEAD) dr_cp4(s_b + kPer * e + 2, decay + (size_t) (c0 + e) * H + h, true);
@@ -515,7 +515,7 @@ __device__ __forceinline__ void delta_scan(float * sm, const float * __restrict_
         const int C = 2 * GD + HV, back = n_taps - 1, L = t1 - t0;
         float * tail = st + tail_off;
         const int part = h * gridDim.x + cb, parts = gridDim.x * gridDim.y;
-        for (int c = part * kScanThreads + threadIdx.x; c < C; c += parts * kScanThreads) {
+        for (int c = part * threads + threadIdx.x; c < C; c += parts * threads) {
             float keep[kMaxTaps];
 #pragma unroll
             for (int i = 0; i < kMaxTaps - 1; i++) {
@@ -651,7 +651,7 @@ delta_scan_kernel(const float * __restrict__ qn, const float * __restrict__ kn, 
     pdl_launch_dependents();
     extern __shared__ __align__(16) float sm[];
     delta_scan<E, VEC, HEAD, A>(sm, qn, kn, vv, beta, decay, qk, state, state_stride, tail_off, proj, ld, col_off, n_taps, cu_q, state_slots, out,
-                                H, G, D, V, chunk);
+                                H, G, D, V, chunk, blockDim.x);
 }
 
 // ---- portions of prompts, four tokens at a time ------------------------------------------------------------------
@@ -764,11 +764,12 @@ delta_block_kernel(const float * __restrict__ qn, const float * __restrict__ kn,
 // Sequences with fewer than at_least tokens are walked token by token as in the scan above, in the same launch: a piece costs more than a
 // token, and a launch of their own would wait for the long ones' chain (a portion of 100 tokens beside 100
 // decoded ones, 16 heads with a decay per channel, through the mixer: 131 us, in two launches 166).  PER: pieces of a stage, 2 where the long
-// walks decide, 1 where many short ones do, so that seven CTAs share an SM and not four (the same 131 us for 142, but 1,500 tokens 386 for 363).
+// walks decide, 1 where many short ones do, so that seven CTAs share an SM and not four (the same 131 us for 142, but 1,500 tokens 386 for 363);
+// the launch bound asks for the registers that leaves (80 a thread are six CTAs: 100 portions of 40 tokens, 16 heads, 605 for 587).
 constexpr int kPairLanes = 16;
 
 template <int E, int PER, bool AHEAD, bool HEAD, typename A>
-__global__ void __launch_bounds__(kCols / 2 * kPairLanes + (AHEAD ? 32 : 0))
+__global__ void __launch_bounds__(kCols / 2 * kPairLanes + (AHEAD ? 32 : 0), PER == 1 ? 7 : 0)
 delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restrict__ qn, const float * __restrict__ kn,
                         const float * __restrict__ vv, const float * __restrict__ beta, const float * __restrict__ decay,
                         const float * __restrict__ qk, float * __restrict__ state, long long state_stride,
@@ -777,6 +778,7 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
                         int from, int pieces, int at_least, int H, int G, int V) {
     constexpr int D = E * kPairLanes, BLOCK = 13 * D + kBlockNumbers, PIECE = BLOCK + 4 * kCols, STAGE = PER * PIECE;
     constexpr int kThreads = kCols / 2 * kPairLanes;         // with AHEAD and a warp that copies
+    constexpr bool EVERY = AHEAD || HEAD;
     extern __shared__ __align__(16) float sm[];
     const int cb = blockIdx.x, h = blockIdx.y, s = blockIdx.z;
     // neighbouring threads have the same entries of two pairs of columns: a 16-byte read then takes 2 clocks a warp, 4 where they lie 16 apart
@@ -788,7 +790,7 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
         static_assert(kCols / 2 * kPairLanes == kCols * kLanes && scan_floats(HEAD, D, CHUNK) <= kBlockStages * STAGE, "both walks fit one launch");
         if (from == 0 && tid < kThreads)
             delta_scan<D / kLanes, true, HEAD, A>(sm, qn, kn, vv, beta, decay, qk, state, state_stride, tail_off, proj, ld, col_off, n_taps, cu_q,
-                                                  state_slots, out, H, G, D, V, CHUNK);
+                                                  state_slots, out, H, G, D, V, CHUNK, AHEAD ? (unsigned) kThreads : blockDim.x);
         return;
     }
     if (t0 >= t1) return;
@@ -911,7 +913,8 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
             }
             const float4 be = *reinterpret_cast<const float4 *>(num), A0 = *reinterpret_cast<const float4 *>(num + 4);
             const float2 A1 = *reinterpret_cast<const float2 *>(num + 8);
-            const float4 B = *reinterpret_cast<const float4 *>(num + 12 + 4 * (lane & 3));
+            float4 B;
+            if (EVERY) B = *reinterpret_cast<const float4 *>(num + 12 + 4 * (lane & 3));
             const float * val = vec + BLOCK + 2 * pair;
             float2 v[4];
 #pragma unroll
@@ -961,13 +964,18 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
                     }
                 }
             }
-            // every lane's sum, so that only the store is under a condition
+            // EVERY: every lane's sum, so that only the store is under a condition.  The other half of the lanes' sums cost more than they save
+            // where many CTAs share the units: 100 portions of 40 tokens, 32 heads with a decay a channel 1,648 -> 1,621 us through the mixer without
+            // them; 16 heads with a decay a head 578 -> 558 with them
             const int t = 4 * c + (lane & 7) - 4;
-            const bool second = lane & 8;
-            const float u0 = second ? u[1][0] : u[0][0], u1 = second ? u[1][1] : u[0][1], u2 = second ? u[1][2] : u[0][2];
-            const float u3 = second ? u[1][3] : u[0][3];
-            const float o = a[0] + (B.x * u0 + B.y * u1 + B.z * u2 + B.w * u3);
-            if ((lane & 4) && t < t1 - t0) to_out[(long long) t * HV] = o;
+            const bool second = lane & 8, mine = (lane & 4) && t < t1 - t0;
+            if (EVERY || mine) {
+                if (!EVERY) B = *reinterpret_cast<const float4 *>(num + 12 + 4 * (lane & 3));
+                const float u0 = second ? u[1][0] : u[0][0], u1 = second ? u[1][1] : u[0][1], u2 = second ? u[1][2] : u[0][2];
+                const float u3 = second ? u[1][3] : u[0][3];
+                const float o = a[0] + (B.x * u0 + B.y * u1 + B.z * u2 + B.w * u3);
+                if (mine) to_out[(long long) t * HV] = o;
+            }
         }
     }
 #pragma unroll

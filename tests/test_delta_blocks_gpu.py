@@ -105,3 +105,38 @@ def test_preparation_of_many_tokens_gives_the_bits_of_few(H, G, V, given, per_he
             k = min(100, m - lo)
             step(slice(cu[i] + lo, cu[i] + lo + k), [0, k], [0] * k, [slots[i]], few, b)
     assert torch.equal(whole, few) and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("H,G,D,V,lens", [(4, 2, 128, 128, [60, 47, 33, 61, 44]), (4, 2, 128, 128, [33 + i % 9 for i in range(12)]),
+                                          (3, 3, 64, 48, [70] + [32 + i for i in range(16)]), (3, 1, 64, 48, [35 + i for i in range(17)])])
+def test_forms_of_the_walk_give_the_same_bits(H, G, D, V, lens, per_head):
+    """Sequences side by side, more CTAs than SMs, two pieces a stage (the first and third) or one, against each sequence alone, where a warp of
+    its own copies the pieces and their vectors are read a step ahead."""
+    K, chosen = CudaKernels(), []
+    K._delta_pieces = lambda *a: chosen.append(CudaKernels._delta_pieces(K, *a)) or chosen[-1]
+    g = torch.Generator("cuda").manual_seed(H + D + len(lens))
+    C, n, S, zw = 2 * G * D + H * V, sum(lens), len(lens), H if per_head else H * D
+    assert V // 16 * H * S > 148 >= V // 16 * H
+    state0 = torch.randn(S, K.delta_state_floats(H, G, D, V, 4), device="cuda", generator=g)
+    proj, z = torch.randn(n, C + H, device="cuda", generator=g).bfloat16(), torch.randn(n, zw, device="cuda", generator=g)
+    taps = torch.randn(C, 4, device="cuda", generator=g) * 0.4
+    a_log, dt_bias = torch.rand(H, device="cuda", generator=g) * 2.5, torch.randn(zw, device="cuda", generator=g) - 2.0
+
+    def step(rows, which, state, out):
+        i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+        mine, cu, bufs = [lens[i] for i in which], [0], {}
+        for m in mine:
+            cu.append(cu[-1] + m)
+        ctx = SimpleNamespace(cu_q=i32(cu), seq_of_token=i32([i for i, m in enumerate(mine) for _ in range(m)]), state_slots=i32(which), max_q_len=max(mine),
+                              buf=lambda name, shape, dt: bufs.setdefault(name, torch.full(shape, float("nan"), dtype=dt, device="cuda")))
+        K.delta_rule(proj[rows], 0, C, z[rows], taps, a_log, dt_bias, state, ctx, out[rows], num_heads=H, num_kv_heads=G, dim=D, v_dim=V)
+
+    whole, alone = state0.clone(), state0.clone()
+    a, b = (torch.full((n, H * V), float("nan"), device="cuda") for _ in range(2))
+    step(slice(0, n), list(range(S)), whole, a)
+    at = 0
+    for i, m in enumerate(lens):
+        step(slice(at, at + m), [i], alone, b)
+        at += m
+    assert set(chosen) == {0} and torch.equal(a, b) and torch.equal(whole, alone)
