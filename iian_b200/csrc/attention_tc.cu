@@ -810,14 +810,6 @@ IIAN_API int iian_attention_tc_masked(const void * q, long long ld_q, const void
                                       float scale, int window, int chunk, int * status, const float * sink, const float * pen1,
                                       const float * pen2, const void * gate, long long ld_gate, cudaStream_t stream);
 
-IIAN_API int iian_attention_tc(const void * q, const void * k_cache, const void * v_cache, void * out,
-                               const int * cu_q, const int * ctx_len, const int * block_table, int max_blocks,
-                               int N, int S, int max_q_len, int nh, int nkv, int hd, int page_size, int num_pages,
-                               float scale, int window, int * status, cudaStream_t stream) {
-    return iian_attention_tc_sink(q, k_cache, v_cache, out, cu_q, ctx_len, block_table, max_blocks, N, S, max_q_len, nh, nkv, hd,
-                                  page_size, num_pages, scale, window, status, nullptr, stream);
-}
-
 // CTAs that should share each row tile's keys, from the step's host numbers (cu_q [S + 1], ctx_len [S]): the one rule, which every caller
 // asks, so that all step functions launch the same form.  us of a launch, as measured: 12 + 2.3 a
 // key tile of the longest walk, or of an SM's share of all of them with 4 tiles' time for every further CTA; split, 19 + 2.3 a tile of a

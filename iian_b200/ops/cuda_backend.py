@@ -2321,6 +2321,8 @@ class CudaKernels:
 
     def sample(self, logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor, top_p: torch.Tensor,
                min_p: torch.Tensor, uniform: torch.Tensor, out: torch.Tensor) -> None:
+        """A token a row, settings and uniform numbers in device arrays: the call that the native engine makes.  The Python engine's is
+        ``sample_rows``; tests hold one against the other."""
         r, v = logits.shape
         if not logits.is_cuda or logits.dtype != torch.float32 or logits.stride(1) != 1:
             raise KernelError("sample: logits must be float32 on CUDA with contiguous rows")

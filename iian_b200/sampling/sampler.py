@@ -40,7 +40,8 @@ def uniform(seed: int, index: int) -> float:
 
 
 def uniforms(seeds: Sequence[int], indices: Sequence[int]) -> np.ndarray:
-    """``uniform`` of every (seed, index) pair, float32: the same integers on arrays (they wrap modulo 2^64)."""
+    """``uniform`` of every (seed, index) pair, float32: the same integers on arrays (they wrap modulo 2^64).  What the sampling
+    kernel computes for itself, for whoever wants to know a draw beforehand; tests hold the kernel to it."""
     def mix(x):
         x = x + np.uint64(GOLDEN)
         x = (x ^ (x >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
