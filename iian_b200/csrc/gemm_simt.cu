@@ -358,6 +358,8 @@ static int launch_rows(const float * x, const float * w, TO * out, int N, int M,
 //   17 x 1,024 x 2,048        130            78               50            28        23
 //   120 x 1,024 x 2,048       130            78               52            29        31
 //   1,024 x 4,096 x 4,096     775           727              781           930     1,070       1,548
+//   256 x 4,096 x 1,024        70            64               70            82        84
+//   1,024 x 1,024 x 3,072     189           177              189           223       234
 //   2,048 x 6,144 x 4,096   2,023         2,107                                                3,996
 template <typename TO>
 static int launch_f32(const float * x, const float * w, TO * out, int N, int M, int K, cudaStream_t stream) {
@@ -373,8 +375,8 @@ static int launch_f32(const float * x, const float * w, TO * out, int N, int M, 
         const long long tiles = (long long) ((N + tn - 1) / tn) * ((M + tm - 1) / tm), further = (tiles - 1) / 148;
         return alone + more * (double) std::min<long long>(further, beside) + then * (double) std::max<long long>(further - beside, 0);
     };
-    const double wide = cost(64, 128, 65.0, 43.0, 1, 43.0), even = cost(64, 64, 40.0, 24.0, 1, 24.0);
-    const double half = cost(32, 64, 24.0, 13.3, 4, 13.3), small = cost(32, 32, 14.5, 6.8, 2, 9.2), least = cost(16, 32, 12.3, 4.3, 4, 5.4);
+    const double wide = cost(64, 128, 65.0, 43.0, 1, 43.0), even = cost(64, 64, 45.0, 13.5, 1, 26.0);
+    const double half = cost(32, 64, 24.5, 12.0, 2, 14.8), small = cost(32, 32, 15.0, 7.7, 2, 9.2), least = cost(16, 32, 11.5, 4.1, 2, 5.5);
     const double best = std::min({wide, even, half, small, least});
     if (wide == best) return launch_tile<64, 128, 8, 8, 1, TO>(x, w, out, N, M, K, stream);
     if (even == best) return launch_tile<64, 64, 8, 4, 3, TO>(x, w, out, N, M, K, stream);
