@@ -736,10 +736,17 @@ done:
     }
 }
 
-// Clusters of `parts` CTAs that the GPU holds at once, asked once (an SM holds one CTA, and a cluster stays inside one GPC).
+// Clusters of `parts` CTAs that the current GPU holds at once, asked once (an SM holds one CTA, and a cluster stays inside one GPC).  Below zero:
+// no answer, so no split of this size now; the next call asks again.
 static int at_clusters(int parts, size_t smem) {
-    static std::atomic<int> known[4];
-    std::atomic<int> & slot = known[parts >= 8 ? 3 : parts >= 4 ? 2 : 1];
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices][4];
+    int device = -1;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kDevices) {
+        cudaGetLastError();
+        return -1;
+    }
+    std::atomic<int> & slot = known[device][parts >= 8 ? 3 : parts >= 4 ? 2 : 1];
     int n = slot.load(std::memory_order_relaxed);
     if (n == 0) {
         cudaLaunchConfig_t cfg = {};
@@ -755,7 +762,7 @@ static int at_clusters(int parts, size_t smem) {
         if (cudaFuncSetAttribute(attention_tc_kernel<AT_SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess ||
             cudaOccupancyMaxActiveClusters(&n, attention_tc_kernel<AT_SPLIT>, &cfg) != cudaSuccess || n <= 0) {
             cudaGetLastError();
-            n = -1;                                          // not to be had: no split of this size
+            return -1;
         }
         slot.store(n, std::memory_order_relaxed);
     }
