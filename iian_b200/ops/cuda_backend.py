@@ -2347,9 +2347,11 @@ class CudaKernels:
         out = torch.empty(r, dtype=torch.int32, pin_memory=True)
         with torch.cuda.device(logits.device):
             stream = torch.cuda.current_stream()
-            _check(fn(logits.data_ptr(), r, v, logits.stride(0), settings.buffer_info()[0], top_k.buffer_info()[0], seeds.buffer_info()[0],
-                      indices.buffer_info()[0], out.data_ptr(), stream.cuda_stream), "sample")
-            stream.synchronize()
+            try:
+                _check(fn(logits.data_ptr(), r, v, logits.stride(0), settings.buffer_info()[0], top_k.buffer_info()[0], seeds.buffer_info()[0],
+                          indices.buffer_info()[0], out.data_ptr(), stream.cuda_stream), "sample")
+            finally:
+                stream.synchronize()         # also where a later launch of several was refused: those before it still write to ``out``
         return out.tolist()
 
 

@@ -204,3 +204,21 @@ def test_sampler_takes_settings_as_numpy_did():
         assert sample(logits, [one(4)], [-1], [0, 1, 2]) == [(0.5, 4, 2 ** 64 - 1, i) for i in range(3)]
         with pytest.raises(ValueError):
             sample(logits, [one(4)] * 2, [1], [0])
+
+
+def test_tokens_are_waited_for_where_a_launch_is_refused(monkeypatch):
+    """Of several launches the first may be under way when a later one is refused: its memory is not let go before it has ended."""
+    import contextlib
+    from array import array
+    from types import SimpleNamespace
+
+    from iian_b200.ops import cuda_backend as cb
+    waited, empty = [], torch.empty
+    monkeypatch.setattr(cb, "_fn", lambda *a: lambda *b: 1002)
+    monkeypatch.setattr(torch, "empty", lambda *a, pin_memory=False, **k: empty(*a, **k))
+    monkeypatch.setattr(torch.cuda, "device", lambda d: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: SimpleNamespace(cuda_stream=0, synchronize=lambda: waited.append(1)))
+    logits = SimpleNamespace(shape=(2, 8), is_cuda=True, dtype=torch.float32, stride=lambda d: (8, 1)[d], data_ptr=lambda: 0, device="cuda")
+    with pytest.raises(cb.KernelError):
+        cb.CudaKernels().sample_rows(logits, array("f", [1.0] * 6), array("i", [0, 0]), array("Q", [1, 2]), array("Q", [0, 0]))
+    assert waited == [1]
