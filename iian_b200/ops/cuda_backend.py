@@ -1245,6 +1245,7 @@ class CudaKernels:
     LATENT_LINE_US = {512: (39.3, 0.2725, 16.0, 68.0, 38.0), 256: (29.5, 0.147, 16.8, 56.0, 16.0)}
 
     _line_floats = {}
+    _LINE_ARGS = [c_void_p] * 9 + [c_int] * 8 + [c_float, c_int, c_void_p, c_void_p]
 
     def latent_line_pays(self, num_seqs: int, max_q_len: int, num_heads: int, rank: int, max_ctx: int, window: Optional[int], ctxs=()) -> bool:
         """``ctxs``: the sequences' contexts where the host has them.  Else (a captured graph) ``max_ctx`` is a bucket that they fill by half
@@ -1284,9 +1285,7 @@ class CudaKernels:
             self._line_floats[size] = floats(*size)
         scratch = self.attention_scratch(q_cat.device, self._line_floats[size])
         bt = meta.block_table
-        fn = _fn("latent_attention_tc", "iian_latent_line",
-                 [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
-                  c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p])
+        fn = _fn("latent_attention_tc", "iian_latent_line", self._LINE_ARGS)
         _check(fn(_cuda(q_cat, "q_cat"), _cuda(cache_rows, "latent cache"), _cuda(out, "attention out"), scratch.data_ptr(),
                   _cuda(sink, "sink", torch.float32), _cuda(meta.cu_q, "cu_q", torch.int32), _cuda(meta.ctx_len, "ctx_len", torch.int32),
                   _cuda(meta.seq_of_token, "seq_of_token", torch.int32), _cuda(bt, "block table", torch.int32), bt.shape[1], n,
