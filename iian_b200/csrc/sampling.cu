@@ -145,8 +145,8 @@ __global__ void argmax_final_kernel(const float * __restrict__ part_val, const i
 // Every sum has an order fixed by V alone (entries of a thread, lanes, warps, CTAs), or is one of integers: the same row gives the same token
 // whatever else is in the batch.
 // What bounds it: latency -- the row's way in (4 us), three scans of a slice (bins 6.5, list 3, draw 4.5 us) and the barriers between them --
-// and two waves of CTAs from 38 rows on.  Rows of 151,936, the usual mix of settings: 48 rows 49 us, 8 rows 35 us, one row with top-k and
-// top-p 16 us (by narrowing alone, some 20 passes: 123, 82 and 51 us).
+// and two waves of CTAs from 38 rows on.  Rows of 151,936, the usual mix of settings, caches flushed: 48 rows 53 us, 8 rows 38 us, one row with
+// top-k and top-p 18 us (by narrowing alone, some 20 passes, caches warm: 123, 82 and 51 us).
 constexpr int kDrawThreads = 512;
 constexpr int kDrawWarps = kDrawThreads / 32;
 constexpr int kDrawCluster = 8;                  // CTAs per row, at most
