@@ -444,7 +444,7 @@ template <int N> __device__ __forceinline__ void dr_wait() { asm volatile("cp.as
 // 16 bytes at a time (E a multiple of 4); else entry d = lane + kLanes * i, word by word.  The tokens of a sequence pass
 // through two stages of shared memory, `chunk` tokens each: while one is worked through, cp.async fills the other.
 // HEAD: one decay per (token, head), decay [N, H]; it sits beside the write strength and q . k of its token.
-// threads: those that call it (a constant only where the CTA has more: written in as one, short portions take 2 to 4 percent longer).
+// threads: those that call it (the launch's own number as a rule: with a constant, short portions take 2 to 4 percent longer).
 __host__ __device__ constexpr int scan_floats(bool head, int Dp, int chunk) { return 2 * chunk * ((head ? 2 : 3) * Dp + kCols + 4); }      // of shared memory
 
 template <int E, bool VEC, bool HEAD, typename A>
@@ -765,11 +765,12 @@ delta_block_kernel(const float * __restrict__ qn, const float * __restrict__ kn,
 // token, and a launch of their own would wait for the long ones' chain (a portion of 100 tokens beside 100
 // decoded ones, 16 heads with a decay per channel, through the mixer: 131 us, in two launches 166).  PER: pieces of a stage, 2 where the long
 // walks decide, 1 where many short ones do, so that seven CTAs share an SM and not four (the same 131 us for 142, but 1,500 tokens 386 for 363);
-// the launch bound asks for the registers that leaves (80 a thread are six CTAs: 100 portions of 40 tokens, 16 heads, 605 for 587).
+// the launch bound asks for the registers that leaves (80 a thread are six CTAs: 100 portions of 40 tokens, 16 heads, 605 for 587).  With a decay a
+// head the compiler finds them by itself, the thread count being a constant, and does better without the bound (562 for 554).
 constexpr int kPairLanes = 16;
 
 template <int E, int PER, bool AHEAD, bool HEAD, typename A>
-__global__ void __launch_bounds__(kCols / 2 * kPairLanes + (AHEAD ? 32 : 0), PER == 1 ? 7 : 0)
+__global__ void __launch_bounds__(kCols / 2 * kPairLanes + (AHEAD ? 32 : 0), PER == 1 && !HEAD ? 7 : 0)
 delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restrict__ qn, const float * __restrict__ kn,
                         const float * __restrict__ vv, const float * __restrict__ beta, const float * __restrict__ decay,
                         const float * __restrict__ qk, float * __restrict__ state, long long state_stride,
@@ -790,7 +791,7 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
         static_assert(kCols / 2 * kPairLanes == kCols * kLanes && scan_floats(HEAD, D, CHUNK) <= kBlockStages * STAGE, "both walks fit one launch");
         if (from == 0 && tid < kThreads)
             delta_scan<D / kLanes, true, HEAD, A>(sm, qn, kn, vv, beta, decay, qk, state, state_stride, tail_off, proj, ld, col_off, n_taps, cu_q,
-                                                  state_slots, out, H, G, D, V, CHUNK, AHEAD ? (unsigned) kThreads : blockDim.x);
+                                                  state_slots, out, H, G, D, V, CHUNK, AHEAD || (HEAD && PER == 1) ? (unsigned) kThreads : blockDim.x);
         return;
     }
     if (t0 >= t1) return;
@@ -966,7 +967,7 @@ delta_block_scan_kernel(const float * __restrict__ blocks, const float * __restr
             }
             // EVERY: every lane's sum, so that only the store is under a condition.  The other half of the lanes' sums cost more than they save
             // where many CTAs share the units: 100 portions of 40 tokens, 32 heads with a decay a channel 1,648 -> 1,621 us through the mixer without
-            // them; 16 heads with a decay a head 578 -> 558 with them
+            // them; 16 heads with a decay a head 578 -> 554 with them
             const int t = 4 * c + (lane & 7) - 4;
             const bool second = lane & 8, mine = (lane & 4) && t < t1 - t0;
             if (EVERY || mine) {
